@@ -261,13 +261,22 @@ int sllm_latent_kv_store(const void* dkv, int64_t row_stride, const void* norm_w
 /* latent_attention: per token i at position p and head h, over the cached positions max(0, p - window + 1) .. p (all of 0 .. p
  * when window <= 0): out[i, h, :r] = sigmoid(gate[i, h]) * sum_j softmax_j((q_lat[i,h] . c_j + rotary(q_rot[i,h]) . k_rot_j) * scale) c_j.
  * q_lat / q_rot / out: element strides per token and per head; gate: [T, num_heads] logits (row stride) or NULL.  r <= 1024. */
-/* 16-bit dtypes with r % 16 == 0 and dr % 16 == 0 run on tensor cores (mma.sync over the heads of a token); other shapes and
- * SLLM_F32 run the fp32 CUDA-core kernel.  sllm_latent_attention_set_simt(1) forces the latter (returns the old setting). */
+/* 16-bit dtypes run on tensor cores: tcgen05 with r % 64 == 0, r <= 512, dr % 16 == 0, dr <= 64, mma.sync with other multiples of 16;
+ * other shapes and SLLM_F32 run the fp32 CUDA-core kernel.  sllm_latent_attention_set_simt(1) forces the latter (returns the old setting). */
 int sllm_latent_attention_set_simt(int on);
 /* sink (fp32 [num_heads], or NULL): the softmax's denominator also contains exp(sink[h]) (no key, no value, not scaled).
  * num_splits > 1 with split_workspace (fp32 [T, num_heads, num_splits, r + 2], device) lets the tensor-core kernel share a
  * query's visible keys between num_splits CTAs (steps with few tokens), merged by a second kernel; ignored by the other path. */
 int sllm_latent_attention(const void* q_lat, int64_t q_lat_stride_t, int64_t q_lat_stride_h, const void* q_rot,
+                          int64_t q_rot_stride_t, int64_t q_rot_stride_h, const void* cosb, const void* sinb,
+                          const void* gate, int64_t gate_stride_t, const void* cache, int n_slots, int slot, int block_size,
+                          const void* block_table, int max_blocks_per_seq, const void* tok_seq, const void* tok_pos,
+                          void* out, int64_t out_stride_t, int64_t out_stride_h, int64_t num_tokens, int num_heads, int r,
+                          int dr, int rot_dims, int window, float scale, const void* sink, int num_splits, void* split_workspace,
+                          sllm_dtype_t dtype, sllm_stream_t stream);
+/* The same for rows that are prompt portions: neighbouring rows of one sequence at consecutive positions share every key tile they
+ * read (r % 64 == 0, r <= 512, dr % 16 == 0, dr <= 64; other shapes as above).  Any order of rows is correct. */
+int sllm_latent_attention_portions(const void* q_lat, int64_t q_lat_stride_t, int64_t q_lat_stride_h, const void* q_rot,
                           int64_t q_rot_stride_t, int64_t q_rot_stride_h, const void* cosb, const void* sinb,
                           const void* gate, int64_t gate_stride_t, const void* cache, int n_slots, int slot, int block_size,
                           const void* block_table, int max_blocks_per_seq, const void* tok_seq, const void* tok_pos,

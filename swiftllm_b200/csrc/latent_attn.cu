@@ -8,6 +8,7 @@
 // position p attends to the positions max(0, p - window + 1) .. p (window <= 0: all of 0 .. p).  With `sink` (fp32 [H]) the softmax's
 // denominator also contains exp(sink[h]): a key of that score without a value, which enters the running (maximum, sum) first.
 // Softmax, the norm of the latent and the rotation run in fp32 for every storage type.
+#include "latent_attn_tc.cuh"
 #include "mma_helpers.cuh"
 #include "typed_io.cuh"
 
@@ -471,7 +472,7 @@ int sllm_latent_kv_store(const void* dkv, int64_t row_stride, const void* norm_w
     return check_launch("latent_kv_store");
 }
 
-int sllm_latent_attention(const void* q_lat, int64_t q_lat_stride_t, int64_t q_lat_stride_h, const void* q_rot,
+static int latent_attention(bool portions, const void* q_lat, int64_t q_lat_stride_t, int64_t q_lat_stride_h, const void* q_rot,
                           int64_t q_rot_stride_t, int64_t q_rot_stride_h, const void* cosb, const void* sinb,
                           const void* gate, int64_t gate_stride_t, const void* cache, int n_slots, int slot, int block_size,
                           const void* block_table, int max_blocks_per_seq, const void* tok_seq, const void* tok_pos,
@@ -489,7 +490,27 @@ int sllm_latent_attention(const void* q_lat, int64_t q_lat_stride_t, int64_t q_l
 #define SLLM_LA_ARGS q_lat, q_lat_stride_t, q_lat_stride_h, q_rot, q_rot_stride_t, q_rot_stride_h, cosb, sinb, gate,            \
                      gate_stride_t, cache, n_slots, slot, block_size, block_table, max_blocks_per_seq, tok_seq, tok_pos, out,   \
                      out_stride_t, out_stride_h, num_tokens, num_heads, r, dr, rot_dims, window, scale, sink, (cudaStream_t)stream
-    // 16-bit storage and 16-element-aligned rows: tensor cores; everything else: the fp32 CUDA-core kernel
+    // 16-bit storage and rows that the products can be cut from: tensor cores; everything else: the fp32 CUDA-core kernel
+    if (dtype != SLLM_F32 && !sllm_latent_attention_force_simt && latent_tc_supported(r, dr) && scale > 0.f && ((uintptr_t)cache & 15) == 0 &&
+        num_tokens < (1ll << 31)) {
+        LatentTc a;
+        a.q_lat = q_lat; a.ql_st = q_lat_stride_t; a.ql_sh = q_lat_stride_h; a.q_rot = q_rot; a.qr_st = q_rot_stride_t; a.qr_sh = q_rot_stride_h;
+        a.cosb = (const float*)cosb; a.sinb = (const float*)sinb; a.gate = gate; a.gate_st = gate_stride_t; a.cache = cache;
+        a.n_slots = n_slots; a.slot = slot; a.block_size = block_size; a.block_table = (const int*)block_table;
+        a.max_blocks_per_seq = max_blocks_per_seq; a.tok_seq = (const int*)tok_seq; a.tok_pos = (const int*)tok_pos; a.out = out;
+        a.out_st = out_stride_t; a.out_sh = out_stride_h; a.num_tokens = (int)num_tokens; a.H = num_heads; a.r = r; a.dr = dr;
+        a.rot_dims = rot_dims; a.window = window; a.scale = scale; a.sink = (const float*)sink;
+        a.nsplit = (num_splits > 1 && split_workspace != nullptr) ? (num_splits > 64 ? 64 : num_splits) : 1;
+        a.partial = (float*)split_workspace;
+        a.q_vec = ((uintptr_t)q_lat & 15) == 0 && q_lat_stride_t % 8 == 0 && q_lat_stride_h % 8 == 0;
+        a.rot_vec = (((uintptr_t)q_rot | (uintptr_t)cosb | (uintptr_t)sinb) & 15) == 0 && q_rot_stride_t % 8 == 0 && q_rot_stride_h % 8 == 0 && rot_dims % 8 == 0;
+        a.out_vec = ((uintptr_t)out & 15) == 0 && out_stride_t % 8 == 0 && out_stride_h % 8 == 0;
+        if (int rc = launch_latent_attn_tc(a, portions, dtype, (cudaStream_t)stream)) return rc;
+        if (a.nsplit > 1)
+            SLLM_DISPATCH_DTYPE(dtype, (latent_attn_combine_kernel<T><<<(unsigned)cdiv(num_tokens * num_heads, 4), 128, 0, (cudaStream_t)stream>>>(
+                a.partial, (const T*)gate, gate_stride_t, (T*)out, out_stride_t, out_stride_h, num_tokens, num_heads, r, a.nsplit)));
+        return check_launch("latent_attention (combine)");
+    }
     const size_t mma_smem = ((size_t)(16 + LM_KT) * (r + dr + 8) + 16 * (LM_KT + 8)) * 2 + (16 * (LM_KT + 1) + 48) * sizeof(float);
     const bool mma = dtype != SLLM_F32 && r % 16 == 0 && dr % 16 == 0 && mma_smem <= 200 * 1024 && !sllm_latent_attention_force_simt;
     if (mma) {
@@ -505,6 +526,36 @@ int sllm_latent_attention(const void* q_lat, int64_t q_lat_stride_t, int64_t q_l
     });
 #undef SLLM_LA_ARGS
     return 0;
+}
+
+int sllm_latent_attention(
+    const void* q_lat, int64_t q_lat_stride_t, int64_t q_lat_stride_h, const void* q_rot,
+    int64_t q_rot_stride_t, int64_t q_rot_stride_h, const void* cosb, const void* sinb,
+    const void* gate, int64_t gate_stride_t, const void* cache, int n_slots, int slot, int block_size,
+    const void* block_table, int max_blocks_per_seq, const void* tok_seq, const void* tok_pos,
+    void* out, int64_t out_stride_t, int64_t out_stride_h, int64_t num_tokens, int num_heads, int r,
+    int dr, int rot_dims, int window, float scale, const void* sink, int num_splits, void* split_workspace,
+    sllm_dtype_t dtype, sllm_stream_t stream) {
+    return latent_attention(false,
+                            q_lat, q_lat_stride_t, q_lat_stride_h, q_rot, q_rot_stride_t, q_rot_stride_h, cosb, sinb, gate,
+                            gate_stride_t, cache, n_slots, slot, block_size, block_table, max_blocks_per_seq, tok_seq, tok_pos,
+                            out, out_stride_t, out_stride_h, num_tokens, num_heads, r, dr, rot_dims, window, scale, sink,
+                            num_splits, split_workspace, dtype, stream);
+}
+
+int sllm_latent_attention_portions(
+    const void* q_lat, int64_t q_lat_stride_t, int64_t q_lat_stride_h, const void* q_rot,
+    int64_t q_rot_stride_t, int64_t q_rot_stride_h, const void* cosb, const void* sinb,
+    const void* gate, int64_t gate_stride_t, const void* cache, int n_slots, int slot, int block_size,
+    const void* block_table, int max_blocks_per_seq, const void* tok_seq, const void* tok_pos,
+    void* out, int64_t out_stride_t, int64_t out_stride_h, int64_t num_tokens, int num_heads, int r,
+    int dr, int rot_dims, int window, float scale, const void* sink, int num_splits, void* split_workspace,
+    sllm_dtype_t dtype, sllm_stream_t stream) {
+    return latent_attention(true,
+                            q_lat, q_lat_stride_t, q_lat_stride_h, q_rot, q_rot_stride_t, q_rot_stride_h, cosb, sinb, gate,
+                            gate_stride_t, cache, n_slots, slot, block_size, block_table, max_blocks_per_seq, tok_seq, tok_pos,
+                            out, out_stride_t, out_stride_h, num_tokens, num_heads, r, dr, rot_dims, window, scale, sink,
+                            num_splits, split_workspace, dtype, stream);
 }
 
 }  // extern "C"

@@ -21,18 +21,24 @@ def latent_kv_store(dkv: torch.Tensor, norm_weight: torch.Tensor, cache: torch.T
 _SM_COUNT = {}
 
 
-def _num_splits(T: int, H: int, window: int, dtype) -> int:
-    """Key splits for the tensor-core kernel: as many CTAs as fit at once (two per SM) when the step has few tokens (decoding),
-    never a second wave; never more than the 64-key tiles a window can hold (16 when there is no window)."""
+def _num_splits(rows: int, H: int, r: int, dr: int, window: int, dtype, portions: bool) -> int:
+    """Key splits of a launch over `rows` tokens (prompt portions or single decoded tokens): as many CTAs as fit at once when the rows
+    alone leave SMs idle, never a second wave; never more than the 64-key tiles a window can hold (16 when there is no window)."""
     if dtype == torch.float32:
         return 1
     dev = torch.cuda.current_device()
     if dev not in _SM_COUNT:
         _SM_COUNT[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
-    ctas = T * ((H + 15) // 16)
-    want = (2 * _SM_COUNT[dev]) // ctas
+    if r % 64 == 0 and r <= 512 and dr % 16 == 0 and dr <= 64:         # one CTA per SM, 64 (token, head) rows each
+        heads = 1
+        while heads < H and heads < 64:
+            heads *= 2
+        per = 64 // heads if portions else 1
+        ctas, room = -(-rows // per) * -(-H // heads), _SM_COUNT[dev]
+    else:                                                              # two CTAs per SM, one token and 16 heads each
+        ctas, room = rows * ((H + 15) // 16), 2 * _SM_COUNT[dev]
     most = (window + 63) // 64 + 1 if window > 0 else 16
-    return max(1, min(want, most, 32))
+    return max(1, min(room // ctas, most, 32))
 
 
 def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, gate, cache: torch.Tensor, slot: int, block_table: torch.Tensor,
@@ -48,12 +54,19 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, gate, cache: torc
     assert gate is None or (gate.shape == (T, H) and gate.stride(1) == 1)
     assert sink is None or (sink.dtype == torch.float32 and sink.shape == (H,) and sink.is_contiguous())
     _lib.require_device(q_lat)
-    nsplit = _num_splits(T, H, window, q_lat.dtype)
-    ws = torch.empty((T, H, nsplit, r + 2), dtype=torch.float32, device=q_lat.device) if nsplit > 1 else None
-    _lib.check(_lib.lib().sllm_latent_attention(
-        q_lat.data_ptr(), q_lat.stride(0), q_lat.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
-        _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(gate), gate.stride(0) if gate is not None else 0,
-        cache.data_ptr(), cache.shape[1], slot, cache.shape[2], block_table.data_ptr(), block_table.shape[1],
-        infer_state.token_seq_ids.data_ptr(), infer_state.token_positions.data_ptr(),
-        out.data_ptr(), out.stride(0), out.stride(1), T, H, r, dr, rot_dims, window, scale, _lib.ptr(sink), nsplit, _lib.ptr(ws),
-        _lib.dtype_tag_f32(q_lat.dtype), _lib.stream()), "latent_attention")
+    npre = min(T, max(0, int(getattr(infer_state, "num_prefill_tokens", 0))))
+    lib, ts, tp = _lib.lib(), infer_state.token_seq_ids, infer_state.token_positions
+    for first, rows, portions in ((0, npre, True), (npre, T - npre, False)):
+        if rows == 0:
+            continue
+        nsplit = _num_splits(rows, H, r, dr, window, q_lat.dtype, portions)
+        ws = torch.empty((rows, H, nsplit, r + 2), dtype=torch.float32, device=q_lat.device) if nsplit > 1 else None
+
+        def at(x):                                                     # the part's first row
+            return None if x is None else x.data_ptr() + first * x.stride(0) * x.element_size()
+        _lib.check((lib.sllm_latent_attention_portions if portions else lib.sllm_latent_attention)(
+            at(q_lat), q_lat.stride(0), q_lat.stride(1), at(q_rot), q_rot.stride(0), q_rot.stride(1),
+            at(cos), at(sin), at(gate), gate.stride(0) if gate is not None else 0,
+            cache.data_ptr(), cache.shape[1], slot, cache.shape[2], block_table.data_ptr(), block_table.shape[1],
+            at(ts), at(tp), at(out), out.stride(0), out.stride(1), rows, H, r, dr, rot_dims, window, scale, _lib.ptr(sink), nsplit,
+            _lib.ptr(ws), _lib.dtype_tag_f32(q_lat.dtype), _lib.stream()), "latent_attention")
