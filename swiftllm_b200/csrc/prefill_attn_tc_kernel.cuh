@@ -1,22 +1,27 @@
-// Causal varlen prefill attention, generation 2 kernel: tcgen05 + TMA, two query tiles per CTA in ping-pong (sm_100a).
+// Causal varlen prefill attention, tcgen05 + TMA kernel, two query tiles per CTA in ping-pong (sm_100a).
 // Shared by prefill_attn_tc.cu (packed k/v of the batch) and prefill_attn_paged.cu (chunked prefill: K/V pages gathered
 // from the KV cache through the block table).
 //
 // Reference being replaced: swiftllm/worker/kernels/prefill_attn.py:9-139 and the flash_attn_varlen_func call at
-// swiftllm/worker/layers/transformer_layer.py:86-96.  head_dim 128, fp16/bf16; numerics per SURVEY.md Appendix A6
-// (fp32 scores, exp2 online softmax in fp32, P rounded to the storage dtype before P.V, o = h(acc / l)).
+// swiftllm/worker/layers/transformer_layer.py:86-96.  head_dim 128, fp16/bf16: fp32 scores, exp2 online softmax in fp32, P rounded
+// to the storage dtype before P.V, o = h(acc / l).
 //
-// CTA = (sequence, q head, 256 query rows) = two 128-row tiles A and B.  352 threads:
-//   warp 0/10   TMA producers: warp 0 loads Q (4 boxes of 128 rows x 64 d) once and then the K tiles, warp 10 the V tiles
-//               (2 boxes of 64 x 64 per 64-token step) into separate 3-stage rings with their own mbarriers.
-//   warp 1      MMA issuer (one thread, polling):  S_X[128 x 64] = Q_X . K_j^T       (8 UMMAs, M=128 N=64 K=16)
-//                                                   O_X[128 x 128] += P_X . V_j       (4 UMMAs, M=128 N=128 K=16, B MN-major)
-//               S_A, S_B (64 TMEM columns each) and O_A, O_B (128 columns each) live in TMEM.
-//   warps 2-5   softmax of tile A, warps 6-9 softmax of tile B: thread = query row = TMEM lane.  Row max and row sum
-//               are thread-local (no shuffles); P (storage dtype) goes to shared memory as the A operand of the PV
-//               UMMA; O is rescaled in TMEM only when the running max grew by more than 2^8 ("lazy rescale": the
+// CTA = (sequence, q head, 256 query rows) = two 128-row tiles A and B, keys in steps of 128.  Three warpgroups:
+//   warp 0 / 2  TMA producers: warp 0 loads Q (4 boxes of 128 rows x 64 d) once and then the K tiles, warp 2 the V tiles
+//               (2 boxes of 128 x 64 per step) into separate two-stage rings with their own mbarriers.
+//   warp 1      product issuer (one elected lane), a fixed order:  O_X += P_X(j) . V(j), then S_X = Q_X . K(j + 1), X = A, B in turn
+//               (8 UMMAs each, M = N = 128, K = 16; B of the former MN-major).
+//   warps 4-7   softmax of tile A, warps 8-11 softmax of tile B: thread = query row = TMEM lane.  Row max and row sum
+//               are thread-local (no shuffles); P goes back into TMEM, over the scores it came from, as the A operand of P . V.
+//               O is rescaled in TMEM only when the running max grew by more than 2^8 ("lazy rescale": the
 //               reference point m_ref trails the true max, exact in the end because l uses the same reference).
-// While one tile's softmax runs on the CUDA cores the tensor pipe works on the other tile.
+// While one tile's softmax runs on the CUDA cores the tensor pipe works on the other tile.  The products of one CTA complete in the
+// order they are issued, so s_full (after S(j)) also says that P . V(j - 1) has been read out and that O is stable.
+// TMEM is full: S_A 0..127, S_B 128..255 (P_X in the first 64 columns of S_X), O_A 256..383, O_B 384..511.
+//
+// Why this split: with P in shared memory and steps of 64 keys the kernel was bound by shared-memory operand reads (96 KiB per tile and 64
+// keys).  P from TMEM and 128 keys per pass over Q need 96 KiB per tile and 128 keys; what is left is the exponentials (128 rows x 128
+// keys per tile and step are 1024 cycles of each scheduler's special-function unit) beside 1024 cycles of products.
 // Roofline: tensor-bound; FLOPs = 4 * nq * D * sum_i L_i (L_i + 1) / 2.
 #pragma once
 #include "tc_helpers.cuh"
@@ -27,20 +32,23 @@ using namespace tc;
 
 constexpr int PT_D = 128;
 constexpr int PT_BQ = 128;                // rows per query tile (two tiles per CTA)
-constexpr int PT_BK = 64;                 // kv tokens per pipeline step
-constexpr int PT_STAGES = 3;               // K and V rings (separate producers): two steps of prefetch ahead of the MMA
-constexpr int PT_THREADS = 352;            // warp 0 K+Q producer, 1 MMA, 2-5 softmax A, 6-9 softmax B, 10 V producer
+constexpr int PT_BK = 128;                // kv tokens per pipeline step
+constexpr int PT_STAGES = 2;              // K and V rings (separate producers)
+constexpr int PT_THREADS = 384;           // warp 0 Q + K producer, 1 products, 2 V producer, 4-7 softmax A, 8-11 softmax B
 constexpr int PT_Q_BYTES = PT_BQ * PT_D * 2;          // 32 KiB per query tile ([half][128 rows][128 B])
-constexpr int PT_KV_BYTES = PT_BK * PT_D * 2;         // 16 KiB per K (or V) tile ([half][64 rows][128 B])
-constexpr int PT_P_BYTES = PT_BQ * PT_BK * 2;         // 16 KiB per P tile ([128 rows][128 B])
-constexpr int PT_SMEM_BYTES = 2 * PT_Q_BYTES + 2 * PT_STAGES * PT_KV_BYTES + 4 * PT_P_BYTES + 1024;   // P double buffered per tile
-constexpr int PT_TMEM_COLS = 512;         // S_A 0..63, S_B 64..127, O_A 128..255, O_B 256..383
+constexpr int PT_KV_BYTES = PT_BK * PT_D * 2;         // 32 KiB per K (or V) tile ([half][128 rows][128 B])
+constexpr int PT_SMEM_BYTES = 2 * PT_Q_BYTES + 2 * PT_STAGES * PT_KV_BYTES + 1024;
+constexpr int PT_TMEM_COLS = 512;
+constexpr int PT_S_COL = 0, PT_O_COL = 256;           // tile B: + 128
 constexpr float PT_RESCALE_THRESHOLD = 8.0f;          // log2 units
+// registers: 384 threads are launched with 168 each; the softmax warpgroups hold a row of 128 scores
+constexpr int PT_REGS_FEW = 72, PT_REGS_MANY = 216;
+static_assert(PT_REGS_FEW + 2 * PT_REGS_MANY <= 3 * 168, "the warpgroups' shares must fit what the block was launched with");
 
 struct PtBarriers {
     uint64_t q_full;
     uint64_t k_full[PT_STAGES], k_empty[PT_STAGES], v_full[PT_STAGES], v_empty[PT_STAGES];
-    uint64_t s_full[2], s_empty[2], p_full[2][2], p_empty[2][2];      // P: [tile][buffer]
+    uint64_t s_full[2], p_full[2][2], o_done[2];      // [tile]; P in two halves of 64 keys
 };
 
 struct PtParams {
@@ -57,11 +65,22 @@ struct PtPaged {
 };
 constexpr int PT_PAGE = 16;               // tokens per KV page (PAGED only)
 
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// (a, b) * c + d in one packed instruction
+__device__ __forceinline__ float2 fma2(float a, float b, float c, float d) {
+    float2 o;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %4};\n mov.b64 z, {%5, %5};\n fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a), "f"(b), "f"(c), "f"(d));
+    return o;
+}
+
 // PAGED = false: K/V tiles come from the packed k/v rows of the batch (the reference's contract).
-// PAGED = true (chunked prefill, SURVEY.md §8 f-1): the chunk's queries sit at positions prefix .. prefix + len - 1 of
-// their sequence; every 64-token K/V step is gathered from four 16-token pages of the KV cache through the block
-// table (lanes 0-3 of the producer warp issue the two d-half boxes of one page each), landing in the SAME
-// [half][64 rows][128 B] layout, so the MMA issuer and its descriptors are shared by both variants.
+// PAGED = true (chunked prefill): the chunk's queries sit at positions prefix .. prefix + len - 1 of
+// their sequence; every 128-token K/V step is gathered from eight 16-token pages of the KV cache through the block
+// table (lanes 0-7 of the producer warp issue the two d-half boxes of one page each), landing in the SAME
+// [half][128 rows][128 B] layout, so the product issuer and its descriptors are shared by both variants.
 template <typename T, bool PAGED>
 __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap qmap,
                                                                         const __grid_constant__ CUtensorMap kmap,
@@ -69,10 +88,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                                                                         const PtParams p, const PtPaged pg) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_sm = smem;                                       // [2 tiles][2 halves][128 rows][128 B]
-    uint8_t* k_sm = q_sm + 2 * PT_Q_BYTES;                      // [stage][2 halves][64 rows][128 B]
+    uint8_t* k_sm = q_sm + 2 * PT_Q_BYTES;                      // [stage][2 halves][128 rows][128 B]
     uint8_t* v_sm = k_sm + PT_STAGES * PT_KV_BYTES;
-    uint8_t* p_sm = v_sm + PT_STAGES * PT_KV_BYTES;             // [2 tiles][2 buffers][128 rows][128 B]
-    uint8_t* misc = p_sm + 4 * PT_P_BYTES;
+    uint8_t* misc = v_sm + PT_STAGES * PT_KV_BYTES;
     PtBarriers* bars = reinterpret_cast<PtBarriers*>(misc);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(misc + 512);
 
@@ -87,8 +105,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     const int pre = PAGED ? pg.prefix_lens[seq] : 0;            // position of query row 0 within its sequence
     const int kvlen = pre + len;
     const bool active_b = q0 + PT_BQ < len;
-    const int nkt_a = (min(kvlen, pre + q0 + PT_BQ) + PT_BK - 1) / PT_BK;   // kv steps tile A takes part in
-    const int nkt_b = active_b ? (min(kvlen, pre + q0 + 2 * PT_BQ) + PT_BK - 1) / PT_BK : 0;
+    const int end_a = min(kvlen, pre + q0 + PT_BQ), end_b = active_b ? min(kvlen, pre + q0 + 2 * PT_BQ) : 0;      // keys a tile can see
+    const int nkt_a = (end_a + PT_BK - 1) / PT_BK, nkt_b = (end_b + PT_BK - 1) / PT_BK;      // kv steps a tile takes part in
     const int nkt = max(nkt_a, nkt_b);
 
     if constexpr (PAGED) {
@@ -103,9 +121,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             mbar_init(smem_u32(&bars->k_full[i]), 1); mbar_init(smem_u32(&bars->k_empty[i]), 1);
             mbar_init(smem_u32(&bars->v_full[i]), 1); mbar_init(smem_u32(&bars->v_empty[i]), 1);
         }
-        for (int i = 0; i < 2; i++) {
-            mbar_init(smem_u32(&bars->s_full[i]), 1); mbar_init(smem_u32(&bars->s_empty[i]), 128);
-            for (int b = 0; b < 2; b++) { mbar_init(smem_u32(&bars->p_full[i][b]), 128); mbar_init(smem_u32(&bars->p_empty[i][b]), 1); }
+        for (int x = 0; x < 2; x++) {
+            mbar_init(smem_u32(&bars->s_full[x]), 1); mbar_init(smem_u32(&bars->o_done[x]), 1);
+            mbar_init(smem_u32(&bars->p_full[x][0]), 128); mbar_init(smem_u32(&bars->p_full[x][1]), 128);
         }
         mbar_fence_init();
         tma_prefetch_desc(&qmap); tma_prefetch_desc(&kmap); tma_prefetch_desc(&vmap);
@@ -116,252 +134,207 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     tc_fence_after();
     const uint32_t tmem = *tmem_base_s;
 
-    // PAGED producer (one whole warp per ring): step j = pages 4j .. 4j+3 of the sequence.  The four block-table
-    // entries of the NEXT step are fetched before this step's stage is waited for; lane 0 arms the mbarrier with the
-    // bytes of the pages that exist, then lanes 0..3 issue the two (64 d x 16 token) boxes of one page each.
-    auto paged_producer = [&](const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty) {
-        const int32_t* bt = pg.block_table + (int64_t)pg.seq_ids[seq] * pg.max_blocks_per_seq;
-        const int npages = (kvlen + PT_PAGE - 1) / PT_PAGE;
-        constexpr int PPS = PT_BK / PT_PAGE;                  // pages per step
-        int nxt = (lane < PPS && lane < npages) ? bt[lane] : 0;
-        for (int j = 0; j < nkt; j++) {
-            const int st = j % PT_STAGES;
-            const int blk = nxt;
-            const int npg = (j + 1) * PPS + lane;
-            nxt = (j + 1 < nkt && lane < PPS && npg < npages) ? bt[npg] : 0;
-            const int valid = min(PPS, npages - j * PPS);      // >= 1: step j exists because page 4j does
-            const uint32_t bar = smem_u32(&full[st]);
-            if (lane == 0) {
-                mbar_wait(smem_u32(&empty[st]), ((j / PT_STAGES) & 1) ^ 1);
-                mbar_arrive_expect_tx(bar, (uint32_t)valid * PT_PAGE * PT_D * 2);
-            }
-            __syncwarp();
-            if (lane < valid) {
-                // row of the cache viewed as [num_blocks * L * nkv * 16 rows, 128]: first token row of this page
-                const int64_t row = (((int64_t)blk * pg.num_layers + pg.cur_layer) * p.nkv + kvh) * PT_PAGE;
-                const uint32_t dst = smem_u32(ring + st * PT_KV_BYTES) + lane * (PT_PAGE * 128);
-                tma_load_2d(dst, &map, bar, 0, (int)row);
-                tma_load_2d(dst + PT_KV_BYTES / 2, &map, bar, 64, (int)row);
-            }
-        }
-    };
-
-    if (warp == 0) {
-        // =========================================================== TMA producer: Q once, then the K tiles
-        if (lane == 0) {
-            const uint32_t qbar = smem_u32(&bars->q_full);
-            mbar_arrive_expect_tx(qbar, 2 * PT_Q_BYTES);
-            for (int x = 0; x < 2; x++)
-                for (int h = 0; h < 2; h++)
-                    tma_load_2d(smem_u32(q_sm + x * PT_Q_BYTES + h * (PT_Q_BYTES / 2)), &qmap, qbar, head * PT_D + h * 64,
-                                tok0 + q0 + x * PT_BQ);
-            if constexpr (!PAGED) {
-                for (int j = 0; j < nkt; j++) {
-                    const int st = j % PT_STAGES;
-                    mbar_wait(smem_u32(&bars->k_empty[st]), ((j / PT_STAGES) & 1) ^ 1);
-                    const uint32_t kb = smem_u32(&bars->k_full[st]);
-                    mbar_arrive_expect_tx(kb, PT_KV_BYTES);
-                    tma_load_2d(smem_u32(k_sm + st * PT_KV_BYTES), &kmap, kb, kvh * PT_D, tok0 + j * PT_BK);
-                    tma_load_2d(smem_u32(k_sm + st * PT_KV_BYTES + PT_KV_BYTES / 2), &kmap, kb, kvh * PT_D + 64, tok0 + j * PT_BK);
-                }
-            }
-        }
-        if constexpr (PAGED) paged_producer(kmap, k_sm, bars->k_full, bars->k_empty);
-    } else if (warp == 10) {
-        // =========================================================== TMA producer: the V tiles (independent of K's progress)
-        if constexpr (PAGED) {
-            paged_producer(vmap, v_sm, bars->v_full, bars->v_empty);
-        } else if (lane == 0) {
+    if (warp < 4) {
+        reg_dec<PT_REGS_FEW>();
+        // PAGED producer (one whole warp per ring): step j = pages 8j .. 8j+7 of the sequence.  The block-table
+        // entries of the NEXT step are fetched before this step's stage is waited for; lane 0 arms the mbarrier with the
+        // bytes of the pages that exist, then lanes 0..7 issue the two (64 d x 16 token) boxes of one page each.
+        auto paged_producer = [&](const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty) {
+            const int32_t* bt = pg.block_table + (int64_t)pg.seq_ids[seq] * pg.max_blocks_per_seq;
+            const int npages = (kvlen + PT_PAGE - 1) / PT_PAGE;
+            constexpr int PPS = PT_BK / PT_PAGE;                  // pages per step
+            int nxt = (lane < PPS && lane < npages) ? bt[lane] : 0;
             for (int j = 0; j < nkt; j++) {
                 const int st = j % PT_STAGES;
-                mbar_wait(smem_u32(&bars->v_empty[st]), ((j / PT_STAGES) & 1) ^ 1);
-                const uint32_t vb = smem_u32(&bars->v_full[st]);
-                mbar_arrive_expect_tx(vb, PT_KV_BYTES);
-                tma_load_2d(smem_u32(v_sm + st * PT_KV_BYTES), &vmap, vb, kvh * PT_D, tok0 + j * PT_BK);
-                tma_load_2d(smem_u32(v_sm + st * PT_KV_BYTES + PT_KV_BYTES / 2), &vmap, vb, kvh * PT_D + 64, tok0 + j * PT_BK);
+                const int blk = nxt;
+                const int npg = (j + 1) * PPS + lane;
+                nxt = (j + 1 < nkt && lane < PPS && npg < npages) ? bt[npg] : 0;
+                const int valid = min(PPS, npages - j * PPS);      // >= 1: step j exists because page 8j does
+                const uint32_t bar = smem_u32(&full[st]);
+                if (lane == 0) {
+                    mbar_wait(smem_u32(&empty[st]), ((j / PT_STAGES) & 1) ^ 1);
+                    mbar_arrive_expect_tx(bar, (uint32_t)valid * PT_PAGE * PT_D * 2);
+                }
+                __syncwarp();
+                if (lane < valid) {
+                    // row of the cache viewed as [num_blocks * L * nkv * 16 rows, 128]: first token row of this page
+                    const int64_t row = (((int64_t)blk * pg.num_layers + pg.cur_layer) * p.nkv + kvh) * PT_PAGE;
+                    const uint32_t dst = smem_u32(ring + st * PT_KV_BYTES) + lane * (PT_PAGE * 128);
+                    tma_load_2d(dst, &map, bar, 0, (int)row);
+                    tma_load_2d(dst + PT_KV_BYTES / 2, &map, bar, 64, (int)row);
+                }
             }
-        }
-    } else if (warp == 1) {
-        // =========================================================== MMA issuer: the whole warp runs the polling loop
-        // converged (votes make the control flow provably uniform); one elected lane issues the UMMAs and commits.
-        {
+        };
+        auto packed_producer = [&](const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty) {
+            for (int j = 0; j < nkt; j++) {
+                const int st = j % PT_STAGES;
+                mbar_wait(smem_u32(&empty[st]), ((j / PT_STAGES) & 1) ^ 1);
+                const uint32_t bar = smem_u32(&full[st]), dst = smem_u32(ring + st * PT_KV_BYTES);
+                mbar_arrive_expect_tx(bar, PT_KV_BYTES);
+                tma_load_2d(dst, &map, bar, kvh * PT_D, tok0 + j * PT_BK);
+                tma_load_2d(dst + PT_KV_BYTES / 2, &map, bar, kvh * PT_D + 64, tok0 + j * PT_BK);
+            }
+        };
+        if (warp == 0) {
+            // ======================================================= TMA producer: Q once, then the K tiles
+            if (lane == 0) {
+                const uint32_t qbar = smem_u32(&bars->q_full);
+                mbar_arrive_expect_tx(qbar, 2 * PT_Q_BYTES);
+                for (int x = 0; x < 2; x++)
+                    for (int h = 0; h < 2; h++)
+                        tma_load_2d(smem_u32(q_sm + x * PT_Q_BYTES + h * (PT_Q_BYTES / 2)), &qmap, qbar, head * PT_D + h * 64,
+                                    tok0 + q0 + x * PT_BQ);
+                if constexpr (!PAGED) packed_producer(kmap, k_sm, bars->k_full, bars->k_empty);
+            }
+            if constexpr (PAGED) paged_producer(kmap, k_sm, bars->k_full, bars->k_empty);
+        } else if (warp == 2) {
+            // ======================================================= TMA producer: the V tiles (independent of K's progress)
+            if constexpr (PAGED) paged_producer(vmap, v_sm, bars->v_full, bars->v_empty);
+            else if (lane == 0) packed_producer(vmap, v_sm, bars->v_full, bars->v_empty);
+        } else if (warp == 1) {
+            // ======================================================= product issuer: the warp stays converged, one elected lane issues
             constexpr uint32_t IDESC_S = make_instr_desc(128, PT_BK, UmmaFmt<T>::value, 0, 0);
             constexpr uint32_t IDESC_O = make_instr_desc(128, PT_D, UmmaFmt<T>::value, 0, 1);      // B = V, MN-major
-            constexpr uint32_t FULL = 0xffffffffu;
-            const uint32_t tm = __shfl_sync(FULL, tmem, 0);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
             // Descriptor bases are loop invariants; per UMMA only the 14-bit address field (16-byte units, low word)
             // advances by a compile-time constant (all tiles live below 256 KiB, so no carry into the LBO field).
             const uint64_t dq0 = make_smem_desc(smem_u32(q_sm), 16, 1024);
             const uint64_t dk0 = make_smem_desc(smem_u32(k_sm), 16, 1024);
             const uint64_t dv0 = make_smem_desc(smem_u32(v_sm), PT_KV_BYTES / 2, 1024);             // MN-major: LBO = d-half stride
-            const uint64_t dp0 = make_smem_desc(smem_u32(p_sm), 16, 1024);
-            mbar_wait(smem_u32(&bars->q_full), 0);
-            int js = 0, jpa = 0, jpb = 0;
-            uint32_t spins = 0;
-            while (jpa < nkt_a || jpb < nkt_b) {
-                bool progressed = false;
-                if (js < nkt) {      // S_A(js), S_B(js)
-                    const int st = js % PT_STAGES;
-                    const bool ua = js < nkt_a, ub = js < nkt_b;
-                    const uint32_t spar = (js & 1) ^ 1;
-                    const bool ready = mbar_test_wait(smem_u32(&bars->k_full[st]), (js / PT_STAGES) & 1) &&
-                                       (!ua || mbar_test_wait(smem_u32(&bars->s_empty[0]), spar)) &&
-                                       (!ub || mbar_test_wait(smem_u32(&bars->s_empty[1]), spar));
-                    if (__all_sync(FULL, ready)) {
-                        tc_fence_after();
-                        if (elect_one()) {
-                            const uint64_t kd = dk0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
+            auto scores = [&](int x, int j) {         // S_X(j)
+                const int st = j % PT_STAGES;
+                const uint64_t kd = dk0 + (uint64_t)((st * PT_KV_BYTES) >> 4), qd = dq0 + (uint64_t)((x * PT_Q_BYTES) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                            for (int x = 0; x < 2; x++) {
-                                if (x == 0 ? ua : ub) {
-                                    const uint64_t qd = dq0 + (uint64_t)((x * PT_Q_BYTES) >> 4);
-#pragma unroll
-                                    for (int ks = 0; ks < 8; ks++)      // 16 d per UMMA; d-half = ks / 4
-                                        umma_ss(tm + x * 64, qd + (uint64_t)(((ks >> 2) * (PT_Q_BYTES / 2) + (ks & 3) * 32) >> 4),
-                                                kd + (uint64_t)(((ks >> 2) * (PT_KV_BYTES / 2) + (ks & 3) * 32) >> 4), IDESC_S, ks > 0);
-                                    umma_commit(smem_u32(&bars->s_full[x]));
-                                }
-                            }
-                            umma_commit(smem_u32(&bars->k_empty[st]));
-                        }
-                        __syncwarp();
-                        js++;
-                        progressed = true;
+                    for (int ks = 0; ks < 8; ks++) {  // 16 d per UMMA; d-half = ks / 4
+                        const uint64_t off = (uint64_t)(((ks >> 2) * (PT_KV_BYTES / 2) + (ks & 3) * 32) >> 4);
+                        umma_ss(tm + PT_S_COL + x * 128, qd + off, kd + off, IDESC_S, ks > 0);
                     }
+                    umma_commit(smem_u32(&bars->s_full[x]));
                 }
+                __syncwarp();
+            };
+            mbar_wait(smem_u32(&bars->q_full), 0);
+            mbar_wait(smem_u32(&bars->k_full[0]), 0);
+            tc_fence_after();
+            scores(0, 0);
+            if (nkt_b > 0) scores(1, 0);
+            if (elect_one()) umma_commit(smem_u32(&bars->k_empty[0]));
+            __syncwarp();
+            for (int j = 0; j < nkt; j++) {
+                const int st = j % PT_STAGES;
+                mbar_wait(smem_u32(&bars->v_full[st]), (j / PT_STAGES) & 1);
 #pragma unroll
-                for (int x = 0; x < 2; x++) {     // PV_X(jp[x])
-                    const int j = x == 0 ? jpa : jpb;
-                    const int nkx = x == 0 ? nkt_a : nkt_b;
-                    if (j < nkx && j < js) {
-                        const int st = j % PT_STAGES;
-                        const int pb = j & 1;
-                        const bool ready = mbar_test_wait(smem_u32(&bars->p_full[x][pb]), (j >> 1) & 1) &&
-                                           mbar_test_wait(smem_u32(&bars->v_full[st]), (j / PT_STAGES) & 1);
-                        if (__all_sync(FULL, ready)) {
+                for (int x = 0; x < 2; x++) {
+                    const int nkx = x == 0 ? nkt_a : nkt_b, end = x == 0 ? end_a : end_b;
+                    if (j < nkx) {
+                        // O_X += P_X(j) V(j): 16 tokens per UMMA, none past the last key the tile can see
+                        const int steps = min(PT_BK / 16, (end - j * PT_BK + 15) / 16);
+                        const uint64_t vd = dv0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
+                        const uint32_t o_addr = tm + PT_O_COL + x * 128, p_addr = tm + PT_S_COL + x * 128;
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            mbar_wait(smem_u32(&bars->p_full[x][h]), j & 1);
                             tc_fence_after();
-                            // the V stage is free once every tile that uses it has issued its PV
-                            const int jo = x == 0 ? jpb : jpa, nko = x == 0 ? nkt_b : nkt_a;
-                            const bool release_v = j >= nko || jo > j;
                             if (elect_one()) {
-                                const uint64_t vd = dv0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
-                                const uint64_t pd = dp0 + (uint64_t)(((x * 2 + pb) * PT_P_BYTES) >> 4);
 #pragma unroll
-                                for (int kt = 0; kt < 4; kt++)       // 16 tokens per UMMA
-                                    umma_ss(tm + 128 + x * 128, pd + (uint64_t)((kt * 32) >> 4), vd + (uint64_t)((kt * 2048) >> 4), IDESC_O,
-                                            (j > 0 || kt > 0) ? 1u : 0u);
-                                umma_commit(smem_u32(&bars->p_empty[x][pb]));
-                                if (release_v) umma_commit(smem_u32(&bars->v_empty[st]));
+                                for (int k = 4 * h; k < 4 * h + 4; k++)
+                                    if (k < steps) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
+                                if (h == 1 && j + 1 == nkx) umma_commit(smem_u32(&bars->o_done[x]));
                             }
                             __syncwarp();
-                            if (x == 0) jpa++; else jpb++;
-                            progressed = true;
+                        }
+                        if (j + 1 < nkx) {
+                            mbar_wait(smem_u32(&bars->k_full[(j + 1) % PT_STAGES]), ((j + 1) / PT_STAGES) & 1);
+                            tc_fence_after();
+                            scores(x, j + 1);
                         }
                     }
                 }
-                if (progressed) spins = 0;
-                else if (++spins > (1u << 24)) {
-                    if (lane == 0) printf("sllm: prefill MMA watchdog (block %d,%d,%d js=%d jpA=%d jpB=%d)\n", blockIdx.x, blockIdx.y, blockIdx.z, js, jpa, jpb);
-                    __trap();
+                if (elect_one()) {
+                    umma_commit(smem_u32(&bars->v_empty[st]));
+                    if (j + 1 < nkt) umma_commit(smem_u32(&bars->k_empty[(j + 1) % PT_STAGES]));
                 }
+                __syncwarp();
             }
         }
     } else {
-        // =========================================================== softmax warps: group x = 0 (tile A) / 1 (tile B)
-        const int x = (warp - 2) >> 2;
+        // =========================================================== softmax warps: tile x = 0 (A) / 1 (B)
+        reg_inc<PT_REGS_MANY>();
+        const int x = (warp - 4) >> 2;
         const int nk_mine = x == 0 ? nkt_a : nkt_b;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;                 // row within the tile = TMEM lane
         const int qi = q0 + x * PT_BQ + row;              // query index within the sequence
         const uint32_t tlane = (uint32_t)(quad * 32) << 16;
-        const uint32_t s_addr = tmem + tlane + x * 64;
-        const uint32_t o_addr = tmem + tlane + 128 + x * 128;
+        const uint32_t s_addr = tmem + tlane + PT_S_COL + x * 128;
+        const uint32_t o_addr = tmem + tlane + PT_O_COL + x * 128;
+        const float c = p.scale_log2e;
         float m_ref = -INFINITY, l = 0.f;
         for (int j = 0; j < nk_mine; j++) {
             mbar_wait(smem_u32(&bars->s_full[x]), j & 1);
             tc_fence_after();
-            uint32_t r0[32], r1[32];
-            tmem_ld32(s_addr, r0);
-            tmem_ld32(s_addr + 32, r1);
+            uint32_t r[4][32];
+#pragma unroll
+            for (int g = 0; g < 4; g++) tmem_ld32(s_addr + g * 32, r[g]);
             tmem_ld_wait();
-            tc_fence_before();
-            mbar_arrive(smem_u32(&bars->s_empty[x]));              // S buffer free: the next S UMMAs may overwrite it
 
             const int c0 = j * PT_BK;
-            const bool need_mask = c0 + PT_BK - 1 > pre + q0 + x * PT_BQ || c0 + PT_BK > kvlen;
-            // column c0+i is visible iff c0+i <= pre+qi and c0+i < kvlen  <=>  i <= lim   (branch-free selects)
-            const int lim = min(pre + qi, kvlen - 1) - c0;
-            float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;   // 4 independent chains
-            if (need_mask) {
+            if (c0 + PT_BK - 1 > pre + q0 + x * PT_BQ || c0 + PT_BK > kvlen) {
+                // column c0+i is visible iff c0+i <= pre+qi and c0+i < kvlen  <=>  i <= lim   (branch-free selects)
+                const int lim = min(pre + qi, kvlen - 1) - c0;
 #pragma unroll
-                for (int i = 0; i < 32; i++) r0[i] = i <= lim ? r0[i] : 0xff800000u;        // -inf
+                for (int i = 0; i < 128; i++) r[i >> 5][i & 31] = i <= lim ? r[i >> 5][i & 31] : 0xff800000u;        // -inf
             }
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // independent chains
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                mx0 = fmaxf(mx0, __uint_as_float(r0[i])); mx1 = fmaxf(mx1, __uint_as_float(r0[i + 1]));
-                mx2 = fmaxf(mx2, __uint_as_float(r0[i + 2])); mx3 = fmaxf(mx3, __uint_as_float(r0[i + 3]));
-            }
-            if (need_mask) {
+            for (int i = 0; i < 32; i += 2)
 #pragma unroll
-                for (int i = 0; i < 32; i++) r1[i] = i + 32 <= lim ? r1[i] : 0xff800000u;
-            }
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                mx0 = fmaxf(mx0, __uint_as_float(r1[i])); mx1 = fmaxf(mx1, __uint_as_float(r1[i + 1]));
-                mx2 = fmaxf(mx2, __uint_as_float(r1[i + 2])); mx3 = fmaxf(mx3, __uint_as_float(r1[i + 3]));
-            }
-            const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));       // max of the RAW scores (scale > 0 commutes with max)
-            const float m_new = fmaxf(m_ref, mx * p.scale_log2e);
+                for (int g = 0; g < 4; g++) mx[g] = fmaxf(mx[g], fmaxf(__uint_as_float(r[g][i]), __uint_as_float(r[g][i + 1])));
+            // max of the RAW scores (scale > 0 commutes with max)
+            const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c);
             // Lazy rescale.  The decision is per row, but tcgen05.ld/st are warp-collective (.sync.aligned): vote, and
             // let rows that do not need it take part with alpha = 1.
             const bool need = m_new > m_ref + PT_RESCALE_THRESHOLD;   // always true on the first tile (m_ref = -inf)
             if (j > 0 && __any_sync(0xffffffffu, need)) {
-                // O must be stable: wait until PV(j-1) of this tile has completed, then rescale this thread's row
-                mbar_wait(smem_u32(&bars->p_empty[x][(j - 1) & 1]), ((j - 1) >> 1) & 1);
                 const float alpha = need ? fast_exp2_tc(m_ref - m_new) : 1.0f;
                 l *= alpha;
-                tc_fence_after();
-#pragma unroll
-                for (int cc = 0; cc < 4; cc++) {
-                    uint32_t t[32];
-                    tmem_ld32(o_addr + cc * 32, t);
+#pragma unroll 1
+                for (int cc = 0; cc < 8; cc++) {
+                    uint32_t t[16];
+                    tmem_ld<16>(o_addr + cc * 16, t);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 32; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-                    tmem_st32(o_addr + cc * 32, t);
+                    for (int i = 0; i < 16; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
+                    tmem_st16(o_addr + cc * 16, t);
                 }
-                tmem_st_wait();
-                tc_fence_before();
             }
             if (need) m_ref = m_new;
-            // P buffer (j & 1) was last read by PV(j-2)
-            const int pb = j & 1;
-            if (j >= 2) mbar_wait(smem_u32(&bars->p_empty[x][pb]), ((j - 2) >> 1) & 1);
-            // p = exp2(s*c - m_ref) (<= 2^8), row sum in fp32, P row -> shared memory ([128 rows][128 B], SWIZZLE_128B)
-            float ls0 = 0.f, ls1 = 0.f;
-            const float neg_m = -m_ref, c = p.scale_log2e;
-            uint8_t* prow = p_sm + (x * 2 + pb) * PT_P_BYTES + row * 128;
+            // p = exp2(s*c - m_ref) (<= 2^8), row sum in fp32, P row over the scores (two keys per column)
+            float ls[4] = {0.f, 0.f, 0.f, 0.f};
+            const float neg_m = -m_ref;
 #pragma unroll
-            for (int ch = 0; ch < 8; ch++) {                       // 8 chunks of 8 tokens
-                uint32_t w[4];
+            for (int h = 0; h < 2; h++) {
+                uint32_t w[32];
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int i = ch * 8 + e * 2;                  // token pair (i, i+1) of this 64-token step
-                    const float a = fast_exp2_tc(fmaf(__uint_as_float(i < 32 ? r0[i] : r1[i - 32]), c, neg_m));
-                    const float b = fast_exp2_tc(fmaf(__uint_as_float(i + 1 < 32 ? r0[i + 1] : r1[i + 1 - 32]), c, neg_m));
-                    ls0 += a; ls1 += b;
+                for (int i = 0; i < 32; i++) {
+                    const int k = 2 * i;                           // keys 64 h + k, + 1
+                    const float2 e = fma2(__uint_as_float(r[2 * h + (k >> 5)][k & 31]), __uint_as_float(r[2 * h + (k >> 5)][(k & 31) + 1]), c, neg_m);
+                    const float a = fast_exp2_tc(e.x), b = fast_exp2_tc(e.y);
+                    ls[i & 1] += a; ls[2 + (i & 1)] += b;
                     typename Traits<T>::T2 v2 = Traits<T>::from_f2(make_float2(a, b));
-                    w[e] = *reinterpret_cast<uint32_t*>(&v2);
+                    w[i] = *reinterpret_cast<uint32_t*>(&v2);
                 }
-                *reinterpret_cast<uint4*>(prow + ((ch ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                tmem_st32(s_addr + 32 * h, w);
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(smem_u32(&bars->p_full[x][h]));
             }
-            l += ls0 + ls1;
-            fence_proxy_async();
-            mbar_arrive(smem_u32(&bars->p_full[x][pb]));
+            l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
         }
         if (nk_mine > 0) {
             // ---- epilogue: O / l -> global (row qi of this head), only rows inside the sequence
-            mbar_wait(smem_u32(&bars->p_empty[x][(nk_mine - 1) & 1]), ((nk_mine - 1) >> 1) & 1);   // PV(last) done => all done
+            mbar_wait(smem_u32(&bars->o_done[x]), 0);
             tc_fence_after();
             const float inv = 1.0f / l;
             T* orow = reinterpret_cast<T*>(p.o) + ((int64_t)(tok0 + qi) * p.nq + head) * PT_D;
@@ -383,6 +356,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                         *reinterpret_cast<uint4*>(orow + cc * 32 + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
+                __syncwarp();
             }
         }
     }
