@@ -6,22 +6,20 @@
 // swiftllm/worker/layers/transformer_layer.py:86-96.  head_dim 128, fp16/bf16: fp32 scores, exp2 online softmax in fp32, P rounded
 // to the storage dtype before P.V, o = h(acc / l).
 //
-// CTA = (sequence, q head, 256 query rows) = two 128-row tiles A and B, keys in steps of 128.  Three warpgroups:
+// CTA = (sequence, q head, 256 query rows) = two 128-row tiles A and B, keys in steps of 80.  Three warpgroups:
 //   warp 0 / 2  TMA producers: warp 0 loads Q (4 boxes of 128 rows x 64 d) once and then the K tiles, warp 2 the V tiles
-//               (2 boxes of 128 x 64 per step) into separate two-stage rings with their own mbarriers.
-//   warp 1      product issuer (one elected lane), a fixed order:  O_X += P_X(j) . V(j), then S_X = Q_X . K(j + 1), X = A, B in turn
-//               (8 UMMAs each, M = N = 128, K = 16; B of the former MN-major).
+//               (2 boxes of 80 x 64 per step) into separate four-stage rings with their own mbarriers.
+//   warp 1 / 3  product issuers of tile A / B (one elected lane):  S_X(j + 1) = Q_X . K(j + 1) as soon as the softmax warps hold S_X(j)
+//               in registers (8 UMMAs, M = 128 N = 80 K = 16), O_X += P_X(j) . V(j) when P_X(j) is there (5 UMMAs, N = 128, B MN-major).
 //   warps 4-7   softmax of tile A, warps 8-11 softmax of tile B: thread = query row = TMEM lane.  Row max and row sum
-//               are thread-local (no shuffles); P goes back into TMEM, over the scores it came from, as the A operand of P . V.
+//               are thread-local (no shuffles); P goes back into TMEM as the A operand of P . V.
 //               O is rescaled in TMEM only when the running max grew by more than 2^8 ("lazy rescale": the
 //               reference point m_ref trails the true max, exact in the end because l uses the same reference).
-// While one tile's softmax runs on the CUDA cores the tensor pipe works on the other tile.  The products of one CTA complete in the
-// order they are issued, so s_full (after S(j)) also says that P . V(j - 1) has been read out and that O is stable.
-// TMEM is full: S_A 0..127, S_B 128..255 (P_X in the first 64 columns of S_X), O_A 256..383, O_B 384..511.
+// TMEM: S_A 0..79, S_B 80..159, P_A 160..199, P_B 200..239, O_A 256..383, O_B 384..511.
 //
-// Why this split: with P in shared memory and steps of 64 keys the kernel was bound by shared-memory operand reads (96 KiB per tile and 64
-// keys).  P from TMEM and 128 keys per pass over Q need 96 KiB per tile and 128 keys; what is left is the exponentials (128 rows x 128
-// keys per tile and step are 1024 cycles of each scheduler's special-function unit) beside 1024 cycles of products.
+// Why steps of 80 keys: scores and P need places of their own, so that the next scores are multiplied while the softmax of the last ones
+// runs.  With 128 keys P has to lie over its scores (TMEM is full), which chains S, softmax and P . V of a tile one after the other: 3510
+// cycles a step where products and exponentials each need 2048.  80 keys are the most that leave room for both.
 // Roofline: tensor-bound; FLOPs = 4 * nq * D * sum_i L_i (L_i + 1) / 2.
 #pragma once
 #include "tc_helpers.cuh"
@@ -32,23 +30,23 @@ using namespace tc;
 
 constexpr int PT_D = 128;
 constexpr int PT_BQ = 128;                // rows per query tile (two tiles per CTA)
-constexpr int PT_BK = 128;                // kv tokens per pipeline step
-constexpr int PT_STAGES = 2;              // K and V rings (separate producers)
+constexpr int PT_BK = 80;                 // kv tokens per pipeline step
+constexpr int PT_STAGES = 4;              // K and V rings (separate producers)
 constexpr int PT_THREADS = 384;           // warp 0 Q + K producer, 1 products, 2 V producer, 4-7 softmax A, 8-11 softmax B
 constexpr int PT_Q_BYTES = PT_BQ * PT_D * 2;          // 32 KiB per query tile ([half][128 rows][128 B])
-constexpr int PT_KV_BYTES = PT_BK * PT_D * 2;         // 32 KiB per K (or V) tile ([half][128 rows][128 B])
+constexpr int PT_KV_BYTES = PT_BK * PT_D * 2;         // 20 KiB per K (or V) tile ([half][80 rows][128 B])
 constexpr int PT_SMEM_BYTES = 2 * PT_Q_BYTES + 2 * PT_STAGES * PT_KV_BYTES + 1024;
 constexpr int PT_TMEM_COLS = 512;
-constexpr int PT_S_COL = 0, PT_O_COL = 256;           // tile B: + 128
+constexpr int PT_S_COL = 0, PT_P_COL = 160, PT_O_COL = 256;      // tile B: + 80, + 40, + 128
 constexpr float PT_RESCALE_THRESHOLD = 8.0f;          // log2 units
-// registers: 384 threads are launched with 168 each; the softmax warpgroups hold a row of 128 scores
+// registers: 384 threads are launched with 168 each; the softmax warpgroups hold a row of scores and of P
 constexpr int PT_REGS_FEW = 72, PT_REGS_MANY = 216;
 static_assert(PT_REGS_FEW + 2 * PT_REGS_MANY <= 3 * 168, "the warpgroups' shares must fit what the block was launched with");
 
 struct PtBarriers {
     uint64_t q_full;
     uint64_t k_full[PT_STAGES], k_empty[PT_STAGES], v_full[PT_STAGES], v_empty[PT_STAGES];
-    uint64_t s_full[2], p_full[2][2], o_done[2];      // [tile]; P in two halves of 64 keys
+    uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2];      // [tile]
 };
 
 struct PtParams {
@@ -68,19 +66,29 @@ constexpr int PT_PAGE = 16;               // tokens per KV page (PAGED only)
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// (a, b) * c + d in one packed instruction
-__device__ __forceinline__ float2 fma2(float a, float b, float c, float d) {
+// two fp32 operations in one packed instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 o;
-    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %4};\n mov.b64 z, {%5, %5};\n fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
-        : "=f"(o.x), "=f"(o.y) : "f"(a), "f"(b), "f"(c), "f"(d));
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return o;
 }
-
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 o;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return o;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float o;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(o) : "f"(a), "f"(b), "f"(c));
+    return o;
+}
 // PAGED = false: K/V tiles come from the packed k/v rows of the batch (the reference's contract).
 // PAGED = true (chunked prefill): the chunk's queries sit at positions prefix .. prefix + len - 1 of
-// their sequence; every 128-token K/V step is gathered from eight 16-token pages of the KV cache through the block
-// table (lanes 0-7 of the producer warp issue the two d-half boxes of one page each), landing in the SAME
-// [half][128 rows][128 B] layout, so the product issuer and its descriptors are shared by both variants.
+// their sequence; every 80-token K/V step is gathered from five 16-token pages of the KV cache through the block
+// table (lanes 0-4 of the producer warp issue the two d-half boxes of one page each), landing in the SAME
+// [half][80 rows][128 B] layout, so the product issuer and its descriptors are shared by both variants.
 template <typename T, bool PAGED>
 __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap qmap,
                                                                         const __grid_constant__ CUtensorMap kmap,
@@ -88,7 +96,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                                                                         const PtParams p, const PtPaged pg) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_sm = smem;                                       // [2 tiles][2 halves][128 rows][128 B]
-    uint8_t* k_sm = q_sm + 2 * PT_Q_BYTES;                      // [stage][2 halves][128 rows][128 B]
+    uint8_t* k_sm = q_sm + 2 * PT_Q_BYTES;                      // [stage][2 halves][80 rows][128 B]
     uint8_t* v_sm = k_sm + PT_STAGES * PT_KV_BYTES;
     uint8_t* misc = v_sm + PT_STAGES * PT_KV_BYTES;
     PtBarriers* bars = reinterpret_cast<PtBarriers*>(misc);
@@ -118,12 +126,13 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     if (tid == 0) {
         mbar_init(smem_u32(&bars->q_full), 1);
         for (int i = 0; i < PT_STAGES; i++) {
-            mbar_init(smem_u32(&bars->k_full[i]), 1); mbar_init(smem_u32(&bars->k_empty[i]), 1);
-            mbar_init(smem_u32(&bars->v_full[i]), 1); mbar_init(smem_u32(&bars->v_empty[i]), 1);
+            const int users = active_b ? 2 : 1;
+            mbar_init(smem_u32(&bars->k_full[i]), 1); mbar_init(smem_u32(&bars->k_empty[i]), users);
+            mbar_init(smem_u32(&bars->v_full[i]), 1); mbar_init(smem_u32(&bars->v_empty[i]), users);
         }
         for (int x = 0; x < 2; x++) {
-            mbar_init(smem_u32(&bars->s_full[x]), 1); mbar_init(smem_u32(&bars->o_done[x]), 1);
-            mbar_init(smem_u32(&bars->p_full[x][0]), 128); mbar_init(smem_u32(&bars->p_full[x][1]), 128);
+            mbar_init(smem_u32(&bars->s_full[x]), 1); mbar_init(smem_u32(&bars->s_empty[x]), 128);
+            mbar_init(smem_u32(&bars->p_full[x]), 128); mbar_init(smem_u32(&bars->p_empty[x]), 1);
         }
         mbar_fence_init();
         tma_prefetch_desc(&qmap); tma_prefetch_desc(&kmap); tma_prefetch_desc(&vmap);
@@ -136,9 +145,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
 
     if (warp < 4) {
         reg_dec<PT_REGS_FEW>();
-        // PAGED producer (one whole warp per ring): step j = pages 8j .. 8j+7 of the sequence.  The block-table
+        // PAGED producer (one whole warp per ring): step j = pages 5j .. 5j+4 of the sequence.  The block-table
         // entries of the NEXT step are fetched before this step's stage is waited for; lane 0 arms the mbarrier with the
-        // bytes of the pages that exist, then lanes 0..7 issue the two (64 d x 16 token) boxes of one page each.
+        // bytes of the pages that exist, then lanes 0..4 issue the two (64 d x 16 token) boxes of one page each.
         auto paged_producer = [&](const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty) {
             const int32_t* bt = pg.block_table + (int64_t)pg.seq_ids[seq] * pg.max_blocks_per_seq;
             const int npages = (kvlen + PT_PAGE - 1) / PT_PAGE;
@@ -149,7 +158,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 const int blk = nxt;
                 const int npg = (j + 1) * PPS + lane;
                 nxt = (j + 1 < nkt && lane < PPS && npg < npages) ? bt[npg] : 0;
-                const int valid = min(PPS, npages - j * PPS);      // >= 1: step j exists because page 8j does
+                const int valid = min(PPS, npages - j * PPS);      // >= 1: step j exists because page 5j does
                 const uint32_t bar = smem_u32(&full[st]);
                 if (lane == 0) {
                     mbar_wait(smem_u32(&empty[st]), ((j / PT_STAGES) & 1) ^ 1);
@@ -191,71 +200,67 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             // ======================================================= TMA producer: the V tiles (independent of K's progress)
             if constexpr (PAGED) paged_producer(vmap, v_sm, bars->v_full, bars->v_empty);
             else if (lane == 0) packed_producer(vmap, v_sm, bars->v_full, bars->v_empty);
-        } else if (warp == 1) {
-            // ======================================================= product issuer: the warp stays converged, one elected lane issues
+        } else {
+            // ======================================================= product issuers: warp 1 for tile A, warp 3 for tile B, so that neither
+            // waits for the other tile; the warp stays converged, one elected lane issues
+            const int x = warp >> 1;
+            const int nkx = x == 0 ? nkt_a : nkt_b, end = x == 0 ? end_a : end_b;
             constexpr uint32_t IDESC_S = make_instr_desc(128, PT_BK, UmmaFmt<T>::value, 0, 0);
             constexpr uint32_t IDESC_O = make_instr_desc(128, PT_D, UmmaFmt<T>::value, 0, 1);      // B = V, MN-major
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint32_t s_addr = tm + PT_S_COL + x * PT_BK, p_addr = tm + PT_P_COL + x * (PT_BK / 2), o_addr = tm + PT_O_COL + x * 128;
             // Descriptor bases are loop invariants; per UMMA only the 14-bit address field (16-byte units, low word)
             // advances by a compile-time constant (all tiles live below 256 KiB, so no carry into the LBO field).
-            const uint64_t dq0 = make_smem_desc(smem_u32(q_sm), 16, 1024);
+            const uint64_t dq0 = make_smem_desc(smem_u32(q_sm + x * PT_Q_BYTES), 16, 1024);
             const uint64_t dk0 = make_smem_desc(smem_u32(k_sm), 16, 1024);
             const uint64_t dv0 = make_smem_desc(smem_u32(v_sm), PT_KV_BYTES / 2, 1024);             // MN-major: LBO = d-half stride
-            auto scores = [&](int x, int j) {         // S_X(j)
+            auto scores = [&](int j) {                // S_X(j)
                 const int st = j % PT_STAGES;
-                const uint64_t kd = dk0 + (uint64_t)((st * PT_KV_BYTES) >> 4), qd = dq0 + (uint64_t)((x * PT_Q_BYTES) >> 4);
+                mbar_wait(smem_u32(&bars->k_full[st]), (j / PT_STAGES) & 1);
+                tc_fence_after();
+                const uint64_t kd = dk0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
                 if (elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < 8; ks++) {  // 16 d per UMMA; d-half = ks / 4
-                        const uint64_t off = (uint64_t)(((ks >> 2) * (PT_KV_BYTES / 2) + (ks & 3) * 32) >> 4);
-                        umma_ss(tm + PT_S_COL + x * 128, qd + off, kd + off, IDESC_S, ks > 0);
-                    }
+                    for (int ks = 0; ks < 8; ks++)    // 16 d per UMMA; d-half = ks / 4
+                        umma_ss(s_addr, dq0 + (uint64_t)(((ks >> 2) * (PT_Q_BYTES / 2) + (ks & 3) * 32) >> 4),
+                                kd + (uint64_t)(((ks >> 2) * (PT_KV_BYTES / 2) + (ks & 3) * 32) >> 4), IDESC_S, ks > 0);
                     umma_commit(smem_u32(&bars->s_full[x]));
+                    umma_commit(smem_u32(&bars->k_empty[st]));
                 }
                 __syncwarp();
             };
-            mbar_wait(smem_u32(&bars->q_full), 0);
-            mbar_wait(smem_u32(&bars->k_full[0]), 0);
-            tc_fence_after();
-            scores(0, 0);
-            if (nkt_b > 0) scores(1, 0);
-            if (elect_one()) umma_commit(smem_u32(&bars->k_empty[0]));
-            __syncwarp();
-            for (int j = 0; j < nkt; j++) {
-                const int st = j % PT_STAGES;
-                mbar_wait(smem_u32(&bars->v_full[st]), (j / PT_STAGES) & 1);
-#pragma unroll
-                for (int x = 0; x < 2; x++) {
-                    const int nkx = x == 0 ? nkt_a : nkt_b, end = x == 0 ? end_a : end_b;
-                    if (j < nkx) {
-                        // O_X += P_X(j) V(j): 16 tokens per UMMA, none past the last key the tile can see
-                        const int steps = min(PT_BK / 16, (end - j * PT_BK + 15) / 16);
-                        const uint64_t vd = dv0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
-                        const uint32_t o_addr = tm + PT_O_COL + x * 128, p_addr = tm + PT_S_COL + x * 128;
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            mbar_wait(smem_u32(&bars->p_full[x][h]), j & 1);
-                            tc_fence_after();
-                            if (elect_one()) {
-#pragma unroll
-                                for (int k = 4 * h; k < 4 * h + 4; k++)
-                                    if (k < steps) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
-                                if (h == 1 && j + 1 == nkx) umma_commit(smem_u32(&bars->o_done[x]));
-                            }
-                            __syncwarp();
-                        }
-                        if (j + 1 < nkx) {
-                            mbar_wait(smem_u32(&bars->k_full[(j + 1) % PT_STAGES]), ((j + 1) / PT_STAGES) & 1);
-                            tc_fence_after();
-                            scores(x, j + 1);
-                        }
+            if (nkx > 0) {
+                mbar_wait(smem_u32(&bars->q_full), 0);
+                scores(0);
+                for (int j = 0; j < nkx; j++) {
+                    if (j + 1 < nkx) {
+                        mbar_wait(smem_u32(&bars->s_empty[x]), j & 1);
+                        scores(j + 1);
                     }
+                    const int st = j % PT_STAGES;
+                    mbar_wait(smem_u32(&bars->v_full[st]), (j / PT_STAGES) & 1);
+                    mbar_wait(smem_u32(&bars->p_full[x]), j & 1);
+                    tc_fence_after();
+                    // O_X += P_X(j) V(j): 16 tokens per UMMA, none past the last key the tile can see
+                    const int steps = min(PT_BK / 16, (end - j * PT_BK + 15) / 16);
+                    const uint64_t vd = dv0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < PT_BK / 16; k++)
+                            if (k < steps) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
+                        umma_commit(smem_u32(&bars->v_empty[st]));
+                        umma_commit(smem_u32(&bars->p_empty[x]));
+                    }
+                    __syncwarp();
                 }
-                if (elect_one()) {
-                    umma_commit(smem_u32(&bars->v_empty[st]));
-                    if (j + 1 < nkt) umma_commit(smem_u32(&bars->k_empty[(j + 1) % PT_STAGES]));
+                // steps the other tile still takes: hand the stages on once they have been filled (never a phase ahead)
+                for (int j = nkx; j < nkt; j++) {
+                    const int st = j % PT_STAGES;
+                    mbar_wait(smem_u32(&bars->k_full[st]), (j / PT_STAGES) & 1);
+                    if (lane == 0) mbar_arrive(smem_u32(&bars->k_empty[st]));
+                    mbar_wait(smem_u32(&bars->v_full[st]), (j / PT_STAGES) & 1);
+                    if (lane == 0) mbar_arrive(smem_u32(&bars->v_empty[st]));
                 }
-                __syncwarp();
             }
         }
     } else {
@@ -267,36 +272,42 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
         const int row = quad * 32 + lane;                 // row within the tile = TMEM lane
         const int qi = q0 + x * PT_BQ + row;              // query index within the sequence
         const uint32_t tlane = (uint32_t)(quad * 32) << 16;
-        const uint32_t s_addr = tmem + tlane + PT_S_COL + x * 128;
+        const uint32_t s_addr = tmem + tlane + PT_S_COL + x * PT_BK;
+        const uint32_t p_addr = tmem + tlane + PT_P_COL + x * (PT_BK / 2);
         const uint32_t o_addr = tmem + tlane + PT_O_COL + x * 128;
         const float c = p.scale_log2e;
         float m_ref = -INFINITY, l = 0.f;
         for (int j = 0; j < nk_mine; j++) {
             mbar_wait(smem_u32(&bars->s_full[x]), j & 1);
             tc_fence_after();
-            uint32_t r[4][32];
-#pragma unroll
-            for (int g = 0; g < 4; g++) tmem_ld32(s_addr + g * 32, r[g]);
+            uint32_t r[PT_BK];
+            tmem_ld32(s_addr, reinterpret_cast<uint32_t(&)[32]>(r[0]));
+            tmem_ld32(s_addr + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+            tmem_ld<16>(s_addr + 64, reinterpret_cast<uint32_t(&)[16]>(r[64]));
             tmem_ld_wait();
+            tc_fence_before();
+            mbar_arrive(smem_u32(&bars->s_empty[x]));
 
             const int c0 = j * PT_BK;
             if (c0 + PT_BK - 1 > pre + q0 + x * PT_BQ || c0 + PT_BK > kvlen) {
                 // column c0+i is visible iff c0+i <= pre+qi and c0+i < kvlen  <=>  i <= lim   (branch-free selects)
                 const int lim = min(pre + qi, kvlen - 1) - c0;
 #pragma unroll
-                for (int i = 0; i < 128; i++) r[i >> 5][i & 31] = i <= lim ? r[i >> 5][i & 31] : 0xff800000u;        // -inf
+                for (int i = 0; i < PT_BK; i++) r[i] = i <= lim ? r[i] : 0xff800000u;        // -inf
             }
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};        // independent chains
 #pragma unroll
-            for (int i = 0; i < 32; i += 2)
+            for (int i = 0; i < PT_BK; i += 8)
 #pragma unroll
-                for (int g = 0; g < 4; g++) mx[g] = fmaxf(mx[g], fmaxf(__uint_as_float(r[g][i]), __uint_as_float(r[g][i + 1])));
+                for (int g = 0; g < 4; g++) mx[g] = max3(mx[g], __uint_as_float(r[i + 2 * g]), __uint_as_float(r[i + 2 * g + 1]));
             // max of the RAW scores (scale > 0 commutes with max)
             const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c);
             // Lazy rescale.  The decision is per row, but tcgen05.ld/st are warp-collective (.sync.aligned): vote, and
             // let rows that do not need it take part with alpha = 1.
             const bool need = m_new > m_ref + PT_RESCALE_THRESHOLD;   // always true on the first tile (m_ref = -inf)
             if (j > 0 && __any_sync(0xffffffffu, need)) {
+                mbar_wait(smem_u32(&bars->p_empty[x]), (j - 1) & 1);       // P . V(j - 1) is done: O is stable
+                tc_fence_after();
                 const float alpha = need ? fast_exp2_tc(m_ref - m_new) : 1.0f;
                 l *= alpha;
 #pragma unroll 1
@@ -310,31 +321,29 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 }
             }
             if (need) m_ref = m_new;
-            // p = exp2(s*c - m_ref) (<= 2^8), row sum in fp32, P row over the scores (two keys per column)
-            float ls[4] = {0.f, 0.f, 0.f, 0.f};
-            const float neg_m = -m_ref;
+            // p = exp2(s*c - m_ref) (<= 2^8), row sum in fp32, P row into TMEM (two keys per column)
+            float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            const float2 neg_m = make_float2(-m_ref, -m_ref), c2 = make_float2(c, c);
+            uint32_t w[PT_BK / 2];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                uint32_t w[32];
-#pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    const int k = 2 * i;                           // keys 64 h + k, + 1
-                    const float2 e = fma2(__uint_as_float(r[2 * h + (k >> 5)][k & 31]), __uint_as_float(r[2 * h + (k >> 5)][(k & 31) + 1]), c, neg_m);
-                    const float a = fast_exp2_tc(e.x), b = fast_exp2_tc(e.y);
-                    ls[i & 1] += a; ls[2 + (i & 1)] += b;
-                    typename Traits<T>::T2 v2 = Traits<T>::from_f2(make_float2(a, b));
-                    w[i] = *reinterpret_cast<uint32_t*>(&v2);
-                }
-                tmem_st32(s_addr + 32 * h, w);
-                tmem_st_wait();
-                tc_fence_before();
-                mbar_arrive(smem_u32(&bars->p_full[x][h]));
+            for (int i = 0; i < PT_BK / 2; i++) {
+                const float2 e = fma2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), c2, neg_m);
+                const float2 v = make_float2(fast_exp2_tc(e.x), fast_exp2_tc(e.y));
+                ls[i & 1] = add2(ls[i & 1], v);
+                typename Traits<T>::T2 v2 = Traits<T>::from_f2(v);
+                w[i] = *reinterpret_cast<uint32_t*>(&v2);
             }
-            l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+            if (j > 0) { mbar_wait(smem_u32(&bars->p_empty[x]), (j - 1) & 1); tc_fence_after(); }      // P(j - 1) has been read
+            tmem_st32(p_addr, reinterpret_cast<uint32_t(&)[32]>(w[0]));
+            tmem_st8(p_addr + 32, reinterpret_cast<uint32_t(&)[8]>(w[32]));
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(smem_u32(&bars->p_full[x]));
+            l += (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y);
         }
         if (nk_mine > 0) {
             // ---- epilogue: O / l -> global (row qi of this head), only rows inside the sequence
-            mbar_wait(smem_u32(&bars->o_done[x]), 0);
+            mbar_wait(smem_u32(&bars->p_empty[x]), (nk_mine - 1) & 1);          // the last P . V
             tc_fence_after();
             const float inv = 1.0f / l;
             T* orow = reinterpret_cast<T*>(p.o) + ((int64_t)(tok0 + qi) * p.nq + head) * PT_D;
