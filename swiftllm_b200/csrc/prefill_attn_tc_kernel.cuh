@@ -66,24 +66,6 @@ constexpr int PT_PAGE = 16;               // tokens per KV page (PAGED only)
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// two fp32 operations in one packed instruction
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 o;
-    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
-        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return o;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 o;
-    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}"
-        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return o;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float o;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(o) : "f"(a), "f"(b), "f"(c));
-    return o;
-}
 // PAGED = false: K/V tiles come from the packed k/v rows of the batch (the reference's contract).
 // PAGED = true (chunked prefill): the chunk's queries sit at positions prefix .. prefix + len - 1 of
 // their sequence; every 80-token K/V step is gathered from five 16-token pages of the KV cache through the block

@@ -160,6 +160,24 @@ __device__ __forceinline__ float fast_exp2_tc(float x) {
     return y;
 }
 
+// two fp32 operations in one packed instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 o;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return o;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 o;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return o;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float o;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(o) : "f"(a), "f"(b), "f"(c));
+    return o;
+}
 // One lane of a CONVERGED warp.  Issuing tcgen05.mma from `if (elect_one())` inside warp-uniform control flow was measured
 // faster than issuing it under a plain `if (lane == 0)`.
 __device__ __forceinline__ bool elect_one() {

@@ -32,8 +32,11 @@
 //                      krot + dk - 1 of the key part) and the value its first dk columns
 //   sinks              a learned number per head: the softmax's denominator also contains exp(sinks[h])
 // diff_combine: per token and head, o = a1 - lambda * a2 of two maps' outputs, o / sqrt(mean(o^2) + eps) * factor * sigmoid(gate).
+#include <type_traits>
+
 #include "mma_helpers.cuh"
 #include "typed_io.cuh"
+#include "window_attn_tc.cuh"
 
 namespace sllm {
 
@@ -1107,6 +1110,25 @@ static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void*
     for (int k = 0; k < 2; k++) {
         const int64_t first = parts[k][0], count = parts[k][1];
         if (count <= 0) continue;
+        // prompt rows: tcgen05 (window_attn_tc.cu) where the products can be cut from the rows
+        if (k == 0 && window_tc_supported(dk, dv, krot, hq, scale, cache, count)) {
+            WindowTc w;
+            w.q = q; w.q_st = q_stride_t; w.cosb = (const float*)cosb; w.sinb = (const float*)sinb; w.gate = gate; w.gate_st = gate_stride_t;
+            w.cache = cache; w.n_slots = n_slots; w.slot = slot; w.block_size = block_size; w.block_table = (const int*)block_table;
+            w.max_blocks_per_seq = max_blocks_per_seq; w.tok_seq = (const int*)tok_seq; w.tok_pos = (const int*)tok_pos; w.out = out;
+            w.out_st = out_stride_t; w.num_rows = (int)count; w.H = H; w.G = G; w.dk = dk; w.dv = dv; w.rot_dims = rot_dims; w.window = window;
+            w.scale = scale; w.sink = sink; w.halves = halves; w.qk_norm_eps = qk_norm_eps; w.softcap = softcap; w.vcos = (const float*)vcos;
+            w.vsin = (const float*)vsin; w.out_scale = out_scale; w.qnorm_w = (const float*)qnorm_w; w.prenorm_eps = prenorm_eps; w.chunk = chunk;
+            w.vshare = vshare; w.out_f32 = out_f32; w.slopes = (const float*)slopes; w.keep_first = keep_first; w.gate_per_head = gate_per_head;
+            w.shared_kv = shared_kv; w.krot = krot; w.sinks = (const float*)sinks;
+            w.row_elems = shared_kv ? shared_kv_row(G, dk + krot) : G * dk + (G / vshare) * dv;
+            w.koff = shared_kv ? shared_kv_key_offset(G) : 0;
+            w.q_vec = ((uintptr_t)q & 15) == 0 && q_stride_t % 8 == 0 && (!halves || rot_dims % 16 == 0);
+            w.gate_vec = ((uintptr_t)gate & 15) == 0 && gate_stride_t % 8 == 0;
+            w.out_vec = ((uintptr_t)out & 15) == 0 && out_stride_t % 8 == 0;
+            if (int rc = launch_window_attn_tc(w, std::is_same<T, __half>::value ? SLLM_F16 : SLLM_BF16, stream)) return rc;
+            continue;
+        }
         if (k == 1 && hq <= 16) {
             size_t smem = 16 * (size_t)(dk * 2 + 16) + WD_WARPS * WD_STAGES * (size_t)KT * (tile_pitch(dk + krot) + (shared_kv ? sizeof(float) : dv * 2 + 16));
             const size_t merge = ((size_t)WD_WARPS * hq * dv + 2 * WD_WARPS * 16) * sizeof(float);

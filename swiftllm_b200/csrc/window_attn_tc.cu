@@ -1,0 +1,542 @@
+// Window attention for prompt rows in 16-bit storage on the fifth-generation tensor cores (tcgen05 + TMEM): the same function as
+// window_attn.cu, whose head comment gives the definition, the cache rows and the options.
+//
+// A CTA owns two tiles of 128 query ROWS of one key/value group, row = (token, head of the group) with the heads padded to a power of
+// two: 64 tokens for four heads per group.  Tokens are walked in segments (runs of one sequence at consecutive positions), so any order
+// of rows is correct; a segment's rows share ONE list of keys (kept first positions, then the window), taken in steps of 80.
+//   warps 0, 2   producers: gather cache rows through the block table by cp.async into a four-stage ring (keys past the segment's last
+//                position are zero)
+//   warps 1, 3   product issuers of tile A / B:  S_X(j + 1) = Q_X . K(j + 1) as soon as S_X(j) is in registers,
+//                O_X += P_X(j) . V(j) when P_X(j) is there; with shared_kv the key tile is also the value tile
+//   warps 4-7    softmax and output of tile A, warps 8-11 of tile B: thread = query row = TMEM lane, P as 16-bit A operand in TMEM,
+//                O rescaled only when the running maximum grew by more than 2^8
+// TMEM: S_A 0..79, S_B 80..159, P_A 160..199, P_B 200..239, O_A 256..383, O_B 384..511 (the layout of the prefill kernel: 80 keys are the
+// most that leave scores and P places of their own).
+//
+// Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
+// ones 317 us with the mma.sync kernel of window_attn.cu for the prompts -> 169 us.
+//
+// EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores.
+#include "mma_helpers.cuh"
+#include "tc_helpers.cuh"
+#include "typed_io.cuh"
+#include "window_attn_tc.cuh"
+
+namespace sllm {
+
+using namespace tc;
+
+constexpr int WX_ROWS = 128, WX_BK = 80, WX_STAGES = 4, WX_THREADS = 384;
+constexpr int WX_QCHUNK = WX_ROWS * 128;              // 128 rows x 64 columns
+constexpr int WX_CHUNK = WX_BK * 128;                 // 80 keys x 64 columns
+constexpr int WX_CHUNKS = 4;                          // 64-column chunks of a stage: keys, then values (shared_kv: keys only)
+constexpr int WX_STAGE = WX_CHUNKS * WX_CHUNK;
+constexpr int WX_Q_BYTES = 2 * WX_QCHUNK;
+constexpr int WX_INV_OFF = 2 * WX_Q_BYTES + WX_STAGES * WX_STAGE;                 // [stage][80] fp32: the keys' 1 / rms
+constexpr int WX_MISC_OFF = WX_INV_OFF + WX_STAGES * WX_BK * 4;
+constexpr int WX_SMEM = WX_MISC_OFF + 256;
+constexpr int WX_S_COL = 0, WX_P_COL = 160, WX_O_COL = 256;      // tile B: + 80, + 40, + 128
+constexpr float WX_RESCALE = 8.0f;                    // log2 units
+constexpr float WX_LOG2E = 1.4426950408889634f;
+constexpr int WX_LAG = 2;                             // steps whose rows are in flight behind the one being asked for
+
+struct WindowTcBars {
+    uint64_t full[WX_STAGES], empty[WX_STAGES];
+    uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2];
+};
+
+__device__ __forceinline__ uint32_t wx_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
+
+template <typename T, bool EXT, bool CAP>
+__global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const WindowTc p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* q_sm = smem;                             // [tile][chunk][128 rows][128 B]
+    uint8_t* kv_sm = smem + 2 * WX_Q_BYTES;           // [stage][chunk][80 keys][128 B]
+    float* inv_sm = reinterpret_cast<float*>(smem + WX_INV_OFF);
+    WindowTcBars* bars = reinterpret_cast<WindowTcBars*>(smem + WX_MISC_OFF);
+    uint32_t* tmem_s = reinterpret_cast<uint32_t*>(smem + WX_MISC_OFF + sizeof(WindowTcBars));
+    static_assert(sizeof(WindowTcBars) + 4 <= 256, "");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool shared_kv = EXT && p.shared_kv;
+    const int krot = EXT ? p.krot : 0, keep_first = EXT ? p.keep_first : 0;
+    const int dk = p.dk, dv = p.dv, KW = dk + krot, hq = p.H / p.G, hqp = 1 << p.hqp_log2, g = blockIdx.y;
+    const int kch = (KW + 63) >> 6, vch = shared_kv ? 0 : (dv + 63) >> 6;         // chunks of a key / value row
+    const int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;                       // the last tokens of a prompt have the most keys: first
+    const int ntok = min(p.qt, p.num_rows - t_first);
+
+    if (tid == 0) {
+        for (int s = 0; s < WX_STAGES; s++) { mbar_init(smem_u32(&bars->full[s]), 2); mbar_init(smem_u32(&bars->empty[s]), 2); }
+        for (int x = 0; x < 2; x++) {
+            mbar_init(smem_u32(&bars->s_full[x]), 1); mbar_init(smem_u32(&bars->s_empty[x]), 128);
+            mbar_init(smem_u32(&bars->p_full[x]), 128); mbar_init(smem_u32(&bars->p_empty[x]), 1);
+        }
+        mbar_fence_init();
+    }
+    if (warp == 1) tmem_alloc<512>(smem_u32(tmem_s));
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_s;
+
+    int n_done = 0, x_done[2] = {0, 0};               // steps of the segments before (of the ring, of each tile): the barriers' phases
+    for (int i0 = 0; i0 < ntok;) {
+        // ---- the segment: tokens ts .. ts + n - 1 of one sequence at positions pos0 ..
+        const int ts = t_first + i0, left = ntok - i0;
+        const int seq = p.tok_seq[ts], pos0 = p.tok_pos[ts];
+        int n = left;
+        for (int b = 0; b < left; b += 32) {
+            const int i = b + min(lane, left - 1 - b);
+            const uint32_t cut = __ballot_sync(0xffffffffu, p.tok_seq[ts + i] != seq || p.tok_pos[ts + i] != pos0 + i);
+            if (cut) { n = b + __ffs(cut) - 1; break; }
+        }
+        const int* bt = p.block_table + (int64_t)seq * p.max_blocks_per_seq;
+        auto first_seen = [&](int pos) {              // first position of the window (and chunk) of a query at `pos`
+            int a = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
+            if (p.chunk > 0) a = max(a, pos / p.chunk * p.chunk);
+            return a;
+        };
+        const int lo = first_seen(pos0), hi = pos0 + n - 1;
+        const int nk = EXT && p.window > 0 ? min(keep_first, lo) : 0;
+        const int vkeep = EXT && p.window > 0 ? keep_first : 0;                    // list entries below it are kept positions
+        const int tpt = WX_ROWS >> p.hqp_log2;                                    // tokens per tile
+        const int na = min(n, tpt), nb = n - na;
+        // entry v of the list of keys is position v (v < nk) or v - nk + lo; entries a tile's last token sees
+        const int end_a = nk + pos0 + na - 1 - lo + 1, end_b = nb > 0 ? nk + hi - lo + 1 : 0;
+        const int steps_a = (end_a + WX_BK - 1) / WX_BK, steps_b = (end_b + WX_BK - 1) / WX_BK;
+        const int nsteps = max(steps_a, steps_b), total = max(end_a, end_b);
+
+        // ---- queries of both tiles, half a warp per row, eight entries a lane: (norm,) rotation, (norm) in fp32, rounded to the storage type
+        if (warp != 0 && warp != 2) {
+            const int me = warp == 1 ? 0 : warp == 3 ? 1 : warp - 2;              // 10 warps
+            const int l16 = lane & 15, d = l16 * 8, half = p.rot_dims >> 1;
+            const int nrows = nb > 0 ? 2 * WX_ROWS : WX_ROWS;
+#pragma unroll 1
+            for (int r0 = 2 * me; r0 < nrows; r0 += 20) {
+                const int row = r0 + (lane >> 4), tr = row >> p.hqp_log2, hh = row & (hqp - 1);
+                const bool live = tr < n && hh < hq && d < dk;
+                const int64_t t = ts + tr;
+                const T* qr = reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + hh) * dk;
+                float x[8], y[8];                     // the lane's entries; with `halves` the partners of those that turn
+                const bool turns = live && d < p.rot_dims;
+                const int dp = d < half ? d + half : d - half;                    // partner group (halves)
+#pragma unroll
+                for (int e = 0; e < 8; e++) { x[e] = 0.f; y[e] = 0.f; }
+                if (live) {
+                    if (p.q_vec) {
+                        const Vec8<T> u = ld_vec8(qr + d);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(u.v[e]); x[2 * e] = f.x; x[2 * e + 1] = f.y; }
+                        if (p.halves && turns) {
+                            const Vec8<T> w = ld_vec8(qr + dp);
+#pragma unroll
+                            for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(w.v[e]); y[2 * e] = f.x; y[2 * e + 1] = f.y; }
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) x[e] = ldf(qr + d + e);
+                        if (p.halves && turns) {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) {
+                                const int j = d + e;
+                                y[e] = j < p.rot_dims ? ldf(qr + (j < half ? j + half : j - half)) : 0.f;
+                            }
+                        }
+                    }
+                }
+                auto sum16 = [&](float v) {
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    return v;
+                };
+                if (p.qnorm_w != nullptr) {
+                    float ss = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                    const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.prenorm_eps);
+                    if (live) {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            x[e] *= inv * p.qnorm_w[d + e];
+                            const int j = d + e;
+                            if (p.halves && j < p.rot_dims) y[e] *= inv * p.qnorm_w[j < half ? j + half : j - half];
+                        }
+                    }
+                }
+                if (turns) {
+                    const float* cs = p.cosb + t * half;
+                    const float* sn = p.sinb + t * half;
+                    if (p.halves) {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            const int j = d + e;
+                            if (j < half) x[e] = x[e] * cs[j] - y[e] * sn[j];
+                            else if (j < p.rot_dims) x[e] = x[e] * cs[j - half] + y[e] * sn[j - half];
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int i = (d >> 1) + e;
+                            if (i < half) {
+                                const float a = x[2 * e], b = x[2 * e + 1];
+                                x[2 * e] = a * cs[i] - b * sn[i]; x[2 * e + 1] = b * cs[i] + a * sn[i];
+                            }
+                        }
+                    }
+                }
+                if (p.qk_norm_eps >= 0.f) {
+                    float ss = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                    const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.qk_norm_eps);
+#pragma unroll
+                    for (int e = 0; e < 8; e++) x[e] *= inv;
+                }
+                if (d < dk) {
+                    const uint4 v = make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
+                    *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + wx_off(row & 127, (d & 63) >> 3)) = v;
+                }
+            }
+            fence_proxy_async();
+            named_bar_sync(1, WX_THREADS - 64);
+        }
+
+        if (warp == 0 || warp == 2) {
+            // ======================================================= producers: keys 40 (warp / 2) .. of every step, eight lanes a 128-byte piece
+            const int r0 = 20 * warp, piece = lane & 7;
+            const T* cache = reinterpret_cast<const T*>(p.cache);
+            auto key_row = [&](int v) {               // cache row of list entry v, -1 past the last
+                if (v >= total) return -1ll;
+                const int kp = v < nk ? v : v - nk + lo;
+                const int b = kp / p.block_size;
+                return ((long long)bt[b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size);
+            };
+            auto signal = [&](int j) {
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bars->full[(n_done + j) % WX_STAGES]));
+            };
+            const int kofs = p.koff + g * KW, vofs = p.G * dk + (g / p.vshare) * dv;
+            long long ra = key_row(r0 + lane), rb = lane < 8 ? key_row(r0 + 32 + lane) : -1ll;
+            for (int j = 0; j < nsteps; j++) {
+                const long long a = ra, b = rb;
+                if (j + 1 < nsteps) {
+                    ra = key_row((j + 1) * WX_BK + r0 + lane);
+                    rb = lane < 8 ? key_row((j + 1) * WX_BK + r0 + 32 + lane) : -1ll;
+                }
+                const int it = n_done + j, st = it % WX_STAGES;
+                mbar_wait(smem_u32(&bars->empty[st]), ((it / WX_STAGES) & 1) ^ 1);
+                const uint32_t stage = smem_u32(kv_sm + st * WX_STAGE);
+#pragma unroll 2
+                for (int i = 0; i < 10; i++) {
+                    const int l = 4 * i + (lane >> 3), row = r0 + l;
+                    const long long ri = __shfl_sync(0xffffffffu, i < 8 ? a : b, l & 31);
+                    const int bytes = ri >= 0 ? 16 : 0;
+                    const T* src = cache + (ri >= 0 ? ri * p.row_elems : 0);
+                    const uint32_t dst = stage + wx_off(row, piece);
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        if (c < kch && c * 64 + piece * 8 < KW) cp_async16(dst + c * WX_CHUNK, bytes ? src + kofs + c * 64 + piece * 8 : src, bytes);
+#pragma unroll
+                    for (int c = 0; c < 2; c++)
+                        if (c < vch && c * 64 + piece * 8 < dv)
+                            cp_async16(dst + (kch + c) * WX_CHUNK, bytes ? src + vofs + c * 64 + piece * 8 : src, bytes);
+                    if (EXT && shared_kv && piece == 0) {
+                        float* to = inv_sm + st * WX_BK + row;
+                        if (bytes) cp_async4(smem_u32(to), src + 2 * g);
+                        else *to = 0.f;
+                    }
+                }
+                cp_async_commit();
+                if (j >= WX_LAG) { cp_async_wait<WX_LAG>(); signal(j - WX_LAG); }
+            }
+            cp_async_wait<0>();
+            for (int j = max(0, nsteps - WX_LAG); j < nsteps; j++) signal(j);
+        } else if (warp < 4) {
+            // ======================================================= product issuers (the warp stays converged, one elected lane issues)
+            const int x = warp >> 1;
+            const int mine = x == 0 ? steps_a : steps_b, end = x == 0 ? end_a : end_b;
+            const uint32_t idesc_s = make_instr_desc(WX_ROWS, WX_BK, UmmaFmt<T>::value, 0, 0);
+            const uint32_t idesc_o = make_instr_desc(WX_ROWS, dv, UmmaFmt<T>::value, 0, 1);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint32_t s_addr = tm + WX_S_COL + x * WX_BK, p_addr = tm + WX_P_COL + x * (WX_BK / 2), o_addr = tm + WX_O_COL + x * 128;
+            const uint64_t dq = make_smem_desc(smem_u32(q_sm + x * WX_Q_BYTES), 16, 1024);
+            const uint64_t dk0 = make_smem_desc(smem_u32(kv_sm), 16, 1024), dv0 = make_smem_desc(smem_u32(kv_sm), WX_CHUNK, 1024);
+            const uint32_t vfirst = (uint32_t)((vch > 0 ? kch : 0) * WX_CHUNK) >> 4;
+            const int kd_steps = dk >> 4;
+            auto scores = [&](int j) {
+                const int it = n_done + j, st = it % WX_STAGES;
+                mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t kd = dk0 + (uint64_t)((st * WX_STAGE) >> 4);
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        if (k < kd_steps) {
+                            const int col = krot + 16 * k;
+                            umma_ss(s_addr, dq + (uint64_t)(((k >> 2) * WX_QCHUNK + (k & 3) * 32) >> 4),
+                                    kd + (uint64_t)(((col >> 6) * WX_CHUNK + (col & 63) * 2) >> 4), idesc_s, k > 0);
+                        }
+                    umma_commit(smem_u32(&bars->s_full[x]));
+                }
+                __syncwarp();
+            };
+            if (mine > 0) {
+                scores(0);
+                for (int j = 0; j < mine; j++) {
+                    const int xi = x_done[x] + j;
+                    if (j + 1 < mine) {
+                        mbar_wait(smem_u32(&bars->s_empty[x]), xi & 1);
+                        scores(j + 1);
+                    }
+                    const int st = (n_done + j) % WX_STAGES;
+                    mbar_wait(smem_u32(&bars->p_full[x]), xi & 1);
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const int k16 = min(WX_BK / 16, (end - j * WX_BK + 15) / 16);     // none past the last key the tile can see
+                        const uint64_t vd = dv0 + (uint64_t)((st * WX_STAGE) >> 4) + vfirst;
+#pragma unroll
+                        for (int k = 0; k < WX_BK / 16; k++)
+                            if (k < k16) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                        umma_commit(smem_u32(&bars->empty[st]));
+                        umma_commit(smem_u32(&bars->p_empty[x]));
+                    }
+                    __syncwarp();
+                }
+                // the last scores' s_empty is waited for by nobody: its phase is taken by the count x_done
+            }
+            // steps that only the other tile takes: hand the stages on once they have been filled (never a phase ahead)
+            for (int j = mine; j < nsteps; j++) {
+                const int it = n_done + j, st = it % WX_STAGES;
+                mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
+                if (lane == 0) mbar_arrive(smem_u32(&bars->empty[st]));
+            }
+        } else {
+            // ======================================================= softmax: tile x, thread = row
+            const int x = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
+            const int mine = x == 0 ? steps_a : steps_b;
+            const int tr = x * tpt + (row >> p.hqp_log2), hh = row & (hqp - 1), h = g * hq + hh;
+            const bool live = tr < n && hh < hq;
+            const int pos = pos0 + tr;
+            // visible list entries: vmin .. vmax, and those below vkeep
+            const int vmax = nk + pos - lo, vmin = nk + first_seen(pos) - lo;
+            // entries every live row of the tile sees without a look
+            const int tr0 = x * tpt, tr1 = min(n, (x + 1) * tpt) - 1;
+            const int all_lo = nk + first_seen(pos0 + tr1) - lo, all_hi = nk + pos0 + tr0 - lo;
+            const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16);
+            const uint32_t s_addr = tl + WX_S_COL + x * WX_BK, p_addr = tl + WX_P_COL + x * (WX_BK / 2), o_addr = tl + WX_O_COL + x * 128;
+            const float c = p.scale * WX_LOG2E, cap_in = CAP ? p.scale / p.softcap : 0.f, cap_out = CAP ? p.softcap * WX_LOG2E : 0.f;
+            const float slope = EXT && p.slopes != nullptr && live ? p.slopes[h] * WX_LOG2E : 0.f;
+            float m_ref = p.sink > 0.f ? 0.f : -INFINITY, l = p.sink;
+            if (EXT && p.sinks != nullptr && live) { m_ref = p.sinks[h] * WX_LOG2E; l = 1.f; }
+            for (int j = 0; j < mine; j++) {
+                const int xi = x_done[x] + j;
+                mbar_wait(smem_u32(&bars->s_full[x]), xi & 1);
+                tc_fence_after();
+                uint32_t r[WX_BK];
+                tmem_ld32(s_addr, reinterpret_cast<uint32_t(&)[32]>(r[0]));
+                tmem_ld32(s_addr + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+                tmem_ld<16>(s_addr + 64, reinterpret_cast<uint32_t(&)[16]>(r[64]));
+                tmem_ld_wait();
+                tc_fence_before();
+                mbar_arrive(smem_u32(&bars->s_empty[x]));
+                const int v0 = j * WX_BK;
+                if constexpr (CAP || EXT) {           // scores in base 2, all factors applied
+                    if (EXT && shared_kv) {
+                        const int it = n_done + j;
+                        mbar_wait(smem_u32(&bars->full[it % WX_STAGES]), (it / WX_STAGES) & 1);      // long there: orders the producers' writes
+                        const float* iv = inv_sm + it % WX_STAGES * WX_BK;
+#pragma unroll
+                        for (int i = 0; i < WX_BK; i += 4) {
+                            const float4 f = *reinterpret_cast<const float4*>(iv + i);
+                            r[i] = __float_as_uint(__uint_as_float(r[i]) * f.x); r[i + 1] = __float_as_uint(__uint_as_float(r[i + 1]) * f.y);
+                            r[i + 2] = __float_as_uint(__uint_as_float(r[i + 2]) * f.z); r[i + 3] = __float_as_uint(__uint_as_float(r[i + 3]) * f.w);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < WX_BK; i++) {
+                        const float s = __uint_as_float(r[i]);
+                        r[i] = __float_as_uint(CAP ? cap_out * tanhf(s * cap_in) : s * c);
+                    }
+                    if (EXT && p.slopes != nullptr) {
+                        const float far = (float)(pos - lo + nk - v0), near = (float)(pos - v0);      // distance of entry v0 (kept: near)
+#pragma unroll
+                        for (int i = 0; i < WX_BK; i++)
+                            r[i] = __float_as_uint(__uint_as_float(r[i]) - slope * ((v0 + i < nk ? near : far) - (float)i));
+                    }
+                }
+                if (v0 + WX_BK - 1 > all_hi || v0 < all_lo) {
+                    const int top = vmax - v0, bottom = vmin - v0, kept = vkeep - v0;
+#pragma unroll
+                    for (int i = 0; i < WX_BK; i++) r[i] = i <= top && (i >= bottom || (EXT && i < kept)) ? r[i] : 0xff800000u;
+                }
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int i = 0; i < WX_BK; i += 8)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) mx[e] = max3(mx[e], __uint_as_float(r[i + 2 * e]), __uint_as_float(r[i + 2 * e + 1]));
+                const float cc = CAP || EXT ? 1.f : c;
+                const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * cc);
+                // true on a row's first visible key; the first step's maximum is taken as it is (a sink may lie far below it)
+                const bool need = m_new > m_ref + (j == 0 ? 0.f : WX_RESCALE);
+                const float alpha = need ? fast_exp2_tc(m_ref - m_new) : 1.f;
+                l *= alpha;
+                if (j > 0 && __any_sync(0xffffffffu, need)) {
+                    mbar_wait(smem_u32(&bars->p_empty[x]), (xi - 1) & 1);          // the products of step j - 1 are done: O is stable
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int d = 0; d < dv; d += 16) {
+                        uint32_t t[16];
+                        tmem_ld<16>(o_addr + d, t);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
+                        tmem_st16(o_addr + d, t);
+                    }
+                }
+                if (need) m_ref = m_new;
+                const float sub = m_ref == -INFINITY ? 0.f : -m_ref;              // nothing seen yet
+                float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                const float2 neg_m = make_float2(sub, sub), c2 = make_float2(cc, cc);
+                uint32_t w[WX_BK / 2];
+#pragma unroll
+                for (int i = 0; i < WX_BK / 2; i++) {
+                    const float2 e = fma2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), c2, neg_m);
+                    const float2 v = make_float2(fast_exp2_tc(e.x), fast_exp2_tc(e.y));
+                    ls[i & 1] = add2(ls[i & 1], v);
+                    w[i] = pack2<T>(v.x, v.y);
+                }
+                if (j > 0) { mbar_wait(smem_u32(&bars->p_empty[x]), (xi - 1) & 1); tc_fence_after(); }      // P of step j - 1 has been read
+                tmem_st32(p_addr, reinterpret_cast<uint32_t(&)[32]>(w[0]));
+                tmem_st8(p_addr + 32, reinterpret_cast<uint32_t(&)[8]>(w[32]));
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(smem_u32(&bars->p_full[x]));
+                l += (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y);
+            }
+            if (mine > 0) {
+                // ---- output row: normalise, (turn back,) gate, store
+                mbar_wait(smem_u32(&bars->p_empty[x]), (x_done[x] + mine - 1) & 1);
+                tc_fence_after();
+                const int64_t t = ts + tr;
+                const T* gate = reinterpret_cast<const T*>(p.gate);
+                float f = 0.f;
+                if (live) {
+                    f = p.out_scale / l;
+                    if (EXT && p.gate_per_head && gate != nullptr) f *= 1.f / (1.f + __expf(-ldf(gate + t * p.gate_st + h)));
+                }
+                const T* grow = gate != nullptr && !(EXT && p.gate_per_head) ? gate + t * p.gate_st + (int64_t)h * dv : nullptr;
+                const int64_t at = t * p.out_st + (int64_t)h * dv;
+                auto put8 = [&](int d, float (&y)[8]) {                            // eight neighbouring entries from d on
+                    if (grow != nullptr) {
+                        if (p.gate_vec) {
+                            const Vec8<T> u = ld_vec8(grow + d);
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const float2 z = Traits<T>::to_f2(u.v[e]);
+                                y[2 * e] *= 1.f / (1.f + __expf(-z.x)); y[2 * e + 1] *= 1.f / (1.f + __expf(-z.y));
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) y[e] *= 1.f / (1.f + __expf(-ldf(grow + d + e)));
+                        }
+                    }
+                    if (p.out_f32) {
+                        float* o = reinterpret_cast<float*>(p.out) + at + d;
+                        if (p.out_vec) {
+                            *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
+                            *reinterpret_cast<float4*>(o + 4) = make_float4(y[4], y[5], y[6], y[7]);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) o[e] = y[e];
+                        }
+                    } else {
+                        T* o = reinterpret_cast<T*>(p.out) + at + d;
+                        if (p.out_vec) {
+                            *reinterpret_cast<uint4*>(o) = make_uint4(pack2<T>(y[0], y[1]), pack2<T>(y[2], y[3]), pack2<T>(y[4], y[5]), pack2<T>(y[6], y[7]));
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) stf(o + e, y[e]);
+                        }
+                    }
+                };
+                const int hv = dv >> 1;
+#pragma unroll 1
+                for (int m = 0; m < hv; m += 8) {     // entries m .. m + 7 and m + hv .. (pairs of halves), or 2 m .. 2 m + 15
+                    const bool split = p.vcos != nullptr && p.halves;
+                    const int da = split ? m : 2 * m, db = split ? m + hv : 2 * m + 8;
+                    uint32_t ua[8], ub[8];
+                    __syncwarp();
+                    tmem_ld<8>(o_addr + da, ua);
+                    tmem_ld<8>(o_addr + db, ub);
+                    tmem_ld_wait();
+                    if (live) {
+                        float a[8], b[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e++) { a[e] = __uint_as_float(ua[e]) * f; b[e] = __uint_as_float(ub[e]) * f; }
+                        if (p.vcos != nullptr) {      // values were stored turned by their position: turned back by the query's
+                            const float* vc = p.vcos + t * hv + m;
+                            const float* vs = p.vsin + t * hv + m;
+#pragma unroll
+                            for (int e = 0; e < 8; e++) {
+                                const float cs = vc[e], sn = vs[e];
+                                float& u = split ? a[e] : (e < 4 ? a[2 * e] : b[2 * e - 8]);
+                                float& w = split ? b[e] : (e < 4 ? a[2 * e + 1] : b[2 * e - 7]);
+                                const float u0 = u, w0 = w;
+                                u = u0 * cs + w0 * sn; w = w0 * cs - u0 * sn;
+                            }
+                        }
+                        put8(da, a);
+                        put8(db, b);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        tc_fence_before();
+        __syncthreads();                              // the next segment overwrites the queries; its first products overwrite O
+        tc_fence_after();
+        n_done += nsteps;
+        x_done[0] += steps_a; x_done[1] += steps_b;
+        i0 += n;
+    }
+    if (warp == 1) tmem_dealloc<512>(tmem);
+}
+
+bool window_tc_supported(int dk, int dv, int krot, int hq, float scale, const void* cache, int64_t num_rows) {
+    return dk % 16 == 0 && dv % 16 == 0 && dk <= 128 && dv <= 128 && krot % 16 == 0 && dk + krot <= 256 && hq <= 64 && scale > 0.f &&
+           ((uintptr_t)cache & 15) == 0 && num_rows < (1ll << 31);
+}
+
+int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) {
+    const int hq = p.H / p.G;
+    p.hqp_log2 = 0;
+    while ((1 << p.hqp_log2) < hq) p.hqp_log2++;
+    int num_sms = 0;
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, current_device());
+    // two full tiles a CTA; fewer tokens while that leaves SMs without one (down to half a tile)
+    p.qt = (2 * WX_ROWS) >> p.hqp_log2;
+    const int least = (WX_ROWS / 2) >> p.hqp_log2;
+    while (p.qt > least && p.qt > 1 && (int64_t)cdiv(p.num_rows, p.qt) * p.G < num_sms) p.qt >>= 1;
+    const dim3 grid((unsigned)cdiv(p.num_rows, p.qt), (unsigned)p.G);
+    const bool ext = p.slopes != nullptr || p.keep_first > 0 || p.gate_per_head || p.shared_kv || p.sinks != nullptr, cap = p.softcap > 0.f;
+#define SLLM_WX(EXT, CAP)                                                                                                          \
+    do {                                                                                                                           \
+        static unsigned long long configured = 0;                                                                                  \
+        auto kern = window_attn_tc_kernel<T, EXT, CAP>;                                                                            \
+        if (first_use_on_this_device(configured)) {                                                                                \
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM);                      \
+            SLLM_REQUIRE(e == cudaSuccess, "window_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));                  \
+        }                                                                                                                          \
+        kern<<<grid, WX_THREADS, WX_SMEM, stream>>>(p);                                                                            \
+    } while (0)
+    SLLM_DISPATCH_DTYPE(dtype, {
+        if (ext && cap) SLLM_WX(true, true);
+        else if (ext) SLLM_WX(true, false);
+        else if (cap) SLLM_WX(false, true);
+        else SLLM_WX(false, false);
+    });
+#undef SLLM_WX
+    return check_launch("window_attention (tcgen05)");
+}
+
+}  // namespace sllm

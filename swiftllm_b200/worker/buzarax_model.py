@@ -26,7 +26,7 @@ LAST_TOKEN = "last_token"
 
 
 class BuzaraxModel(TokenBatchModel):
-    NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("parallel_block.cu", "stream_ops.cu", "recurrent.cu", "window_attn.cu")
+    NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("parallel_block.cu", "stream_ops.cu", "recurrent.cu", "window_attn.cu", "window_attn_tc.cu")
     CONFIG_CLASS = BuzaraxModelConfig
 
     @staticmethod

@@ -25,7 +25,7 @@ from .token_model import TokenBatchModel
 
 class NaforaxModel(TokenBatchModel):
     NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("parallel_block.cu", "stream_ops.cu", "sandwich_ops.cu", "scan_ops.cu",
-                                                       "window_attn.cu")
+                                                       "window_attn.cu", "window_attn_tc.cu")
     CONFIG_CLASS = NaforaxModelConfig
 
     @staticmethod

@@ -8,7 +8,7 @@ from swiftllm_b200.worker.weight import load_rivudra_weights
 
 
 class RivudraModel(ParallelBlockModel):
-    NATIVE_SOURCES = ParallelBlockModel.NATIVE_SOURCES + ("window_attn.cu",)
+    NATIVE_SOURCES = ParallelBlockModel.NATIVE_SOURCES + ("window_attn.cu", "window_attn_tc.cu",)
     CONFIG_CLASS = RivudraModelConfig
 
     @staticmethod

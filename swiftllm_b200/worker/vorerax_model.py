@@ -26,7 +26,7 @@ LAST_TOKEN = "last_token"
 
 
 class VoreraxModel(TokenBatchModel):
-    NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("stream_ops.cu", "hyper_streams.cu", "window_attn.cu", "scan_ops.cu", "delta_rule.cu",
+    NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("stream_ops.cu", "hyper_streams.cu", "window_attn.cu", "window_attn_tc.cu", "scan_ops.cu", "delta_rule.cu",
                                                        "matrix_memory.cu")
     CONFIG_CLASS = VoreraxModelConfig
 
