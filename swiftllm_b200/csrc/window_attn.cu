@@ -1124,6 +1124,7 @@ static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void*
             w.row_elems = shared_kv ? shared_kv_row(G, dk + krot) : G * dk + (G / vshare) * dv;
             w.koff = shared_kv ? shared_kv_key_offset(G) : 0;
             w.q_vec = ((uintptr_t)q & 15) == 0 && q_stride_t % 8 == 0 && (!halves || rot_dims % 16 == 0);
+            w.q_fast = w.q_vec && (rot_dims == 0 || (!halves && rot_dims % 8 == 0 && (((uintptr_t)cosb | (uintptr_t)sinb) & 15) == 0));
             w.gate_vec = ((uintptr_t)gate & 15) == 0 && gate_stride_t % 8 == 0;
             w.out_vec = ((uintptr_t)out & 15) == 0 && out_stride_t % 8 == 0;
             if (int rc = launch_window_attn_tc(w, std::is_same<T, __half>::value ? SLLM_F16 : SLLM_BF16, stream)) return rc;

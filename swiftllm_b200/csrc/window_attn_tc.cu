@@ -16,7 +16,8 @@
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
 // ones 317 us with the mma.sync kernel of window_attn.cu for the prompts -> 169 us.
 //
-// EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores.
+// EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores;
+// FULL: heads of 128 + 128 entries without turned ones beside shared keys (the producers are bound by their instructions).
 #include "mma_helpers.cuh"
 #include "tc_helpers.cuh"
 #include "typed_io.cuh"
@@ -47,7 +48,7 @@ struct WindowTcBars {
 
 __device__ __forceinline__ uint32_t wx_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
 
-template <typename T, bool EXT, bool CAP>
+template <typename T, bool EXT, bool CAP, bool FULL>
 __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const WindowTc p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_sm = smem;                             // [tile][chunk][128 rows][128 B]
@@ -58,8 +59,8 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
     static_assert(sizeof(WindowTcBars) + 4 <= 256, "");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool shared_kv = EXT && p.shared_kv;
-    const int krot = EXT ? p.krot : 0, keep_first = EXT ? p.keep_first : 0;
-    const int dk = p.dk, dv = p.dv, KW = dk + krot, hq = p.H / p.G, hqp = 1 << p.hqp_log2, g = blockIdx.y;
+    const int krot = EXT && !FULL ? p.krot : 0, keep_first = EXT ? p.keep_first : 0;
+    const int dk = FULL ? 128 : p.dk, dv = FULL ? 128 : p.dv, KW = dk + krot, hq = p.H / p.G, hqp = 1 << p.hqp_log2, g = blockIdx.y;
     const int kch = (KW + 63) >> 6, vch = shared_kv ? 0 : (dv + 63) >> 6;         // chunks of a key / value row
     const int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;                       // the last tokens of a prompt have the most keys: first
     const int ntok = min(p.qt, p.num_rows - t_first);
@@ -110,6 +111,76 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
             const int me = warp == 1 ? 0 : warp == 3 ? 1 : warp - 2;              // 10 warps
             const int l16 = lane & 15, d = l16 * 8, half = p.rot_dims >> 1;
             const int nrows = nb > 0 ? 2 * WX_ROWS : WX_ROWS;
+            auto sum16 = [&](float v) {
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                return v;
+            };
+            auto stage_row = [&](int row, const float (&x)[8]) {
+                if (d < dk) {
+                    const uint4 v = make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
+                    *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + wx_off(row & 127, (d & 63) >> 3)) = v;
+                }
+            };
+            if (p.q_fast) {
+                // neighbouring pairs turn, 16-byte loads: four rows' loads are in flight before the first is used
+                const int dc = min(d, dk - 8), dr = min(d, p.rot_dims - 8) >> 1;
+                float nw[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) nw[e] = p.qnorm_w != nullptr ? p.qnorm_w[dc + e] : 1.f;
+                const bool turns = d < p.rot_dims;
+#pragma unroll 1
+                for (int r0 = 2 * me + (lane >> 4); r0 < nrows; r0 += 80) {
+                    Vec8<T> u[4];
+                    float4 c4[4], s4[4];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        const int row = r0 + 20 * b;
+                        const int64_t t = ts + min(row >> p.hqp_log2, n - 1);
+                        u[b] = ld_vec8(reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + min(row & (hqp - 1), hq - 1)) * dk + dc);
+                        if (p.rot_dims > 0) {
+                            c4[b] = *reinterpret_cast<const float4*>(p.cosb + t * half + dr);
+                            s4[b] = *reinterpret_cast<const float4*>(p.sinb + t * half + dr);
+                        }
+                    }
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        const int row = r0 + 20 * b;
+                        const bool live = (row >> p.hqp_log2) < n && (row & (hqp - 1)) < hq && d < dk;
+                        float x[8];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const float2 f = Traits<T>::to_f2(u[b].v[e]);
+                            x[2 * e] = live ? f.x : 0.f; x[2 * e + 1] = live ? f.y : 0.f;
+                        }
+                        if (p.qnorm_w != nullptr) {
+                            float ss = 0.f;
+#pragma unroll
+                            for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                            const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.prenorm_eps);
+#pragma unroll
+                            for (int e = 0; e < 8; e++) x[e] *= inv * nw[e];
+                        }
+                        if (turns) {
+                            const float cs[4] = {c4[b].x, c4[b].y, c4[b].z, c4[b].w}, sn[4] = {s4[b].x, s4[b].y, s4[b].z, s4[b].w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const float v = x[2 * e], w = x[2 * e + 1];
+                                x[2 * e] = v * cs[e] - w * sn[e]; x[2 * e + 1] = w * cs[e] + v * sn[e];
+                            }
+                        }
+                        if (p.qk_norm_eps >= 0.f) {
+                            float ss = 0.f;
+#pragma unroll
+                            for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                            const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.qk_norm_eps);
+#pragma unroll
+                            for (int e = 0; e < 8; e++) x[e] *= inv;
+                        }
+                        if (row < nrows) stage_row(row, x);
+                    }
+                }
+            } else
 #pragma unroll 1
             for (int r0 = 2 * me; r0 < nrows; r0 += 20) {
                 const int row = r0 + (lane >> 4), tr = row >> p.hqp_log2, hh = row & (hqp - 1);
@@ -143,11 +214,6 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                         }
                     }
                 }
-                auto sum16 = [&](float v) {
-#pragma unroll
-                    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    return v;
-                };
                 if (p.qnorm_w != nullptr) {
                     float ss = 0.f;
 #pragma unroll
@@ -191,10 +257,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
 #pragma unroll
                     for (int e = 0; e < 8; e++) x[e] *= inv;
                 }
-                if (d < dk) {
-                    const uint4 v = make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
-                    *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + wx_off(row & 127, (d & 63) >> 3)) = v;
-                }
+                stage_row(row, x);
             }
             fence_proxy_async();
             named_bar_sync(1, WX_THREADS - 64);
@@ -226,20 +289,27 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                 const int it = n_done + j, st = it % WX_STAGES;
                 mbar_wait(smem_u32(&bars->empty[st]), ((it / WX_STAGES) & 1) ^ 1);
                 const uint32_t stage = smem_u32(kv_sm + st * WX_STAGE);
-#pragma unroll 2
+#pragma unroll
                 for (int i = 0; i < 10; i++) {
                     const int l = 4 * i + (lane >> 3), row = r0 + l;
                     const long long ri = __shfl_sync(0xffffffffu, i < 8 ? a : b, l & 31);
                     const int bytes = ri >= 0 ? 16 : 0;
-                    const T* src = cache + (ri >= 0 ? ri * p.row_elems : 0);
+                    const T* src = ri >= 0 ? cache + ri * p.row_elems : cache;
                     const uint32_t dst = stage + wx_off(row, piece);
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        if (c < kch && c * 64 + piece * 8 < KW) cp_async16(dst + c * WX_CHUNK, bytes ? src + kofs + c * 64 + piece * 8 : src, bytes);
-#pragma unroll
-                    for (int c = 0; c < 2; c++)
-                        if (c < vch && c * 64 + piece * 8 < dv)
-                            cp_async16(dst + (kch + c) * WX_CHUNK, bytes ? src + vofs + c * 64 + piece * 8 : src, bytes);
+                    if constexpr (FULL) {             // (a row that is not there reads nothing, wherever src points)
+                        const T* ks = src + kofs + piece * 8;
+                        cp_async16(dst, ks, bytes); cp_async16(dst + WX_CHUNK, ks + 64, bytes);
+                        if (!shared_kv) {
+                            const T* vs = src + vofs + piece * 8;
+                            cp_async16(dst + 2 * WX_CHUNK, vs, bytes); cp_async16(dst + 3 * WX_CHUNK, vs + 64, bytes);
+                        }
+                    } else {
+                        for (int c = 0; c < kch; c++)
+                            if (c * 64 + piece * 8 < KW) cp_async16(dst + c * WX_CHUNK, bytes ? src + kofs + c * 64 + piece * 8 : src, bytes);
+                        for (int c = 0; c < vch; c++)
+                            if (c * 64 + piece * 8 < dv)
+                                cp_async16(dst + (kch + c) * WX_CHUNK, bytes ? src + vofs + c * 64 + piece * 8 : src, bytes);
+                    }
                     if (EXT && shared_kv && piece == 0) {
                         float* to = inv_sm + st * WX_BK + row;
                         if (bytes) cp_async4(smem_u32(to), src + 2 * g);
@@ -426,22 +496,22 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                 }
                 const T* grow = gate != nullptr && !(EXT && p.gate_per_head) ? gate + t * p.gate_st + (int64_t)h * dv : nullptr;
                 const int64_t at = t * p.out_st + (int64_t)h * dv;
-                auto put8 = [&](int d, float (&y)[8]) {                            // eight neighbouring entries from d on
-                    if (grow != nullptr) {
+                auto store8 = [&](const T* gr, int64_t to, float (&y)[8]) {        // eight neighbouring entries (gated unless gr is null)
+                    if (gr != nullptr) {
                         if (p.gate_vec) {
-                            const Vec8<T> u = ld_vec8(grow + d);
+                            const Vec8<T> u = ld_vec8(gr);
 #pragma unroll
                             for (int e = 0; e < 4; e++) {
                                 const float2 z = Traits<T>::to_f2(u.v[e]);
-                                y[2 * e] *= 1.f / (1.f + __expf(-z.x)); y[2 * e + 1] *= 1.f / (1.f + __expf(-z.y));
+                                y[2 * e] = __fdividef(y[2 * e], 1.f + __expf(-z.x)); y[2 * e + 1] = __fdividef(y[2 * e + 1], 1.f + __expf(-z.y));
                             }
                         } else {
 #pragma unroll
-                            for (int e = 0; e < 8; e++) y[e] *= 1.f / (1.f + __expf(-ldf(grow + d + e)));
+                            for (int e = 0; e < 8; e++) y[e] *= 1.f / (1.f + __expf(-ldf(gr + e)));
                         }
                     }
                     if (p.out_f32) {
-                        float* o = reinterpret_cast<float*>(p.out) + at + d;
+                        float* o = reinterpret_cast<float*>(p.out) + to;
                         if (p.out_vec) {
                             *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
                             *reinterpret_cast<float4*>(o + 4) = make_float4(y[4], y[5], y[6], y[7]);
@@ -450,7 +520,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                             for (int e = 0; e < 8; e++) o[e] = y[e];
                         }
                     } else {
-                        T* o = reinterpret_cast<T*>(p.out) + at + d;
+                        T* o = reinterpret_cast<T*>(p.out) + to;
                         if (p.out_vec) {
                             *reinterpret_cast<uint4*>(o) = make_uint4(pack2<T>(y[0], y[1]), pack2<T>(y[2], y[3]), pack2<T>(y[4], y[5]), pack2<T>(y[6], y[7]));
                         } else {
@@ -459,6 +529,41 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                         }
                     }
                 };
+                auto put8 = [&](int d, float (&y)[8]) { store8(grow != nullptr ? grow + d : nullptr, at + d, y); };
+                if (p.vcos == nullptr && p.out_vec && (grow == nullptr || p.gate_vec)) {
+                    // 64 columns at a time through this tile's query buffer (its products are done), so that a row's gate and output move
+                    // as whole lines: eight lanes a row, rows swizzled by 16 bytes
+                    float* xs = reinterpret_cast<float*>(q_sm + x * WX_Q_BYTES);
+                    auto cell = [&](int rr, int quarter) { return reinterpret_cast<float4*>(xs + rr * 64 + ((quarter ^ (rr & 15)) << 2)); };
+                    for (int d0 = 0; d0 < dv; d0 += 64) {
+                        const int cols = min(64, dv - d0);
+#pragma unroll 1
+                        for (int d = 0; d < cols; d += 16) {
+                            uint32_t v[16];
+                            tmem_ld<16>(o_addr + d0 + d, v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 4; e++)
+                                *cell(row, (d >> 2) + e) = make_float4(__uint_as_float(v[4 * e]) * f, __uint_as_float(v[4 * e + 1]) * f,
+                                                                       __uint_as_float(v[4 * e + 2]) * f, __uint_as_float(v[4 * e + 3]) * f);
+                        }
+                        named_bar_sync(2 + x, 128);
+                        const int l8 = lane & 7, d = d0 + 8 * l8;
+#pragma unroll 4
+                        for (int i = 0; i < 8; i++) {
+                            const int rr = quad * 32 + 4 * i + (lane >> 3), rt = x * tpt + (rr >> p.hqp_log2), rh = rr & (hqp - 1);
+                            if (rt < n && rh < hq && d < dv) {
+                                const int64_t tt = ts + rt;
+                                const int head = g * hq + rh;
+                                const float4 lo4 = *cell(rr, 2 * l8), hi4 = *cell(rr, 2 * l8 + 1);
+                                float y[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+                                store8(gate != nullptr && !(EXT && p.gate_per_head) ? gate + tt * p.gate_st + (int64_t)head * dv + d : nullptr,
+                                       tt * p.out_st + (int64_t)head * dv + d, y);
+                            }
+                        }
+                        named_bar_sync(2 + x, 128);
+                    }
+                } else {
                 const int hv = dv >> 1;
 #pragma unroll 1
                 for (int m = 0; m < hv; m += 8) {     // entries m .. m + 7 and m + hv .. (pairs of halves), or 2 m .. 2 m + 15
@@ -490,6 +595,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                     }
                 }
                 __syncwarp();
+                }
             }
         }
         tc_fence_before();
@@ -519,15 +625,20 @@ int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) 
     while (p.qt > least && p.qt > 1 && (int64_t)cdiv(p.num_rows, p.qt) * p.G < num_sms) p.qt >>= 1;
     const dim3 grid((unsigned)cdiv(p.num_rows, p.qt), (unsigned)p.G);
     const bool ext = p.slopes != nullptr || p.keep_first > 0 || p.gate_per_head || p.shared_kv || p.sinks != nullptr, cap = p.softcap > 0.f;
-#define SLLM_WX(EXT, CAP)                                                                                                          \
+#define SLLM_WX3(EXT, CAP, FULL)                                                                                                          \
     do {                                                                                                                           \
         static unsigned long long configured = 0;                                                                                  \
-        auto kern = window_attn_tc_kernel<T, EXT, CAP>;                                                                            \
+        auto kern = window_attn_tc_kernel<T, EXT, CAP, FULL>;                                                                            \
         if (first_use_on_this_device(configured)) {                                                                                \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM);                      \
             SLLM_REQUIRE(e == cudaSuccess, "window_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));                  \
         }                                                                                                                          \
         kern<<<grid, WX_THREADS, WX_SMEM, stream>>>(p);                                                                            \
+    } while (0)
+#define SLLM_WX(EXT, CAP)                                                                                                          \
+    do {                                                                                                                           \
+        if (p.dk == 128 && p.dv == 128 && p.krot == 0) SLLM_WX3(EXT, CAP, true);                                                   \
+        else SLLM_WX3(EXT, CAP, false);                                                                                            \
     } while (0)
     SLLM_DISPATCH_DTYPE(dtype, {
         if (ext && cap) SLLM_WX(true, true);
@@ -536,6 +647,7 @@ int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) 
         else SLLM_WX(false, false);
     });
 #undef SLLM_WX
+#undef SLLM_WX3
     return check_launch("window_attention (tcgen05)");
 }
 

@@ -27,7 +27,8 @@ struct WindowTc {
     const float* sinks;
     int row_elems, koff;                             // entries of a cache row; first key entry
     int qt, hqp_log2;                                // tokens per CTA; heads per group, padded to a power of two
-    int q_vec, gate_vec, out_vec;                    // 16-byte accesses of q and its angles / gate / out are aligned
+    // 16-byte accesses of q / gate / out are aligned; q_fast: of q and its angles, whose pairs are neighbours
+    int q_vec, q_fast, gate_vec, out_vec;
 };
 
 // what the products can be cut from (see the kernel); everything else takes the mma.sync kernel
