@@ -63,9 +63,6 @@ struct PtPaged {
 };
 constexpr int PT_PAGE = 16;               // tokens per KV page (PAGED only)
 
-template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-
 // PAGED = false: K/V tiles come from the packed k/v rows of the batch (the reference's contract).
 // PAGED = true (chunked prefill): the chunk's queries sit at positions prefix .. prefix + len - 1 of
 // their sequence; every 80-token K/V step is gathered from five 16-token pages of the KV cache through the block

@@ -160,6 +160,10 @@ __device__ __forceinline__ float fast_exp2_tc(float x) {
     return y;
 }
 
+// registers of every warp of a warpgroup (what one gives back another may take; the sum is bounded by the block's launch)
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // two fp32 operations in one packed instruction
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 o;

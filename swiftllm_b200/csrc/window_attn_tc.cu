@@ -8,13 +8,14 @@
 //                position are zero)
 //   warps 1, 3   product issuers of tile A / B:  S_X(j + 1) = Q_X . K(j + 1) as soon as S_X(j) is in registers,
 //                O_X += P_X(j) . V(j) when P_X(j) is there; with shared_kv the key tile is also the value tile
-//   warps 4-7    softmax and output of tile A, warps 8-11 of tile B: thread = query row = TMEM lane, P as 16-bit A operand in TMEM,
+//   warps 4-7    queries, softmax and output of tile A, warps 8-11 of tile B: thread = query row = TMEM lane, P as 16-bit A operand in TMEM,
 //                O rescaled only when the running maximum grew by more than 2^8
 // TMEM: S_A 0..79, S_B 80..159, P_A 160..199, P_B 200..239, O_A 256..383, O_B 384..511 (the layout of the prefill kernel: 80 keys are the
 // most that leave scores and P places of their own).
 //
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
-// ones 317 us with the mma.sync kernel of window_attn.cu for the prompts -> 169 us.
+// ones 317 us with the mma.sync kernel of window_attn.cu for the prompts -> 114 us (95 of them this kernel, two rounds of CTAs; a CTA's
+// step of 80 keys is about 2200 cycles, its queries and first keys 12 k, its output 5 k).
 //
 // EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores;
 // FULL: heads of 128 + 128 entries without turned ones beside shared keys (the producers are bound by their instructions).
@@ -39,7 +40,10 @@ constexpr int WX_SMEM = WX_MISC_OFF + 256;
 constexpr int WX_S_COL = 0, WX_P_COL = 160, WX_O_COL = 256;      // tile B: + 80, + 40, + 128
 constexpr float WX_RESCALE = 8.0f;                    // log2 units
 constexpr float WX_LOG2E = 1.4426950408889634f;
-constexpr int WX_LAG = 2;                             // steps whose rows are in flight behind the one being asked for
+// registers: 384 threads are launched with 168 each; the softmax warpgroups hold a row of scores and of P
+constexpr int WX_REGS_FEW = 72, WX_REGS_MANY = 216;
+static_assert(WX_REGS_FEW + 2 * WX_REGS_MANY <= 3 * 168, "the warpgroups' shares must fit what the block was launched with");
+constexpr int WX_LAG = 1;                             // steps whose rows are in flight behind the one being asked for
 
 struct WindowTcBars {
     uint64_t full[WX_STAGES], empty[WX_STAGES];
@@ -79,311 +83,332 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
     tc_fence_after();
     const uint32_t tmem = *tmem_s;
 
-    int n_done = 0, x_done[2] = {0, 0};               // steps of the segments before (of the ring, of each tile): the barriers' phases
-    for (int i0 = 0; i0 < ntok;) {
-        // ---- the segment: tokens ts .. ts + n - 1 of one sequence at positions pos0 ..
-        const int ts = t_first + i0, left = ntok - i0;
-        const int seq = p.tok_seq[ts], pos0 = p.tok_pos[ts];
-        int n = left;
+    // ---- a segment: tokens ts .. ts + n - 1 of one sequence at positions pos0 ..
+    struct Segment { int ts, n, seq, pos0, lo, hi, nk, steps_a, steps_b, end_a, end_b; };
+    const int tpt = WX_ROWS >> p.hqp_log2;                                        // tokens per tile
+    const int vkeep = EXT && p.window > 0 ? keep_first : 0;                        // list entries below it are kept positions
+    auto first_seen = [&](int pos) {                  // first position of the window (and chunk) of a query at `pos`
+        int a = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
+        if (p.chunk > 0) a = max(a, pos / p.chunk * p.chunk);
+        return a;
+    };
+    auto segment = [&](int i0) {
+        Segment s;
+        s.ts = t_first + i0;
+        const int left = ntok - i0;
+        s.seq = p.tok_seq[s.ts]; s.pos0 = p.tok_pos[s.ts];
+        s.n = left;
         for (int b = 0; b < left; b += 32) {
             const int i = b + min(lane, left - 1 - b);
-            const uint32_t cut = __ballot_sync(0xffffffffu, p.tok_seq[ts + i] != seq || p.tok_pos[ts + i] != pos0 + i);
-            if (cut) { n = b + __ffs(cut) - 1; break; }
+            const uint32_t cut = __ballot_sync(0xffffffffu, p.tok_seq[s.ts + i] != s.seq || p.tok_pos[s.ts + i] != s.pos0 + i);
+            if (cut) { s.n = b + __ffs(cut) - 1; break; }
         }
-        const int* bt = p.block_table + (int64_t)seq * p.max_blocks_per_seq;
-        auto first_seen = [&](int pos) {              // first position of the window (and chunk) of a query at `pos`
-            int a = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
-            if (p.chunk > 0) a = max(a, pos / p.chunk * p.chunk);
-            return a;
-        };
-        const int lo = first_seen(pos0), hi = pos0 + n - 1;
-        const int nk = EXT && p.window > 0 ? min(keep_first, lo) : 0;
-        const int vkeep = EXT && p.window > 0 ? keep_first : 0;                    // list entries below it are kept positions
-        const int tpt = WX_ROWS >> p.hqp_log2;                                    // tokens per tile
-        const int na = min(n, tpt), nb = n - na;
+        s.lo = first_seen(s.pos0); s.hi = s.pos0 + s.n - 1;
+        s.nk = EXT && p.window > 0 ? min(keep_first, s.lo) : 0;
+        const int na = min(s.n, tpt), nb = s.n - na;
         // entry v of the list of keys is position v (v < nk) or v - nk + lo; entries a tile's last token sees
-        const int end_a = nk + pos0 + na - 1 - lo + 1, end_b = nb > 0 ? nk + hi - lo + 1 : 0;
-        const int steps_a = (end_a + WX_BK - 1) / WX_BK, steps_b = (end_b + WX_BK - 1) / WX_BK;
-        const int nsteps = max(steps_a, steps_b), total = max(end_a, end_b);
-
-        // ---- queries of both tiles, half a warp per row, eight entries a lane: (norm,) rotation, (norm) in fp32, rounded to the storage type
-        if (warp != 0 && warp != 2) {
-            const int me = warp == 1 ? 0 : warp == 3 ? 1 : warp - 2;              // 10 warps
-            const int l16 = lane & 15, d = l16 * 8, half = p.rot_dims >> 1;
-            const int nrows = nb > 0 ? 2 * WX_ROWS : WX_ROWS;
-            auto sum16 = [&](float v) {
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                return v;
-            };
-            auto stage_row = [&](int row, const float (&x)[8]) {
-                if (d < dk) {
-                    const uint4 v = make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
-                    *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + wx_off(row & 127, (d & 63) >> 3)) = v;
-                }
-            };
-            if (p.q_fast) {
-                // neighbouring pairs turn, 16-byte loads: four rows' loads are in flight before the first is used
-                const int dc = min(d, dk - 8), dr = min(d, p.rot_dims - 8) >> 1;
-                float nw[8];
-#pragma unroll
-                for (int e = 0; e < 8; e++) nw[e] = p.qnorm_w != nullptr ? p.qnorm_w[dc + e] : 1.f;
-                const bool turns = d < p.rot_dims;
-#pragma unroll 1
-                for (int r0 = 2 * me + (lane >> 4); r0 < nrows; r0 += 80) {
-                    Vec8<T> u[4];
-                    float4 c4[4], s4[4];
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        const int row = r0 + 20 * b;
-                        const int64_t t = ts + min(row >> p.hqp_log2, n - 1);
-                        u[b] = ld_vec8(reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + min(row & (hqp - 1), hq - 1)) * dk + dc);
-                        if (p.rot_dims > 0) {
-                            c4[b] = *reinterpret_cast<const float4*>(p.cosb + t * half + dr);
-                            s4[b] = *reinterpret_cast<const float4*>(p.sinb + t * half + dr);
+        s.end_a = s.nk + s.pos0 + na - s.lo; s.end_b = nb > 0 ? s.nk + s.hi - s.lo + 1 : 0;
+        s.steps_a = (s.end_a + WX_BK - 1) / WX_BK; s.steps_b = (s.end_b + WX_BK - 1) / WX_BK;
+        return s;
+    };
+    // steps of the segments before (of the ring, of each tile): the barriers' phases follow from them
+    int n_done = 0, done_a = 0, done_b = 0;
+    if (warp < 4) {
+        reg_dec<WX_REGS_FEW>();
+        for (int i0 = 0; i0 < ntok;) {
+            const Segment sg = segment(i0);
+            const int n = sg.n, lo = sg.lo, nk = sg.nk, nsteps = max(sg.steps_a, sg.steps_b);
+            const int total = max(sg.end_a, sg.end_b);
+            const int* bt = p.block_table + (int64_t)sg.seq * p.max_blocks_per_seq;
+            if (warp == 0 || warp == 2) {
+                // ======================================================= producers: keys 40 (warp / 2) .. of every step, eight lanes a 128-byte piece
+                const int r0 = 20 * warp, piece = lane & 7;
+                const T* cache = reinterpret_cast<const T*>(p.cache);
+                auto key_row = [&](int v) {               // cache row of list entry v, -1 past the last
+                    if (v >= total) return -1ll;
+                    const int kp = v < nk ? v : v - nk + lo;
+                    const int b = kp / p.block_size;
+                    return ((long long)bt[b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size);
+                };
+                auto signal = [&](int j) {
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&bars->full[(n_done + j) % WX_STAGES]));
+                };
+                const int kofs = p.koff + g * KW, vofs = p.G * dk + (g / p.vshare) * dv;
+                long long ra = key_row(r0 + lane), rb = lane < 8 ? key_row(r0 + 32 + lane) : -1ll;
+                for (int j = 0; j < nsteps; j++) {
+                    const long long a = ra, b = rb;
+                    if (j + 1 < nsteps) {
+                        ra = key_row((j + 1) * WX_BK + r0 + lane);
+                        rb = lane < 8 ? key_row((j + 1) * WX_BK + r0 + 32 + lane) : -1ll;
+                    }
+                    const int it = n_done + j, st = it % WX_STAGES;
+                    mbar_wait(smem_u32(&bars->empty[st]), ((it / WX_STAGES) & 1) ^ 1);
+                    const uint32_t stage = smem_u32(kv_sm + st * WX_STAGE);
+#pragma unroll 2
+                    for (int i = 0; i < 10; i++) {
+                        const int l = 4 * i + (lane >> 3), row = r0 + l;
+                        const long long ri = __shfl_sync(0xffffffffu, i < 8 ? a : b, l & 31);
+                        const int bytes = ri >= 0 ? 16 : 0;
+                        const T* src = ri >= 0 ? cache + ri * p.row_elems : cache;
+                        const uint32_t dst = stage + wx_off(row, piece);
+                        if constexpr (FULL) {             // (a row that is not there reads nothing, wherever src points)
+                            const T* ks = src + kofs + piece * 8;
+                            cp_async16(dst, ks, bytes); cp_async16(dst + WX_CHUNK, ks + 64, bytes);
+                            if (!shared_kv) {
+                                const T* vs = src + vofs + piece * 8;
+                                cp_async16(dst + 2 * WX_CHUNK, vs, bytes); cp_async16(dst + 3 * WX_CHUNK, vs + 64, bytes);
+                            }
+                        } else {
+                            for (int c = 0; c < kch; c++)
+                                if (c * 64 + piece * 8 < KW) cp_async16(dst + c * WX_CHUNK, bytes ? src + kofs + c * 64 + piece * 8 : src, bytes);
+                            for (int c = 0; c < vch; c++)
+                                if (c * 64 + piece * 8 < dv)
+                                    cp_async16(dst + (kch + c) * WX_CHUNK, bytes ? src + vofs + c * 64 + piece * 8 : src, bytes);
+                        }
+                        if (EXT && shared_kv && piece == 0) {
+                            float* to = inv_sm + st * WX_BK + row;
+                            if (bytes) cp_async4(smem_u32(to), src + 2 * g);
+                            else *to = 0.f;
                         }
                     }
+                    cp_async_commit();
+                    if (j >= WX_LAG) { cp_async_wait<WX_LAG>(); signal(j - WX_LAG); }
+                }
+                cp_async_wait<0>();
+                for (int j = max(0, nsteps - WX_LAG); j < nsteps; j++) signal(j);
+            } else {
+                // ======================================================= product issuers (the warp stays converged, one elected lane issues)
+                const int x = warp >> 1;
+                const int mine = x == 0 ? sg.steps_a : sg.steps_b, end = x == 0 ? sg.end_a : sg.end_b, x_done = x == 0 ? done_a : done_b;
+                const uint32_t idesc_s = make_instr_desc(WX_ROWS, WX_BK, UmmaFmt<T>::value, 0, 0);
+                const uint32_t idesc_o = make_instr_desc(WX_ROWS, dv, UmmaFmt<T>::value, 0, 1);
+                const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+                const uint32_t s_addr = tm + WX_S_COL + x * WX_BK, p_addr = tm + WX_P_COL + x * (WX_BK / 2), o_addr = tm + WX_O_COL + x * 128;
+                const uint64_t dq = make_smem_desc(smem_u32(q_sm + x * WX_Q_BYTES), 16, 1024);
+                const uint64_t dk0 = make_smem_desc(smem_u32(kv_sm), 16, 1024), dv0 = make_smem_desc(smem_u32(kv_sm), WX_CHUNK, 1024);
+                const uint32_t vfirst = (uint32_t)((vch > 0 ? kch : 0) * WX_CHUNK) >> 4;
+                const int kd_steps = dk >> 4;
+                auto scores = [&](int j) {
+                    const int it = n_done + j, st = it % WX_STAGES;
+                    mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint64_t kd = dk0 + (uint64_t)((st * WX_STAGE) >> 4);
 #pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        const int row = r0 + 20 * b;
-                        const bool live = (row >> p.hqp_log2) < n && (row & (hqp - 1)) < hq && d < dk;
-                        float x[8];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float2 f = Traits<T>::to_f2(u[b].v[e]);
-                            x[2 * e] = live ? f.x : 0.f; x[2 * e + 1] = live ? f.y : 0.f;
+                        for (int k = 0; k < 8; k++)
+                            if (k < kd_steps) {
+                                const int col = krot + 16 * k;
+                                umma_ss(s_addr, dq + (uint64_t)(((k >> 2) * WX_QCHUNK + (k & 3) * 32) >> 4),
+                                        kd + (uint64_t)(((col >> 6) * WX_CHUNK + (col & 63) * 2) >> 4), idesc_s, k > 0);
+                            }
+                        umma_commit(smem_u32(&bars->s_full[x]));
+                    }
+                    __syncwarp();
+                };
+                named_bar_sync(1, WX_THREADS - 64);       // the queries are staged
+                if (mine > 0) {
+                    scores(0);
+                    for (int j = 0; j < mine; j++) {
+                        const int xi = x_done + j;
+                        if (j + 1 < mine) {
+                            mbar_wait(smem_u32(&bars->s_empty[x]), xi & 1);
+                            scores(j + 1);
                         }
-                        if (p.qnorm_w != nullptr) {
-                            float ss = 0.f;
+                        const int st = (n_done + j) % WX_STAGES;
+                        mbar_wait(smem_u32(&bars->p_full[x]), xi & 1);
+                        tc_fence_after();
+                        if (elect_one()) {
+                            const int k16 = min(WX_BK / 16, (end - j * WX_BK + 15) / 16);     // none past the last key the tile can see
+                            const uint64_t vd = dv0 + (uint64_t)((st * WX_STAGE) >> 4) + vfirst;
 #pragma unroll
-                            for (int e = 0; e < 8; e++) ss += x[e] * x[e];
-                            const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.prenorm_eps);
-#pragma unroll
-                            for (int e = 0; e < 8; e++) x[e] *= inv * nw[e];
+                            for (int k = 0; k < WX_BK / 16; k++)
+                                if (k < k16) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                            umma_commit(smem_u32(&bars->empty[st]));
+                            umma_commit(smem_u32(&bars->p_empty[x]));
                         }
-                        if (turns) {
-                            const float cs[4] = {c4[b].x, c4[b].y, c4[b].z, c4[b].w}, sn[4] = {s4[b].x, s4[b].y, s4[b].z, s4[b].w};
+                        __syncwarp();
+                    }
+                    // the last scores' s_empty is waited for by nobody: its phase is taken by the count x_done
+                }
+                // steps that only the other tile takes: hand the stages on once they have been filled (never a phase ahead)
+                for (int j = mine; j < nsteps; j++) {
+                    const int it = n_done + j, st = it % WX_STAGES;
+                    mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
+                    if (lane == 0) mbar_arrive(smem_u32(&bars->empty[st]));
+                }
+            }
+            tc_fence_before();
+            __syncthreads();                          // the next segment overwrites the queries; its first products overwrite O
+            tc_fence_after();
+            n_done += nsteps; done_a += sg.steps_a; done_b += sg.steps_b;
+            i0 += n;
+        }
+    } else {
+        reg_inc<WX_REGS_MANY>();
+        const int x = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
+        for (int i0 = 0; i0 < ntok;) {
+            const Segment sg = segment(i0);
+            const int ts = sg.ts, n = sg.n, pos0 = sg.pos0, lo = sg.lo, nk = sg.nk, nsteps = max(sg.steps_a, sg.steps_b);
+            // ---- queries of both tiles, half a warp per row, eight entries a lane: (norm,) rotation, (norm) in fp32, rounded to the storage type
+            {
+                const int me = warp - 4;
+                const int l16 = lane & 15, d = l16 * 8, half = p.rot_dims >> 1;
+                const int nrows = n > tpt ? 2 * WX_ROWS : WX_ROWS;
+                auto sum16 = [&](float v) {
 #pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                const float v = x[2 * e], w = x[2 * e + 1];
-                                x[2 * e] = v * cs[e] - w * sn[e]; x[2 * e + 1] = w * cs[e] + v * sn[e];
+                    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    return v;
+                };
+                auto stage_row = [&](int row, const float (&x)[8]) {
+                    if (d < dk) {
+                        const uint4 v = make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
+                        *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + wx_off(row & 127, (d & 63) >> 3)) = v;
+                    }
+                };
+                if (p.q_fast) {
+                    // neighbouring pairs turn, 16-byte loads: four rows' loads are in flight before the first is used
+                    const int dc = min(d, dk - 8), dr = min(d, p.rot_dims - 8) >> 1;
+                    float nw[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) nw[e] = p.qnorm_w != nullptr ? p.qnorm_w[dc + e] : 1.f;
+                    const bool turns = d < p.rot_dims;
+#pragma unroll 1
+                    for (int r0 = 2 * me + (lane >> 4); r0 < nrows; r0 += 64) {
+                        Vec8<T> u[4];
+                        float4 c4[4], s4[4];
+#pragma unroll
+                        for (int b = 0; b < 4; b++) {
+                            const int row = r0 + 16 * b;
+                            const int64_t t = ts + min(row >> p.hqp_log2, n - 1);
+                            u[b] = ld_vec8(reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + min(row & (hqp - 1), hq - 1)) * dk + dc);
+                            if (p.rot_dims > 0) {
+                                c4[b] = *reinterpret_cast<const float4*>(p.cosb + t * half + dr);
+                                s4[b] = *reinterpret_cast<const float4*>(p.sinb + t * half + dr);
                             }
                         }
-                        if (p.qk_norm_eps >= 0.f) {
-                            float ss = 0.f;
 #pragma unroll
-                            for (int e = 0; e < 8; e++) ss += x[e] * x[e];
-                            const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.qk_norm_eps);
+                        for (int b = 0; b < 4; b++) {
+                            const int row = r0 + 16 * b;
+                            const bool live = (row >> p.hqp_log2) < n && (row & (hqp - 1)) < hq && d < dk;
+                            float x[8];
 #pragma unroll
-                            for (int e = 0; e < 8; e++) x[e] *= inv;
+                            for (int e = 0; e < 4; e++) {
+                                const float2 f = Traits<T>::to_f2(u[b].v[e]);
+                                x[2 * e] = live ? f.x : 0.f; x[2 * e + 1] = live ? f.y : 0.f;
+                            }
+                            if (p.qnorm_w != nullptr) {
+                                float ss = 0.f;
+#pragma unroll
+                                for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                                const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.prenorm_eps);
+#pragma unroll
+                                for (int e = 0; e < 8; e++) x[e] *= inv * nw[e];
+                            }
+                            if (turns) {
+                                const float cs[4] = {c4[b].x, c4[b].y, c4[b].z, c4[b].w}, sn[4] = {s4[b].x, s4[b].y, s4[b].z, s4[b].w};
+#pragma unroll
+                                for (int e = 0; e < 4; e++) {
+                                    const float v = x[2 * e], w = x[2 * e + 1];
+                                    x[2 * e] = v * cs[e] - w * sn[e]; x[2 * e + 1] = w * cs[e] + v * sn[e];
+                                }
+                            }
+                            if (p.qk_norm_eps >= 0.f) {
+                                float ss = 0.f;
+#pragma unroll
+                                for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                                const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.qk_norm_eps);
+#pragma unroll
+                                for (int e = 0; e < 8; e++) x[e] *= inv;
+                            }
+                            if (row < nrows) stage_row(row, x);
                         }
-                        if (row < nrows) stage_row(row, x);
                     }
-                }
-            } else
+                } else
 #pragma unroll 1
-            for (int r0 = 2 * me; r0 < nrows; r0 += 20) {
-                const int row = r0 + (lane >> 4), tr = row >> p.hqp_log2, hh = row & (hqp - 1);
-                const bool live = tr < n && hh < hq && d < dk;
-                const int64_t t = ts + tr;
-                const T* qr = reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + hh) * dk;
-                float x[8], y[8];                     // the lane's entries; with `halves` the partners of those that turn
-                const bool turns = live && d < p.rot_dims;
-                const int dp = d < half ? d + half : d - half;                    // partner group (halves)
+                for (int r0 = 2 * me; r0 < nrows; r0 += 16) {
+                    const int row = r0 + (lane >> 4), tr = row >> p.hqp_log2, hh = row & (hqp - 1);
+                    const bool live = tr < n && hh < hq && d < dk;
+                    const int64_t t = ts + tr;
+                    const T* qr = reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + hh) * dk;
+                    float x[8], y[8];                     // the lane's entries; with `halves` the partners of those that turn
+                    const bool turns = live && d < p.rot_dims;
+                    const int dp = d < half ? d + half : d - half;                    // partner group (halves)
 #pragma unroll
-                for (int e = 0; e < 8; e++) { x[e] = 0.f; y[e] = 0.f; }
-                if (live) {
-                    if (p.q_vec) {
-                        const Vec8<T> u = ld_vec8(qr + d);
+                    for (int e = 0; e < 8; e++) { x[e] = 0.f; y[e] = 0.f; }
+                    if (live) {
+                        if (p.q_vec) {
+                            const Vec8<T> u = ld_vec8(qr + d);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(u.v[e]); x[2 * e] = f.x; x[2 * e + 1] = f.y; }
-                        if (p.halves && turns) {
-                            const Vec8<T> w = ld_vec8(qr + dp);
+                            for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(u.v[e]); x[2 * e] = f.x; x[2 * e + 1] = f.y; }
+                            if (p.halves && turns) {
+                                const Vec8<T> w = ld_vec8(qr + dp);
 #pragma unroll
-                            for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(w.v[e]); y[2 * e] = f.x; y[2 * e + 1] = f.y; }
+                                for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(w.v[e]); y[2 * e] = f.x; y[2 * e + 1] = f.y; }
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) x[e] = ldf(qr + d + e);
+                            if (p.halves && turns) {
+#pragma unroll
+                                for (int e = 0; e < 8; e++) {
+                                    const int j = d + e;
+                                    y[e] = j < p.rot_dims ? ldf(qr + (j < half ? j + half : j - half)) : 0.f;
+                                }
+                            }
                         }
-                    } else {
+                    }
+                    if (p.qnorm_w != nullptr) {
+                        float ss = 0.f;
 #pragma unroll
-                        for (int e = 0; e < 8; e++) x[e] = ldf(qr + d + e);
-                        if (p.halves && turns) {
+                        for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                        const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.prenorm_eps);
+                        if (live) {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) {
+                                x[e] *= inv * p.qnorm_w[d + e];
+                                const int j = d + e;
+                                if (p.halves && j < p.rot_dims) y[e] *= inv * p.qnorm_w[j < half ? j + half : j - half];
+                            }
+                        }
+                    }
+                    if (turns) {
+                        const float* cs = p.cosb + t * half;
+                        const float* sn = p.sinb + t * half;
+                        if (p.halves) {
 #pragma unroll
                             for (int e = 0; e < 8; e++) {
                                 const int j = d + e;
-                                y[e] = j < p.rot_dims ? ldf(qr + (j < half ? j + half : j - half)) : 0.f;
+                                if (j < half) x[e] = x[e] * cs[j] - y[e] * sn[j];
+                                else if (j < p.rot_dims) x[e] = x[e] * cs[j - half] + y[e] * sn[j - half];
+                            }
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const int i = (d >> 1) + e;
+                                if (i < half) {
+                                    const float a = x[2 * e], b = x[2 * e + 1];
+                                    x[2 * e] = a * cs[i] - b * sn[i]; x[2 * e + 1] = b * cs[i] + a * sn[i];
+                                }
                             }
                         }
                     }
-                }
-                if (p.qnorm_w != nullptr) {
-                    float ss = 0.f;
+                    if (p.qk_norm_eps >= 0.f) {
+                        float ss = 0.f;
 #pragma unroll
-                    for (int e = 0; e < 8; e++) ss += x[e] * x[e];
-                    const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.prenorm_eps);
-                    if (live) {
+                        for (int e = 0; e < 8; e++) ss += x[e] * x[e];
+                        const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.qk_norm_eps);
 #pragma unroll
-                        for (int e = 0; e < 8; e++) {
-                            x[e] *= inv * p.qnorm_w[d + e];
-                            const int j = d + e;
-                            if (p.halves && j < p.rot_dims) y[e] *= inv * p.qnorm_w[j < half ? j + half : j - half];
-                        }
+                        for (int e = 0; e < 8; e++) x[e] *= inv;
                     }
+                    stage_row(row, x);
                 }
-                if (turns) {
-                    const float* cs = p.cosb + t * half;
-                    const float* sn = p.sinb + t * half;
-                    if (p.halves) {
-#pragma unroll
-                        for (int e = 0; e < 8; e++) {
-                            const int j = d + e;
-                            if (j < half) x[e] = x[e] * cs[j] - y[e] * sn[j];
-                            else if (j < p.rot_dims) x[e] = x[e] * cs[j - half] + y[e] * sn[j - half];
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int i = (d >> 1) + e;
-                            if (i < half) {
-                                const float a = x[2 * e], b = x[2 * e + 1];
-                                x[2 * e] = a * cs[i] - b * sn[i]; x[2 * e + 1] = b * cs[i] + a * sn[i];
-                            }
-                        }
-                    }
-                }
-                if (p.qk_norm_eps >= 0.f) {
-                    float ss = 0.f;
-#pragma unroll
-                    for (int e = 0; e < 8; e++) ss += x[e] * x[e];
-                    const float inv = 1.f / sqrtf(sum16(ss) / (float)dk + p.qk_norm_eps);
-#pragma unroll
-                    for (int e = 0; e < 8; e++) x[e] *= inv;
-                }
-                stage_row(row, x);
-            }
-            fence_proxy_async();
-            named_bar_sync(1, WX_THREADS - 64);
-        }
-
-        if (warp == 0 || warp == 2) {
-            // ======================================================= producers: keys 40 (warp / 2) .. of every step, eight lanes a 128-byte piece
-            const int r0 = 20 * warp, piece = lane & 7;
-            const T* cache = reinterpret_cast<const T*>(p.cache);
-            auto key_row = [&](int v) {               // cache row of list entry v, -1 past the last
-                if (v >= total) return -1ll;
-                const int kp = v < nk ? v : v - nk + lo;
-                const int b = kp / p.block_size;
-                return ((long long)bt[b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size);
-            };
-            auto signal = [&](int j) {
                 fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->full[(n_done + j) % WX_STAGES]));
-            };
-            const int kofs = p.koff + g * KW, vofs = p.G * dk + (g / p.vshare) * dv;
-            long long ra = key_row(r0 + lane), rb = lane < 8 ? key_row(r0 + 32 + lane) : -1ll;
-            for (int j = 0; j < nsteps; j++) {
-                const long long a = ra, b = rb;
-                if (j + 1 < nsteps) {
-                    ra = key_row((j + 1) * WX_BK + r0 + lane);
-                    rb = lane < 8 ? key_row((j + 1) * WX_BK + r0 + 32 + lane) : -1ll;
-                }
-                const int it = n_done + j, st = it % WX_STAGES;
-                mbar_wait(smem_u32(&bars->empty[st]), ((it / WX_STAGES) & 1) ^ 1);
-                const uint32_t stage = smem_u32(kv_sm + st * WX_STAGE);
-#pragma unroll
-                for (int i = 0; i < 10; i++) {
-                    const int l = 4 * i + (lane >> 3), row = r0 + l;
-                    const long long ri = __shfl_sync(0xffffffffu, i < 8 ? a : b, l & 31);
-                    const int bytes = ri >= 0 ? 16 : 0;
-                    const T* src = ri >= 0 ? cache + ri * p.row_elems : cache;
-                    const uint32_t dst = stage + wx_off(row, piece);
-                    if constexpr (FULL) {             // (a row that is not there reads nothing, wherever src points)
-                        const T* ks = src + kofs + piece * 8;
-                        cp_async16(dst, ks, bytes); cp_async16(dst + WX_CHUNK, ks + 64, bytes);
-                        if (!shared_kv) {
-                            const T* vs = src + vofs + piece * 8;
-                            cp_async16(dst + 2 * WX_CHUNK, vs, bytes); cp_async16(dst + 3 * WX_CHUNK, vs + 64, bytes);
-                        }
-                    } else {
-                        for (int c = 0; c < kch; c++)
-                            if (c * 64 + piece * 8 < KW) cp_async16(dst + c * WX_CHUNK, bytes ? src + kofs + c * 64 + piece * 8 : src, bytes);
-                        for (int c = 0; c < vch; c++)
-                            if (c * 64 + piece * 8 < dv)
-                                cp_async16(dst + (kch + c) * WX_CHUNK, bytes ? src + vofs + c * 64 + piece * 8 : src, bytes);
-                    }
-                    if (EXT && shared_kv && piece == 0) {
-                        float* to = inv_sm + st * WX_BK + row;
-                        if (bytes) cp_async4(smem_u32(to), src + 2 * g);
-                        else *to = 0.f;
-                    }
-                }
-                cp_async_commit();
-                if (j >= WX_LAG) { cp_async_wait<WX_LAG>(); signal(j - WX_LAG); }
+                named_bar_sync(1, WX_THREADS - 64);
             }
-            cp_async_wait<0>();
-            for (int j = max(0, nsteps - WX_LAG); j < nsteps; j++) signal(j);
-        } else if (warp < 4) {
-            // ======================================================= product issuers (the warp stays converged, one elected lane issues)
-            const int x = warp >> 1;
-            const int mine = x == 0 ? steps_a : steps_b, end = x == 0 ? end_a : end_b;
-            const uint32_t idesc_s = make_instr_desc(WX_ROWS, WX_BK, UmmaFmt<T>::value, 0, 0);
-            const uint32_t idesc_o = make_instr_desc(WX_ROWS, dv, UmmaFmt<T>::value, 0, 1);
-            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-            const uint32_t s_addr = tm + WX_S_COL + x * WX_BK, p_addr = tm + WX_P_COL + x * (WX_BK / 2), o_addr = tm + WX_O_COL + x * 128;
-            const uint64_t dq = make_smem_desc(smem_u32(q_sm + x * WX_Q_BYTES), 16, 1024);
-            const uint64_t dk0 = make_smem_desc(smem_u32(kv_sm), 16, 1024), dv0 = make_smem_desc(smem_u32(kv_sm), WX_CHUNK, 1024);
-            const uint32_t vfirst = (uint32_t)((vch > 0 ? kch : 0) * WX_CHUNK) >> 4;
-            const int kd_steps = dk >> 4;
-            auto scores = [&](int j) {
-                const int it = n_done + j, st = it % WX_STAGES;
-                mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
-                tc_fence_after();
-                if (elect_one()) {
-                    const uint64_t kd = dk0 + (uint64_t)((st * WX_STAGE) >> 4);
-#pragma unroll
-                    for (int k = 0; k < 8; k++)
-                        if (k < kd_steps) {
-                            const int col = krot + 16 * k;
-                            umma_ss(s_addr, dq + (uint64_t)(((k >> 2) * WX_QCHUNK + (k & 3) * 32) >> 4),
-                                    kd + (uint64_t)(((col >> 6) * WX_CHUNK + (col & 63) * 2) >> 4), idesc_s, k > 0);
-                        }
-                    umma_commit(smem_u32(&bars->s_full[x]));
-                }
-                __syncwarp();
-            };
-            if (mine > 0) {
-                scores(0);
-                for (int j = 0; j < mine; j++) {
-                    const int xi = x_done[x] + j;
-                    if (j + 1 < mine) {
-                        mbar_wait(smem_u32(&bars->s_empty[x]), xi & 1);
-                        scores(j + 1);
-                    }
-                    const int st = (n_done + j) % WX_STAGES;
-                    mbar_wait(smem_u32(&bars->p_full[x]), xi & 1);
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const int k16 = min(WX_BK / 16, (end - j * WX_BK + 15) / 16);     // none past the last key the tile can see
-                        const uint64_t vd = dv0 + (uint64_t)((st * WX_STAGE) >> 4) + vfirst;
-#pragma unroll
-                        for (int k = 0; k < WX_BK / 16; k++)
-                            if (k < k16) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-                        umma_commit(smem_u32(&bars->empty[st]));
-                        umma_commit(smem_u32(&bars->p_empty[x]));
-                    }
-                    __syncwarp();
-                }
-                // the last scores' s_empty is waited for by nobody: its phase is taken by the count x_done
-            }
-            // steps that only the other tile takes: hand the stages on once they have been filled (never a phase ahead)
-            for (int j = mine; j < nsteps; j++) {
-                const int it = n_done + j, st = it % WX_STAGES;
-                mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
-                if (lane == 0) mbar_arrive(smem_u32(&bars->empty[st]));
-            }
-        } else {
             // ======================================================= softmax: tile x, thread = row
-            const int x = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
-            const int mine = x == 0 ? steps_a : steps_b;
+            const int mine = x == 0 ? sg.steps_a : sg.steps_b, x_done = x == 0 ? done_a : done_b;
             const int tr = x * tpt + (row >> p.hqp_log2), hh = row & (hqp - 1), h = g * hq + hh;
             const bool live = tr < n && hh < hq;
             const int pos = pos0 + tr;
@@ -399,7 +424,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
             float m_ref = p.sink > 0.f ? 0.f : -INFINITY, l = p.sink;
             if (EXT && p.sinks != nullptr && live) { m_ref = p.sinks[h] * WX_LOG2E; l = 1.f; }
             for (int j = 0; j < mine; j++) {
-                const int xi = x_done[x] + j;
+                const int xi = x_done + j;
                 mbar_wait(smem_u32(&bars->s_full[x]), xi & 1);
                 tc_fence_after();
                 uint32_t r[WX_BK];
@@ -485,7 +510,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
             }
             if (mine > 0) {
                 // ---- output row: normalise, (turn back,) gate, store
-                mbar_wait(smem_u32(&bars->p_empty[x]), (x_done[x] + mine - 1) & 1);
+                mbar_wait(smem_u32(&bars->p_empty[x]), (x_done + mine - 1) & 1);
                 tc_fence_after();
                 const int64_t t = ts + tr;
                 const T* gate = reinterpret_cast<const T*>(p.gate);
@@ -494,22 +519,17 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                     f = p.out_scale / l;
                     if (EXT && p.gate_per_head && gate != nullptr) f *= 1.f / (1.f + __expf(-ldf(gate + t * p.gate_st + h)));
                 }
-                const T* grow = gate != nullptr && !(EXT && p.gate_per_head) ? gate + t * p.gate_st + (int64_t)h * dv : nullptr;
+                const bool gated = gate != nullptr && !(EXT && p.gate_per_head);
+                const T* grow = gated ? gate + t * p.gate_st + (int64_t)h * dv : nullptr;
                 const int64_t at = t * p.out_st + (int64_t)h * dv;
-                auto store8 = [&](const T* gr, int64_t to, float (&y)[8]) {        // eight neighbouring entries (gated unless gr is null)
-                    if (gr != nullptr) {
-                        if (p.gate_vec) {
-                            const Vec8<T> u = ld_vec8(gr);
+                auto gate8 = [&](const Vec8<T>& u, float (&y)[8]) {
 #pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                const float2 z = Traits<T>::to_f2(u.v[e]);
-                                y[2 * e] = __fdividef(y[2 * e], 1.f + __expf(-z.x)); y[2 * e + 1] = __fdividef(y[2 * e + 1], 1.f + __expf(-z.y));
-                            }
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 8; e++) y[e] *= 1.f / (1.f + __expf(-ldf(gr + e)));
-                        }
+                    for (int e = 0; e < 4; e++) {
+                        const float2 z = Traits<T>::to_f2(u.v[e]);
+                        y[2 * e] = __fdividef(y[2 * e], 1.f + __expf(-z.x)); y[2 * e + 1] = __fdividef(y[2 * e + 1], 1.f + __expf(-z.y));
                     }
+                };
+                auto store8 = [&](int64_t to, float (&y)[8]) {
                     if (p.out_f32) {
                         float* o = reinterpret_cast<float*>(p.out) + to;
                         if (p.out_vec) {
@@ -529,13 +549,34 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                         }
                     }
                 };
-                auto put8 = [&](int d, float (&y)[8]) { store8(grow != nullptr ? grow + d : nullptr, at + d, y); };
-                if (p.vcos == nullptr && p.out_vec && (grow == nullptr || p.gate_vec)) {
+                auto put8 = [&](int d, float (&y)[8]) {                            // eight neighbouring entries of this thread's row
+                    if (gated) {
+                        if (p.gate_vec) {
+                            gate8(ld_vec8(grow + d), y);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) y[e] *= 1.f / (1.f + __expf(-ldf(grow + d + e)));
+                        }
+                    }
+                    store8(at + d, y);
+                };
+                if (p.vcos == nullptr && p.out_vec && (!gated || p.gate_vec)) {
                     // 64 columns at a time through this tile's query buffer (its products are done), so that a row's gate and output move
                     // as whole lines: eight lanes a row, rows swizzled by 16 bytes
                     float* xs = reinterpret_cast<float*>(q_sm + x * WX_Q_BYTES);
                     auto cell = [&](int rr, int quarter) { return reinterpret_cast<float4*>(xs + rr * 64 + ((quarter ^ (rr & 15)) << 2)); };
+                    const int l8 = lane & 7;
+                    // this lane's part of row 32 quad + 4 i + lane / 8: its index in gate and out, -1 where there is nothing to store
+                    auto part = [&](int i, int d0, int64_t stride) {
+                        const int rr = quad * 32 + 4 * i + (lane >> 3), rt = x * tpt + (rr >> p.hqp_log2), rh = rr & (hqp - 1);
+                        return rt < n && rh < hq && d0 + 8 * l8 < dv ? (ts + rt) * stride + (int64_t)(g * hq + rh) * dv + d0 + 8 * l8 : -1ll;
+                    };
                     for (int d0 = 0; d0 < dv; d0 += 64) {
+                        Vec8<T> z[8];                 // all gates of the pass are asked for before the first is used
+                        if (gated) {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) z[i] = ld_vec8(gate + max(part(i, d0, p.gate_st), 0ll));
+                        }
                         const int cols = min(64, dv - d0);
 #pragma unroll 1
                         for (int d = 0; d < cols; d += 16) {
@@ -547,21 +588,17 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                                 *cell(row, (d >> 2) + e) = make_float4(__uint_as_float(v[4 * e]) * f, __uint_as_float(v[4 * e + 1]) * f,
                                                                        __uint_as_float(v[4 * e + 2]) * f, __uint_as_float(v[4 * e + 3]) * f);
                         }
-                        named_bar_sync(2 + x, 128);
-                        const int l8 = lane & 7, d = d0 + 8 * l8;
-#pragma unroll 4
+                        __syncwarp();                 // a warp reads the rows that it wrote
+#pragma unroll
                         for (int i = 0; i < 8; i++) {
-                            const int rr = quad * 32 + 4 * i + (lane >> 3), rt = x * tpt + (rr >> p.hqp_log2), rh = rr & (hqp - 1);
-                            if (rt < n && rh < hq && d < dv) {
-                                const int64_t tt = ts + rt;
-                                const int head = g * hq + rh;
-                                const float4 lo4 = *cell(rr, 2 * l8), hi4 = *cell(rr, 2 * l8 + 1);
-                                float y[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
-                                store8(gate != nullptr && !(EXT && p.gate_per_head) ? gate + tt * p.gate_st + (int64_t)head * dv + d : nullptr,
-                                       tt * p.out_st + (int64_t)head * dv + d, y);
-                            }
+                            const int rr = quad * 32 + 4 * i + (lane >> 3);
+                            const float4 lo4 = *cell(rr, 2 * l8), hi4 = *cell(rr, 2 * l8 + 1);
+                            float y[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+                            if (gated) gate8(z[i], y);
+                            const int64_t to = part(i, d0, p.out_st);
+                            if (to >= 0) store8(to, y);
                         }
-                        named_bar_sync(2 + x, 128);
+                        __syncwarp();
                     }
                 } else {
                 const int hv = dv >> 1;
@@ -597,13 +634,12 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                 __syncwarp();
                 }
             }
+            tc_fence_before();
+            __syncthreads();                          // the next segment overwrites the queries; its first products overwrite O
+            tc_fence_after();
+            n_done += nsteps; done_a += sg.steps_a; done_b += sg.steps_b;
+            i0 += n;
         }
-        tc_fence_before();
-        __syncthreads();                              // the next segment overwrites the queries; its first products overwrite O
-        tc_fence_after();
-        n_done += nsteps;
-        x_done[0] += steps_a; x_done[1] += steps_b;
-        i0 += n;
     }
     if (warp == 1) tmem_dealloc<512>(tmem);
 }
