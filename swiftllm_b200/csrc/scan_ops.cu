@@ -90,19 +90,20 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TI* __restrict__ 
     }
 }
 
-// The same for prompt rows where rows are 16-byte pieces: a thread walks SV_TOKENS rows of VW neighbouring channels (16 bytes of input),
-// four of them in flight while four are multiplied; where the rows of the tile break (another sequence) is found once per warp.  The products
+// The same for prompt rows where rows are whole pieces of four channels: a thread walks SV_TOKENS rows of four neighbouring channels, eight
+// rows' loads in flight together (wider pieces need 154 registers and leave ten warps on an SM: 96 us); where the rows of the tile break (another sequence) is found once per warp.  The products
 // and their order are those above; for 16-bit results the SiLU takes the special-function unit's exponential and quotient (a few units
-// of 2^-22).  Bound: the input and output bytes.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 186 -> 33 us (4.1 TB/s).
+// of 2^-22).  Bound: bytes, of which enough
+// are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 -> 59 us (2.3 TB/s).
 constexpr int SV_TOKENS = 16;
 template <typename TI, typename TO, int K>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restrict__ xin, int64_t xin_stride, const float* __restrict__ w,
                                                              const float* __restrict__ bias, const TI* __restrict__ tail,
                                                              const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                                                              TO* __restrict__ out, int64_t row_end, int C, int add_input, int act_silu) {
-    constexpr int VW = 16 / sizeof(TI), H = K - 1;
-    struct alignas(16) In { TI e[VW]; };
-    struct alignas(VW * sizeof(TO) < 16 ? VW * sizeof(TO) : 16) Out { TO e[VW]; };
+    constexpr int VW = 4, H = K - 1;
+    struct alignas(VW * sizeof(TI)) In { TI e[VW]; };
+    struct alignas(VW * sizeof(TO)) Out { TO e[VW]; };
     const int64_t tile0 = (int64_t)blockIdx.x * SV_TOKENS;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VW, lane = threadIdx.x & 31;
     const int nrows = (int)min((int64_t)SV_TOKENS, row_end - tile0);
@@ -119,15 +120,15 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restric
     const bool live = c < C;
     const int cc = live ? c : 0;
     const TI* col = xin + cc;
-    constexpr int AT_ONCE = 4;                          // rows in flight while as many are multiplied
-    In cur[AT_ONCE], nxt[AT_ONCE];
-    auto load = [&](In (&to)[AT_ONCE], int i0) {
+    constexpr int AT_ONCE = 8;                          // rows whose loads are in flight together
+    In cur[AT_ONCE];
+    auto load = [&](int i0) {
+        const TI* at = col + (tile0 + i0) * xin_stride;
 #pragma unroll
-        for (int u = 0; u < AT_ONCE; u++)
-            if (i0 + u < nrows) to[u] = *reinterpret_cast<const In*>(col + (tile0 + i0 + u) * xin_stride);
+        for (int u = 0; u < AT_ONCE; u++, at += xin_stride)
+            if (i0 + u < nrows) cur[u] = *reinterpret_cast<const In*>(at);
     };
-    load(cur, 0);
-    load(nxt, AT_ONCE);
+    load(0);
     float wk[K][VW], b0[VW];
 #pragma unroll
     for (int e = 0; e < VW; e++) {
@@ -185,9 +186,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restric
             }
             if (live) *reinterpret_cast<Out*>(out + (tile0 + i) * C + c) = o;
         }
-#pragma unroll
-        for (int u = 0; u < AT_ONCE; u++) cur[u] = nxt[u];
-        load(nxt, i0 + 2 * AT_ONCE);
+        load(i0 + AT_ONCE);
     }
 }
 
@@ -373,14 +372,18 @@ constexpr int SS_BCR = 4;
 //
 // VEC (16-bit rows in 16-byte pieces, states in whole eights): a thread brings eight neighbouring channels of ONE token and eight entries of
 // B or C per tile, with one address each, and stores eight outputs; the SiLU of the gate takes the special-function unit's exponential
-// and quotient.  Measured on B200, bf16, 4 x 2048 tokens, 4096 channels, 16 states: SCAN_MEASURED.
-template <typename T, typename TD, bool VEC>
+// and quotient.  Measured on B200, bf16, 4 x 2048 tokens, 4096 channels, 16 states: 813 -> 370 us (staging took 85
+// of 125 instructions per token; with the shape unknown to the compiler 541 us); one segment of 1024 tokens 426 -> 122 us.  What
+// remains is issue and the special-function unit (21 results per token and channel: 150 us).
+// NSL >= 0: 16 states on 2^NSL lanes, known to the compiler.
+template <typename T, typename TD, bool VEC, int NSL>
 __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
     const T* __restrict__ x, int64_t x_stride, const TD* __restrict__ dtl, int64_t dt_stride, const float* __restrict__ dt_bias,
     const float* __restrict__ A, const T* __restrict__ bc, int64_t bc_stride, int b_off, int c_off, const float* __restrict__ D,
     const T* __restrict__ z, int64_t z_stride, float* __restrict__ state, const int* __restrict__ seg_starts,
-    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C, int N, int ns_log2, int tt) {
+    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C, int N_, int ns_log2_, int tt_) {
     extern __shared__ __align__(16) float ssm[];
+    const int N = NSL >= 0 ? 16 : N_, ns_log2 = NSL >= 0 ? NSL : ns_log2_, tt = NSL >= 0 ? (NSL >= 2 ? 32 : SS_ITEMS << NSL) : tt_;
     const int NS = 1 << ns_log2, ch_log2 = 7 - ns_log2, CH = 1 << ch_log2, RE = (N + NS - 1) >> ns_log2;
     // whole groups of four states per lane, on 16-byte boundaries of the staged rows: B and C are read four at a time
     const bool vec = (N & 3) == 0 && (RE & 3) == 0;
@@ -525,20 +528,20 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
         const float* bp = bs + s * RE;
         const float* cp = cs + s * RE;
         const bool lane_live = s * RE < N;
-        if (vec && ns_log2 >= 2 && (tt & 3) == 0) {
+        if (NSL >= 0 || (vec && ns_log2 >= 2 && (tt & 3) == 0)) {
             // four tokens at a time, packed arithmetic; the four sums over the lanes of a channel are taken together, each lane quarter
             // keeping the token (2 (s & 1) + (s >> 1 & 1)) that it writes
-            for (int j = 0; j < nt; j += 4) {
+            auto four = [&](int j, bool whole) {        // tokens j .. j + 3 (those below nt)
                 float y[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     y[u] = 0.f;
-                    if (j + u < nt) {
+                    if (whole || j + u < nt) {
                         const float dt = ds[((j + u) << ch_log2) + cl], dx = dt * xs[((j + u) << ch_log2) + cl];
                         float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-                        for (int q = 0; q < SS_R / 4; q++) {
-                            if (4 * q < RE && lane_live) {
+                        for (int q = 0; q < (NSL >= 0 ? (16 >> NSL) / 4 : SS_R / 4); q++) {
+                            if (NSL >= 0 || (4 * q < RE && lane_live)) {
                                 const float4 b4 = reinterpret_cast<const float4*>(bp + (j + u) * N)[q], c4 = reinterpret_cast<const float4*>(cp + (j + u) * N)[q];
                                 float2 s0 = make_float2(S[4 * q], S[4 * q + 1]), s1 = make_float2(S[4 * q + 2], S[4 * q + 3]);
                                 const float2 e0 = make_float2(exp2_neg(dt * a[4 * q]), exp2_neg(dt * a[4 * q + 1]));
@@ -556,13 +559,25 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                 const bool odd = s & 1, high = s & 2;
                 const float k0 = odd ? y[2] : y[0], k1 = odd ? y[3] : y[1];                          // kept pair
                 const float p0 = k0 + __shfl_xor_sync(0xffffffffu, odd ? y[0] : y[2], 1), p1 = k1 + __shfl_xor_sync(0xffffffffu, odd ? y[1] : y[3], 1);
-                float v = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
-                for (int o = NS >> 1; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                const int mine = j + 2 * (s & 1) + ((s >> 1) & 1);
-                if (s < 4 && mine < nt) {
-                    const int at = (mine << ch_log2) + cl;
-                    ys[at] = (v + dd * xs[at]) * zs[at];
+                if (NSL == 1) {
+                    const int mine = j + 2 * (s & 1), at = (mine << ch_log2) + cl;
+                    if (whole || mine < nt) ys[at] = (p0 + dd * xs[at]) * zs[at];
+                    if (whole || mine + 1 < nt) ys[at + CH] = (p1 + dd * xs[at + CH]) * zs[at + CH];
+                } else {
+                    float v = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
+                    if (NSL < 0) for (int o = NS >> 1; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    const int mine = j + 2 * (s & 1) + ((s >> 1) & 1);
+                    if ((NSL >= 0 || s < 4) && (whole || mine < nt)) {
+                        const int at = (mine << ch_log2) + cl;
+                        ys[at] = (v + dd * xs[at]) * zs[at];
+                    }
                 }
+            };
+            if (nt == tt) {
+#pragma unroll 2
+                for (int j = 0; j < tt; j += 4) four(j, true);
+            } else {
+                for (int j = 0; j < nt; j += 4) four(j, false);
             }
         } else
         for (int j = 0; j < nt; j++, bp += N, cp += N) {
@@ -641,12 +656,11 @@ int sllm_short_conv(const void* xin, int64_t xin_stride, sllm_dtype_t in_dtype, 
         (const TI*)xin, xin_stride, (const float*)w, (const float*)bias, (TI*)tail, (const int*)tok_seq,                        \
         (const int*)tok_pos, (T*)out, (int64_t)(r0), (int64_t)(r1), channels, taps, add_input, act_silu,                        \
         (TOKENS == 1 && move_decode_tails && taps > 1) ? 1 : 0)
-    // prompt rows in 16-byte pieces: three or four taps (what the workers have) take the vector kernel, others a channel per thread
-    const int vw = in_dtype == SLLM_F32 ? 4 : 8;
-    const bool vec = (taps == 3 || taps == 4) && channels % vw == 0 && xin_stride % vw == 0 &&
+    // prompt rows in pieces of four channels: three or four taps (what the workers have) take the vector kernel, others a channel per thread
+    const bool vec = (taps == 3 || taps == 4) && channels % 4 == 0 && xin_stride % 4 == 0 &&
                      (((uintptr_t)xin | (uintptr_t)tail | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
 #define SC_VEC(TI, K)                                                                                                          \
-    short_conv_vec_kernel<TI, T, K><<<dim3((unsigned)cdiv(num_prefill_tokens, SV_TOKENS), (unsigned)cdiv(channels, 128 * vw)), 128, 0, st>>>( \
+    short_conv_vec_kernel<TI, T, K><<<dim3((unsigned)cdiv(num_prefill_tokens, SV_TOKENS), (unsigned)cdiv(channels, 512)), 128, 0, st>>>( \
         (const TI*)xin, xin_stride, (const float*)w, (const float*)bias, (const TI*)tail, (const int*)tok_seq, (const int*)tok_pos, \
         (T*)out, num_prefill_tokens, channels, add_input, act_silu)
     if (num_prefill_tokens > 0 && vec) {
@@ -716,7 +730,8 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
     int ns_tiled = ns_plain;
     if (num_prefill_segs > 0) {
         // prompt portions walk their tokens one after the other: with few (segment, channel) pairs more lanes per channel (fewer
-        // states per thread) put more warps on the SMs
+        // states per thread) put more warps on the SMs, but not below four states a lane, which are read and multiplied together
+        // (one segment of 1024 tokens, 4096 channels: 389 us with two states a lane, 229 with four)
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
         while (ns_tiled < 5 && (2 << ns_tiled) <= states &&
@@ -737,12 +752,15 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
         const bool vec = dtype != SLLM_F32 && states % 8 == 0 && channels % 8 == 0 && ns_tiled <= 4 && x_stride % 8 == 0 && z_stride % 8 == 0 &&
                          bc_stride % 8 == 0 && b_off % 8 == 0 && c_off % 8 == 0 && dt_stride % dv == 0 &&
                          (((uintptr_t)x | (uintptr_t)dt | (uintptr_t)z | (uintptr_t)bc | (uintptr_t)out) & 15) == 0;
-#define SS_TILED(TT, TD, VEC) selective_scan_tiled_kernel<TT, TD, VEC><<<SS_GRID(num_prefill_segs, ns_tiled), smem, st>>>(SS_ARGS(TD, 0, ns_tiled), tt)
+#define SS_TILED(TT, TD, VEC, NSL) selective_scan_tiled_kernel<TT, TD, VEC, NSL><<<SS_GRID(num_prefill_segs, ns_tiled), smem, st>>>(SS_ARGS(TD, 0, ns_tiled), tt)
+        const bool n16 = states == 16 && (ns_tiled == 1 || ns_tiled == 2);
         if (vec) {
-            if (dt_f32) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true))); }
-            else { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, T, true))); }
-        } else if (dt_f32) { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, float, false))); }
-        else { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, T, false))); }
+            if (dt_f32 && n16 && ns_tiled == 1) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, 1))); }
+            else if (dt_f32 && n16) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, 2))); }
+            else if (dt_f32) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, -1))); }
+            else { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, T, true, -1))); }
+        } else if (dt_f32) { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, float, false, -1))); }
+        else { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, T, false, -1))); }
 #undef SS_TILED
         if (check_launch("selective_scan (prompt portions)")) return 1;
     }
