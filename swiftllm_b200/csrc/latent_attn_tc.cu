@@ -8,8 +8,9 @@
 //   O[64, r]       += P K[:, :r]   M = 64, N = 256 twice; P from TMEM, the SAME key tile (now MN-major: a latent is key and value at once)
 // Accumulators and P stay in TMEM: an M = 64 operand fills 16 of every 32 lanes, so the two halves of O lie in the same 256 columns (lane
 // offsets 0 and 16); P (16-bit, two buffers) is written to both lane offsets, because an A operand lies in its accumulator's lanes; S has
-// two buffers beside them.  The running maximum may trail the true one by 2^8 before O is rescaled ("lazy": numerator and denominator
-// use the same reference, so the result does not change).
+// two buffers beside them.  The reference of the exponentials is the running maximum itself: a reference that trails it (by up to 2^8, say)
+// would save most rescales of O (486 instead of 530 us below), but then the largest weight is not 1 and takes a rounding as well,
+// 2.15e-3 instead of 2.01e-3 off 64-bit arithmetic in bf16.
 //
 // Shared memory is what decides the shape: 64 rows of Q (576 entries: 72 KiB) and two stages of 64 keys (72 KiB each) fill it.  A stage
 // therefore is handed back in two pieces, each as soon as the product that reads it last is done: the first 256 columns after the first
@@ -38,7 +39,6 @@ constexpr int LT_MAX_CHUNKS = 9;
 constexpr int LT_STAGE = LT_MAX_CHUNKS * LT_CHUNK;
 constexpr int LT_SMEM = 3 * LT_STAGE + 1024;
 constexpr int LT_S_COL = 256, LT_P_COL = 384;       // TMEM columns: O 0..255, S two of 64, P two of 32
-constexpr float LT_RESCALE = 8.0f;                  // log2 units
 constexpr float LT_LOG2E = 1.4426950408889634f, LT_LN2 = 0.6931471805599453f;
 
 struct LatentTcBars {
@@ -154,8 +154,26 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             mbar_wait(smem_u32(&bars->empty[n_done & 1][g]), ((n_done >> 1) & 1) ^ 1);
             load(n_done & 1, first);
         }
-        // ---- queries: [q_lat | rotated q_rot], zeros in rows without a (token, head)
+        // ---- queries: [q_lat | rotated q_rot], zeros in rows without a (token, head).  The rotated entries (eight at a time; pairs
+        // (2i, 2i + 1) below rot_dims turn) and their angles are asked for first and used last
         {
+            const int half = p.rot_dims >> 1, eighths = dr >> 3;
+            constexpr int AT_ONCE = (LT_ROWS * 8 + LT_THREADS - 1) / LT_THREADS;
+            Vec8<T> u[AT_ONCE];
+            float4 c4[AT_ONCE], s4[AT_ONCE];
+#pragma unroll
+            for (int b = 0; b < AT_ONCE; b++) {
+                const int i = tid + b * LT_THREADS, row = eighths > 0 ? i / eighths : LT_ROWS, d = (i - row * eighths) * 8;
+                const int j = row >> p.hp_log2, h = h0 + (row & (hp - 1));
+                c4[b] = make_float4(1.f, 1.f, 1.f, 1.f); s4[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p.rot_vec && row < LT_ROWS && j < n && h < p.H) {
+                    u[b] = ld_vec8(reinterpret_cast<const T*>(p.q_rot) + (int64_t)(ts + j) * p.qr_st + (int64_t)h * p.qr_sh + d);
+                    if (d < p.rot_dims) {
+                        const int64_t ang = (int64_t)(ts + j) * half + (d >> 1);
+                        c4[b] = *reinterpret_cast<const float4*>(p.cosb + ang); s4[b] = *reinterpret_cast<const float4*>(p.sinb + ang);
+                    }
+                }
+            }
 #pragma unroll 1
             for (int row = warp; row < LT_ROWS; row += LT_THREADS / 32) {
                 const int j = row >> p.hp_log2, h = h0 + (row & (hp - 1));
@@ -177,39 +195,33 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 }
             }
             cp_async_commit();
-            // eight rotated entries at a time; pairs (2i, 2i + 1) below rot_dims turn
-            const int half = p.rot_dims >> 1, eighths = dr >> 3;
-            for (int i = tid; i < LT_ROWS * eighths; i += LT_THREADS) {
-                const int row = i / eighths, d = (i - row * eighths) * 8;
+#pragma unroll
+            for (int b = 0; b < AT_ONCE; b++) {
+                const int i = tid + b * LT_THREADS, row = eighths > 0 ? i / eighths : LT_ROWS, d = (i - row * eighths) * 8;
+                if (row >= LT_ROWS) continue;
                 const int j = row >> p.hp_log2, h = h0 + (row & (hp - 1));
                 const int64_t t = ts + j;
                 uint4 v = make_uint4(0, 0, 0, 0);
                 if (j < n && h < p.H) {
-                    const T* qr = reinterpret_cast<const T*>(p.q_rot) + t * p.qr_st + (int64_t)h * p.qr_sh + d;
-                    const int64_t ang = t * half + (d >> 1);
-                    float x[8], cs[4], sn[4];
+                    float x[8], cs[4] = {c4[b].x, c4[b].y, c4[b].z, c4[b].w}, sn[4] = {s4[b].x, s4[b].y, s4[b].z, s4[b].w};
                     if (p.rot_vec) {
-                        const Vec8<T> u = ld_vec8(qr);
-                        float4 c4 = make_float4(1.f, 1.f, 1.f, 1.f), s4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (d < p.rot_dims) { c4 = *reinterpret_cast<const float4*>(p.cosb + ang); s4 = *reinterpret_cast<const float4*>(p.sinb + ang); }
-                        cs[0] = c4.x; cs[1] = c4.y; cs[2] = c4.z; cs[3] = c4.w;
-                        sn[0] = s4.x; sn[1] = s4.y; sn[2] = s4.z; sn[3] = s4.w;
 #pragma unroll
-                        for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(u.v[e]); x[2 * e] = f.x; x[2 * e + 1] = f.y; }
+                        for (int e = 0; e < 4; e++) { const float2 f = Traits<T>::to_f2(u[b].v[e]); x[2 * e] = f.x; x[2 * e + 1] = f.y; }
                     } else {
+                        const T* qr = reinterpret_cast<const T*>(p.q_rot) + t * p.qr_st + (int64_t)h * p.qr_sh + d;
+                        const int64_t ang = t * half + (d >> 1);
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
-                            const bool turns = d + 2 * e < p.rot_dims;
                             x[2 * e] = ldf(qr + 2 * e); x[2 * e + 1] = ldf(qr + 2 * e + 1);
-                            cs[e] = turns ? p.cosb[ang + e] : 1.f; sn[e] = turns ? p.sinb[ang + e] : 0.f;
+                            if (d + 2 * e < p.rot_dims) { cs[e] = p.cosb[ang + e]; sn[e] = p.sinb[ang + e]; }
                         }
                     }
                     uint32_t w[4];
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
                         const bool turns = d + 2 * e < p.rot_dims;
-                        const float a = x[2 * e], b = x[2 * e + 1];
-                        w[e] = turns ? pack2<T>(a * cs[e] - b * sn[e], b * cs[e] + a * sn[e]) : pack2<T>(a, b);
+                        const float a = x[2 * e], b2 = x[2 * e + 1];
+                        w[e] = turns ? pack2<T>(a * cs[e] - b2 * sn[e], b2 * cs[e] + a * sn[e]) : pack2<T>(a, b2);
                     }
                     v = make_uint4(w[0], w[1], w[2], w[3]);
                 }
@@ -366,9 +378,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, 1)); xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, 2));
                 xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, 1)); xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, 2));
                 const float na = fmaxf(ma, xa * c), nb = fmaxf(mb, xb * c);
-                // true on a row's first visible key; the first tile's maximum is taken as it is (a sink may lie far below it)
-                const float slack = j == 0 ? 0.f : LT_RESCALE;
-                const bool need_a = na > ma + slack, need_b = nb > mb + slack;
+                const bool need_a = na > ma, need_b = nb > mb;
                 const float al_a = need_a ? fast_exp2_tc(ma - na) : 1.f, al_b = need_b ? fast_exp2_tc(mb - nb) : 1.f;
                 if (need_a) { ma = na; la *= al_a; }
                 if (need_b) { mb = nb; lb *= al_b; }
@@ -391,13 +401,18 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                     const float f0 = __shfl_sync(0xffffffffu, al_a, from), f1 = __shfl_sync(0xffffffffu, al_b, from);
                     const float f = orow < 8 ? f0 : f1;
 #pragma unroll 1
-                    for (int cc = 0; cc < n0; cc += 32) {
-                        uint32_t o[32];
-                        tmem_ld32(tlane + cc, o);
+                    for (int cc = 0; cc < n0; cc += 64) {      // n0 is in whole 64-column chunks
+                        uint32_t o0[32], o1[32];
+                        tmem_ld32(tlane + cc, o0);
+                        tmem_ld32(tlane + cc + 32, o1);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int e = 0; e < 32; e++) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-                        tmem_st32(tlane + cc, o);
+                        for (int e = 0; e < 32; e++) {
+                            o0[e] = __float_as_uint(__uint_as_float(o0[e]) * f);
+                            o1[e] = __float_as_uint(__uint_as_float(o1[e]) * f);
+                        }
+                        tmem_st32(tlane + cc, o0);
+                        tmem_st32(tlane + cc + 32, o1);
                     }
                 }
                 tmem_st_16x32(tlane + LT_P_COL + 32 * st, w);

@@ -30,6 +30,30 @@ static int launch_prefill_paged(const void* q, const void* k_cache, const void* 
     return check_launch("prefill_attention_paged");
 }
 
+// One warp per (token, head), four entries a lane: the splits' rows on their common maximum.  A split that saw no key of the row has
+// maximum -infinity and wrote no O.
+template <typename T>
+__global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+                                                            T* __restrict__ o, int64_t units, int nsplit) {
+    const int lane = threadIdx.x & 31;
+    const int64_t u = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (u >= units) return;
+    float M = -INFINITY, L = 0.f;
+    for (int z = 0; z < nsplit; z++) M = fmaxf(M, part_ml[2 * (z * units + u)]);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int z = 0; z < nsplit; z++) {
+        const float2 ml = *reinterpret_cast<const float2*>(part_ml + 2 * (z * units + u));
+        if (ml.x == -INFINITY) continue;
+        const float f = exp2f(ml.x - M);
+        const float4 v = *reinterpret_cast<const float4*>(part_o + (z * units + u) * PT_D + 4 * lane);
+        L += f * ml.y;
+        a.x += f * v.x; a.y += f * v.y; a.z += f * v.z; a.w += f * v.w;
+    }
+    const float inv = 1.f / L;
+    typename Traits<T>::T2 lo = Traits<T>::from_f2(make_float2(a.x * inv, a.y * inv)), hi = Traits<T>::from_f2(make_float2(a.z * inv, a.w * inv));
+    *reinterpret_cast<uint2*>(o + u * PT_D + 4 * lane) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+
 static bool tc_prefill_paged_supported(int head_dim, int block_size, int64_t num_tokens, int64_t cache_rows) {
     return head_dim == PT_D && block_size == PT_PAGE && num_tokens > 0 && num_tokens < (1LL << 31) &&
            cache_rows < (1LL << 31) && get_tensor_map_encoder() != nullptr;      // TMA coordinates are int32
@@ -46,7 +70,7 @@ static int launch_prefill_paged_tc(const void* q, const void* k_cache, const voi
                  "prefill_attention_paged: cuTensorMapEncodeTiled failed");
     PtParams p;
     p.o = o; p.start_locs = start_locs; p.seq_lens = chunk_lens; p.scale_log2e = scale_log2e; p.nq = nq; p.nkv = nkv;
-    dim3 grid((max_chunk_len + 2 * PT_BQ - 1) / (2 * PT_BQ), nq, num_seqs);
+    dim3 grid((max_chunk_len + 2 * PT_BQ - 1) / (2 * PT_BQ), nq, num_seqs * pg.nsplit);
     if (dtype == SLLM_F16) {
         static unsigned long long c = 0;
         if (first_use_on_this_device(c)) cudaFuncSetAttribute(prefill_attn_tc_kernel<__half, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
@@ -56,20 +80,27 @@ static int launch_prefill_paged_tc(const void* q, const void* k_cache, const voi
         if (first_use_on_this_device(c)) cudaFuncSetAttribute(prefill_attn_tc_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
         prefill_attn_tc_kernel<__nv_bfloat16, true><<<grid, PT_THREADS, PT_SMEM_BYTES, stream>>>(qmap, kmap, vmap, p, pg);
     }
-    return check_launch("prefill_attention_paged(tcgen05)");
+    if (check_launch("prefill_attention_paged(tcgen05)")) return 1;
+    if (pg.nsplit > 1) {
+        const int64_t units = num_tokens * nq;
+        SLLM_DISPATCH_DTYPE(dtype, (prefill_merge_kernel<T><<<(unsigned)cdiv(units, 8), 256, 0, stream>>>(pg.part_o, pg.part_ml, (T*)o, units, pg.nsplit)));
+        return check_launch("prefill_attention_paged(merge)");
+    }
+    return 0;
 }
 
 }  // namespace sllm
 
 using namespace sllm;
 
-extern "C" int sllm_prefill_attention_paged(const void* q, const void* k_cache, const void* v_cache, void* o,
+static int prefill_attention_paged(const void* q, const void* k_cache, const void* v_cache, void* o,
                                             const int32_t* block_table, const int32_t* seq_ids,
                                             const int32_t* prefill_seq_start_locs, const int32_t* prefill_seq_lens,
                                             const int32_t* prefill_prefix_lens, float softmax_scale, int num_prefill_seqs,
                                             int max_prefill_len, int64_t num_prefill_tokens, int cur_layer, int num_layers,
                                             int nq, int nkv, int block_size, int head_dim, int max_blocks_per_seq,
-                                            int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, sllm_stream_t stream) {
+                                            int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, sllm_stream_t stream,
+                                   int num_splits, void* workspace) {
     SLLM_REQUIRE(num_prefill_seqs >= 0 && max_prefill_len >= 0, "prefill_attention_paged: negative sizes");
     if (num_prefill_seqs == 0 || max_prefill_len == 0) return 0;
     SLLM_REQUIRE(q && k_cache && v_cache && o && block_table && seq_ids && prefill_seq_start_locs && prefill_seq_lens &&
@@ -85,7 +116,10 @@ extern "C" int sllm_prefill_attention_paged(const void* q, const void* k_cache, 
     const int gen = (gen_env && gen_env[0] == '1') ? 1 : (gen_env && gen_env[0] == '2') ? 2 : 0;
     const int64_t cache_rows = num_blocks * num_layers * nkv * block_size;
     if (gen != 1 && dtype <= SLLM_BF16 && tc_prefill_paged_supported(head_dim, block_size, num_prefill_tokens, cache_rows)) {
-        PtPaged pg{block_table, seq_ids, prefill_prefix_lens, cur_layer, num_layers, max_blocks_per_seq};
+        PtPaged pg{block_table, seq_ids, prefill_prefix_lens, cur_layer, num_layers, max_blocks_per_seq, 1, num_prefill_tokens, nullptr, nullptr};
+        if (num_splits > 1 && workspace != nullptr && (int64_t)num_prefill_seqs * num_splits <= 65535) {
+            pg.nsplit = num_splits; pg.part_o = (float*)workspace; pg.part_ml = pg.part_o + (int64_t)num_splits * num_prefill_tokens * nq * PT_D;
+        }
         return launch_prefill_paged_tc(q, k_cache, v_cache, o, prefill_seq_start_locs, prefill_seq_lens,
                                        softmax_scale * 1.4426950408889634f, num_prefill_seqs, max_prefill_len, num_prefill_tokens,
                                        nq, nkv, q_row_stride, cache_rows, pg, dtype, st);
@@ -95,4 +129,34 @@ extern "C" int sllm_prefill_attention_paged(const void* q, const void* k_cache, 
     if (head_dim == 128) { SLLM_DISPATCH_DTYPE(dtype, return (launch_prefill_paged<T, 128>(q, k_cache, v_cache, o, prefill_seq_start_locs, prefill_seq_lens, softmax_scale, num_prefill_seqs, max_prefill_len, nq, nkv, q_row_stride, pk, st))); }
     else { SLLM_DISPATCH_DTYPE(dtype, return (launch_prefill_paged<T, 64>(q, k_cache, v_cache, o, prefill_seq_start_locs, prefill_seq_lens, softmax_scale, num_prefill_seqs, max_prefill_len, nq, nkv, q_row_stride, pk, st))); }
     return 0;
+}
+
+extern "C" int sllm_prefill_attention_paged(
+    const void* q, const void* k_cache, const void* v_cache, void* o,
+    const int32_t* block_table, const int32_t* seq_ids,
+    const int32_t* prefill_seq_start_locs, const int32_t* prefill_seq_lens,
+    const int32_t* prefill_prefix_lens, float softmax_scale, int num_prefill_seqs,
+    int max_prefill_len, int64_t num_prefill_tokens, int cur_layer, int num_layers,
+    int nq, int nkv, int block_size, int head_dim, int max_blocks_per_seq,
+    int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, sllm_stream_t stream) {
+    return prefill_attention_paged(q, k_cache, v_cache, o, block_table, seq_ids, prefill_seq_start_locs, prefill_seq_lens,
+                                   prefill_prefix_lens, softmax_scale, num_prefill_seqs, max_prefill_len, num_prefill_tokens,
+                                   cur_layer, num_layers, nq, nkv, block_size, head_dim, max_blocks_per_seq, num_blocks,
+                                   q_row_stride, dtype, stream, 1, nullptr);
+}
+
+extern "C" int sllm_prefill_attention_paged_split(
+    const void* q, const void* k_cache, const void* v_cache, void* o,
+    const int32_t* block_table, const int32_t* seq_ids,
+    const int32_t* prefill_seq_start_locs, const int32_t* prefill_seq_lens,
+    const int32_t* prefill_prefix_lens, float softmax_scale, int num_prefill_seqs,
+    int max_prefill_len, int64_t num_prefill_tokens, int cur_layer, int num_layers,
+    int nq, int nkv, int block_size, int head_dim, int max_blocks_per_seq,
+    int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, sllm_stream_t stream,
+    int num_splits, void* workspace) {
+    SLLM_REQUIRE(num_splits >= 1 && num_splits <= 64, "prefill_attention_paged: 1 <= splits <= 64 (got %d)", num_splits);
+    return prefill_attention_paged(q, k_cache, v_cache, o, block_table, seq_ids, prefill_seq_start_locs, prefill_seq_lens,
+                                   prefill_prefix_lens, softmax_scale, num_prefill_seqs, max_prefill_len, num_prefill_tokens,
+                                   cur_layer, num_layers, nq, nkv, block_size, head_dim, max_blocks_per_seq, num_blocks,
+                                   q_row_stride, dtype, stream, num_splits, workspace);
 }

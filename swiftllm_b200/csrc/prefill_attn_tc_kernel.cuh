@@ -60,6 +60,10 @@ struct PtParams {
 struct PtPaged {
     const int32_t* block_table; const int32_t* seq_ids; const int32_t* prefix_lens;
     int cur_layer, num_layers, max_blocks_per_seq;
+    // key splits (steps with few query blocks): blockIdx.z = sequence * nsplit + split; nsplit > 1 leaves fp32 rows of unnormalised O
+    // [nsplit, tokens, nq, 128] and their (reference maximum in base 2, sum) [nsplit, tokens, nq, 2] for prefill_merge_kernel
+    int nsplit; int64_t num_tokens;
+    float* part_o; float* part_ml;
 };
 constexpr int PT_PAGE = 16;               // tokens per KV page (PAGED only)
 
@@ -83,7 +87,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int qblk = gridDim.x - 1 - blockIdx.x;                // latest (heaviest) query blocks first
-    const int head = blockIdx.y, seq = blockIdx.z;
+    const int nsplit = PAGED ? pg.nsplit : 1;
+    const int head = blockIdx.y, seq = PAGED ? blockIdx.z / nsplit : blockIdx.z, split = PAGED ? blockIdx.z - seq * nsplit : 0;
     const int len = p.seq_lens[seq];                            // query rows of this sequence in the batch
     const int q0 = qblk * 2 * PT_BQ;
     if (q0 >= len) return;
@@ -93,8 +98,16 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     const int kvlen = pre + len;
     const bool active_b = q0 + PT_BQ < len;
     const int end_a = min(kvlen, pre + q0 + PT_BQ), end_b = active_b ? min(kvlen, pre + q0 + 2 * PT_BQ) : 0;      // keys a tile can see
-    const int nkt_a = (end_a + PT_BK - 1) / PT_BK, nkt_b = (end_b + PT_BK - 1) / PT_BK;      // kv steps a tile takes part in
+    const int all_a = (end_a + PT_BK - 1) / PT_BK, all_b = (end_b + PT_BK - 1) / PT_BK;      // kv steps a tile takes part in
+    // this CTA's steps of them: j0 .. (all of them without splits); the loops below count from j0
+    const int per = PAGED ? (max(all_a, all_b) + nsplit - 1) / nsplit : 0, j0 = split * per;
+    const int nkt_a = PAGED ? min(max(all_a - j0, 0), per) : all_a, nkt_b = PAGED ? min(max(all_b - j0, 0), per) : all_b;
     const int nkt = max(nkt_a, nkt_b);
+    if (PAGED && nkt == 0) {                                    // a split past the last key: nothing to add
+        if (q0 + tid < len && tid < 2 * PT_BQ)
+            *reinterpret_cast<float2*>(pg.part_ml + 2 * (((int64_t)split * pg.num_tokens + tok0 + q0 + tid) * p.nq + head)) = make_float2(-INFINITY, 0.f);
+        return;
+    }
 
     if constexpr (PAGED) {
         // page slots that a tail step never loads must hold finite data (their P columns are exactly 0)
@@ -131,13 +144,13 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             const int32_t* bt = pg.block_table + (int64_t)pg.seq_ids[seq] * pg.max_blocks_per_seq;
             const int npages = (kvlen + PT_PAGE - 1) / PT_PAGE;
             constexpr int PPS = PT_BK / PT_PAGE;                  // pages per step
-            int nxt = (lane < PPS && lane < npages) ? bt[lane] : 0;
+            int nxt = (lane < PPS && j0 * PPS + lane < npages) ? bt[j0 * PPS + lane] : 0;
             for (int j = 0; j < nkt; j++) {
                 const int st = j % PT_STAGES;
                 const int blk = nxt;
-                const int npg = (j + 1) * PPS + lane;
+                const int npg = (j0 + j + 1) * PPS + lane;
                 nxt = (j + 1 < nkt && lane < PPS && npg < npages) ? bt[npg] : 0;
-                const int valid = min(PPS, npages - j * PPS);      // >= 1: step j exists because page 5j does
+                const int valid = min(PPS, npages - (j0 + j) * PPS);      // >= 1: step j exists because page 5j does
                 const uint32_t bar = smem_u32(&full[st]);
                 if (lane == 0) {
                     mbar_wait(smem_u32(&empty[st]), ((j / PT_STAGES) & 1) ^ 1);
@@ -221,7 +234,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                     mbar_wait(smem_u32(&bars->p_full[x]), j & 1);
                     tc_fence_after();
                     // O_X += P_X(j) V(j): 16 tokens per UMMA, none past the last key the tile can see
-                    const int steps = min(PT_BK / 16, (end - j * PT_BK + 15) / 16);
+                    const int steps = min(PT_BK / 16, (end - (j0 + j) * PT_BK + 15) / 16);
                     const uint64_t vd = dv0 + (uint64_t)((st * PT_KV_BYTES) >> 4);
                     if (elect_one()) {
 #pragma unroll
@@ -232,7 +245,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                     }
                     __syncwarp();
                 }
-                // steps the other tile still takes: hand the stages on once they have been filled (never a phase ahead)
+            }
+            // steps that only the other tile takes: hand the stages on once they have been filled (never a phase ahead)
+            if (x == 0 || active_b) {
                 for (int j = nkx; j < nkt; j++) {
                     const int st = j % PT_STAGES;
                     mbar_wait(smem_u32(&bars->k_full[st]), (j / PT_STAGES) & 1);
@@ -267,7 +282,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             tc_fence_before();
             mbar_arrive(smem_u32(&bars->s_empty[x]));
 
-            const int c0 = j * PT_BK;
+            const int c0 = (j0 + j) * PT_BK;
             if (c0 + PT_BK - 1 > pre + q0 + x * PT_BQ || c0 + PT_BK > kvlen) {
                 // column c0+i is visible iff c0+i <= pre+qi and c0+i < kvlen  <=>  i <= lim   (branch-free selects)
                 const int lim = min(pre + qi, kvlen - 1) - c0;
@@ -302,7 +317,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             if (need) m_ref = m_new;
             // p = exp2(s*c - m_ref) (<= 2^8), row sum in fp32, P row into TMEM (two keys per column)
             float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            const float2 neg_m = make_float2(-m_ref, -m_ref), c2 = make_float2(c, c);
+            const float sub = PAGED && m_ref == -INFINITY ? 0.f : -m_ref;      // (a split whose keys so far are all behind the row)
+            const float2 neg_m = make_float2(sub, sub), c2 = make_float2(c, c);
             uint32_t w[PT_BK / 2];
 #pragma unroll
             for (int i = 0; i < PT_BK / 2; i++) {
@@ -320,7 +336,24 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             mbar_arrive(smem_u32(&bars->p_full[x]));
             l += (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y);
         }
-        if (nk_mine > 0) {
+        if (PAGED && nsplit > 1) {
+            // ---- a split's part of the row
+            const int64_t at = ((int64_t)split * pg.num_tokens + tok0 + qi) * p.nq + head;
+            if (nk_mine > 0) { mbar_wait(smem_u32(&bars->p_empty[x]), (nk_mine - 1) & 1); tc_fence_after(); }
+            if (qi < len) *reinterpret_cast<float2*>(pg.part_ml + 2 * at) = make_float2(m_ref, l);
+#pragma unroll 1
+            for (int cc = 0; cc < 4 && nk_mine > 0; cc++) {
+                uint32_t t[32];
+                tmem_ld32(o_addr + cc * 32, t);
+                tmem_ld_wait();
+                if (qi < len) {
+#pragma unroll
+                    for (int v = 0; v < 32; v += 4)
+                        *reinterpret_cast<uint4*>(pg.part_o + at * PT_D + cc * 32 + v) = make_uint4(t[v], t[v + 1], t[v + 2], t[v + 3]);
+                }
+                __syncwarp();
+            }
+        } else if (nk_mine > 0) {
             // ---- epilogue: O / l -> global (row qi of this head), only rows inside the sequence
             mbar_wait(smem_u32(&bars->p_empty[x]), (nk_mine - 1) & 1);          // the last P . V
             tc_fence_after();

@@ -29,6 +29,19 @@ def prefill_attention(
         _lib.dtype_tag(q.dtype), _lib.stream()), "prefill_attention")
 
 
+_SM_COUNT = {}
+
+
+def _key_splits(heads: int, longest: int, kv_len: int) -> int:
+    """CTAs that share a query block's keys: as many as keep one CTA (256 query rows of a head) per SM when the portions alone leave SMs
+    idle, each with at least eight steps of 80 keys (shorter ones do not pay for the merge)."""
+    dev = torch.cuda.current_device()
+    if dev not in _SM_COUNT:
+        _SM_COUNT[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+    blocks = heads * -(-longest // 256)
+    return max(1, min(_SM_COUNT[dev] // max(1, blocks), kv_len // 640, 16))
+
+
 def prefill_attention_paged(
     q: torch.Tensor,            # [num_prefill_tokens, num_q_heads, head_dim]  (the chunks' queries, packed)
     k_cache: torch.Tensor,      # [num_blocks, num_layers, num_kv_heads, block_size, head_dim]
@@ -53,9 +66,12 @@ def prefill_attention_paged(
     if infer_state.num_prefill_seqs == 0:
         return
     num_blocks, num_layers, nkv, bs, _ = k_cache.shape
-    _lib.check(_lib.lib().sllm_prefill_attention_paged(
+    nsplit = _key_splits(nq * infer_state.num_prefill_seqs, infer_state.max_prefill_len, getattr(infer_state, "max_prefill_kv_len", 0)) \
+        if D == 128 and bs == 16 else 1
+    ws = torch.empty((nsplit * Tp * nq * (D + 2),), dtype=torch.float32, device=q.device) if nsplit > 1 else None
+    _lib.check(_lib.lib().sllm_prefill_attention_paged_split(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr(), block_table.data_ptr(),
         infer_state.seq_ids.data_ptr(), infer_state.prefill_seq_start_locs.data_ptr(), infer_state.prefill_seq_lens.data_ptr(),
         prefix.data_ptr(), infer_state.softmax_scale, infer_state.num_prefill_seqs, infer_state.max_prefill_len, Tp,
         cur_layer, num_layers, nq, nkv, bs, D, block_table.shape[1], num_blocks, qs,
-        _lib.dtype_tag(q.dtype), _lib.stream()), "prefill_attention_paged")
+        _lib.dtype_tag(q.dtype), _lib.stream(), nsplit, _lib.ptr(ws)), "prefill_attention_paged")
