@@ -345,29 +345,44 @@ __global__ void __launch_bounds__(LM_NW * 32) latent_attn_mma_kernel(
     }
 }
 
-// One warp per (token, head): merge the key splits.  partial [T, H, nsplit, r + 2] = (sum_j e^(s_j - m) c_j, m, sum_j e^(s_j - m));
-// a split that saw no key has m = -inf and contributes nothing.
+// One CTA per (token, head): merge the key splits (at most 64).  partial [T, H, nsplit, r + 2] = (sum_j e^(s_j - m) c_j, m, sum_j e^(s_j - m));
+// a split that saw no key has m = -inf and is not read.  Every warp weighs the splits by itself (lane = split), then a thread adds two
+// neighbouring columns of all of them, four splits' loads in flight.  With a warp per (token, head) that took the weights anew for every
+// column, sixteen splits of one token took 11 to 45 us (most of it waiting for the weights); now 4.
 template <typename T>
 __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* __restrict__ partial, const T* __restrict__ gate,
                                                                   int64_t gate_stride_t, T* __restrict__ out, int64_t out_stride_t,
-                                                                  int64_t out_stride_h, int64_t num_tokens, int H, int r, int nsplit) {
+                                                                  int64_t out_stride_h, int H, int r, int nsplit) {
     const int lane = threadIdx.x & 31;
-    const int64_t idx = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (idx >= num_tokens * H) return;
-    const int64_t t = idx / H;
+    const int64_t idx = blockIdx.x, t = idx / H;
     const int h = (int)(idx - t * H);
     const float* pr = partial + idx * nsplit * (r + 2);
-    float M = -INFINITY;
-    for (int z = 0; z < nsplit; z++) M = fmaxf(M, pr[z * (r + 2) + r]);
-    float L = 0.f;
-    for (int z = 0; z < nsplit; z++) L += expf(pr[z * (r + 2) + r] - M) * pr[z * (r + 2) + r + 1];
-    float gt = 1.f;
-    if (gate != nullptr) gt = 1.f / (1.f + expf(-ldf(gate + t * gate_stride_t + h)));
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    if (lane < nsplit) { const float2 f = *reinterpret_cast<const float2*>(pr + lane * (r + 2) + r); m0 = f.x; l0 = f.y; }
+    if (lane + 32 < nsplit) { const float2 f = *reinterpret_cast<const float2*>(pr + (lane + 32) * (r + 2) + r); m1 = f.x; l1 = f.y; }
+    const float M = warp_max(fmaxf(m0, m1));
+    const float w0 = expf(m0 - M), w1 = expf(m1 - M);
+    float f = 1.f / warp_sum(w0 * l0 + w1 * l1);
+    if (gate != nullptr) f *= 1.f / (1.f + expf(-ldf(gate + t * gate_stride_t + h)));
     T* o = out + t * out_stride_t + (int64_t)h * out_stride_h;
-    for (int d = lane; d < r; d += 32) {
-        float a = 0.f;
-        for (int z = 0; z < nsplit; z++) a += expf(pr[z * (r + 2) + r] - M) * pr[z * (r + 2) + d];
-        stf(o + d, a / L * gt);
+    const int turns = (r + 2 * blockDim.x - 1) / (2 * blockDim.x);
+    for (int i = 0; i < turns; i++) {
+        const int d = 2 * (threadIdx.x + i * blockDim.x);
+        float2 a = make_float2(0.f, 0.f);
+        for (int z = 0; z < nsplit; z += 4) {
+            float2 v[4];
+            float w[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float wa = __shfl_sync(0xffffffffu, w0, (z + u) & 31), wb = __shfl_sync(0xffffffffu, w1, (z + u) & 31);
+                w[u] = z + u >= nsplit ? 0.f : z + u < 32 ? wa : wb;
+                v[u] = make_float2(0.f, 0.f);
+                if (w[u] != 0.f && d < r) v[u] = *reinterpret_cast<const float2*>(pr + (z + u) * (r + 2) + d);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) { a.x += w[u] * v[u].x; a.y += w[u] * v[u].y; }
+        }
+        if (d < r) { stf(o + d, a.x * f); stf(o + d + 1, a.y * f); }
     }
 }
 
@@ -395,8 +410,8 @@ static int launch_latent_attn_mma(const void* q_lat, int64_t ql_st, int64_t ql_s
         (const float*)sink);
     if (int rc = check_launch("latent_attention (mma)")) return rc;
     if (nsplit > 1) {
-        latent_attn_combine_kernel<T><<<(unsigned)cdiv(num_tokens * H, 4), 128, 0, stream>>>(
-            (const float*)partial, (const T*)gate, gate_st, (T*)out, out_st, out_sh, num_tokens, H, r, nsplit);
+        latent_attn_combine_kernel<T><<<(unsigned)(num_tokens * H), 128, 0, stream>>>(
+            (const float*)partial, (const T*)gate, gate_st, (T*)out, out_st, out_sh, H, r, nsplit);
         return check_launch("latent_attention (combine)");
     }
     return 0;
@@ -507,8 +522,8 @@ static int latent_attention(bool portions, const void* q_lat, int64_t q_lat_stri
         a.out_vec = ((uintptr_t)out & 15) == 0 && out_stride_t % 8 == 0 && out_stride_h % 8 == 0;
         if (int rc = launch_latent_attn_tc(a, portions, dtype, (cudaStream_t)stream)) return rc;
         if (a.nsplit > 1)
-            SLLM_DISPATCH_DTYPE(dtype, (latent_attn_combine_kernel<T><<<(unsigned)cdiv(num_tokens * num_heads, 4), 128, 0, (cudaStream_t)stream>>>(
-                a.partial, (const T*)gate, gate_stride_t, (T*)out, out_stride_t, out_stride_h, num_tokens, num_heads, r, a.nsplit)));
+            SLLM_DISPATCH_DTYPE(dtype, (latent_attn_combine_kernel<T><<<(unsigned)(num_tokens * num_heads), 128, 0, (cudaStream_t)stream>>>(
+                a.partial, (const T*)gate, gate_stride_t, (T*)out, out_stride_t, out_stride_h, num_heads, r, a.nsplit)));
         return check_launch("latent_attention (combine)");
     }
     const size_t mma_smem = ((size_t)(16 + LM_KT) * (r + dr + 8) + 16 * (LM_KT + 8)) * 2 + (16 * (LM_KT + 1) + 48) * sizeof(float);

@@ -55,18 +55,21 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, gate, cache: torc
     assert sink is None or (sink.dtype == torch.float32 and sink.shape == (H,) and sink.is_contiguous())
     _lib.require_device(q_lat)
     npre = min(T, max(0, int(getattr(infer_state, "num_prefill_tokens", 0))))
-    lib, ts, tp = _lib.lib(), infer_state.token_seq_ids, infer_state.token_positions
-    for first, rows, portions in ((0, npre, True), (npre, T - npre, False)):
+    lib, es = _lib.lib(), q_lat.element_size()
+    (ql_t, ql_h, _), (qr_t, qr_h, _), (o_t, o_h, _) = q_lat.stride(), q_rot.stride(), out.stride()
+    gate_t = gate.stride(0) if gate is not None else 0
+    half = rot_dims // 2 * 4
+    ql, qr, o, g, c, sn = q_lat.data_ptr(), q_rot.data_ptr(), out.data_ptr(), _lib.ptr(gate), _lib.ptr(cos), _lib.ptr(sin)
+    ts, tp = infer_state.token_seq_ids.data_ptr(), infer_state.token_positions.data_ptr()
+    _, n_slots, bs, _ = cache.shape
+    dtype, stream = _lib.dtype_tag_f32(q_lat.dtype), _lib.stream()
+    for i, rows, portions in ((0, npre, True), (npre, T - npre, False)):       # i: the part's first row
         if rows == 0:
             continue
         nsplit = _num_splits(rows, H, r, dr, window, q_lat.dtype, portions)
         ws = torch.empty((rows, H, nsplit, r + 2), dtype=torch.float32, device=q_lat.device) if nsplit > 1 else None
-
-        def at(x):                                                     # the part's first row
-            return None if x is None else x.data_ptr() + first * x.stride(0) * x.element_size()
         _lib.check((lib.sllm_latent_attention_portions if portions else lib.sllm_latent_attention)(
-            at(q_lat), q_lat.stride(0), q_lat.stride(1), at(q_rot), q_rot.stride(0), q_rot.stride(1),
-            at(cos), at(sin), at(gate), gate.stride(0) if gate is not None else 0,
-            cache.data_ptr(), cache.shape[1], slot, cache.shape[2], block_table.data_ptr(), block_table.shape[1],
-            at(ts), at(tp), at(out), out.stride(0), out.stride(1), rows, H, r, dr, rot_dims, window, scale, _lib.ptr(sink), nsplit,
-            _lib.ptr(ws), _lib.dtype_tag_f32(q_lat.dtype), _lib.stream()), "latent_attention")
+            ql + i * ql_t * es, ql_t, ql_h, qr + i * qr_t * es, qr_t, qr_h, c + i * half if c else None, sn + i * half if sn else None,
+            g + i * gate_t * es if g else None, gate_t, cache.data_ptr(), n_slots, slot, bs, block_table.data_ptr(), block_table.shape[1],
+            ts + 4 * i, tp + 4 * i, o + i * o_t * es, o_t, o_h, rows, H, r, dr, rot_dims, window, scale, _lib.ptr(sink), nsplit,
+            _lib.ptr(ws), dtype, stream), "latent_attention")
