@@ -9,7 +9,7 @@
 // Accumulators and P stay in TMEM: an M = 64 operand fills 16 of every 32 lanes, so the two halves of O lie in the same 256 columns (lane
 // offsets 0 and 16); P (16-bit, two buffers) is written to both lane offsets, because an A operand lies in its accumulator's lanes; S has
 // two buffers beside them.  The reference of the exponentials is the running maximum itself: a reference that trails it (by up to 2^8, say)
-// would save most rescales of O (486 instead of 530 us below), but then the largest weight is not 1 and takes a rounding as well,
+// would save most rescales of O (490 instead of 580 us below), but then the largest weight is not 1 and takes a rounding as well,
 // 2.15e-3 instead of 2.01e-3 off 64-bit arithmetic in bf16.
 //
 // Shared memory is what decides the shape: 64 rows of Q (576 entries: 72 KiB) and two stages of 64 keys (72 KiB each) fill it.  A stage
@@ -19,8 +19,8 @@
 //
 // Bound: at M = 64 the tensor core runs at half rate, (D + r) * 64 * 64 multiply-adds per tile = 2176 cycles at D = 576, r = 512, and
 // S's operands are 4 KiB of shared memory per 32 cycles; a decoded token is bound by its rows' bytes.  Measured on B200, bf16, 16 heads,
-// r = 512: four prompts of 2048 tokens 3217 us with the mma.sync kernel of latent_attn.cu -> 486 us (600 TFLOP/s); 64 decoded tokens at
-// 2048 keys 95 -> 63 us.
+// r = 512: four prompts of 2048 tokens 3217 us with the mma.sync kernel of latent_attn.cu -> 580 us (504 TFLOP/s); 64 decoded tokens at
+// 2048 keys 95 -> 67 us.
 #include "latent_attn_tc.cuh"
 #include "mma_helpers.cuh"
 #include "tc_helpers.cuh"
@@ -447,16 +447,11 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 tc_fence_after();
             }
 #pragma unroll 1
-            for (int cc = 0; cc < n0; cc += 32) {
+            for (int cc = 0; cc < n0 && ntiles > 0; cc += 32) {      // (a split without keys leaves its sums alone: m = -inf is not read)
                 uint32_t v[32];
                 __syncwarp();
-                if (ntiles > 0) {
-                    tmem_ld32(tlane + cc, v);
-                    tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 32; e++) v[e] = 0u;
-                }
+                tmem_ld32(tlane + cc, v);
+                tmem_ld_wait();
                 if (live && cc < cols) {
                     if (p.nsplit > 1) {
 #pragma unroll
