@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TI* __restrict__ 
 // The same for prompt rows where rows are whole pieces of four channels: a thread walks SV_TOKENS rows of four neighbouring channels, eight
 // rows' loads in flight together (wider pieces need 154 registers and leave ten warps on an SM: 96 us); where the rows of the tile break (another sequence) is found once per warp.  The products,
 // their order and the SiLU are those above (a quicker quotient turns some roundings, which a state behind the convolution keeps).  Bound: bytes, of which enough
-// are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 -> 59 us (2.3 TB/s).
+// are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 -> about 80 us (59 with a quicker quotient).
 constexpr int SV_TOKENS = 16;
 template <typename TI, typename TO, int K>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restrict__ xin, int64_t xin_stride, const float* __restrict__ w,
