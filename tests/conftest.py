@@ -18,8 +18,8 @@ def pytest_configure(config):
 
 
 def pytest_collection_modifyitems(config, items):
-    """Tests of kernels that have never run on a GPU must not be able to turn the validated suite red (the driver runs
-    `-m gpu -x`).  They are opted into with SLLM_RUN_PENDING=1 (scripts/gpu_validate_pending.sh) and lose the marker once
+    """Tests of kernels that have never run on a GPU must not be able to turn the validated suite red (it runs with
+    `-m gpu -x`).  They are opted into with SLLM_RUN_PENDING=1 and lose the marker once
     they have passed on a B200."""
     import torch
     lib_built = os.path.exists(os.path.join(ROOT, "swiftllm_b200", "libswiftllm_b200.so"))
