@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                 for (int e = 0; e < 8; e++) f[e] = softplus_fn(cvt_f(rd[e]) + vbias[e]);
                 put(ds + at, f);
 #pragma unroll
-                for (int e = 0; e < 8; e++) { const float g = cvt_f(rz[e]); f[e] = __fdividef(g, 1.f + __expf(-g)); }
+                for (int e = 0; e < 8; e++) f[e] = silu_fn(cvt_f(rz[e]));
                 put(zs + at, f);
             }
             auto stage_bc = [&](const T* from, int j, int k, bool of_c) {
