@@ -17,6 +17,10 @@
 // half of O, the rest after the second; producer warps gather each piece through the block table by cp.async (rows past the last
 // visible key are zero).
 //
+// A weight of exactly 0 times a key row that is not finite is NaN, so a key that one row of a pass sees and another does not may reach both.
+// Key and value are one row: a masked score that is not finite gives such a key away, and the segment is then done over, token by token,
+// with the keys that the token does not see left zero (same tiles, same key splits).  A result depends on its own keys only.
+//
 // Bound: at M = 64 the tensor core runs at half rate, (D + r) * 64 * 64 multiply-adds per tile = 2176 cycles at D = 576, r = 512, and
 // S's operands are 4 KiB of shared memory per 32 cycles; a decoded token is bound by its rows' bytes.  Measured on B200, bf16, 16 heads,
 // r = 512: four prompts of 2048 tokens 3217 us with the mma.sync kernel of latent_attn.cu -> 580 us (504 TFLOP/s); 64 decoded tokens at
@@ -73,6 +77,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     uint8_t* k_sm = smem + LT_STAGE;                 // [stage][chunk][64 keys][128 B]
     LatentTcBars* bars = reinterpret_cast<LatentTcBars*>(smem + 3 * LT_STAGE);
     uint32_t* tmem_s = reinterpret_cast<uint32_t*>(smem + 3 * LT_STAGE + 512);
+    volatile int* tainted = reinterpret_cast<int*>(tmem_s + 1);      // the last pass over a segment that met such a key
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r = FULL ? 512 : p.r, dr = FULL ? 64 : p.dr, D = r + dr;
     const int n0 = r < 256 ? r : 256, n1 = r - n0;   // columns of O in its two halves
@@ -82,6 +87,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     const int ntok = min(p.qt, p.num_tokens - t_first);
 
     if (tid == 0) {
+        *tainted = 0;
         for (int s = 0; s < 2; s++) {
             for (int g = 0; g < 2; g++) { mbar_init(smem_u32(&bars->full[s][g]), LT_PW); mbar_init(smem_u32(&bars->empty[s][g]), 1); }
             mbar_init(smem_u32(&bars->s_full[s]), 1); mbar_init(smem_u32(&bars->s_empty[s]), 128);
@@ -95,8 +101,10 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     tc_fence_after();
     const uint32_t tmem = *tmem_s;
 
-    int n_done = 0;                                  // tiles of the segments before: every barrier's phase follows from it
+    int n_done = 0;                                  // tiles of the passes before: every barrier's phase follows from it
+    int pass = 0, solo = -1;                         // solo >= 0: the pass is for this token of the segment alone
     for (int i0 = 0; i0 < ntok;) {
+        pass++;
         // ---- the segment: tokens ts .. ts + n - 1 of one sequence at positions pos0 ..; its keys lo .. hi, this CTA's tiles of them
         const int ts = t_first + i0, left = ntok - i0;
         int n, seq, pos0;
@@ -114,13 +122,15 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
         const int all = (hi - lo) / LT_KEYS + 1, per = (all + p.nsplit - 1) / p.nsplit;
         const int tile0 = min(all, (int)blockIdx.z * per), ntiles = min(all, tile0 + per) - tile0;
         const int key0 = lo + tile0 * LT_KEYS;
+        const int see_hi = solo < 0 ? hi : pos0 + solo;                        // keys outside are left zero
+        const int see_lo = solo < 0 || p.window <= 0 ? lo : max(lo, pos0 + solo - p.window + 1);
 
         // producers: piece g of every tile, rows r0 .. r0 + 64 / LT_PW - 1; eight lanes a 128-byte row piece
         const bool producer = warp >= 4 && warp < LT_MMA_WARP;
         const int g = (warp - 4) / LT_PW, r0 = (64 / LT_PW) * ((warp - 4) % LT_PW), piece = lane & 7;
-        auto key_row = [&](int j) {                  // cache row of key r0 + lane of tile j, -1 past the last visible one
+        auto key_row = [&](int j) {                  // cache row of key r0 + lane of tile j, -1 for one that is not visible
             const int kp = key0 + j * LT_KEYS + r0 + lane;
-            if (lane >= 64 / LT_PW || kp > hi) return -1ll;
+            if (lane >= 64 / LT_PW || kp > see_hi || kp < see_lo) return -1ll;
             const int b = kp / p.block_size;
             return ((long long)bt[b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size);
         };
@@ -348,6 +358,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             const uint32_t tlane = tmem + ((uint32_t)(32 * warp) << 16);
             // the row whose part of O this lane owns (lanes 16.. : its second half), and the lane that holds the row's state
             const int orow = lane & 15, from = 4 * (orow & 7);
+            uint32_t top_a = 0, top_b = 0;           // the largest magnitude (as bits) among the masked scores
             for (int j = 0; j < ntiles; j++) {
                 const int it = n_done + j, st = it & 1;
                 mbar_wait(smem_u32(&bars->s_full[st]), (it >> 1) & 1);
@@ -365,8 +376,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
                             const int kp = cb + 8 * i + e;
-                            if (kp > last_a || kp < first_a) s[4 * i + e] = 0xff800000u;
-                            if (kp > last_b || kp < first_b) s[4 * i + 2 + e] = 0xff800000u;
+                            if (kp > last_a || kp < first_a) { top_a = max(top_a, s[4 * i + e] & 0x7fffffffu); s[4 * i + e] = 0xff800000u; }
+                            if (kp > last_b || kp < first_b) { top_b = max(top_b, s[4 * i + 2 + e] & 0x7fffffffu); s[4 * i + 2 + e] = 0xff800000u; }
                         }
                 }
                 float xa = -INFINITY, xb = -INFINITY;
@@ -421,14 +432,17 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 tc_fence_before();
                 mbar_arrive(smem_u32(&bars->p_full[st]));
             }
+            // a row whose sum is NaN is NaN by its own keys
+            const bool odd_a = live_a && top_a >= 0x7f800000u, odd_b = live_b && top_b >= 0x7f800000u;
             // ---- output: the lane owns row orow, columns n0 * (lane / 16) ..
             la += __shfl_xor_sync(0xffffffffu, la, 1); la += __shfl_xor_sync(0xffffffffu, la, 2);
             lb += __shfl_xor_sync(0xffffffffu, lb, 1); lb += __shfl_xor_sync(0xffffffffu, lb, 2);
             const float l0 = __shfl_sync(0xffffffffu, la, from), l1 = __shfl_sync(0xffffffffu, lb, from);
             const float m0 = __shfl_sync(0xffffffffu, ma, from), m1 = __shfl_sync(0xffffffffu, mb, from);
             const float l = orow < 8 ? l0 : l1, m = orow < 8 ? m0 : m1;
+            if (solo < 0 && n > 1 && ((odd_a && la == la) || (odd_b && lb == lb))) *tainted = pass;
             const int row = 16 * warp + orow, jj = row >> p.hp_log2, h = h0 + (row & (hp - 1));
-            const bool live = jj < n && h < p.H;
+            const bool live = jj < n && h < p.H && (solo < 0 || jj == solo);
             const int64_t t = ts + jj;
             const int col0 = lane < 16 ? 0 : n0, cols = lane < 16 ? n0 : n1;
             float f = 0.f;
@@ -477,6 +491,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
         __syncthreads();                             // the next segment overwrites the queries; its first products overwrite O
         tc_fence_after();
         n_done += ntiles;
+        if ((solo >= 0 || *tainted == pass) && ++solo < n) continue;
+        solo = -1;
         i0 += n;
     }
     if (warp == LT_MMA_WARP) tmem_dealloc<512>(tmem);

@@ -28,3 +28,38 @@ def test_selective_scan_gate_is_the_plain_one(dtype, C, N):
         outs.append(selective_scan(torch.ones(T, C, dtype=dtype, device=DEV), dt, one, A, zero, 0, N, one, gate,
                                    torch.zeros(st.batch_size, C, N, device=DEV), st))
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+# ---------------------------------------------------------------- keys that are not finite reach nobody who does not see them
+def _poisoned(c, spots, cols, value):
+    """The case's cache with `value` in columns `cols` of the rows of (sequence, position)s."""
+    cache = c.cache.clone()
+    bs = cache.shape[2]
+    for s, p in spots:
+        cache[int(c.bt[s, p // bs]), :, p % bs, cols] = value
+    return cache
+
+
+def _sees(c, spots, keep=0, chunk=0):
+    """[rows] whether a row sees one of the (sequence, position)s."""
+    out = []
+    for s, (n, first) in enumerate(c.rows):
+        for q in range(first, first + n):
+            out.append(any(s == t and p <= q and (c.window <= 0 or q - p < c.window or p < keep) and (chunk <= 0 or p >= q // chunk * chunk)
+                           for t, p in spots))
+    return torch.tensor(out, device=DEV)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H,r,dr,window,portions", [
+    (16, 512, 64, 0, [(130, 5), (7, 90)]), (16, 512, 64, 33, [(130, 5), (7, 90)]), (1, 64, 16, 0, [(130, 0), (64, 3)]),
+    (5, 192, 48, 20, [(100, 0)]), (16, 512, 64, 0, [(1200, 0)])])
+def test_latent_keys_reach_only_rows_that_see_them(dtype, value, H, r, dr, window, portions):
+    c = latent_case(dtype, portions, [77, 0], H, r, dr, dr, window, sink=True)
+    spots = [(0, 43), (0, 66), (0, portions[0][0] - 2)]
+    clean, got = latent_run(c), latent_run(c, _poisoned(c, spots, [3, r - 1], value))
+    sees = _sees(c, spots)
+    # a row that does not see the key: the same tiles, the same splits, zeros in place of a key with the weight 0
+    assert torch.equal(got[~sees], clean[~sees])
+    assert bool((~torch.isfinite(got[sees])).flatten(1).any(1).all())
