@@ -13,6 +13,9 @@
 //                largest weight is then not 1 and takes a rounding as well: 2.38e-3 instead of 2.33e-3 off 64 bits in bf16)
 // TMEM: S_A 0..79, S_B 80..159, P_A 160..199, P_B 200..239, O_A 256..383, O_B 384..511 (the layout of the prefill kernel: 80 keys are the
 // most that leave scores and P places of their own).
+// A weight of exactly 0 times a value that is not finite is NaN, so a key that one row of a pass sees and another does not may reach both.
+// Where a row's sum of weights is finite but its O is not, and such a value is found among the keys that only some tokens of the segment
+// see, the segment is done over, token by token, with the keys that the token does not see left zero: a result depends on its own keys only.
 //
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
 // ones 317 us with the mma.sync kernel of window_attn.cu for the prompts -> 114 us (95 of them this kernel, two rounds of CTAs; a CTA's
@@ -60,7 +63,8 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
     float* inv_sm = reinterpret_cast<float*>(smem + WX_INV_OFF);
     WindowTcBars* bars = reinterpret_cast<WindowTcBars*>(smem + WX_MISC_OFF);
     uint32_t* tmem_s = reinterpret_cast<uint32_t*>(smem + WX_MISC_OFF + sizeof(WindowTcBars));
-    static_assert(sizeof(WindowTcBars) + 4 <= 256, "");
+    volatile int* tainted = reinterpret_cast<int*>(tmem_s + 1);      // [2]: the last pass in which O was not finite; ... that is done over
+    static_assert(sizeof(WindowTcBars) + 12 <= 256, "");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool shared_kv = EXT && p.shared_kv;
     const int krot = EXT && !FULL ? p.krot : 0, keep_first = EXT ? p.keep_first : 0;
@@ -70,6 +74,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
     const int ntok = min(p.qt, p.num_rows - t_first);
 
     if (tid == 0) {
+        tainted[0] = tainted[1] = 0;
         for (int s = 0; s < WX_STAGES; s++) { mbar_init(smem_u32(&bars->full[s]), 2); mbar_init(smem_u32(&bars->empty[s]), 2); }
         for (int x = 0; x < 2; x++) {
             mbar_init(smem_u32(&bars->s_full[x]), 1); mbar_init(smem_u32(&bars->s_empty[x]), 128);
@@ -111,31 +116,56 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
         s.steps_a = (s.end_a + WX_BK - 1) / WX_BK; s.steps_b = (s.end_b + WX_BK - 1) / WX_BK;
         return s;
     };
-    // steps of the segments before (of the ring, of each tile): the barriers' phases follow from them
+    // steps of the passes before (of the ring, of each tile): the barriers' phases follow from them
     int n_done = 0, done_a = 0, done_b = 0;
+    int pass = 0, solo = -1;                          // solo >= 0: the pass is for this token of the segment alone
+    const int kofs = p.koff + g * KW, vofs = p.G * dk + (g / p.vshare) * dv;       // the group's keys and values in a cache row
+    auto row_of = [&](const Segment& s, int v) {      // cache row of list entry v
+        const int kp = v < s.nk ? v : v - s.nk + s.lo;
+        const int b = kp / p.block_size;
+        return ((long long)p.block_table[(int64_t)s.seq * p.max_blocks_per_seq + b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size);
+    };
+    // what a pass ends with: true if the segment is taken once more (its end was a barrier)
+    auto again = [&](const Segment& s, bool search) {
+        if (solo < 0) {
+            if (tainted[0] != pass) return false;
+            if (search) {
+                const int all_lo = s.nk + first_seen(s.hi) - s.lo, all_hi = s.nk + s.pos0 - s.lo, total = max(s.end_a, s.end_b);
+                const T* values = reinterpret_cast<const T*>(p.cache) + (shared_kv ? kofs : vofs);
+                for (int v = vkeep + warp - 4; v < total; v += WX_THREADS / 32 - 4) {
+                    if (v >= all_lo && v <= all_hi) continue;
+                    const T* row = values + row_of(s, v) * p.row_elems;
+                    bool odd = false;
+                    for (int d = lane; d < dv; d += 32) { const float x = ldf(row + d); odd |= x - x != 0.f; }
+                    if (odd) tainted[1] = pass;
+                }
+            }
+            __syncthreads();
+            if (tainted[1] != pass) return false;
+        }
+        if (++solo < s.n) return true;
+        solo = -1;
+        return false;
+    };
     if (warp < 4) {
         reg_dec<WX_REGS_FEW>();
         for (int i0 = 0; i0 < ntok;) {
+            pass++;
             const Segment sg = segment(i0);
             const int n = sg.n, lo = sg.lo, nk = sg.nk, nsteps = max(sg.steps_a, sg.steps_b);
-            const int total = max(sg.end_a, sg.end_b);
-            const int* bt = p.block_table + (int64_t)sg.seq * p.max_blocks_per_seq;
+            // list entries that are visible: all of them, or those of one token
+            const int own = sg.pos0 + max(solo, 0), total = solo < 0 ? max(sg.end_a, sg.end_b) : nk + own - lo + 1;
+            const int hidden = solo < 0 ? 0 : nk + first_seen(own) - lo;             // entries vkeep .. hidden - 1 are not
             if (warp == 0 || warp == 2) {
                 // ======================================================= producers: keys 40 (warp / 2) .. of every step, eight lanes a 128-byte piece
                 const int r0 = 20 * warp, piece = lane & 7;
                 const T* cache = reinterpret_cast<const T*>(p.cache);
-                auto key_row = [&](int v) {               // cache row of list entry v, -1 past the last
-                    if (v >= total) return -1ll;
-                    const int kp = v < nk ? v : v - nk + lo;
-                    const int b = kp / p.block_size;
-                    return ((long long)bt[b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size);
-                };
+                auto key_row = [&](int v) { return v >= total || (v < hidden && v >= vkeep) ? -1ll : row_of(sg, v); };      // -1: not visible
                 auto signal = [&](int j) {
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bars->full[(n_done + j) % WX_STAGES]));
                 };
-                const int kofs = p.koff + g * KW, vofs = p.G * dk + (g / p.vshare) * dv;
                 long long ra = key_row(r0 + lane), rb = lane < 8 ? key_row(r0 + 32 + lane) : -1ll;
                 for (int j = 0; j < nsteps; j++) {
                     const long long a = ra, b = rb;
@@ -243,12 +273,13 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
             __syncthreads();                          // the next segment overwrites the queries; its first products overwrite O
             tc_fence_after();
             n_done += nsteps; done_a += sg.steps_a; done_b += sg.steps_b;
-            i0 += n;
+            if (!again(sg, false)) i0 += n;
         }
     } else {
         reg_inc<WX_REGS_MANY>();
         const int x = (warp - 4) >> 2, quad = warp & 3, row = quad * 32 + lane;
         for (int i0 = 0; i0 < ntok;) {
+            pass++;
             const Segment sg = segment(i0);
             const int ts = sg.ts, n = sg.n, pos0 = sg.pos0, lo = sg.lo, nk = sg.nk, nsteps = max(sg.steps_a, sg.steps_b);
             // ---- queries of both tiles, half a warp per row, eight entries a lane: (norm,) rotation, (norm) in fp32, rounded to the storage type
@@ -518,6 +549,9 @@ const bool need = m_new > m_ref;
                     f = p.out_scale / l;
                     if (EXT && p.gate_per_head && gate != nullptr) f *= 1.f / (1.f + __expf(-ldf(gate + t * p.gate_st + h)));
                 }
+                const bool stored = live && (solo < 0 || tr == solo);
+                float2 odd = make_float2(0.f, 0.f);       // NaN once an entry of O is not finite
+                auto look = [&](uint32_t a, uint32_t b) { odd = fma2(make_float2(__uint_as_float(a), __uint_as_float(b)), make_float2(0.f, 0.f), odd); };
                 const bool gated = gate != nullptr && !(EXT && p.gate_per_head);
                 const T* grow = gated ? gate + t * p.gate_st + (int64_t)h * dv : nullptr;
                 const int64_t at = t * p.out_st + (int64_t)h * dv;
@@ -568,7 +602,7 @@ const bool need = m_new > m_ref;
                     // this lane's part of row 32 quad + 4 i + lane / 8: its index in gate and out, -1 where there is nothing to store
                     auto part = [&](int i, int d0, int64_t stride) {
                         const int rr = quad * 32 + 4 * i + (lane >> 3), rt = x * tpt + (rr >> p.hqp_log2), rh = rr & (hqp - 1);
-                        return rt < n && rh < hq && d0 + 8 * l8 < dv ? (ts + rt) * stride + (int64_t)(g * hq + rh) * dv + d0 + 8 * l8 : -1ll;
+                        return rt < n && rh < hq && (solo < 0 || rt == solo) && d0 + 8 * l8 < dv ? (ts + rt) * stride + (int64_t)(g * hq + rh) * dv + d0 + 8 * l8 : -1ll;
                     };
                     for (int d0 = 0; d0 < dv; d0 += 64) {
                         Vec8<T> z[8];                 // all gates of the pass are asked for before the first is used
@@ -582,6 +616,8 @@ const bool need = m_new > m_ref;
                             uint32_t v[16];
                             tmem_ld<16>(o_addr + d0 + d, v);
                             tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 16; e += 2) look(v[e], v[e + 1]);
 #pragma unroll
                             for (int e = 0; e < 4; e++)
                                 *cell(row, (d >> 2) + e) = make_float4(__uint_as_float(v[4 * e]) * f, __uint_as_float(v[4 * e + 1]) * f,
@@ -610,7 +646,9 @@ const bool need = m_new > m_ref;
                     tmem_ld<8>(o_addr + da, ua);
                     tmem_ld<8>(o_addr + db, ub);
                     tmem_ld_wait();
-                    if (live) {
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) { look(ua[e], ua[e + 1]); look(ub[e], ub[e + 1]); }
+                    if (stored) {
                         float a[8], b[8];
 #pragma unroll
                         for (int e = 0; e < 8; e++) { a[e] = __uint_as_float(ua[e]) * f; b[e] = __uint_as_float(ub[e]) * f; }
@@ -632,12 +670,14 @@ const bool need = m_new > m_ref;
                 }
                 __syncwarp();
                 }
+                // (a row whose sum is NaN is NaN by its own keys)
+                if (live && n > 1 && solo < 0 && l == l && odd.x + odd.y != 0.f) tainted[0] = pass;
             }
             tc_fence_before();
             __syncthreads();                          // the next segment overwrites the queries; its first products overwrite O
             tc_fence_after();
             n_done += nsteps; done_a += sg.steps_a; done_b += sg.steps_b;
-            i0 += n;
+            if (!again(sg, true)) i0 += n;
         }
     }
     if (warp == 1) tmem_dealloc<512>(tmem);

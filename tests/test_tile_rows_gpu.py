@@ -63,3 +63,24 @@ def test_latent_keys_reach_only_rows_that_see_them(dtype, value, H, r, dr, windo
     # a row that does not see the key: the same tiles, the same splits, zeros in place of a key with the weight 0
     assert torch.equal(got[~sees], clean[~sees])
     assert bool((~torch.isfinite(got[sees])).flatten(1).any(1).all())
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("where", ["keys", "values"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H,G,dk,dv,rot,window,opts", [
+    (16, 4, 128, 128, 64, 33, {}), (4, 4, 16, 48, 16, 0, {"pair_halves": True, "out_f32": True}),
+    (8, 4, 64, 128, 32, 0, {"vshare": 2, "chunk": 64}), (4, 2, 128, 128, 64, 50, {"pair_halves": True, "turned_values": True}),
+    (8, 2, 128, 128, 0, 40, {"shared": True, "keep_first": 4, "slopes": True, "gate_per_head": True}),
+    (8, 2, 96, 96, 0, 0, {"shared": True, "key_turned": 32, "sinks": True, "gate_per_head": True}), (64, 1, 64, 64, 64, 40, {"gate": False})])
+def test_window_keys_reach_only_rows_that_see_them(dtype, where, value, H, G, dk, dv, rot, window, opts):
+    # 700 tokens of 64 heads a group fill both tiles of a CTA; with fewer heads a CTA has half a tile
+    c = window_case(dtype, [(700, 5), (7, 90)], [77, 0], H, G, dk, dv, rot, window, opts)
+    k0, kw, v0, _ = window_columns(c)
+    spots = [(0, 43), (0, 66), (0, 299), (0, 300), (0, 702)]
+    cols = [k0 + kw - 1] if where == "keys" else [v0 + 3, v0 + dv - 1]
+    clean, got = window_run(c), window_run(c, _poisoned(c, spots, cols, value))
+    sees = _sees(c, spots, c.opt.keep_first, c.opt.chunk)
+    assert torch.equal(got[~sees], clean[~sees])
+    if where == "values" or value != value:                  # (a score of -infinity is a weight of 0)
+        assert bool((~torch.isfinite(got[sees])).any(1).all())
