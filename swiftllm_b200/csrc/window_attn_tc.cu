@@ -559,7 +559,7 @@ const bool need = m_new > m_ref;
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
                         const float2 z = Traits<T>::to_f2(u.v[e]);
-                        y[2 * e] = __fdividef(y[2 * e], 1.f + __expf(-z.x)); y[2 * e + 1] = __fdividef(y[2 * e + 1], 1.f + __expf(-z.y));
+                        y[2 * e] *= 1.f / (1.f + __expf(-z.x)); y[2 * e + 1] *= 1.f / (1.f + __expf(-z.y));
                     }
                 };
                 auto store8 = [&](int64_t to, float (&y)[8]) {

@@ -84,3 +84,13 @@ def test_window_keys_reach_only_rows_that_see_them(dtype, where, value, H, G, dk
     assert torch.equal(got[~sees], clean[~sees])
     if where == "values" or value != value:                  # (a score of -infinity is a weight of 0)
         assert bool((~torch.isfinite(got[sees])).any(1).all())
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("H,G,d", [(16, 4, 128), (4, 4, 48)])
+def test_window_gate_of_prompt_rows_is_that_of_decoded_rows(dtype, H, G, d):
+    # a window of one token: the weight is exactly 1 and O the value itself, so the fp32 output is the value times the gate
+    c = window_case(dtype, [(150, 5)], [], H, G, d, d, 16, 1, {"out_f32": True, "sink": False, "slopes": True})
+    prompt = window_run(c)
+    c.st.num_prefill_tokens = 0
+    assert torch.equal(prompt, window_run(c))
