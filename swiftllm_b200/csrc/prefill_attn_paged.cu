@@ -30,14 +30,16 @@ static int launch_prefill_paged(const void* q, const void* k_cache, const void* 
     return check_launch("prefill_attention_paged");
 }
 
-// One warp per (token, head), four entries a lane: the splits' rows on their common maximum.  A split that saw no key of the row has
-// maximum -infinity and wrote no O.
+// One warp per (row of sequence blockIdx.y, head), four entries a lane: the splits' rows on their common maximum.  A split that saw no key
+// of the row has maximum -infinity and wrote no O.  Rows of no sequence are left alone.
 template <typename T>
 __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                            T* __restrict__ o, int64_t units, int nsplit) {
+                                                            T* __restrict__ o, const int32_t* __restrict__ start_locs,
+                                                            const int32_t* __restrict__ seq_lens, int nq, int64_t units, int nsplit) {
     const int lane = threadIdx.x & 31;
-    const int64_t u = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (u >= units) return;
+    const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= (int64_t)seq_lens[blockIdx.y] * nq) return;
+    const int64_t u = (int64_t)start_locs[blockIdx.y] * nq + i;
     float M = -INFINITY, L = 0.f;
     for (int z = 0; z < nsplit; z++) M = fmaxf(M, part_ml[2 * (z * units + u)]);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -82,8 +84,8 @@ static int launch_prefill_paged_tc(const void* q, const void* k_cache, const voi
     }
     if (check_launch("prefill_attention_paged(tcgen05)")) return 1;
     if (pg.nsplit > 1) {
-        const int64_t units = num_tokens * nq;
-        SLLM_DISPATCH_DTYPE(dtype, (prefill_merge_kernel<T><<<(unsigned)cdiv(units, 8), 256, 0, stream>>>(pg.part_o, pg.part_ml, (T*)o, units, pg.nsplit)));
+        const dim3 rows((unsigned)cdiv((int64_t)max_chunk_len * nq, 8), (unsigned)num_seqs);
+        SLLM_DISPATCH_DTYPE(dtype, (prefill_merge_kernel<T><<<rows, 256, 0, stream>>>(pg.part_o, pg.part_ml, (T*)o, start_locs, chunk_lens, nq, num_tokens * nq, pg.nsplit)));
         return check_launch("prefill_attention_paged(merge)");
     }
     return 0;

@@ -94,3 +94,37 @@ def test_window_gate_of_prompt_rows_is_that_of_decoded_rows(dtype, H, G, d):
     prompt = window_run(c)
     c.st.num_prefill_tokens = 0
     assert torch.equal(prompt, window_run(c))
+
+
+# ---------------------------------------------------------------- portions whose keys are split between CTAs
+def _split_case(dtype, lens, prefix, H=4, G=2):
+    T, totals = sum(lens) + 3, [a + b for a, b in zip(lens, prefix)]              # three rows belong to no sequence
+    bt, nb = table(totals, 16, T)
+    kc, vc = (normal(nb, 1, G, 16, 128, seed=T + i, dtype=dtype) for i in (1, 2))
+    return normal(T, H, 128, seed=T, dtype=dtype), kc, vc, bt
+
+
+def _split_run(q, kc, vc, bt, lens, prefix, splits):
+    from swiftllm_b200 import _lib
+    T, H, D = q.shape
+    starts = ints(sum(lens[:i]) for i in range(len(lens)))
+    out, n = torch.full_like(q, 7.0), ints(lens)
+    ws = torch.full((splits * T * H * (D + 2),), float("nan"), device=DEV)        # what nobody wrote is not read
+    seqs, pre = ints(range(len(lens))), ints(prefix)
+    _lib.check(_lib.lib().sllm_prefill_attention_paged_split(
+        q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), bt.data_ptr(), seqs.data_ptr(), starts.data_ptr(), n.data_ptr(),
+        pre.data_ptr(), D ** -0.5, len(lens), max(lens), T, 0, 1, H, kc.shape[2], 16, D, bt.shape[1], kc.shape[0], H * D,
+        _lib.dtype_tag(q.dtype), _lib.stream(), splits, ws.data_ptr()))
+    torch.cuda.synchronize()
+    return out
+
+
+SPLIT_SHAPES = [((1, 300, 81), (0, 1000, 4000)), ((512,), (3584,)), ((257, 16, 1), (63, 4000, 700)), ((80, 130), (0, 31))]
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("splits", [2, 3, 16, 64])
+def test_split_keys_leave_other_rows_alone(dtype, splits):
+    lens, prefix = SPLIT_SHAPES[0]
+    q, kc, vc, bt = _split_case(dtype, lens, prefix)
+    assert bool((_split_run(q, kc, vc, bt, lens, prefix, splits)[sum(lens):] == 7).all())
