@@ -31,7 +31,7 @@ static int launch_prefill_paged(const void* q, const void* k_cache, const void* 
 }
 
 // One warp per (row of sequence blockIdx.y, head), four entries a lane: the splits' rows on their common maximum.  A split that saw no key
-// of the row has maximum -infinity and wrote no O.  Rows of no sequence are left alone.
+// of the row has the sum 0 and may have written no O (a sum that is NaN belongs to keys that it saw).  Rows of no sequence are left alone.
 template <typename T>
 __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                             T* __restrict__ o, const int32_t* __restrict__ start_locs,
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restr
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int z = 0; z < nsplit; z++) {
         const float2 ml = *reinterpret_cast<const float2*>(part_ml + 2 * (z * units + u));
-        if (ml.x == -INFINITY) continue;
+        if (ml.y == 0.f) continue;
         const float f = exp2f(ml.x - M);
         const float4 v = *reinterpret_cast<const float4*>(part_o + (z * units + u) * PT_D + 4 * lane);
         L += f * ml.y;

@@ -128,3 +128,13 @@ def test_split_keys_leave_other_rows_alone(dtype, splits):
     lens, prefix = SPLIT_SHAPES[0]
     q, kc, vc, bt = _split_case(dtype, lens, prefix)
     assert bool((_split_run(q, kc, vc, bt, lens, prefix, splits)[sum(lens):] == 7).all())
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("splits", [1, 2, 5, 16])
+def test_split_of_keys_that_are_not_finite_is_not_lost(dtype, splits):
+    # every key of the first splits is NaN: so is every row, however the keys were split
+    lens, prefix = (33,), (2000,)
+    q, kc, vc, bt = _split_case(dtype, lens, prefix)
+    kc[bt[0, :80].long()] = float("nan")
+    assert bool(torch.isnan(_split_run(q, kc, vc, bt, lens, prefix, splits)[:33]).all())
