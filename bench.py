@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py - decode tokens/s of the paged-attention data plane (BASELINE.json metric).
+"""bench.py - decode tokens/s of the paged-attention data plane.
 
   python bench.py [--gpus N] [--steps K] [--warmup W]            # this implementation
   python bench.py --impl reference ...                            # CPU arm: torch-eager oracle port on host cores
@@ -7,7 +7,7 @@
   python bench.py --arch-compare all [--steps K] [--warmup W]     # NOT the headline: Bupozen / Rivudra / Buzarax / Naforax / Zuzezen / Vorerax workers beside the Llama worker
                                                                   # (prefill / decode tok/s, attention roofline), 1 GPU
 
-Workload (BASELINE.json configs[1]): Llama-3-8B shapes, bf16, pure decode, batch 256, every sequence at
+Workload: Llama-3-8B shapes, bf16, pure decode, batch 256, every sequence at
 seq_len 4096, block_size 16, synthetic seeded weights N(0, 0.02) and a KV cache pre-filled with N(0, 1).
 A "step" is one LlamaModel.forward over the batch = one new token per sequence.
 
@@ -601,7 +601,7 @@ def cpu_decode_sample(cfg_full: dict, batch: int, seqlen: int, sample_seqs: int,
         m.forward(ids, sids, lens)
         tl.append(m.last_times["layers"] / NL); tp.append(m.last_times["pre_post"])
     # the least-disturbed of the repetitions: the host cores are shared with whatever else runs on the box (the value moved 2x
-    # between boxes in round 1 when a median over 1-3 steps was used)
+    # between boxes when a median over 1-3 steps was used)
     t_layer, t_prepost = min(tl), min(tp)
     del m, w
     t_full_sample = L * t_layer + t_prepost
@@ -642,8 +642,8 @@ def workload_config(args, cfg, n):
 
 
 
-# --------------------------------------------------------------------------- reference Triton arm (north_star: "next to the
-# reference's own Triton path on one B200"): the UNMODIFIED reference under baseline/_ref/src, in its own process
+# --------------------------------------------------------------------------- reference Triton arm, beside this
+# implementation on one B200: the UNMODIFIED reference under baseline/_ref/src, in its own process
 def run_reference_triton(args, dtypes):
     """Runs scripts/ref_triton_bench.py once per dtype BEFORE this process allocates its own 143 GB (both need most of the
     GPU).  Same workload, same public call (LlamaModel.forward: host lists in, host ints out), same step count and
@@ -1041,7 +1041,7 @@ def run_ours(args):
     kname = "paged_attn_kernel (gen 1: cp.async + mma.sync)" if pa_gen == "1" else \
         "paged_attn_tc_kernel (gen 2: tcgen05 + TMA, persistent)"
 
-    # ---- optional: prefill tokens/s (secondary metric of BASELINE.json)
+    # ---- optional: prefill tokens/s (secondary metric)
     prefill = None
     if not args.no_prefill:
         stage("prefill tokens/s")

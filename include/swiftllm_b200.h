@@ -104,7 +104,7 @@ int sllm_prefill_attention(const void* q, const void* k, const void* v, void* o,
                            int head_dim, int64_t q_row_stride, int64_t k_row_stride, int64_t v_row_stride,
                            sllm_dtype_t dtype, sllm_stream_t stream);
 
-/* ---- Chunked ("prefix-aware") prefill - SURVEY.md §8 f-1.  NEW: the reference's forward cannot express a partial prompt
+/* ---- Chunked ("prefix-aware") prefill.  NEW: the reference's forward cannot express a partial prompt
  * (its prefill attention only sees the packed k/v of the batch: swiftllm/worker/kernels/prefill_attn.py:102-139,
  * swiftllm/worker/layers/transformer_layer.py:86-96; its store always starts at position 0: kvcache_mgmt.py:10-48).
  * Prefill entry i of the batch is the CHUNK of its prompt that covers positions
@@ -218,7 +218,7 @@ int sllm_swap_blocks(const int64_t* host_src_ids, const int64_t* host_dst_ids, i
                      void* k_cache, void* v_cache, void* host_k_swap, void* host_v_swap, int64_t block_bytes,
                      sllm_stream_t stream);
 
-/* Sync-free variant (new, SURVEY.md §8 f-4): src_ids / dst_ids are DEVICE arrays (int64) - the gathered source ids and the
+/* Sync-free variant (new): src_ids / dst_ids are DEVICE arrays (int64) - the gathered source ids and the
  * newly allocated target ids never travel to the host (the reference does `.tolist()` twice per swap, model.py:374-377) - and
  * one kernel moves every block between the cache and the swap space, which must be pinned, device-mapped host memory
  * (cudaHostAlloc / torch pin_memory).  Same data movement as sllm_swap_blocks. */

@@ -1,7 +1,7 @@
 """
 Golden-vector generator.  TEST INFRASTRUCTURE ONLY.
 
-Executes the UNMODIFIED reference (swiftLLM at /root/reference) on CPU -- Triton kernels under
+Executes the UNMODIFIED reference (swiftLLM) on CPU -- Triton kernels under
 TRITON_INTERPRET=1, `LlamaModel` under the cuda->cpu shim of `oracle/ref_shim.py` -- on seeded
 inputs and stores inputs + outputs under `tests/golden/*.npz`.  Run in the build container:
 
@@ -114,7 +114,7 @@ def gen_kvcache_and_paged(swiftllm):
          prefill_seq_lens=st.prefill_seq_lens, decoding_seq_lens=st.decoding_seq_lens, cur_layer=1, block_size=bs,
          k_cache_out=kc, v_cache_out=vc)
 
-    # ---- paged attention, BASELINE config 1: 1 request x 1 KV block  (paged_attn.py:152-222)
+    # ---- paged attention: 1 request x 1 KV block  (paged_attn.py:152-222)
     out = {}
     L, nq, nkv, bs, D, nblk = 2, 4, 2, 16, 64, 4
     mc = _NS(num_layers=L, num_kv_heads=nkv, head_dim=D, num_q_heads=nq)

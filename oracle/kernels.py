@@ -3,7 +3,7 @@ CPU restatements (torch-CPU / numpy) of every kernel in the reference's
 `swiftllm/worker/kernels/`.  TEST INFRASTRUCTURE ONLY (see oracle/__init__.py).
 
 Each function follows the rounding order of the reference kernel it cites
-(SURVEY.md Appendix A).  `h(.)` below means "round to the storage dtype"
+`h(.)` below means "round to the storage dtype"
 (fp16 in the reference; bf16 in the bf16 build), `f(.)` means fp32.
 
 All functions are functional (return new tensors) unless they end in
@@ -36,7 +36,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
 def fused_add_rmsnorm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float):
     """rmsnorm.py:39-65: s = h(x + r) (add in the storage dtype, stored to the
     residual), then rmsnorm(s).  Returns (x_out, residual_out)."""
-    s = x + residual           # storage-dtype add, correctly rounded (see DESIGN.md numerics)
+    s = x + residual           # storage-dtype add, correctly rounded
     return rmsnorm(s, weight, eps), s
 
 
@@ -114,7 +114,7 @@ def store_kvcache_inplace(k, v, k_cache, v_cache, block_table, seq_ids, prefill_
     """kvcache_mgmt.py:10-79 (+ the commented torch loop at :124-132).
     k,v [T,nkv,D]; caches [num_blocks, L, nkv, bs, D]; block_table int32 [max_seqs, max_blocks_per_seq].
     Exact copies.
-    `prefill_prefix_lens` (chunked prefill; not in the reference): token t of prefill chunk i goes to
+    `prefill_prefix_lens` (chunked prefill, not in the reference): token t of prefill chunk i goes to
     position prefill_prefix_lens[i] + t of its sequence (the reference always writes a prompt from position 0)."""
     seq_ids = [int(s) for s in seq_ids]
     for i in range(num_prefill_seqs):
@@ -303,8 +303,8 @@ def prefill_attention_exact(q, k, v, start_locs, seq_lens, softmax_scale, out_dt
 
 def prefix_prefill_attention_exact(q, k_cache, v_cache, block_table, seq_ids, start_locs, chunk_lens, prefix_lens,
                                    softmax_scale, block_size, cur_layer, out_dtype=None, compute_dtype=torch.float64):
-    """Chunked ("prefix-aware") prefill attention - SURVEY.md §8 f-1.  The reference has no such kernel (its prefill
-    attention never reads the KV cache, SURVEY.md §3.1); the definition is the one that makes a prompt processed in
+    """Chunked ("prefix-aware") prefill attention.  The reference has no such kernel (its prefill
+    attention never reads the KV cache); the definition is the one that makes a prompt processed in
     chunks equal to the same prompt processed at once by `prefill_attention_exact`: chunk b holds the tokens at
     positions [prefix_lens[b], prefix_lens[b] + chunk_lens[b]) of sequence seq_ids[b]; the keys/values of ALL positions
     below prefix + chunk are read from the paged cache (the chunk's own K/V are stored first, like decode tokens,

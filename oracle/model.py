@@ -30,7 +30,7 @@ class OracleWeights:
 
     @staticmethod
     def random(cfg: dict, dtype=torch.float16, seed=0, std=0.02):
-        """Seeded synthetic weights (N(0,std) projections, 1+N(0,std) norms; SURVEY.md §8d)."""
+        """Seeded synthetic weights (N(0,std) projections, 1+N(0,std) norms)."""
         g = torch.Generator().manual_seed(seed)
         H, nq = cfg["hidden_size"], cfg["num_attention_heads"]
         nkv = cfg.get("num_key_value_heads", nq)
@@ -89,7 +89,7 @@ class OracleLlama:
     @torch.inference_mode()
     def forward(self, input_ids_list, seq_ids_list, decoding_seq_lens_list, ignore_kvcache=False,
                 prefill_prefix_lens_list=None):
-        """`prefill_prefix_lens_list` (chunked prefill; not in the reference): prefill entry i is the
+        """`prefill_prefix_lens_list` (chunked prefill, not in the reference): prefill entry i is the
         chunk of its prompt that starts at position prefill_prefix_lens_list[i]; the earlier positions are already in
         the KV cache.  None = the reference's contract (every prefill entry is a whole prompt)."""
         num_prefill_seqs = len(input_ids_list) - len(decoding_seq_lens_list)

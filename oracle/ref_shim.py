@@ -1,9 +1,9 @@
 """
-Import shim that lets the UNMODIFIED reference (`/root/reference`, swiftLLM) execute on CPU in
+Import shim that lets the UNMODIFIED reference (swiftLLM) execute on CPU in
 the build container.  TEST INFRASTRUCTURE ONLY; used by `oracle/gen_golden.py` to produce the
-fixtures in `tests/golden/`.  It never runs on the GPU box (`/root/reference` is absent there).
+fixtures in `tests/golden/`.  It needs the reference's sources (SWIFTLLM_REFERENCE_ROOT) and no GPU.
 
-What it does (SURVEY.md §8c):
+What it does:
   * TRITON_INTERPRET=1 so every `@triton.jit` kernel runs in Triton's numpy interpreter;
   * stub modules for imports that are not installable here: `ray` (tokenizer actor only),
     `swiftllm_c` (swap_blocks; restated with torch copies below), `vllm_flash_attn`
@@ -53,7 +53,7 @@ def _install_stubs():
 
         def flash_attn_varlen_func(q, k, v, cu_q, cu_k, max_q, max_k, softmax_scale=None, causal=False, **kw):
             # fp32 stand-in for the third-party kernel (transformer_layer.py:86-96).  The last
-            # cu_seqlen is clamped to the sliced q length (SURVEY.md §3.1 quirk).
+            # cu_seqlen is clamped to the sliced q length.
             T, nq, D = q.shape
             nkv = k.shape[1]
             g = nq // nkv

@@ -5,7 +5,7 @@
 //      for sizes from 256 KiB (a decode exchange at TP 8: 32 rows x 8 KiB) to 128 MiB (a prefill exchange);
 //   3. peer write bandwidth: 16-byte stores into GPU1's memory (the two-shot path's all-gather half).
 // Build: nvcc -gencode arch=compute_100a,code=sm_100a -O2 -std=c++17 -o probes/build/p2p_latency probes/p2p_latency.cu
-// Run on a box with >= 2 GPUs: gpurun --gpus 2 -- 'probes/build/p2p_latency'
+// Run on a box with >= 2 GPUs: probes/build/p2p_latency
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>

@@ -1,5 +1,5 @@
 """HBM roofline of the elementwise / copy kernels at prefill-size T (Llama-3-8B shapes, bf16): achieved GB/s =
-algorithmic bytes (SURVEY.md §8d) / CUDA-event time, against the measured copy peak.  One JSON line per kernel."""
+algorithmic bytes / CUDA-event time, against the measured copy peak.  One JSON line per kernel."""
 import json, os, sys, types
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__))); sys.path.insert(0, ROOT)
 import torch

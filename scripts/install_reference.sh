@@ -5,7 +5,7 @@
 # The reference installs itself with `pip install -e .` + `pip install -e csrc` (its README, "Build and Run"): an editable install
 # exposes the source tree itself, and its setup.py depends on that (packages=["swiftllm"] leaves out swiftllm.server / swiftllm.worker,
 # so a regular `pip install --target` yields a package that cannot be imported).  The offline equivalent of the editable install is
-# what this script does: a verbatim copy of the tree at baseline/_ref/src (git-ignored, travels with gpurun) that the bench script
+# what this script does: a verbatim copy of the tree at baseline/_ref/src (git-ignored, travels with the tree) that the bench script
 # puts on sys.path, and an in-place build of the `swiftllm_c` extension (host-only C++, builds without a GPU).
 # baseline/_ref is NOT part of the product: nothing under swiftllm_b200/, tests/ or bench.py reads it.
 set -euo pipefail

@@ -1,7 +1,7 @@
 """One launch of the paged-decode kernel at the benchmarked geometry, for `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum`
 (bench.py runs this under ncu as a subprocess to fill `roofline.traffic` live; it is never timed).
 
-The KV cache here holds ONE layer ([blocks, 1, nkv, 16, D]: 2 x 4.3 GB at BASELINE configs[1]) instead of the 32 of the
+The KV cache here holds ONE layer ([blocks, 1, nkv, 16, D]: 2 x 4.3 GB at batch 256 x 4096) instead of the 32 of the
 benchmark, because the benchmark process still owns its 128 GiB cache while this runs.  Bytes per launch do not depend on the
 layer count: the kernel reads the same sum(len) * nkv * D * 2 * 2 bytes of pages, block-table entries and q, and writes o.
 Blocks are assigned to sequences through a random permutation so the page gather is as scattered as in a served cache."""

@@ -1,14 +1,14 @@
 """Times the UNMODIFIED reference (swiftLLM, placed under baseline/_ref/src by scripts/install_reference.sh; git-ignored) on the GPU:
-its own Triton kernels + cuBLAS, BASELINE config 2 (Llama-3-8B shapes, pure decode, batch 256, seq_len 4096) through its
+its own Triton kernels + cuBLAS, Llama-3-8B shapes, pure decode, batch 256, seq_len 4096, through its
 own public API (`LlamaModel.forward`: host lists in, host ints out - the same call bench.py's `e2e` leg makes).
 bench.py runs this as a subprocess (N = 1, before it allocates its own model) and reports the result as `reference_triton`;
 the contract's `--impl reference` arm stays the CPU port.  Prints one JSON line: decode step time, tokens/s and the time of
 its paged_attention (phase 1 + 2, CUDA events on the stream the reference launches it on).
 
-REF_DTYPE=fp16 (default): the tree exactly as shipped (it hard-codes fp16, SURVEY.md "Facts").
-REF_DTYPE=bf16: a throw-away COPY of the tree (temp dir, never written back) in which the fp16 literals SURVEY.md lists
+REF_DTYPE=fp16 (default): the tree exactly as shipped (it hard-codes fp16).
+REF_DTYPE=bf16: a throw-away COPY of the tree (temp dir, never written back) in which the fp16 literals
 (`torch.float16` / `tl.float16` in swiftllm/**.py) are replaced by their bf16 counterparts - the "dtype-patched reference"
-BASELINE's bf16 metric needs; nothing else is changed."""
+the bf16 metric needs; nothing else is changed."""
 import json, os, re, shutil, statistics, sys, tempfile, types
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -34,7 +34,7 @@ if DTYPE == "bf16":
 # paged_attn.py:88) and is specialised three times on cur_layer: ~8 minutes of ptxas on a cold cache.  A cache built once on a
 # B200 box of this image is kept under baseline/_ref/triton_cache/<dtype> (git-ignored,
 # travels with the repo snapshot): the UNMODIFIED kernels, compiled by the same Triton, only not recompiled.
-# REF_TRITON_CACHE_DIR overrides the location (the warm-up script points it at gpurun_out/).
+# REF_TRITON_CACHE_DIR overrides the location.
 cache = os.environ.get("REF_TRITON_CACHE_DIR") or os.path.join(ROOT, "baseline", "_ref", "triton_cache", DTYPE)
 packed = os.path.join(ROOT, "baseline", "_ref", f"triton_cache_{DTYPE}.tar.gz")     # how the cache travels (it compresses 8x)
 if not os.environ.get("REF_TRITON_CACHE_DIR") and not os.path.isdir(cache) and os.path.exists(packed):

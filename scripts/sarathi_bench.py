@@ -1,13 +1,13 @@
 #!/usr/bin/env python
-"""BASELINE.json configs[2]: Llama-3-8B bf16, SARATHI-style piggybacking - every step carries one 512-token CHUNK of a
-4096-token prompt plus 64 decoding sequences at seq_len 4096 (chunked prefill through the paged cache: SURVEY.md §8 f-1,
+"""Llama-3-8B bf16, SARATHI-style piggybacking - every step carries one 512-token CHUNK of a
+4096-token prompt plus 64 decoding sequences at seq_len 4096 (chunked prefill through the paged cache,
 `LlamaModel.forward(..., prefill_prefix_lens_list=...)`).  Not the headline bench (that is bench.py / configs[1]); one JSON
 line with the mean step time over whole prompts (8 chunk positions each), tokens/s = (chunk + decodes) / step, and the
 same schedule with the chunk and the decodes issued as two separate calls (what the reference would have to do).
 
     python scripts/sarathi_bench.py [--chunk 512] [--decodes 64] [--prompt 4096] [--prompts 3]
     torchrun --nproc-per-node 8 scripts/sarathi_bench.py --gpus 8 --model llama3-70b --prompt 8192 --seqlen 8192
-        (BASELINE.json configs[4]: Llama-3-70B, TP = 8, mixed prefill/decode at seq_len 8192)
+        (Llama-3-70B, TP = 8, mixed prefill/decode at seq_len 8192)
 """
 import argparse
 import json
@@ -104,7 +104,7 @@ def main():
     if rank != 0:
         torch.cuda.synchronize(); dist.barrier(); os._exit(0)
     print(json.dumps({"metric": "sarathi_step_tokens_per_s", "config": {"workload": f"{args.model} bf16, {args.chunk}-token chunk of a "
-                      f"{args.prompt}-token prompt + {Bd} decodes at seq_len {S} per step (BASELINE.json configs[2] / [4])", "layers": cfg["num_hidden_layers"]},
+                      f"{args.prompt}-token prompt + {Bd} decodes at seq_len {S} per step", "layers": cfg["num_hidden_layers"]},
                       "piggybacked": {"ms_per_step": ms_pig, "tokens_per_s": tok / (ms_pig * 1e-3)},
                       "separate_calls": {"ms_per_step": ms_sep, "tokens_per_s": tok / (ms_sep * 1e-3)},
                       "steps_timed": args.prompts * nchunks, "n_gpus": n, "parallelism": f"tp{n}", "data": "synthetic",

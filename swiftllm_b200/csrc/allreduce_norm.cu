@@ -1,4 +1,4 @@
-// Tensor-parallel exchange fused with the op that always follows it (SURVEY.md §8 f-3):
+// Tensor-parallel exchange fused with the op that always follows it:
 //     x_sum = sum over ranks of the partial GEMM output   (one-shot all-reduce over NVLink peer memory)
 //     residual <- h(x_sum) + residual ;  x_out <- rmsnorm(residual) * weight       (rmsnorm.py:39-65 semantics)
 // in ONE kernel, instead of ncclAllReduce + fused_add_rmsnorm.  Every rank's partial lives in a symmetric buffer

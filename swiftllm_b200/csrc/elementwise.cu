@@ -1,6 +1,6 @@
 // HBM-bound elementwise kernels: RMSNorm, fused add+RMSNorm, rotary embedding, SiLU-and-mul.
 // All are 128-bit vectorised (8 half/bf16 values per load/store), coalesced, and follow the rounding
-// order of the reference Triton kernels (SURVEY.md Appendix A; oracle/kernels.py restates them):
+// order of the reference Triton kernels (oracle/kernels.py restates them):
 //   rmsnorm.py:5-24, :39-65   rotary_emb.py:7-41   silu_and_mul.py:5-23
 // Algorithmic bytes (s = 2): rmsnorm 2*T*H*s + H*s, fused 4*T*H*s + H*s, rotary 2*T*(nq+nkv)*D*s + T*D*s,
 // silu_and_mul 3*T*F*s.

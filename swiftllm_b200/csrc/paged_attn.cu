@@ -10,7 +10,7 @@
 //   * v1 (single pass, writes o directly) when the batch alone fills the GPU, v2 (flash-decoding split +
 //     merge kernel, same (normalised o, log2-sum-exp) partial format as the reference) otherwise.
 // HBM roofline: algorithmic bytes per launch = sum_i len_i * nkv * D * 2 (K and V) * sizeof(T)
-//               + 2 * Bd * nq * D * sizeof(T)  (SURVEY.md §8d).
+//               + 2 * Bd * nq * D * sizeof(T).
 #include <stdlib.h>
 
 #include "mma_helpers.cuh"

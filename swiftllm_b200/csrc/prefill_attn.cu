@@ -3,10 +3,10 @@
 //
 // Reference: swiftllm/worker/kernels/prefill_attn.py:9-139 (the Triton kernel) and the flash_attn_varlen_func
 // call that stands in for it at swiftllm/worker/layers/transformer_layer.py:86-96.  Numerics follow
-// SURVEY.md Appendix A6: S = f32(QK^T) * (scale*log2e); online softmax in fp32 with exp2; P rounded to the
+// S = f32(QK^T) * (scale*log2e); online softmax in fp32 with exp2; P rounded to the
 // storage dtype before P.V; o = h(acc / l).
 // The sequence END is taken from prefill_seq_lens (never from a cu_seqlens array that includes decode tokens:
-// the reference's mixed-batch quirk, SURVEY.md §3.1).
+// the reference's mixed-batch quirk).
 // Roofline: tensor-bound; FLOPs = 4 * nq * D * sum_i L_i (L_i + 1) / 2.
 #include <stdlib.h>
 

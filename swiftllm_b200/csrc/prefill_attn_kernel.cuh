@@ -4,10 +4,10 @@
 //
 // Reference: swiftllm/worker/kernels/prefill_attn.py:9-139 (the Triton kernel) and the flash_attn_varlen_func
 // call that stands in for it at swiftllm/worker/layers/transformer_layer.py:86-96.  Numerics follow
-// SURVEY.md Appendix A6: S = f32(QK^T) * (scale*log2e); online softmax in fp32 with exp2; P rounded to the
+// S = f32(QK^T) * (scale*log2e); online softmax in fp32 with exp2; P rounded to the
 // storage dtype before P.V; o = h(acc / l).
 // The sequence END is taken from prefill_seq_lens (never from a cu_seqlens array that includes decode tokens:
-// the reference's mixed-batch quirk, SURVEY.md §3.1).
+// the reference's mixed-batch quirk).
 // Roofline: tensor-bound; FLOPs = 4 * nq * D * sum_i L_i (L_i + 1) / 2  (+ 4 * nq * D * sum_i prefix_i * L_i when PAGED).
 #pragma once
 #include "mma_helpers.cuh"
@@ -25,7 +25,7 @@ struct PfPagedKV {
 };
 
 // PAGED = false: k, v are the packed [T, nkv, D] rows of this very batch (the reference's contract).
-// PAGED = true (chunked prefill, SURVEY.md §8 f-1): k, v are the paged caches [num_blocks, L, nkv, bs, D]; the chunk's
+// PAGED = true (chunked prefill): k, v are the paged caches [num_blocks, L, nkv, bs, D]; the chunk's
 // queries sit at positions prefix .. prefix + len - 1 of their sequence and attend to positions <= their own.
 template <typename T, int D, bool PAGED>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_attn_kernel(

@@ -1,7 +1,7 @@
 // Chunked ("prefix-aware") prefill attention: the queries of a prompt CHUNK attend to the whole prefix + chunk through
-// the paged KV cache.  SURVEY.md §8 f-1: the reference's forward cannot express a partial prompt (its prefill attention,
+// the paged KV cache.  The reference's forward cannot express a partial prompt (its prefill attention,
 // swiftllm/worker/kernels/prefill_attn.py:102-139 / transformer_layer.py:86-96, only ever sees the packed k/v of the
-// batch), which is what SARATHI-style piggybacking (BASELINE.json configs[2]) needs.  Definition = the one that makes
+// batch), which is what SARATHI-style piggybacking needs.  Definition = the one that makes
 // a prompt processed in chunks equal to the same prompt processed at once (oracle/kernels.py:
 // prefix_prefill_attention_exact).  Both generations of the prefill kernel are instantiated with PAGED = true:
 //   gen 2 (prefill_attn_tc_kernel.cuh): tcgen05 + TMA page gather, head_dim 128, block_size 16

@@ -1,4 +1,4 @@
-// Block swapping with DEVICE-resident id lists (SURVEY.md §8 f-4).  The reference (csrc/src/block_swapping.cpp:22-85, driven by
+// Block swapping with DEVICE-resident id lists.  The reference (csrc/src/block_swapping.cpp:22-85, driven by
 // swiftllm/worker/model.py:361-379) reads the gathered source ids and the newly allocated target ids back to the host
 // (`.tolist()` x 2: two device syncs per swap) and issues two cudaMemcpyAsync per run of consecutive blocks.  Here the ids
 // never leave the GPU: ONE kernel moves all blocks of the swap between the paged cache and the PINNED, device-mapped swap space

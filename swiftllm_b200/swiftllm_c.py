@@ -31,7 +31,7 @@ def swap_blocks_device(source_block_ids: torch.Tensor, target_block_ids: torch.T
                        k_cache: torch.Tensor, v_cache: torch.Tensor, k_swap: torch.Tensor, v_swap: torch.Tensor):
     """Same data movement as swap_blocks, but the id lists are DEVICE tensors (int64) and one kernel moves all blocks through the
     pinned, device-mapped swap space: no `.tolist()` syncs (the reference does two per swap, model.py:374-377).  Addition of this
-    implementation (SURVEY.md §8 f-4); needs `pin_swap_space`."""
+    implementation; needs `pin_swap_space`."""
     n = source_block_ids.numel()
     assert n == target_block_ids.numel()
     if n == 0:

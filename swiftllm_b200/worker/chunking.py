@@ -1,4 +1,4 @@
-"""SARATHI-style piggybacking on top of `LlamaModel.forward(..., prefill_prefix_lens_list=...)` (SURVEY.md §8 f-1).
+"""SARATHI-style piggybacking on top of `LlamaModel.forward(..., prefill_prefix_lens_list=...)`.
 
 The reference's scheduler launches whole-prompt prefill batches and marks where piggybacking would go
 (swiftllm/server/scheduler.py:93-94: "If you want decoding requests to be piggybacked, you can do it here"), but its worker

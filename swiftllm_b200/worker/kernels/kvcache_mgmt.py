@@ -27,7 +27,7 @@ def store_kvcache(
     num_layers, nkv, bs, D = k_cache.shape[1:]
     prefix = getattr(infer_state, "prefill_prefix_lens", None)
     if prefix is not None:
-        # chunked prefill (SURVEY.md §8 f-1, not in the reference): chunk token t goes to position prefix + t
+        # chunked prefill (not in the reference): chunk token t goes to position prefix + t
         assert prefix.dtype == torch.int32 and prefix.is_contiguous() and prefix.shape[0] == infer_state.num_prefill_seqs
         _lib.check(_lib.lib().sllm_store_kvcache_chunked(
             k.data_ptr(), v.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(),

@@ -1,5 +1,5 @@
 """Reference: swiftllm/worker/kernels/linear.py:3-12.  A plain library GEMM (cuBLAS through torch), exactly as in
-the reference; the hot-path scope keeps it a library call."""
+the reference; it stays a library call."""
 import torch
 
 

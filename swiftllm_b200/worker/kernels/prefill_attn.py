@@ -53,7 +53,7 @@ def prefill_attention_paged(
     infer_state: LlamaInferState,
     cur_layer: int,
 ):
-    """Chunked ("prefix-aware") prefill attention (SURVEY.md §8 f-1; no counterpart in the reference, whose prefill attention
+    """Chunked ("prefix-aware") prefill attention (no counterpart in the reference, whose prefill attention
     never reads the KV cache): the chunk's queries sit at positions prefill_prefix_lens[i] + t of their sequence and attend
     to positions <= their own, keys / values read from the paged cache (the chunk's own K/V are stored first)."""
     assert o.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous() and block_table.is_contiguous()

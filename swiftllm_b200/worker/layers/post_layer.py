@@ -1,6 +1,6 @@
 """Reference: swiftllm/worker/layers/post_layer.py:9-40 (last-token gather, final RMSNorm, lm_head, greedy argmax).
 
-Addition (tensor parallelism, SURVEY.md §8 f-3): with a vocabulary-sharded lm_head every rank computes the logits of its
+Addition (tensor parallelism): with a vocabulary-sharded lm_head every rank computes the logits of its
 V / tp_size rows only and the greedy token is found with ONE all-gather of per-rank (max logit, global index) pairs
 (8 bytes per sequence and rank) instead of every rank streaming the whole lm_head."""
 import torch

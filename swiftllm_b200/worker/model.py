@@ -7,7 +7,7 @@
 
 and the same observable state (k_cache, v_cache, k_swap, v_swap, gpu_block_manager, cpu_block_manager).
 
-B200-first host path (SURVEY.md §8 f-2): all per-step metadata travels in ONE pinned staging buffer and one
+B200-first host path: all per-step metadata travels in ONE pinned staging buffer and one
 H2D copy (the reference issues ~6 small copies, model.py:272-297); block allocation is one sync-free kernel
 (three syncs + torch.nonzero in the reference, block_manager.py:50,70,75); pure-decode steps can be replayed
 from a CUDA graph; the only sync of a step is the final `.tolist()` of the sampled tokens.
@@ -258,7 +258,7 @@ class LlamaModel(PagedModelBase):
         """model.py:252-359.  Batch layout contract: prefill sequences first (full prompt each), then decoding
         sequences (exactly one token each); decoding_seq_lens_list[i] includes the new token.
 
-        `prefill_prefix_lens_list` (addition, SURVEY.md §8 f-1: chunked / SARATHI-style prefill, which the reference's
+        `prefill_prefix_lens_list` (addition: chunked / SARATHI-style prefill, which the reference's
         forward cannot express): when given, prefill entry i is the CHUNK of its prompt that starts at position
         prefill_prefix_lens_list[i]; positions below it were written to the KV cache by earlier calls.  The chunk's
         K/V are stored at their positions and its queries attend to the whole prefix + chunk through the block
@@ -315,7 +315,7 @@ class LlamaModel(PagedModelBase):
             num_prefill_seqs=num_prefill_seqs, num_prefill_tokens=num_prefill_tokens,
             prefill_seq_start_locs=p_starts,
             # ends at num_prefill_tokens (the reference puts num_tokens there, model.py:336-339, which over-declares
-            # the last prompt by the number of decoding tokens on mixed batches; SURVEY.md §3.1)
+            # the last prompt by the number of decoding tokens on mixed batches)
             prefill_seq_start_locs_with_end=torch.cat([p_starts, p_starts.new_tensor([num_prefill_tokens])])
             if num_prefill_seqs > 0 else p_starts,
             prefill_seq_lens=p_lens, max_prefill_len=max_prefill_len,

@@ -1,5 +1,5 @@
-"""Tensor-parallel exchange over NVLink peer memory, fused with the residual add + RMSNorm that follows it
-(SURVEY.md §8 f-3).  torch.distributed symmetric memory is the plumbing (buffer allocation + handle exchange); the
+"""Tensor-parallel exchange over NVLink peer memory, fused with the residual add + RMSNorm that follows it.
+torch.distributed symmetric memory is the plumbing (buffer allocation + handle exchange); the
 data movement and the reduction are this library's own kernel (`sllm_allreduce_add_rmsnorm`, csrc/allreduce_norm.cu).
 
 Two symmetric buffers alternate: slot 0 holds the o_proj partials, slot 1 the down_proj partials of a layer.  The GEMM

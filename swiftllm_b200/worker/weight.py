@@ -609,7 +609,7 @@ def dummy_getter(device="cuda"):
 
 
 def synthetic_getter(seed: int = 0, std: float = 0.02, device="cuda", norm_offset: float = 1.0):
-    """Seeded synthetic weights of realistic scale (SURVEY.md §8d): N(0, std) projections, norm_offset + N(0, std) norms
+    """Seeded synthetic weights of realistic scale: N(0, std) projections, norm_offset + N(0, std) norms
     (0 for designs that store norm weights around zero).
     Deterministic per tensor key, so every TP rank generates the same full tensor before slicing."""
     import zlib

@@ -1,4 +1,4 @@
-"""CPU: chunked ("prefix-aware", SARATHI-style) prefill - SURVEY.md §8 f-1.
+"""CPU: chunked ("prefix-aware", SARATHI-style) prefill.
 
 The reference cannot express a partial prompt, so there is no reference output to pin against; the definition is
 "processing a prompt in chunks gives what processing it at once gives".  These tests hold (a) the oracle's chunked path to

@@ -295,7 +295,7 @@ def _gz(z, c):
 @pytest.mark.parametrize("sbs", [0, "ref"])
 def test_paged_attention_golden(golden, case, sbs, paged_gen):
     """vs the reference's own outputs.  The reference accumulates q.k in fp16 (its own error vs fp64 is 1-3e-3 of
-    max|o|, SURVEY.md §7); this kernel accumulates in fp32, so the tolerance is 3e-3 * max|o| against the reference
+    max|o|); this kernel accumulates in fp32, so the tolerance is 3e-3 * max|o| against the reference
     and 1e-3 * max|o| against the fp64 definition."""
     z = golden("paged_attention")
     args = _gz(z, case)
@@ -345,7 +345,7 @@ def test_paged_attention_vs_exact_oracle(dtype, geom, sbs, paged_gen):
 
 
 def test_paged_attention_full_length_properties(paged_gen):
-    """BASELINE config-2 sequence length (4096) at a reduced batch, Llama-3-8B head geometry, bf16:
+    """The benchmark's sequence length (4096) at a reduced batch, Llama-3-8B head geometry, bf16:
     (a) vs the fp64 oracle, (b) v1 vs v2 agree, (c) result is invariant under a permutation of the physical blocks,
     (d) linear in V."""
     dtype, nq, nkv, D, bs, L = torch.bfloat16, 32, 8, 128, 16, 2

@@ -94,7 +94,7 @@ def test_model_matches_reference_golden_trace(golden):
             e_prod = float((got.double() - tru).abs().max() / tru.abs().max())
             worst_prod, worst_ref = max(worst_prod, e_prod), max(worst_ref, e_ref)
             _log("golden_trace_vs_exact_arithmetic", step=i, reference_trace_err=e_ref, product_err=e_prod)
-            # north_star asks for logits "within 1e-3 relative": the reference's own trace is this far from exact arithmetic,
+            # The target is logits "within 1e-3 relative": the reference's own trace is this far from exact arithmetic,
             # (1.0-1.4e-3 on this trace), and the product - whose fp16 storage roundings are as many but not the same - must not be
             # materially further: 1.5 x the reference's own error + one fp16 ulp of the largest logit
             assert e_prod <= 1.5 * e_ref + 2 ** -11, (i, e_prod, e_ref)
@@ -102,7 +102,7 @@ def test_model_matches_reference_golden_trace(golden):
             margin = float((top2[:, 0] - top2[:, 1]).min() / ref.abs().max())
             _log("golden_trace", step=i, rel_logit_err=rel, top1_margin_rel=margin, tokens_equal=toks == z[f"t{i}_tokens"].tolist())
             assert toks == z[f"t{i}_tokens"].tolist(), (i, toks, z[f"t{i}_tokens"].tolist())     # greedy ids bit-exact
-            # the reference's own fp16-accumulated decode attention is 1-3e-3 off the fp64 definition (SURVEY §7)
+            # the reference's own fp16-accumulated decode attention is 1-3e-3 off the fp64 definition
             assert rel <= 4e-3, rel
         elif c["op"] == "swap_out":
             m.swap_out_seqs(c["seq_ids"])

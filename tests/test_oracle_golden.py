@@ -58,7 +58,7 @@ def _paged(z, c):
 
 
 def test_paged_attention_config1_one_req_one_block(golden):
-    """single paged_attention decode, 1 req x 1 KV block, TRITON_INTERPRET=1."""
+    """Single paged_attention decode, 1 req x 1 KV block, TRITON_INTERPRET=1."""
     args, S, nsb, o_ref = _paged(golden("paged_attention"), "c1")
     o = K.paged_attention_ref_order(*args, S, nsb)
     assert torch.equal(bits(o), bits(o_ref))          # rounding order reproduced bit for bit

@@ -194,7 +194,7 @@ def test_product_model_fused_exchange_host_path_on_cpu(world, comm):
 @pytest.mark.slow_cpu
 @pytest.mark.parametrize("comm", ["two_shot", "one_shot", None], ids=["row-owner", "one-shot", "all-reduce"])
 def test_product_model_world8_host_path_on_cpu(comm):
-    """World 8 (the TP degree of BASELINE configs[3] / [4]): the host path with the row-owner exchange family that is the default
+    """World 8 (the largest TP degree of one box): the host path with the row-owner exchange family that is the default
     there (two-shot semantics: 2-row decode steps leave six ranks without a row to own) and the vocabulary-sharded lm_head, over
     gloo with oracle-backed kernels.  8 processes on the CPU container."""
     world = 8
