@@ -1,9 +1,9 @@
-"""GPU: chunked ("prefix-aware") prefill - SURVEY.md §8 f-1 - through the C ABI:
+"""GPU: chunked ("prefix-aware") prefill through the C ABI:
   sllm_store_kvcache_chunked      bit-exact vs the oracle (pages entered in the middle, ragged chunks, mixed with decode rows)
   sllm_prefill_attention_paged    both kernel generations vs the fp64 definition; with prefix 0 vs sllm_prefill_attention
   LlamaModel.forward(..., prefill_prefix_lens_list=...)   chunked == whole-prompt (tokens exact, logits within tolerance)
 
-First executed on a B200 in round 2 (green on the first run: profiles/r2_pytest_pending_1gpu.log); part of the default `-m gpu` suite."""
+Part of the default `-m gpu` suite."""
 import types
 
 import numpy as np
@@ -135,8 +135,9 @@ def test_prefill_attention_paged_nan_in_unowned_pages_is_harmless(dtype, prefill
 
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_prefill_attention_paged_zero_prefix_equals_packed_kernel(dtype, prefill_gen):
-    """With every prefix 0 the paged kernel sees exactly the keys the packed kernel sees, in the same 64-token steps: the two
-    must agree to the last bit (same MMA shapes, same softmax code; only the producer differs)."""
+    """With every prefix 0 and keys that are not split (the state names no max_prefill_kv_len) the paged kernel sees exactly the keys
+    the packed kernel sees, in the same steps: the two must agree to the last bit (same MMA shapes, same softmax code; only the producer
+    differs).  Split keys agree up to rounding: tests/test_tile_rows_gpu.py."""
     from swiftllm_b200.worker.kernels.prefill_attn import prefill_attention
     from swiftllm_b200.worker.kernels.kvcache_mgmt import store_kvcache
     nq, nkv, D, bs, L = 8, 2, 128, 16, 2
@@ -160,7 +161,7 @@ def test_prefill_attention_paged_zero_prefix_equals_packed_kernel(dtype, prefill
 
 
 def test_prefill_attention_paged_sarathi_shape_property(prefill_gen):
-    """BASELINE configs[2] geometry: a 512-token chunk at the end of a 4096-token prompt (Llama-3-8B heads, bf16).  The last
+    """A 512-token chunk at the end of a 4096-token prompt (Llama-3-8B heads, bf16).  The last
     row of the chunk equals decode attention over the same 4096 keys (paged decode kernel and fp64 definition)."""
     from swiftllm_b200.worker.kernels.paged_attn import paged_attention
     dtype, nq, nkv, D, bs = torch.bfloat16, 32, 8, 128, 16

@@ -22,54 +22,85 @@ def _gather_page(cache, blk, layer, kvh):
     return cache[blk, layer, kvh].double().numpy()          # [16, D]
 
 
-def mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, scale, layer):
-    """prefill_attn_tc_kernel<T, PAGED=true>: CTA = (seq, head, 256 query rows = tiles A and B), 64-token kv steps."""
+def mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, scale, layer, nsplit=1):
+    """prefill_attn_tc_kernel<T, PAGED=true>: CTA = (seq and key split, head, 256 query rows = tiles A and B), 80-token kv steps of which a
+    split takes `per`; then prefill_merge_kernel over the splits' (maximum, sum, O), which start as NaN: what nobody wrote is not read."""
     Tn, nq, D = q.shape
     nkv = kc.shape[2]
     out = np.zeros((Tn, nq, D))
-    BQ, BK = 128, 64
+    BQ, BK = 128, 80
+    PPS = BK // BS                                                     # pages per step
+    part_m, part_l, part_o = np.full((nsplit, Tn, nq), np.nan), np.full((nsplit, Tn, nq), np.nan), np.full((nsplit, Tn, nq, D), np.nan)
+    cdiv = lambda a, b: (a + b - 1) // b
     for seq in range(len(chunk)):
         ln, pre, tok0 = chunk[seq], prefix[seq], starts[seq]
         kvlen = pre + ln
-        npages = (kvlen + BS - 1) // BS
+        npages = cdiv(kvlen, BS)
         for head in range(nq):
             kvh = head // (nq // nkv)
-            for qblk in range((max(chunk) + 2 * BQ - 1) // (2 * BQ)):
+            for qblk, split in ((b, z) for b in range(cdiv(max(chunk), 2 * BQ)) for z in range(nsplit)):
                 q0 = qblk * 2 * BQ
                 if q0 >= ln:
                     continue
                 active_b = q0 + BQ < ln
-                nkt = [(min(kvlen, pre + q0 + BQ) + BK - 1) // BK, (min(kvlen, pre + q0 + 2 * BQ) + BK - 1) // BK if active_b else 0]
+                end = [min(kvlen, pre + q0 + BQ), min(kvlen, pre + q0 + 2 * BQ) if active_b else 0]
+                steps = [cdiv(e, BK) for e in end]
+                per = cdiv(max(steps), nsplit)
+                j0 = split * per
+                nkt = [min(max(n - j0, 0), per) for n in steps]
+                if max(nkt) == 0:                                      # a split past the last key: thread tid < 256 answers for row tid
+                    n = min(2 * BQ, ln - q0)
+                    part_m[split, tok0 + q0:tok0 + q0 + n, head], part_l[split, tok0 + q0:tok0 + q0 + n, head] = -np.inf, 0.0
+                    continue
                 for x in range(2):
                     rows = q0 + x * BQ + np.arange(BQ)                 # chunk-relative query rows of this tile
-                    S_all, V_all = [], []
-                    for j in range(nkt[x]):
-                        # producer: pages 4j .. 4j+3 that exist are loaded WHOLE; the rest of the stage is zero (or stale, finite)
+                    ok = tok0 + rows < Tn
+                    qrow = np.zeros((BQ, D))
+                    qrow[ok] = q[tok0 + rows[ok], head].double().numpy()          # TMA: rows past the tensor are zero-filled
+                    m, l, O = np.full((BQ, 1), -np.inf), np.zeros((BQ, 1)), np.zeros((BQ, D))
+                    for j in range(j0, j0 + nkt[x]):
+                        # producer: pages 5j .. 5j+4 that exist are loaded WHOLE; the rest of the stage is zero (or stale, finite)
                         Kt, Vt = np.zeros((BK, D)), np.zeros((BK, D))
-                        for pg in range(min(4, npages - 4 * j)):
-                            blk = int(bt[sids[seq], 4 * j + pg])
+                        valid = min(PPS, npages - j * PPS)
+                        assert valid >= 1
+                        for pg in range(valid):
+                            blk = int(bt[sids[seq], PPS * j + pg])
                             Kt[pg * BS:(pg + 1) * BS] = _gather_page(kc, blk, layer, kvh)
                             Vt[pg * BS:(pg + 1) * BS] = _gather_page(vc, blk, layer, kvh)
-                        qrow = np.zeros((BQ, D))
-                        ok = tok0 + rows < Tn
-                        qrow[ok] = q[tok0 + rows[ok], head].double().numpy()      # TMA: rows past the tensor are zero-filled
                         with np.errstate(invalid="ignore"):
                             S = qrow @ Kt.T
                         c0 = j * BK
-                        need_mask = c0 + BK - 1 > pre + q0 + x * BQ or c0 + BK > kvlen
-                        if need_mask:
+                        if c0 + BK - 1 > pre + q0 + x * BQ or c0 + BK > kvlen:
                             lim = np.minimum(pre + rows, kvlen - 1) - c0
                             S = np.where(np.arange(BK)[None, :] <= lim[:, None], S, -np.inf)
-                        S_all.append(S); V_all.append(Vt)
-                    if not S_all:
-                        continue
-                    S = np.concatenate(S_all, 1) * scale
-                    Vt = np.concatenate(V_all, 0)
-                    P = np.exp(S - S.max(1, keepdims=True))
-                    with np.errstate(invalid="ignore"):
-                        O = (P @ Vt) / P.sum(1, keepdims=True)         # 0 * NaN = NaN here exactly as on the tensor core
+                        m_new = np.maximum(m, S.max(1, keepdims=True) * scale)
+                        with np.errstate(invalid="ignore"):
+                            alpha = np.where(m_new > m, np.exp(m - m_new), 1.0)
+                        m, l, O = m_new, l * alpha, O * alpha
+                        P = np.exp(S * scale - np.where(np.isneginf(m), 0.0, m))         # nothing seen yet: weights of 0
+                        l = l + P.sum(1, keepdims=True)
+                        k16 = min(PPS, cdiv(end[x] - c0, 16))          # P . V: none past the last key the tile can see
+                        assert k16 >= 1
+                        O = O + P[:, :16 * k16] @ Vt[:16 * k16]
                     wr = rows < ln                                      # epilogue: only rows inside the chunk are written
-                    out[tok0 + rows[wr], head] = O[wr]
+                    at = tok0 + rows[wr]
+                    if nsplit > 1:
+                        part_m[split, at, head], part_l[split, at, head] = m[wr, 0], l[wr, 0]
+                        if nkt[x] > 0:
+                            part_o[split, at, head] = O[wr]
+                    elif nkt[x] > 0:
+                        out[at, head] = O[wr] / l[wr]
+    if nsplit > 1:
+        for seq in range(len(chunk)):                                   # merge: the rows of the sequences, no others
+            for u in range(starts[seq], starts[seq] + chunk[seq]):
+                for head in range(nq):
+                    M, L, a = part_m[:, u, head].max(), 0.0, np.zeros(D)
+                    for z in range(nsplit):
+                        if part_l[z, u, head] == 0:
+                            continue
+                        f = np.exp(part_m[z, u, head] - M)
+                        L, a = L + f * part_l[z, u, head], a + f * part_o[z, u, head]
+                    out[u, head] = a / L
     return out
 
 
@@ -160,9 +191,10 @@ def test_mirror_of_the_tcgen05_paged_prefill_kernel_matches_the_definition(seed)
     rng = np.random.default_rng(seed)
     q, kc, vc, bt, sids, starts, chunk, prefix = _case(rng, BS, 32, 4, 2, 3)
     ref = K.prefix_prefill_attention_exact(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, BS, 1).numpy()
-    got = mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, 1)
-    assert np.isfinite(got).all()
-    assert np.abs(got - ref).max() < 1e-9
+    for nsplit in (1, 2, 5, 16):
+        got = mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, 1, nsplit)
+        assert np.isfinite(got).all()
+        assert np.abs(got - ref).max() < 1e-9
 
 
 @pytest.mark.parametrize("seed,bs", [(0, 16), (1, 16), (2, 32), (3, 4)])
