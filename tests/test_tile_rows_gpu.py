@@ -138,3 +138,95 @@ def test_split_of_keys_that_are_not_finite_is_not_lost(dtype, splits):
     q, kc, vc, bt = _split_case(dtype, lens, prefix)
     kc[bt[0, :80].long()] = float("nan")
     assert bool(torch.isnan(_split_run(q, kc, vc, bt, lens, prefix, splits)[:33]).all())
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("H,r,dr,dims,window,portions", [
+    (16, 512, 64, 64, 0, [(130, 5), (7, 90), (1, 3)]), (16, 512, 64, 32, 100, [(600, 200), (95, 0)]), (1, 64, 16, 8, 50, [(130, 0), (65, 70)]),
+    (5, 192, 48, 48, 0, [(33, 63), (64, 0)]), (40, 256, 64, 32, 70, [(31, 200), (2, 0)]), (70, 320, 0, 0, 0, [(20, 44)])])
+def test_latent_rows_against_64_bits(dtype, H, r, dr, dims, window, portions):
+    # weights and output are rounded to 16 bits, and the turned queries: three roundings of at most half a unit, that add as squares
+    c = latent_case(dtype, portions, [77, 0, 500], H, r, dr, dims, window, sink=True)
+    assert rel(latent_run(c), latent_exact(c)) < UNIT[dtype]
+
+
+# CTAs of two full tiles: 16 heads on 4 groups need more than 36 x 64 prompt rows on 148 SMs, one group of 64 heads more than 147 x 4.
+# Sequences end inside tile A (33 tokens), inside tile B (63) and beside whole CTAs
+FULL = [(33, 0), (63, 5), (1, 0), (700, 90), (1500, 30), (95, 0)]
+SHORT = [(1, 0), (3, 5), (130, 0), (65, 17)]
+WINDOWS = [
+    (16, 4, 128, 128, 64, 100, {}, FULL), (64, 1, 64, 64, 64, 40, {"gate": False}, [(3, 0), (1, 7), (600, 90), (2, 0), (5, 200)]),
+    (16, 4, 128, 128, 0, 90, {"shared": True, "keep_first": 4, "slopes": True, "gate_per_head": True, "prenorm": True}, FULL),
+    (16, 4, 128, 128, 0, 300, {"shared": True, "key_turned": 32, "sinks": True, "gate_per_head": True}, FULL),
+    (16, 4, 128, 128, 64, 0, {"pair_halves": True, "turned_values": True, "qk_norm_eps": 1e-5, "softcap": 5.0, "sink": False}, FULL),
+    (16, 4, 64, 128, 32, 0, {"vshare": 2, "chunk": 64, "prenorm": True, "out_f32": True, "gate": False}, FULL),
+    (16, 4, 80, 112, 16, 50, {"softcap": 5.0, "out_scale": 0.5, "slopes": True}, FULL),
+    (16, 4, 128, 128, 64, 100, {}, SHORT), (3, 1, 64, 128, 32, 0, {"out_f32": True}, SHORT),
+    (4, 4, 16, 48, 16, 33, {"pair_halves": True, "qk_norm_eps": 1e-5}, SHORT), (8, 2, 96, 96, 0, 90, {"shared": True, "key_turned": 16}, SHORT)]
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("H,G,dk,dv,rot,window,opts,portions", WINDOWS)
+def test_window_rows_against_64_bits(dtype, H, G, dk, dv, rot, window, opts, portions):
+    # as above: queries after norm and rotation, weights, and the output
+    c = window_case(dtype, portions, [77, 0], H, G, dk, dv, rot, window, opts)
+    got, ref = window_run(c), window_exact(c)
+    at = 0
+    for n, p in c.rows:                                      # a fault in a short sequence does not hide behind a long one
+        assert rel(got[at:at + n], ref[at:at + n]) < UNIT[dtype], (n, p)
+        at += n
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("splits", [1, 2, 3, 7, 16, 64])
+@pytest.mark.parametrize("lens,prefix", SPLIT_SHAPES)
+def test_split_keys_against_64_bits(dtype, splits, lens, prefix):
+    # splits beyond the steps, one-row portions beside long ones, boundaries inside a query block's diagonal
+    q, kc, vc, bt = _split_case(dtype, lens, prefix)
+    got, at, H = _split_run(q, kc, vc, bt, lens, prefix, splits), 0, q.shape[1]
+    for s, (n, p) in enumerate(zip(lens, prefix)):
+        k, v = (c[bt[s, :-(-(n + p) // 16)].long(), 0].transpose(1, 2).flatten(0, 1)[:n + p].repeat_interleave(H // kc.shape[2], 1).double()
+                for c in (kc, vc))
+        score = torch.einsum("nhd,lhd->nhl", q[at:at + n].double(), k) * 128 ** -0.5
+        seen = torch.arange(n + p, device=DEV)[None] <= p + torch.arange(n, device=DEV)[:, None]
+        assert rel(got[at:at + n], attend(score, seen, v, None)) < UNIT[dtype], (n, p)
+        at += n
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("lens,prefix", SPLIT_SHAPES)
+def test_portions_of_a_step_split_their_keys(dtype, lens, prefix):
+    # the entry point that the worker calls, with the length that it gives: the split count is its own
+    import types
+    from swiftllm_b200.worker.kernels.prefill_attn import _key_splits, prefill_attention_paged
+    q, kc, vc, bt = _split_case(dtype, lens, prefix)
+    longest = max(a + b for a, b in zip(lens, prefix))
+    st = types.SimpleNamespace(
+        num_prefill_seqs=len(lens), num_prefill_tokens=sum(lens), max_prefill_len=max(lens), seq_ids=ints(range(len(lens))), prefill_seq_lens=ints(lens),
+        prefill_seq_start_locs=ints(sum(lens[:i]) for i in range(len(lens))), prefill_prefix_lens=ints(prefix), softmax_scale=128 ** -0.5,
+        max_prefill_kv_len=longest)
+    splits = _key_splits(4 * len(lens), max(lens), longest)
+    assert splits > 1 or longest < 1280
+    out = torch.full_like(q, 7.0)
+    prefill_attention_paged(q, kc, vc, bt, out, None, types.SimpleNamespace(block_size=16), st, 0)
+    assert torch.equal(out, _split_run(q, kc, vc, bt, lens, prefix, splits))
+
+
+# ---------------------------------------------------------------- selective scan: the instances that other tests do not reach
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("dt_wide", [True, False])
+@pytest.mark.parametrize("lens,C,N", [((15, 16, 17, 33), 8192, 16), ((32, 1, 31), 8192, 16), ((33, 70), 64, 16), ((9,), 128, 8)])
+def test_selective_scan_lanes_and_step_types(dtype, dt_wide, lens, C, N):
+    # four (three) segments of 8192 channels leave two lanes to a channel on 148 SMs; step sizes of the storage type
+    from swiftllm_b200.worker.kernels.scan_ops import selective_scan
+    st, T = segments(lens, [0] * (len(lens) - 1) + [5]), sum(lens)
+    base = normal(T, 2 * C + 2 * N + 8, seed=C + N, dtype=dtype)
+    dt, bias = normal(T, C, seed=1, dtype=torch.float32 if dt_wide else dtype), normal(C, seed=2) - 3
+    A, D = -(normal(C, N, seed=3).abs() + 0.1), normal(C, seed=4)
+    outs = []
+    for off in (0, 1):                                       # a view that is not aligned takes the plain path
+        x = torch.zeros_like(base)[:, off:off + C]
+        x.copy_(base[:, :C])
+        state = normal(len(lens), C, N, seed=5)
+        outs.append((selective_scan(x, dt, bias, A, base[:, 2 * C:], 0, N, D, base[:, C:2 * C], state, st), state))
+    assert rel(outs[0][0], outs[1][0]) < UNIT[dtype] and rel(outs[0][1], outs[1][1]) < 1e-6
