@@ -3,10 +3,10 @@
 // Keys and values are never expanded: the caller folds the key up-projection into the query (q_lat[h] = W_uk[h]^T q_nope[h])
 // and applies the value up-projection to the attention-weighted sum of latents, so per head
 //     score(i, j) = (q_lat[i,h] . c[j] + rope(q_rot[i,h]) . k_rot[j]) * scale,   out_lat[i,h] = sum_j softmax_j(score) c[j].
-// Every token of the step is a query with its own (block-table row, position): prompt portions and single decoded tokens go
-// through the same kernel, so the result for a position does not depend on how its sequence was cut into steps.  A query at
-// position p attends to the positions max(0, p - window + 1) .. p (window <= 0: all of 0 .. p).  With `sink` (fp32 [H]) the softmax's
-// denominator also contains exp(sink[h]): a key of that score without a value, which enters the running (maximum, sum) first.
+// Every token of the step is a query with its own (block-table row, position), whose result depends on its own keys only; how its
+// sequence was cut into steps changes it by rounding (tiles and key splits follow the rows of a launch).  A query at position p attends
+// to the positions max(0, p - window + 1) .. p (window <= 0: all of 0 .. p).  With `sink` (fp32 [H]) the softmax's denominator also contains
+// exp(sink[h]): a key of that score without a value, which enters the running (maximum, sum) first.
 // Softmax, the norm of the latent and the rotation run in fp32 for every storage type.
 #include "latent_attn_tc.cuh"
 #include "mma_helpers.cuh"
