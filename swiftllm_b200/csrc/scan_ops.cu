@@ -729,12 +729,15 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
     int ns_tiled = ns_plain;
     if (num_prefill_segs > 0) {
         // prompt portions walk their tokens one after the other: with few (segment, channel) pairs more lanes per channel (fewer
-        // states per thread) put more warps on the SMs, but not below four states a lane, which are read and multiplied together
-        // (one segment of 1024 tokens, 4096 channels: 389 us with two states a lane, 229 with four)
+        // states per thread) put more warps on the SMs, but not below four states a lane where these are read and multiplied together, four
+        // tokens at a time, which takes 16 states or more (512 tokens, 16 states, us: 162 with one state a lane, 68 with four; 24: 174 and
+        // 167; 32: 193 and 113; 64: 248 and 134), or where one state a lane would be more than eight warps an SM (8 states: 64 to
+        // 4096 channels 156 - 170 and 168, f32 152 - 168 and 195; 8192 channels 215 and 168, f32 211 and 195; 4 states 162 and 287)
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
-        while (ns_tiled < 5 && (2 << ns_tiled) <= states &&
-               (((int64_t)num_prefill_segs * channels) << ns_tiled) / 32 < 8 * (int64_t)sms && !((states & 3) == 0 && (states >> ns_tiled) <= 4)) ns_tiled++;
+        const int64_t pairs = (int64_t)num_prefill_segs * channels, few = 8 * (int64_t)sms;
+        const bool fours = (states & 3) == 0 && (states >= 16 || (states >= 8 && pairs * states / 32 > few));
+        while (ns_tiled < 5 && (2 << ns_tiled) <= states && (pairs << ns_tiled) / 32 < few && !(fours && (states >> ns_tiled) <= 4)) ns_tiled++;
     }
     int tt = SS_ITEMS << ns_tiled;                     // tt * (128 >> ns_tiled) = 128 SS_ITEMS entries per staged array ...
     if (tt > 32) tt = 32;

@@ -230,3 +230,18 @@ def test_selective_scan_lanes_and_step_types(dtype, dt_wide, lens, C, N):
         state = normal(len(lens), C, N, seed=5)
         outs.append((selective_scan(x, dt, bias, A, base[:, 2 * C:], 0, N, D, base[:, C:2 * C], state, st), state))
     assert rel(outs[0][0], outs[1][0]) < UNIT[dtype] and rel(outs[0][1], outs[1][1]) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("lens,C,N", [((40, 9), 64, 4), ((40, 9), 64, 8), ((33, 8, 20, 15), 2048, 8), ((17, 40), 8192, 4)])
+def test_selective_scan_of_few_states_against_32_bit_rows(dtype, lens, C, N):
+    # one state a lane, or four: the same steps as fp32 rows of the same values, to the output's rounding
+    from swiftllm_b200.worker.kernels.scan_ops import selective_scan
+    st, T = segments(lens, [0] * (len(lens) - 1) + [5]), sum(lens)
+    x, z, bc = (normal(T, n, seed=n + i, dtype=dtype) for i, n in enumerate((C, C, 2 * N)))
+    dt, bias, A, D = normal(T, C, seed=1), normal(C, seed=2) - 3, -(normal(C, N, seed=3).abs() + 0.1), normal(C, seed=4)
+    outs = []
+    for t in (dtype, torch.float32):
+        state = normal(len(lens), C, N, seed=5)
+        outs.append((selective_scan(x.to(t), dt, bias, A, bc.to(t), 0, N, D, z.to(t), state, st), state))
+    assert rel(outs[0][0], outs[1][0]) < UNIT[dtype] and rel(outs[0][1], outs[1][1]) < 1e-6
