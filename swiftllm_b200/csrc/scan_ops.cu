@@ -91,9 +91,10 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TI* __restrict__ 
 }
 
 // The same for prompt rows where rows are whole pieces of four channels: a thread walks SV_TOKENS rows of four neighbouring channels, eight
-// rows' loads in flight together (wider pieces need 154 registers and leave ten warps on an SM: 96 us); where the rows of the tile break (another sequence) is found once per warp.  The products,
-// their order and the SiLU are those above (a quicker quotient turns some roundings, which a state behind the convolution keeps).  Bound: bytes, of which enough
-// are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 -> about 80 us (59 with a quicker quotient).
+// rows' loads in flight together (wider pieces need 154 registers and leave ten warps on an SM: 96 us); where the rows of the tile break
+// (another sequence) is found once per warp.  The products, their order and the SiLU are those above (a quicker quotient turns some
+// roundings, which a state behind the convolution keeps).  Bound: bytes, of which enough are in flight only with many warps.  Measured on
+// B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 -> about 80 us (59 with a quicker quotient).
 constexpr int SV_TOKENS = 16;
 template <typename TI, typename TO, int K>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restrict__ xin, int64_t xin_stride, const float* __restrict__ w,
@@ -368,7 +369,6 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(
 constexpr int SS_ITEMS = 8;
 constexpr int SS_BCR = 4;
 
-//
 // VEC (16-bit rows in 16-byte pieces, states in whole eights): a thread brings eight neighbouring channels of ONE token and eight entries of
 // B or C per tile, with one address each, and stores eight outputs; the SiLU of the gate takes the special-function unit's exponential
 // and quotient.  Measured on B200, bf16, 4 x 2048 tokens, 4096 channels, 16 states: 813 -> 370 us (staging took 85
@@ -655,8 +655,10 @@ int sllm_short_conv(const void* xin, int64_t xin_stride, sllm_dtype_t in_dtype, 
         (const TI*)xin, xin_stride, (const float*)w, (const float*)bias, (TI*)tail, (const int*)tok_seq,                        \
         (const int*)tok_pos, (T*)out, (int64_t)(r0), (int64_t)(r1), channels, taps, add_input, act_silu,                        \
         (TOKENS == 1 && move_decode_tails && taps > 1) ? 1 : 0)
-    // prompt rows in pieces of four channels: three or four taps (what the workers have) take the vector kernel, others a channel per thread
-    const bool vec = (taps == 3 || taps == 4) && channels % 4 == 0 && xin_stride % 4 == 0 &&
+    // prompt rows in pieces of four channels: three or four taps (what the workers have) take the vector kernel, others a channel per thread,
+    // which also starts sooner where there are few entries (4 taps, bf16, us: 300 x 2048 12 against 16, 300 x 4096 16 both, 2048 x 516 16
+    // both, 2048 x 2048 31 against 18)
+    const bool vec = num_prefill_tokens * channels >= (1 << 20) && (taps == 3 || taps == 4) && channels % 4 == 0 && xin_stride % 4 == 0 &&
                      (((uintptr_t)xin | (uintptr_t)tail | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
 #define SC_VEC(TI, K)                                                                                                          \
     short_conv_vec_kernel<TI, T, K><<<dim3((unsigned)cdiv(num_prefill_tokens, SV_TOKENS), (unsigned)cdiv(channels, 512)), 128, 0, st>>>( \

@@ -245,3 +245,20 @@ def test_selective_scan_of_few_states_against_32_bit_rows(dtype, lens, C, N):
         state = normal(len(lens), C, N, seed=5)
         outs.append((selective_scan(x.to(t), dt, bias, A, bc.to(t), 0, N, D, z.to(t), state, st), state))
     assert rel(outs[0][0], outs[1][0]) < UNIT[dtype] and rel(outs[0][1], outs[1][1]) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("lens,C,taps,wide", [((1, 2, 3, 250, 44), 4096, 4, False), ((17, 184), 5252, 3, False), ((16, 15, 241), 4096, 4, True)])
+def test_short_convolution_of_many_rows(dtype, lens, C, taps, wide):
+    # 2^20 entries and more go in pieces of four channels, with the sums and the SiLU of the plain path, which other views take
+    from swiftllm_b200.worker.kernels.scan_ops import short_conv
+    st, T = segments(lens, [0, 7, 2, 0, 1][:len(lens)]), sum(lens)
+    tin = torch.float32 if wide else dtype
+    base, w, b = normal(T, C + 8, seed=C, dtype=tin), normal(C, taps, seed=1) * 0.4, normal(C, seed=2)
+    outs = []
+    for off in (0, 1):
+        x = torch.zeros_like(base)[:, off:off + C]
+        x.copy_(base[:, :C])
+        tail = normal(len(lens), taps - 1, C, seed=3, dtype=tin)
+        outs.append((short_conv(x, w, b, tail, st, dtype, add_input=wide, silu=True, move_tail=True), tail))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
