@@ -265,3 +265,13 @@ def test_short_convolution_of_many_rows(dtype, lens, C, taps, wide):
         tail = normal(len(lens), taps - 1, C, seed=3, dtype=tin)
         outs.append((short_conv(x, w, b, tail, st, dtype, add_input=wide, silu=True, move_tail=True), tail))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+# ---------------------------------------------------------------- how often a result is rounded
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("opts", [{}, {"softcap": 5.0}, {"slopes": True}])
+def test_window_weights_sum_to_one(dtype, opts):
+    # equal values come out as they are, whatever the weights were rounded to: sum and product take the same weights
+    c = window_case(dtype, [(300, 5), (1, 0), (700, 90)], [], 16, 4, 128, 128, 0, 200, {"out_f32": True, "gate": False, "sink": False, **opts})
+    c.cache[..., 4 * 128:] = 1.5
+    assert float((window_run(c) - 1.5).abs().max()) < 1e-5
