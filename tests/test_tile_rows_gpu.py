@@ -69,7 +69,7 @@ def test_latent_keys_reach_only_rows_that_see_them(dtype, value, H, r, dr, windo
 @pytest.mark.parametrize("where", ["keys", "values"])
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("H,G,dk,dv,rot,window,opts", [
-    (16, 4, 128, 128, 64, 33, {}), (4, 4, 16, 48, 16, 0, {"pair_halves": True, "out_f32": True}),
+    (16, 4, 128, 128, 64, 33, {}), (4, 4, 80, 48, 16, 0, {"pair_halves": True, "out_f32": True}),
     (8, 4, 64, 128, 32, 0, {"vshare": 2, "chunk": 64}), (4, 2, 128, 128, 64, 50, {"pair_halves": True, "turned_values": True}),
     (8, 2, 128, 128, 0, 40, {"shared": True, "keep_first": 4, "slopes": True, "gate_per_head": True}),
     (8, 2, 96, 96, 0, 0, {"shared": True, "key_turned": 32, "sinks": True, "gate_per_head": True}), (64, 1, 64, 64, 64, 40, {"gate": False})])
@@ -165,7 +165,7 @@ WINDOWS = [
     (16, 4, 64, 128, 32, 0, {"vshare": 2, "chunk": 64, "prenorm": True, "out_f32": True, "gate": False}, FULL),
     (16, 4, 80, 112, 16, 50, {"softcap": 5.0, "out_scale": 0.5, "slopes": True}, FULL),
     (16, 4, 128, 128, 64, 100, {}, SHORT), (3, 1, 64, 128, 32, 0, {"out_f32": True}, SHORT),
-    (4, 4, 16, 48, 16, 33, {"pair_halves": True, "qk_norm_eps": 1e-5}, SHORT), (8, 2, 96, 96, 0, 90, {"shared": True, "key_turned": 16}, SHORT)]
+    (4, 4, 80, 48, 16, 33, {"pair_halves": True, "qk_norm_eps": 1e-5}, SHORT), (4, 4, 16, 48, 16, 33, {"pair_halves": True}, SHORT), (8, 2, 96, 96, 0, 90, {"shared": True, "key_turned": 16}, SHORT)]
 
 
 @pytest.mark.parametrize("dtype", TYPES)
