@@ -38,18 +38,31 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restr
                                                             const int32_t* __restrict__ seq_lens, int nq, int64_t units, int nsplit) {
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (i >= (int64_t)seq_lens[blockIdx.y] * nq) return;
-    const int64_t u = (int64_t)start_locs[blockIdx.y] * nq + i;
+    const int start = start_locs[blockIdx.y], len = seq_lens[blockIdx.y];
+    if (i >= (int64_t)len * nq) return;
+    const int64_t u = (int64_t)start * nq + i;
     float M = -INFINITY, L = 0.f;
-    for (int z = 0; z < nsplit; z++) M = fmaxf(M, part_ml[2 * (z * units + u)]);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int z = 0; z < nsplit; z++) {
-        const float2 ml = *reinterpret_cast<const float2*>(part_ml + 2 * (z * units + u));
-        if (ml.y == 0.f) continue;
-        const float f = exp2f(ml.x - M);
-        const float4 v = *reinterpret_cast<const float4*>(part_o + (z * units + u) * PT_D + 4 * lane);
-        L += f * ml.y;
-        a.x += f * v.x; a.y += f * v.y; a.z += f * v.z; a.w += f * v.w;
+    for (int z = 0; z < nsplit; z += 2) {            // two splits' loads in flight, none waits for another
+        float2 ml[2];
+        float4 v[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int64_t at = min(z + k, nsplit - 1) * units + u;
+            ml[k] = *reinterpret_cast<const float2*>(part_ml + 2 * at);
+            v[k] = *reinterpret_cast<const float4*>(part_o + at * PT_D + 4 * lane);
+        }
+        if (z + 1 == nsplit) ml[1] = make_float2(-INFINITY, 0.f);
+        const float m = fmaxf(M, fmaxf(ml[0].x, ml[1].x)), keep = M == m ? 1.f : exp2f(M - m);
+        M = m; L *= keep;
+        a.x *= keep; a.y *= keep; a.z *= keep; a.w *= keep;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (ml[k].y == 0.f) continue;            // (its O is whatever lay there)
+            const float f = exp2f(ml[k].x - m);
+            L += f * ml[k].y;
+            a.x += f * v[k].x; a.y += f * v[k].y; a.z += f * v[k].z; a.w += f * v[k].w;
+        }
     }
     const float inv = 1.f / L;
     typename Traits<T>::T2 lo = Traits<T>::from_f2(make_float2(a.x * inv, a.y * inv)), hi = Traits<T>::from_f2(make_float2(a.z * inv, a.w * inv));
