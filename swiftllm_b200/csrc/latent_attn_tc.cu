@@ -12,6 +12,10 @@
 // would save most rescales of O (490 instead of 580 us below), but then the largest weight is not 1 and takes a rounding as well,
 // 2.15e-3 instead of 2.01e-3 off 64-bit arithmetic in bf16.
 //
+// Single tokens of at most 16 heads fill one warp's 16 rows.  The next warp's rows repeat them and take as P what the rounding of the first
+// left over, at no further product: weights of 8 and 8 bits (bf16).  With one rounding, fewer key splits (each rounds against its own
+// maximum) cost precision: 64 tokens at 2048 keys 1.919e-3 off 64 bits in four splits of the mma.sync kernel, 1.945e-3 in two, now 1.791e-3.
+//
 // Shared memory is what decides the shape: 64 rows of Q (576 entries: 72 KiB) and two stages of 64 keys (72 KiB each) fill it.  A stage
 // therefore is handed back in two pieces, each as soon as the product that reads it last is done: the first 256 columns after the first
 // half of O, the rest after the second; producer warps gather each piece through the block table by cp.async (rows past the last
@@ -42,6 +46,7 @@ constexpr int LT_CHUNK = 64 * 128;                  // bytes of 64 rows x 64 col
 constexpr int LT_MAX_CHUNKS = 9;
 constexpr int LT_STAGE = LT_MAX_CHUNKS * LT_CHUNK;
 constexpr int LT_SMEM = 3 * LT_STAGE + 1024;
+constexpr int LT_REST_PITCH = 512 + 4;              // floats of a row on its way from rows 16 .. 31 to rows 0 .. 15: O, then the sum
 constexpr int LT_S_COL = 256, LT_P_COL = 384;       // TMEM columns: O 0..255, S two of 64, P two of 32
 constexpr float LT_LOG2E = 1.4426950408889634f, LT_LN2 = 0.6931471805599453f;
 
@@ -69,8 +74,9 @@ __device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const uint32_t (&r
 // byte offset of 16-byte piece `piece` (of 8) of row `row` in a chunk of 64 rows x 128 bytes, SWIZZLE_128B
 __device__ __forceinline__ uint32_t lt_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
 
-// FULL: r = 512 and dr = 64, known to the compiler (the producers' and the issuer's loops are bound by their instructions)
-template <typename T, bool FULL>
+// FULL: r = 512 and dr = 64, known to the compiler (the producers' and the issuer's loops are bound by their instructions).  DUP: single
+// tokens of at most 16 heads, whose rows 16 .. 31 repeat rows 0 .. 15
+template <typename T, bool FULL, bool DUP>
 __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const LatentTc p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_sm = smem;                            // [chunk][64 rows][128 B]
@@ -85,6 +91,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     const int hp = 1 << p.hp_log2, h0 = blockIdx.y * hp;
     const int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;      // the last tokens of a prompt have the most keys: first
     const int ntok = min(p.qt, p.num_tokens - t_first);
+    auto head_row = [&](int row) { return DUP && row < 32 ? row & 15 : row; };      // the row whose token and head it is
 
     if (tid == 0) {
         *tainted = 0;
@@ -104,7 +111,6 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     int n_done = 0;                                  // tiles of the passes before: every barrier's phase follows from it
     int pass = 0, solo = -1;                         // solo >= 0: the pass is for this token of the segment alone
     for (int i0 = 0; i0 < ntok;) {
-        pass++;
         // ---- the segment: tokens ts .. ts + n - 1 of one sequence at positions pos0 ..; its keys lo .. hi, this CTA's tiles of them
         const int ts = t_first + i0, left = ntok - i0;
         int n, seq, pos0;
@@ -116,6 +122,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             const uint32_t cut_b = __ballot_sync(0xffffffffu, lane + 32 >= left || sb != seq || qb != pos0 + lane + 32);
             n = cut_a ? __ffs(cut_a) - 1 : cut_b ? 31 + __ffs(cut_b) : 64;
         }
+        pass++;
         const int* bt = p.block_table + (int64_t)seq * p.max_blocks_per_seq;
         const int hi = pos0 + n - 1;
         const int lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
@@ -174,7 +181,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
 #pragma unroll
             for (int b = 0; b < AT_ONCE; b++) {
                 const int i = tid + b * LT_THREADS, row = eighths > 0 ? i / eighths : LT_ROWS, d = (i - row * eighths) * 8;
-                const int j = row >> p.hp_log2, h = h0 + (row & (hp - 1));
+                const int j = head_row(row) >> p.hp_log2, h = h0 + (head_row(row) & (hp - 1));
                 c4[b] = make_float4(1.f, 1.f, 1.f, 1.f); s4[b] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (p.rot_vec && row < LT_ROWS && j < n && h < p.H) {
                     u[b] = ld_vec8(reinterpret_cast<const T*>(p.q_rot) + (int64_t)(ts + j) * p.qr_st + (int64_t)h * p.qr_sh + d);
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             }
 #pragma unroll 1
             for (int row = warp; row < LT_ROWS; row += LT_THREADS / 32) {
-                const int j = row >> p.hp_log2, h = h0 + (row & (hp - 1));
+                const int j = head_row(row) >> p.hp_log2, h = h0 + (head_row(row) & (hp - 1));
                 const bool live = j < n && h < p.H;
                 const T* ql = reinterpret_cast<const T*>(p.q_lat) + (live ? (int64_t)(ts + j) * p.ql_st + (int64_t)h * p.ql_sh : 0);
                 for (int c = lane; c < (r >> 3); c += 32) {
@@ -209,7 +216,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             for (int b = 0; b < AT_ONCE; b++) {
                 const int i = tid + b * LT_THREADS, row = eighths > 0 ? i / eighths : LT_ROWS, d = (i - row * eighths) * 8;
                 if (row >= LT_ROWS) continue;
-                const int j = row >> p.hp_log2, h = h0 + (row & (hp - 1));
+                const int j = head_row(row) >> p.hp_log2, h = h0 + (head_row(row) & (hp - 1));
                 const int64_t t = ts + j;
                 uint4 v = make_uint4(0, 0, 0, 0);
                 if (j < n && h < p.H) {
@@ -343,8 +350,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
         } else {
             // ======================================================= softmax: rows 16 w + lane / 4 (a) and + 8 (b), four lanes a row
             const int ra = 16 * warp + (lane >> 2), rb = ra + 8;
-            const int ja = ra >> p.hp_log2, jb = rb >> p.hp_log2;
-            const int ha = h0 + (ra & (hp - 1)), hb = h0 + (rb & (hp - 1));
+            const int ja = head_row(ra) >> p.hp_log2, jb = head_row(rb) >> p.hp_log2;
+            const int ha = h0 + (head_row(ra) & (hp - 1)), hb = h0 + (head_row(rb) & (hp - 1));
+            const bool rest = DUP && warp == 1;      // P is what the rounding of rows 0 .. 15 left over
             const bool live_a = ja < n && ha < p.H, live_b = jb < n && hb < p.H;
             // a row sees the keys first .. last (none in a dead row)
             const int last_a = live_a ? pos0 + ja : -1, last_b = live_b ? pos0 + jb : -1;
@@ -352,13 +360,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             const float c = p.scale * LT_LOG2E;
             float ma = -INFINITY, mb = -INFINITY, la = 0.f, lb = 0.f;
             if (p.sink != nullptr && blockIdx.z == 0) {                        // the sink counts in ONE key split
-                if (live_a) { ma = p.sink[ha] * LT_LOG2E; la = (lane & 3) == 0 ? 1.f : 0.f; }
-                if (live_b) { mb = p.sink[hb] * LT_LOG2E; lb = (lane & 3) == 0 ? 1.f : 0.f; }
+                if (live_a) { ma = p.sink[ha] * LT_LOG2E; la = (lane & 3) == 0 && !rest ? 1.f : 0.f; }
+                if (live_b) { mb = p.sink[hb] * LT_LOG2E; lb = (lane & 3) == 0 && !rest ? 1.f : 0.f; }
             }
             const uint32_t tlane = tmem + ((uint32_t)(32 * warp) << 16);
             // the row whose part of O this lane owns (lanes 16.. : its second half), and the lane that holds the row's state
             const int orow = lane & 15, from = 4 * (orow & 7);
-            uint32_t top_a = 0, top_b = 0;           // the largest magnitude (as bits) among the masked scores
+            uint32_t top = 0;                        // the largest magnitude (as bits) among the masked scores
             for (int j = 0; j < ntiles; j++) {
                 const int it = n_done + j, st = it & 1;
                 mbar_wait(smem_u32(&bars->s_full[st]), (it >> 1) & 1);
@@ -376,8 +384,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
                             const int kp = cb + 8 * i + e;
-                            if (kp > last_a || kp < first_a) { top_a = max(top_a, s[4 * i + e] & 0x7fffffffu); s[4 * i + e] = 0xff800000u; }
-                            if (kp > last_b || kp < first_b) { top_b = max(top_b, s[4 * i + 2 + e] & 0x7fffffffu); s[4 * i + 2 + e] = 0xff800000u; }
+                            if (kp > last_a || kp < first_a) { if (!DUP) top = max(top, s[4 * i + e] & 0x7fffffffu); s[4 * i + e] = 0xff800000u; }
+                            if (kp > last_b || kp < first_b) { if (!DUP) top = max(top, s[4 * i + 2 + e] & 0x7fffffffu); s[4 * i + 2 + e] = 0xff800000u; }
                         }
                 }
                 float xa = -INFINITY, xb = -INFINITY;
@@ -396,12 +404,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 const float sub_a = ma == -INFINITY ? 0.f : -ma, sub_b = mb == -INFINITY ? 0.f : -mb;      // nothing seen yet
                 uint32_t w[16];                      // P in the storage type; the sums take the rounded values
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    w[2 * i] = pack2<T>(fast_exp2_tc(fmaf(__uint_as_float(s[4 * i]), c, sub_a)), fast_exp2_tc(fmaf(__uint_as_float(s[4 * i + 1]), c, sub_a)));
-                    w[2 * i + 1] = pack2<T>(fast_exp2_tc(fmaf(__uint_as_float(s[4 * i + 2]), c, sub_b)), fast_exp2_tc(fmaf(__uint_as_float(s[4 * i + 3]), c, sub_b)));
-                    const float2 fa = Traits<T>::to_f2(*reinterpret_cast<typename Traits<T>::T2*>(&w[2 * i]));
-                    const float2 fb = Traits<T>::to_f2(*reinterpret_cast<typename Traits<T>::T2*>(&w[2 * i + 1]));
-                    la += fa.x + fa.y; lb += fb.x + fb.y;
+                for (int i = 0; i < 16; i++) {       // two keys of row a (even i) or b
+                    const float sub = i & 1 ? sub_b : sub_a;
+                    const float p0 = fast_exp2_tc(fmaf(__uint_as_float(s[2 * i]), c, sub)), p1 = fast_exp2_tc(fmaf(__uint_as_float(s[2 * i + 1]), c, sub));
+                    w[i] = pack2<T>(p0, p1);
+                    float2 f = Traits<T>::to_f2(*reinterpret_cast<typename Traits<T>::T2*>(&w[i]));
+                    if (DUP && rest) {
+                        w[i] = pack2<T>(p0 - f.x, p1 - f.y);
+                        f = Traits<T>::to_f2(*reinterpret_cast<typename Traits<T>::T2*>(&w[i]));
+                    }
+                    (i & 1 ? lb : la) += f.x + f.y;
                 }
                 // P's buffer was last read by the products of tile j - 2; a rescale needs those of tile j - 1 to be done
                 const bool rescale = j > 0 && __any_sync(0xffffffffu, need_a || need_b);
@@ -432,41 +444,69 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 tc_fence_before();
                 mbar_arrive(smem_u32(&bars->p_full[st]));
             }
-            // a row whose sum is NaN is NaN by its own keys
-            const bool odd_a = live_a && top_a >= 0x7f800000u, odd_b = live_b && top_b >= 0x7f800000u;
             // ---- output: the lane owns row orow, columns n0 * (lane / 16) ..
             la += __shfl_xor_sync(0xffffffffu, la, 1); la += __shfl_xor_sync(0xffffffffu, la, 2);
             lb += __shfl_xor_sync(0xffffffffu, lb, 1); lb += __shfl_xor_sync(0xffffffffu, lb, 2);
             const float l0 = __shfl_sync(0xffffffffu, la, from), l1 = __shfl_sync(0xffffffffu, lb, from);
             const float m0 = __shfl_sync(0xffffffffu, ma, from), m1 = __shfl_sync(0xffffffffu, mb, from);
-            const float l = orow < 8 ? l0 : l1, m = orow < 8 ? m0 : m1;
-            if (solo < 0 && n > 1 && ((odd_a && la == la) || (odd_b && lb == lb))) *tainted = pass;
-            const int row = 16 * warp + orow, jj = row >> p.hp_log2, h = h0 + (row & (hp - 1));
+            const float m = orow < 8 ? m0 : m1;
+            float l = orow < 8 ? l0 : l1;
+            // (a row whose sum is NaN is NaN by its own keys)
+            if (!DUP && solo < 0 && n > 1 && top >= 0x7f800000u && ((live_a && la == la) || (live_b && lb == lb))) *tainted = pass;
+            const int row = head_row(16 * warp + orow), jj = row >> p.hp_log2, h = h0 + (row & (hp - 1));
             const bool live = jj < n && h < p.H && (solo < 0 || jj == solo);
+            float* xs = reinterpret_cast<float*>(q_sm) + orow * LT_REST_PITCH;      // (the queries are done with)
             const int64_t t = ts + jj;
             const int col0 = lane < 16 ? 0 : n0, cols = lane < 16 ? n0 : n1;
-            float f = 0.f;
-            float* pr = nullptr;
-            if (p.nsplit > 1) {
-                pr = p.partial + ((t * p.H + h) * p.nsplit + blockIdx.z) * (r + 2);
-                if (live && lane < 16) { pr[r] = m * LT_LN2; pr[r + 1] = l; }
-            } else if (live) {
-                f = 1.f / l;
-                if (p.gate != nullptr) f *= 1.f / (1.f + expf(-ldf(reinterpret_cast<const T*>(p.gate) + t * p.gate_st + h)));
-            }
-            T* o = reinterpret_cast<T*>(p.out) + t * p.out_st + (int64_t)h * p.out_sh + col0;
             if (ntiles > 0) {
                 const int last = n_done + ntiles - 1;
                 mbar_wait(smem_u32(&bars->o_done[last & 1]), (last >> 1) & 1);
                 tc_fence_after();
             }
+            // DUP: warps 0 and 1 hold two parts of the same rows.  Each hands the other the columns that it finishes (of either half the
+            // first or the last), and both the sums
+            const int mid = DUP ? (n0 + 32) >> 6 << 5 : 0, begin = rest ? mid : 0, end = DUP && !rest ? mid : n0;
+            if (DUP && warp < 2 && ntiles > 0) {
 #pragma unroll 1
-            for (int cc = 0; cc < n0 && ntiles > 0; cc += 32) {      // (a split without keys leaves its sums alone: m = -inf is not read)
+                for (int cc = rest ? 0 : mid; cc < (rest ? mid : n0); cc += 32) {
+                    uint32_t v[32];
+                    __syncwarp();
+                    tmem_ld32(tlane + cc, v);
+                    tmem_ld_wait();
+                    if (cc < cols) {
+#pragma unroll
+                        for (int e = 0; e < 32; e += 4) *reinterpret_cast<uint4*>(xs + col0 + cc + e) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+                    }
+                }
+                if (lane < 16) xs[LT_REST_PITCH - 4 + warp] = l;
+                named_bar_sync(1, 64);
+                l += xs[LT_REST_PITCH - 3 - warp];
+            }
+            float f = 0.f;
+            float* pr = nullptr;
+            if (p.nsplit > 1) {
+                pr = p.partial + ((t * p.H + h) * p.nsplit + blockIdx.z) * (r + 2);
+                if (live && lane < 16 && !rest) { pr[r] = m * LT_LN2; pr[r + 1] = l; }
+            } else if (live) {
+                f = 1.f / l;
+                if (p.gate != nullptr) f *= 1.f / (1.f + expf(-ldf(reinterpret_cast<const T*>(p.gate) + t * p.gate_st + h)));
+            }
+            T* o = reinterpret_cast<T*>(p.out) + t * p.out_st + (int64_t)h * p.out_sh + col0;
+#pragma unroll 1
+            for (int cc = begin; cc < end && ntiles > 0; cc += 32) {      // (a split without keys leaves its sums alone: m = -inf is not read)
                 uint32_t v[32];
                 __syncwarp();
                 tmem_ld32(tlane + cc, v);
                 tmem_ld_wait();
                 if (live && cc < cols) {
+                    if (DUP) {
+#pragma unroll
+                        for (int e = 0; e < 32; e += 4) {
+                            const float4 x = *reinterpret_cast<const float4*>(xs + col0 + cc + e);
+                            v[e] = __float_as_uint(__uint_as_float(v[e]) + x.x); v[e + 1] = __float_as_uint(__uint_as_float(v[e + 1]) + x.y);
+                            v[e + 2] = __float_as_uint(__uint_as_float(v[e + 2]) + x.z); v[e + 3] = __float_as_uint(__uint_as_float(v[e + 3]) + x.w);
+                        }
+                    }
                     if (p.nsplit > 1) {
 #pragma unroll
                         for (int e = 0; e < 32; e += 2)
@@ -504,17 +544,21 @@ int launch_latent_attn_tc(LatentTc& p, bool portions, sllm_dtype_t dtype, cudaSt
     p.hp_log2 = 0;
     while ((1 << p.hp_log2) < p.H && p.hp_log2 < 6) p.hp_log2++;
     p.qt = portions ? LT_ROWS >> p.hp_log2 : 1;
+    const bool dup = !portions && p.hp_log2 <= 4;
     const dim3 grid((unsigned)cdiv(p.num_tokens, p.qt), (unsigned)cdiv(p.H, 1 << p.hp_log2), (unsigned)p.nsplit);
+    const bool full = p.r == 512 && p.dr == 64;
     SLLM_DISPATCH_DTYPE(dtype, {
         static unsigned long long configured = 0;
-        auto full = latent_attn_tc_kernel<T, true>;
-        auto any = latent_attn_tc_kernel<T, false>;
+        void (*kernels[2][2])(LatentTc) = {{latent_attn_tc_kernel<T, false, false>, latent_attn_tc_kernel<T, false, true>},
+                                           {latent_attn_tc_kernel<T, true, false>, latent_attn_tc_kernel<T, true, true>}};
         if (first_use_on_this_device(configured)) {
-            cudaError_t e = cudaFuncSetAttribute(full, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(any, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
-            SLLM_REQUIRE(e == cudaSuccess, "latent_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+            for (auto& row : kernels)
+                for (auto k : row) {
+                    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
+                    SLLM_REQUIRE(e == cudaSuccess, "latent_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+                }
         }
-        (p.r == 512 && p.dr == 64 ? full : any)<<<grid, LT_THREADS, LT_SMEM, stream>>>(p);
+        kernels[full][dup]<<<grid, LT_THREADS, LT_SMEM, stream>>>(p);
     });
     return check_launch("latent_attention (tcgen05)");
 }

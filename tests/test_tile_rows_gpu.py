@@ -269,6 +269,16 @@ def test_short_convolution_of_many_rows(dtype, lens, C, taps, wide):
 
 # ---------------------------------------------------------------- how often a result is rounded
 @pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("H,T,length", [(16, 64, 2000), (5, 40, 700), (1, 9, 3000)])
+def test_latent_decoded_tokens_round_their_weights_finely(dtype, H, T, length):
+    # without turned entries nothing but the output is rounded to 16 bits: values spread evenly over a binade's logarithm are then off by
+    # unit / sqrt(12) * sqrt(0.75 / (2 ln 2)) = 0.2123 units (root of the mean square, relative); 6 % for the draw.  Weights rounded to
+    # 16 bits, but for the largest of every key split, added a sixth
+    c = latent_case(dtype, [], [length - 7 * i for i in range(T)], H, 512, 0, 0, 0, sink=False, gated=False)
+    assert rel(latent_run(c), latent_exact(c)) < 1.06 * 0.2123 * 2 * UNIT[dtype]
+
+
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("opts", [{}, {"softcap": 5.0}, {"slopes": True}])
 def test_window_weights_sum_to_one(dtype, opts):
     # equal values come out as they are, whatever the weights were rounded to: sum and product take the same weights
