@@ -27,8 +27,8 @@
 //
 // Bound: at M = 64 the tensor core runs at half rate, (D + r) * 64 * 64 multiply-adds per tile = 2176 cycles at D = 576, r = 512, and
 // S's operands are 4 KiB of shared memory per 32 cycles; a decoded token is bound by its rows' bytes.  Measured on B200, bf16, 16 heads,
-// r = 512: four prompts of 2048 tokens 3217 us with the mma.sync kernel of latent_attn.cu -> 580 us (504 TFLOP/s); 64 decoded tokens at
-// 2048 keys 95 -> 67 us.
+// r = 512: four prompts of 2048 tokens 3214 us with the mma.sync kernel of latent_attn.cu -> 577 us (505 TFLOP/s); 64 decoded tokens at
+// 2048 keys 88 -> 54 us with the merge.
 #include "latent_attn_tc.cuh"
 #include "mma_helpers.cuh"
 #include "tc_helpers.cuh"
@@ -74,10 +74,13 @@ __device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const uint32_t (&r
 // byte offset of 16-byte piece `piece` (of 8) of row `row` in a chunk of 64 rows x 128 bytes, SWIZZLE_128B
 __device__ __forceinline__ uint32_t lt_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
 
-// FULL: r = 512 and dr = 64, known to the compiler (the producers' and the issuer's loops are bound by their instructions).  DUP: single
-// tokens of at most 16 heads, whose rows 16 .. 31 repeat rows 0 .. 15
-template <typename T, bool FULL, bool DUP>
+// FULL: r = 512 and dr = 64, known to the compiler (the producers' and the issuer's loops are bound by their instructions).  ROWS: prompt
+// rows (and single tokens of more heads); LT_SINGLES: single tokens of at most 16 heads, whose rows 16 .. 31 repeat rows 0 .. 15; LT_SHARED: prompt
+// rows of a launch that leaves SMs over, whose CTAs of the same tokens take one segment each (in the first kernel this costs 3 %)
+enum LatentRows { LT_PROMPTS, LT_SINGLES, LT_SHARED };
+template <typename T, bool FULL, LatentRows ROWS>
 __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const LatentTc p) {
+    constexpr bool DUP = ROWS == LT_SINGLES;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_sm = smem;                            // [chunk][64 rows][128 B]
     uint8_t* k_sm = smem + LT_STAGE;                 // [stage][chunk][64 keys][128 B]
@@ -89,8 +92,24 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     const int n0 = r < 256 ? r : 256, n1 = r - n0;   // columns of O in its two halves
     const int c0 = n0 >> 6, chunks = (D + 63) >> 6;  // chunks of the first piece, of a row
     const int hp = 1 << p.hp_log2, h0 = blockIdx.y * hp;
-    const int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;      // the last tokens of a prompt have the most keys: first
-    const int ntok = min(p.qt, p.num_tokens - t_first);
+    auto split = [&] { return (int)(ROWS == LT_SHARED ? blockIdx.z % p.nsplit : blockIdx.z); };      // (found where it is used)
+    int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;            // the last tokens of a prompt have the most keys: first
+    int ntok = min(p.qt, p.num_tokens - t_first);
+    if constexpr (ROWS == LT_SHARED) {               // one segment each, the last CTA what is left
+        auto length = [&](int left) {                // tokens of the segment at t_first
+            const int a = t_first + min(lane, left - 1), b = t_first + min(lane + 32, left - 1);
+            const int sa = p.tok_seq[a], sb = p.tok_seq[b], qa = p.tok_pos[a], qb = p.tok_pos[b];
+            const int seq = __shfl_sync(0xffffffffu, sa, 0), pos = __shfl_sync(0xffffffffu, qa, 0);
+            const uint32_t cut_a = __ballot_sync(0xffffffffu, lane >= left || sa != seq || qa != pos + lane);
+            const uint32_t cut_b = __ballot_sync(0xffffffffu, lane + 32 >= left || sb != seq || qb != pos + lane + 32);
+            return cut_a ? __ffs(cut_a) - 1 : cut_b ? 31 + __ffs(cut_b) : 64;
+        };
+        for (int k = blockIdx.z / p.nsplit; k > 0 && ntok > 0; k--) {
+            const int n = length(ntok);
+            t_first += n; ntok -= n;
+        }
+        if (blockIdx.z + p.nsplit < gridDim.z && ntok > 0) ntok = length(ntok);
+    }
     auto head_row = [&](int row) { return DUP && row < 32 ? row & 15 : row; };      // the row whose token and head it is
 
     if (tid == 0) {
@@ -127,7 +146,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
         const int hi = pos0 + n - 1;
         const int lo = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
         const int all = (hi - lo) / LT_KEYS + 1, per = (all + p.nsplit - 1) / p.nsplit;
-        const int tile0 = min(all, (int)blockIdx.z * per), ntiles = min(all, tile0 + per) - tile0;
+        const int tile0 = min(all, split() * per), ntiles = min(all, tile0 + per) - tile0;
         const int key0 = lo + tile0 * LT_KEYS;
         const int see_hi = solo < 0 ? hi : pos0 + solo;                        // keys outside are left zero
         const int see_lo = solo < 0 || p.window <= 0 ? lo : max(lo, pos0 + solo - p.window + 1);
@@ -359,7 +378,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             const int first_a = p.window > 0 ? last_a - p.window + 1 : 0, first_b = p.window > 0 ? last_b - p.window + 1 : 0;
             const float c = p.scale * LT_LOG2E;
             float ma = -INFINITY, mb = -INFINITY, la = 0.f, lb = 0.f;
-            if (p.sink != nullptr && blockIdx.z == 0) {                        // the sink counts in ONE key split
+            if (p.sink != nullptr && split() == 0) {                        // the sink counts in ONE key split
                 if (live_a) { ma = p.sink[ha] * LT_LOG2E; la = (lane & 3) == 0 && !rest ? 1.f : 0.f; }
                 if (live_b) { mb = p.sink[hb] * LT_LOG2E; lb = (lane & 3) == 0 && !rest ? 1.f : 0.f; }
             }
@@ -485,7 +504,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
             float f = 0.f;
             float* pr = nullptr;
             if (p.nsplit > 1) {
-                pr = p.partial + ((t * p.H + h) * p.nsplit + blockIdx.z) * (r + 2);
+                pr = p.partial + ((t * p.H + h) * p.nsplit + split()) * (r + 2);
                 if (live && lane < 16 && !rest) { pr[r] = m * LT_LN2; pr[r + 1] = l; }
             } else if (live) {
                 f = 1.f / l;
@@ -544,13 +563,19 @@ int launch_latent_attn_tc(LatentTc& p, bool portions, sllm_dtype_t dtype, cudaSt
     p.hp_log2 = 0;
     while ((1 << p.hp_log2) < p.H && p.hp_log2 < 6) p.hp_log2++;
     p.qt = portions ? LT_ROWS >> p.hp_log2 : 1;
-    const bool dup = !portions && p.hp_log2 <= 4;
-    const dim3 grid((unsigned)cdiv(p.num_tokens, p.qt), (unsigned)cdiv(p.H, 1 << p.hp_log2), (unsigned)p.nsplit);
-    const bool full = p.r == 512 && p.dr == 64;
+    dim3 grid((unsigned)cdiv(p.num_tokens, p.qt), (unsigned)cdiv(p.H, 1 << p.hp_log2), (unsigned)p.nsplit);
+    // SMs that are left over take segments of CTAs in whose tokens a sequence ends: their passes would come one after the other (three prompts
+    // of 33 tokens, 32 heads: 38 us in 50 CTAs, 16 in 100)
+    int num_sms = 0;
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, current_device());
+    const int64_t share = portions ? num_sms / ((int64_t)grid.x * grid.y * grid.z) : 1;
+    if (share > 1) grid.z *= (unsigned)(share > p.qt ? p.qt : share);
+    const int full = p.r == 512 && p.dr == 64, rows = grid.z > (unsigned)p.nsplit ? LT_SHARED : !portions && p.hp_log2 <= 4 ? LT_SINGLES : LT_PROMPTS;
     SLLM_DISPATCH_DTYPE(dtype, {
         static unsigned long long configured = 0;
-        void (*kernels[2][2])(LatentTc) = {{latent_attn_tc_kernel<T, false, false>, latent_attn_tc_kernel<T, false, true>},
-                                           {latent_attn_tc_kernel<T, true, false>, latent_attn_tc_kernel<T, true, true>}};
+        void (*kernels[2][3])(LatentTc) = {
+            {latent_attn_tc_kernel<T, false, LT_PROMPTS>, latent_attn_tc_kernel<T, false, LT_SINGLES>, latent_attn_tc_kernel<T, false, LT_SHARED>},
+            {latent_attn_tc_kernel<T, true, LT_PROMPTS>, latent_attn_tc_kernel<T, true, LT_SINGLES>, latent_attn_tc_kernel<T, true, LT_SHARED>}};
         if (first_use_on_this_device(configured)) {
             for (auto& row : kernels)
                 for (auto k : row) {
@@ -558,7 +583,7 @@ int launch_latent_attn_tc(LatentTc& p, bool portions, sllm_dtype_t dtype, cudaSt
                     SLLM_REQUIRE(e == cudaSuccess, "latent_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
                 }
         }
-        kernels[full][dup]<<<grid, LT_THREADS, LT_SMEM, stream>>>(p);
+        kernels[full][rows]<<<grid, LT_THREADS, LT_SMEM, stream>>>(p);
     });
     return check_launch("latent_attention (tcgen05)");
 }

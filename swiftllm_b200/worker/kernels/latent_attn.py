@@ -21,9 +21,10 @@ def latent_kv_store(dkv: torch.Tensor, norm_weight: torch.Tensor, cache: torch.T
 _SM_COUNT = {}
 
 
-def _num_splits(rows: int, H: int, r: int, dr: int, window: int, dtype, portions: bool) -> int:
-    """Key splits of a launch over `rows` tokens (prompt portions or single decoded tokens): as many CTAs as fit at once when the rows
-    alone leave SMs idle, never a second wave; never more than the 64-key tiles a window can hold (16 when there is no window)."""
+def _num_splits(rows: int, H: int, r: int, dr: int, window: int, dtype, portions: bool, seqs: int = 1) -> int:
+    """Key splits of a launch over `rows` tokens (portions of `seqs` prompts, or single decoded tokens): as many CTAs as fit at once when
+    the rows alone leave SMs idle, never a second wave; never more than the 64-key tiles a window can hold (16 when there is no window).
+    Several prompts leave half the SMs to the second segments of CTAs in which one ends (three of 33 tokens, 16 heads: 38 -> 32 us)."""
     if dtype == torch.float32:
         return 1
     dev = torch.cuda.current_device()
@@ -34,7 +35,7 @@ def _num_splits(rows: int, H: int, r: int, dr: int, window: int, dtype, portions
         while heads < H and heads < 64:
             heads *= 2
         per = 64 // heads if portions else 1
-        ctas, room = -(-rows // per) * -(-H // heads), _SM_COUNT[dev]
+        ctas, room = -(-rows // per) * -(-H // heads), _SM_COUNT[dev] // (2 if portions and seqs > 1 else 1)
     else:                                                              # two CTAs per SM, one token and 16 heads each
         ctas, room = rows * ((H + 15) // 16), 2 * _SM_COUNT[dev]
     most = (window + 63) // 64 + 1 if window > 0 else 16
@@ -66,7 +67,7 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, gate, cache: torc
     for i, rows, portions in ((0, npre, True), (npre, T - npre, False)):       # i: the part's first row
         if rows == 0:
             continue
-        nsplit = _num_splits(rows, H, r, dr, window, q_lat.dtype, portions)
+        nsplit = _num_splits(rows, H, r, dr, window, q_lat.dtype, portions, int(getattr(infer_state, "num_prefill_seqs", 1)))
         ws = torch.empty((rows, H, nsplit, r + 2), dtype=torch.float32, device=q_lat.device) if nsplit > 1 else None
         _lib.check((lib.sllm_latent_attention_portions if portions else lib.sllm_latent_attention)(
             ql + i * ql_t * es, ql_t, ql_h, qr + i * qr_t * es, qr_t, qr_h, c + i * half if c else None, sn + i * half if sn else None,
