@@ -130,7 +130,8 @@ int sllm_prefill_attention_paged(const void* q, const void* k_cache, const void*
                                  int max_blocks_per_seq, int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype,
                                  sllm_stream_t stream);
 /* The same; with num_splits > 1 and a workspace of num_splits * num_prefill_tokens * nq * (head_dim + 2) floats the tcgen05 kernel shares a
- * query block's keys between num_splits CTAs (steps with few query blocks), merged by a second kernel.  Other shapes ignore both. */
+ * query block's keys between num_splits CTAs (steps with few query blocks), merged by a second kernel over the rows of the sequences.  Other
+ * shapes ignore both. */
 int sllm_prefill_attention_paged_split(const void* q, const void* k_cache, const void* v_cache, void* o,
                                  const int32_t* block_table, const int32_t* seq_ids,
                                  const int32_t* prefill_seq_start_locs, const int32_t* prefill_seq_lens,
@@ -138,8 +139,7 @@ int sllm_prefill_attention_paged_split(const void* q, const void* k_cache, const
                                  int max_prefill_len, int64_t num_prefill_tokens, int cur_layer, int num_layers,
                                  int num_q_heads, int num_kv_heads, int block_size, int head_dim,
                                  int max_blocks_per_seq, int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype,
-                                 sllm_stream_t stream,
-                                       int num_splits, void* workspace);
+                                 sllm_stream_t stream, int num_splits, void* workspace);
 
 /* ---- Block-table maintenance: swiftllm/worker/kernels/block_mgmt.py:26-46, :66-80, :106-127
  * block_table int32 [max_seqs, max_blocks_per_seq]; num_seq_allocated_blocks int32 [max_seqs];

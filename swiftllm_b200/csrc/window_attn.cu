@@ -3,8 +3,9 @@
 //   score(i, j) = rope(q[i,h]) . k[j, g(h)] * scale          g(h) = h / (H / G)
 //   p(i, j)     = exp(score) / (sink + sum_j' exp(score))     sink = 1 when the softmax has a value-less sink of score 0, else 0
 //   out[i, h]   = sigmoid(gate[i, h, :]) * sum_j p(i, j) v[j, g(h)]          (element-wise gate; no gate when null)
-// Every token of the step is a query with its own (block-table row, position), whose result depends on its own keys only; how its
-// sequence was cut into steps changes it by rounding (prompt rows and decoded rows run different kernels in 16 bits).  A query at
+// Every token of the step is a query with its own (block-table row, position), whose result depends on its own keys only (values that are
+// not finite reach the tokens of a common 64-row tile in the mma.sync kernel of prompt rows); how its sequence was cut into steps
+// changes it by rounding (prompt rows and decoded rows run different kernels in 16 bits).  A query at
 // position p sees the positions max(0, p - window + 1) .. p (window <= 0: all of 0 .. p).  Rotary pairs are interleaved
 // ((2i, 2i+1)) or halves ((i, i + rot_dims/2)) of the first rot_dims entries of a head; the rest pass through; the caller's
 // cos / sin tables carry the frequencies (and any common factor on both).  Softmax, rotation and the weighted sum of values

@@ -40,7 +40,7 @@ def token_state(portions, decodes):
     rows = portions + [(1, p) for p in decodes]
     return rows, types.SimpleNamespace(
         token_seq_ids=ints(i for i, (n, _) in enumerate(rows) for _ in range(n)),
-        token_positions=ints(p + j for n, p in rows for j in range(n)), num_prefill_tokens=sum(n for n, _ in portions))
+        token_positions=ints(p + j for n, p in rows for j in range(n)), num_prefill_tokens=sum(n for n, _ in portions), num_prefill_seqs=len(portions))
 
 
 def angles(positions, dims):
