@@ -380,10 +380,10 @@ constexpr int SS_ITEMS = 8;
 constexpr int SS_BCR = 4;
 
 // VEC (16-bit rows in 16-byte pieces, states in whole eights): a thread brings eight neighbouring channels of ONE token and eight entries of
-// B or C per tile, with one address each, and stores eight outputs; the SiLU of the gate takes the special-function unit's exponential
-// and quotient.  Measured on B200, bf16, 4 x 2048 tokens, 4096 channels, 16 states: 813 -> 370 us (staging took 85
-// of 125 instructions per token; with the shape unknown to the compiler 541 us); one segment of 1024 tokens 426 -> 122 us.  What
-// remains is issue and the special-function unit (21 results per token and channel: 150 us).
+// B or C per tile, with one address each, and stores eight outputs.  Measured on B200, bf16, 4 x 2048 tokens, 4096 channels, 16 states: 813 ->
+// 380 us (staging took 85 of 125 instructions per token; with the shape unknown to the compiler 541 us; a quick SiLU of the gate instead of
+// the exact one 370); one segment of 1024 tokens 426 -> 122 us.  What remains is shared memory (76 % of its rate), then issue and the
+// special-function unit (21 results per token and channel: 150 us).
 // NSL >= 0: 16 states on 2^NSL lanes, known to the compiler.
 template <typename T, typename TD, bool VEC, int NSL>
 __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
