@@ -45,6 +45,20 @@ int sllm_rmsnorm_inplace(void* x, const void* weight, float eps, int64_t num_tok
 int sllm_fused_add_rmsnorm_inplace(void* x, void* residual, const void* weight, float eps, int64_t num_tokens,
                                    int hidden, sllm_dtype_t dtype, sllm_stream_t stream);
 
+/* add_rmsnorm_rows: out [num_rows, hidden] <- rmsnorm(x + residual, rounded to dtype) * weight of the rows rows[] (int32) of x, residual
+ * [num_tokens, hidden], which stay as they are: final add, last-token gather and norm (swiftllm/worker/layers/post_layer.py:19-33). */
+int sllm_add_rmsnorm_rows(const void* x, const void* residual, const void* rows, const void* weight, float eps, int64_t num_rows,
+                          int64_t num_tokens, int hidden, void* out, sllm_dtype_t dtype, sllm_stream_t stream);
+
+/* ---- Rows around the layers (pre_layer.py:17-20, model.py:341-342, post_layer.py:37-39)
+ * gather_rows: out_a[t] <- table_a[idx[t] + offset] (idx int32), out_b[t] <- the same row of table_b, or zeros (table_b NULL);
+ * row lengths in bytes, even; row_bytes_b 0: no second output.
+ * argmax_rows: out int64 [num_rows] <- the index of the largest of n entries (the smallest index among equals, NaN above all). */
+int sllm_gather_rows(const void* idx, int offset, int64_t num_rows, int64_t table_rows, const void* table_a, void* out_a,
+                     int64_t row_bytes_a, const void* table_b, void* out_b, int64_t row_bytes_b, sllm_stream_t stream);
+int sllm_argmax_rows(const void* x, int64_t row_stride, int64_t num_rows, int64_t n, void* out, sllm_dtype_t dtype,
+                     sllm_stream_t stream);
+
 /* ---- Rotary embedding: swiftllm/worker/kernels/rotary_emb.py:44-58 (rotary_embedding_inplace)
  * q [T, nq, D], k [T, nkv, D] in place; cos/sin [T, D/2] (infer_state.position_cos/sin).  NeoX half-split.
  * D % 16 == 0.  *_row_stride: elements between consecutive token rows (nq*D / nkv*D when contiguous, as in the

@@ -25,6 +25,9 @@ SIGNATURES = {
     "sllm_device_check": (_I, [_I]),
     "sllm_rmsnorm_inplace": (_I, [_P, _P, _F, _L, _I, _I, _P]),
     "sllm_fused_add_rmsnorm_inplace": (_I, [_P, _P, _P, _F, _L, _I, _I, _P]),
+    "sllm_add_rmsnorm_rows": (_I, [_P, _P, _P, _P, _F, _L, _L, _I, _P, _I, _P]),
+    "sllm_gather_rows": (_I, [_P, _I, _L, _L, _P, _P, _L, _P, _P, _L, _P]),
+    "sllm_argmax_rows": (_I, [_P, _L, _L, _L, _P, _I, _P]),
     "sllm_rotary_embedding_inplace": (_I, [_P, _P, _P, _P, _L, _I, _I, _I, _L, _L, _I, _P]),
     "sllm_silu_and_mul_inplace": (_I, [_P, _L, _L, _I, _P]),
     "sllm_store_kvcache": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _L, _I, _I, _I, _I, _I, _I, _I, _L, _L, _I, _P]),

@@ -3,12 +3,15 @@
 Addition (tensor parallelism): with a vocabulary-sharded lm_head every rank computes the logits of its
 V / tp_size rows only and the greedy token is found with ONE all-gather of per-rank (max logit, global index) pairs
 (8 bytes per sequence and rank) instead of every rank streaming the whole lm_head."""
+from typing import Optional
+
 import torch
 import torch.distributed as dist
 
 from swiftllm_b200.worker.infer_state import LlamaInferState
 from swiftllm_b200.worker.kernels.linear import linear
 from swiftllm_b200.worker.kernels.rmsnorm import rmsnorm_inplace
+from swiftllm_b200.worker.kernels.row_ops import add_rmsnorm_rows, argmax_rows
 
 
 def merge_sharded_argmax(pairs: torch.Tensor) -> torch.Tensor:
@@ -31,8 +34,10 @@ class LlamaPostLayer:
         self.last_logits = None     # kept for parity tests (the reference discards them)
         self.keep_logits = False
 
-    def forward(self, input_embds: torch.Tensor, infer_state: LlamaInferState, already_normed: bool = False) -> torch.Tensor:
-        """`already_normed`: input_embds rows are rmsnorm(final residual) already (TP fused-exchange path; RMSNorm is
+    def forward(self, input_embds: torch.Tensor, infer_state: LlamaInferState, already_normed: bool = False,
+                residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """`residual`: the stream that the last layer's output has yet to be added to.
+        `already_normed`: input_embds rows are rmsnorm(final residual) already (TP fused-exchange path; RMSNorm is
         row-wise, so normalising before or after the last-token gather is the same computation)."""
         idx = infer_state.last_token_indices
         if idx is None:
@@ -40,17 +45,21 @@ class LlamaPostLayer:
                 infer_state.prefill_seq_start_locs + infer_state.prefill_seq_lens - 1,
                 torch.arange(infer_state.num_prefill_tokens, infer_state.num_tokens, device=input_embds.device, dtype=torch.int32)
             ), dim=0)
-        last_input = input_embds.index_select(0, idx)          # [batch_size, hidden_size], fresh contiguous buffer
-        if not already_normed:
-            rmsnorm_inplace(last_input, self.weights.final_norm, self.model_config.rms_norm_eps)
+        # last_input [batch_size, hidden_size]: a fresh contiguous buffer
+        if residual is not None and input_embds.is_cuda:
+            last_input = add_rmsnorm_rows(input_embds, residual, idx, self.weights.final_norm, self.model_config.rms_norm_eps)
+        else:
+            last_input = (input_embds if residual is None else input_embds + residual).index_select(0, idx)
+            if not already_normed:
+                rmsnorm_inplace(last_input, self.weights.final_norm, self.model_config.rms_norm_eps)
         logits = linear(last_input, self.weights.lm_head)      # [batch_size, vocab_size] (or this rank's V / tp_size columns)
         if not self.sharded:
             if self.keep_logits:
                 self.last_logits = logits
-            return torch.argmax(logits, dim=1)
+            return argmax_rows(logits)
 
         B, Vs = logits.shape
-        local = torch.argmax(logits, dim=1)
+        local = argmax_rows(logits)
         mine = torch.stack((logits.gather(1, local[:, None]).squeeze(1).float(),
                             (local + self.tp_rank * Vs).float()), dim=1)             # [B, 2]
         # outputs in the concatenated form ([ranks * B, ...]): accepted by both NCCL and gloo

@@ -30,6 +30,7 @@ from swiftllm_b200.worker.block_manager import BlockManager
 from swiftllm_b200.worker.weight import load_weights
 
 from .infer_state import LlamaInferState
+from .kernels.row_ops import gather_two
 from .model_base import PagedModelBase
 from .layers.post_layer import LlamaPostLayer
 from .layers.pre_layer import LlamaPreLayer
@@ -235,9 +236,8 @@ class LlamaModel(PagedModelBase):
     def _forward(self, input_ids: torch.Tensor, infer_state: LlamaInferState, k_cache=None, v_cache=None,
                  block_table=None) -> torch.Tensor:
         """model.py:228-249."""
-        input_embds = self.pre_layer.forward(input_ids)
+        input_embds, residual_buf = self.pre_layer.forward_with_residual(input_ids)
         self._wait_for_swaps()          # first KV-cache access of the step is layer 0's store: pending swap copies must be done
-        residual_buf = torch.zeros_like(input_embds)
         k_cache = self.k_cache if k_cache is None else k_cache
         v_cache = self.v_cache if v_cache is None else v_cache
         if block_table is None and not infer_state.ignore_kvcache:
@@ -249,8 +249,7 @@ class LlamaModel(PagedModelBase):
             normed = self.comm.reduce_add_norm(1, residual_buf.shape[0], residual_buf, self.weight.final_norm,
                                                self.model_config.rms_norm_eps)
             return self.post_layer.forward(normed, infer_state, already_normed=True)
-        input_embds += residual_buf
-        return self.post_layer.forward(input_embds, infer_state)
+        return self.post_layer.forward(input_embds, infer_state, residual=residual_buf)
 
     @torch.inference_mode()
     def forward(self, input_ids_list: list, seq_ids_list: list, decoding_seq_lens_list: list,
@@ -309,6 +308,7 @@ class LlamaModel(PagedModelBase):
                                                             target_lens_list=seq_lengths_list, want_new_blocks=False)
 
         seq_block_size = select_seq_block_size(mc.num_kv_heads, list(decoding_seq_lens_list), max_decoding_len)
+        position_cos, position_sin = gather_two(self._cos_cached, self._sin_cached, pos)
         infer_state = LlamaInferState(
             batch_size=batch_size, num_tokens=num_tokens,
             seq_ids=seq_ids, softmax_scale=mc.head_dim ** -0.5,
@@ -322,7 +322,7 @@ class LlamaModel(PagedModelBase):
             num_decoding_seqs=batch_size - num_prefill_seqs, decoding_seq_lens=seq_lengths[num_prefill_seqs:],
             max_decoding_len=max_decoding_len,
             seq_block_size=seq_block_size, num_seq_blocks=(max_decoding_len + seq_block_size - 1) // seq_block_size,
-            position_cos=self._cos_cached.index_select(0, pos), position_sin=self._sin_cached.index_select(0, pos),
+            position_cos=position_cos, position_sin=position_sin,
             ignore_kvcache=ignore_kvcache,
             paged_attn_seq_block_size=0, last_token_indices=last,
             prefill_prefix_lens=p_prefix if chunked else None,
@@ -392,14 +392,14 @@ class LlamaModel(PagedModelBase):
         def step(bm, k_cache, v_cache):
             alloc_kernel(bm.num_seq_allocated_blocks, bm.block_table, bm.is_block_free, seq_ids, lens, bm.block_size,
                          None, bm._status)
-            pos = (lens - 1).long()
+            position_cos, position_sin = gather_two(self._cos_cached, self._sin_cached, lens, -1)
             st = LlamaInferState(
                 batch_size=B, num_tokens=B, seq_ids=seq_ids, softmax_scale=mc.head_dim ** -0.5,
                 num_prefill_seqs=0, num_prefill_tokens=0, prefill_seq_start_locs=empty,
                 prefill_seq_start_locs_with_end=empty, prefill_seq_lens=empty, max_prefill_len=0,
                 num_decoding_seqs=B, decoding_seq_lens=lens, max_decoding_len=bucket_len,
                 seq_block_size=2048, num_seq_blocks=(bucket_len + 2047) // 2048,
-                position_cos=self._cos_cached.index_select(0, pos), position_sin=self._sin_cached.index_select(0, pos),
+                position_cos=position_cos, position_sin=position_sin,
                 ignore_kvcache=False, paged_attn_seq_block_size=0, last_token_indices=last)
             return self._forward(ids, st, k_cache=k_cache, v_cache=v_cache, block_table=bm.block_table)
 

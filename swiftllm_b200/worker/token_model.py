@@ -36,6 +36,7 @@ from swiftllm_b200.worker.block_manager import BlockManager
 from swiftllm_b200.worker.state_manager import SequenceStateManager
 
 from .infer_state import TokenInferState
+from .kernels.row_ops import argmax_rows
 from .model_base import PagedModelBase
 
 _DTYPES = {"float16": torch.float16, "bfloat16": torch.bfloat16, "float32": torch.float32}
@@ -79,7 +80,7 @@ def rotary_frequencies(base: float, dims: int, scaling: Optional[tuple] = None):
 
 class TokenBatchModel(PagedModelBase):
     # CUDA sources this worker's kernels live in (build(only=...) compiles just these in a fresh checkout)
-    NATIVE_SOURCES = ("host.cu", "kvcache.cu")
+    NATIVE_SOURCES = ("host.cu", "kvcache.cu", "row_ops.cu")
     DTYPES = tuple(_DTYPES)
     CONFIG_CLASS = None         # the design's configuration class (model_config.py)
 
@@ -238,7 +239,7 @@ class TokenBatchModel(PagedModelBase):
             max_prefill_len=max(prefill_lens, default=0), seg_starts=seg)
         logits = self._forward(ids, st)
         self.last_logits = logits[batch_size:].float() if logit_rows else None
-        return torch.argmax(logits[:batch_size], dim=1)
+        return argmax_rows(logits[:batch_size])
 
     # ------------------------------------------------------------------ CUDA-graph decode path
     def _decode_step(self, ids, seq_ids, lens, bm, caches, states=None):
@@ -258,7 +259,7 @@ class TokenBatchModel(PagedModelBase):
             logits = self._forward(ids, st)
         finally:
             self.caches, self.gpu_block_manager, self.seq_states = saved
-        return torch.argmax(logits, dim=1)
+        return argmax_rows(logits)
 
     def _forward_decode_graph(self, flat_ids, seq_ids_list, lens_list) -> torch.Tensor:
         """Pure-decode step replayed from a CUDA graph (one graph per batch size; nothing in the step depends on the lengths
