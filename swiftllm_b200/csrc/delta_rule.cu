@@ -1,5 +1,5 @@
-// Gated delta rule with one decay per head (head_decay.cuh, DELTA).
-#include "head_decay.cuh"
+// Gated delta rule with one decay per head (head_decay.cuh, DELTA; prompt portions of 16-bit rows: delta_chunk.cuh).
+#include "delta_chunk.cuh"
 
 using namespace sllm;
 
@@ -19,5 +19,9 @@ extern "C" int sllm_delta_rule(const void* q, int64_t q_stride, const void* k, i
     a.seg_starts = (const int*)seg_starts; a.seq_ids = (const int*)seq_ids; a.tok_pos = (const int*)tok_pos;
     a.o_raw = (float*)workspace; a.out = out; a.out_stride = out_stride;
     a.num_segs = num_segs; a.H = num_heads; a.G = num_kv_heads; a.dk = dk; a.dv = dv;
-    return hd_run<true>(a, dtype, num_tokens, num_prefill_tokens, num_prefill_segs, workspace_floats, (cudaStream_t)stream);
+    return hd_run<true>(a, dtype, num_tokens, num_prefill_tokens, num_prefill_segs, workspace_floats, (cudaStream_t)stream,
+                        [&](const HeadDecayArgs& x, int num_sms, cudaStream_t s) {
+                            if (!delta_chunk_takes(x, dtype)) return 0;
+                            return dtype == SLLM_F16 ? delta_chunk<__half>(x, num_sms, s) : delta_chunk<__nv_bfloat16>(x, num_sms, s);
+                        });
 }

@@ -177,6 +177,12 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
         : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return o;
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 o;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return o;
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float o;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(o) : "f"(a), "f"(b), "f"(c));
