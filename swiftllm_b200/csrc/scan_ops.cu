@@ -23,14 +23,30 @@ __device__ __forceinline__ float silu_fn(float z) { return z / (1.f + expf(-z));
 // The same for eight entries at a time: a quotient without a branch, by one step of Newton's iteration for the reciprocal and Markstein's
 // correction of the quotient by its remainder, which rounds it as the exact one (4 x 2048 tokens x 4096 channels 470 -> 460 us in all).
 // The factors of 1/4 keep the reciprocal of a denominator near 2^128 in range.
-__device__ __forceinline__ float silu_rows(float z) {
-    const float d = 1.f + expf(-z), df = fminf(d, 0x1p127f);        // (d = infinity: reciprocal and quotient 0)
-    float r = __fdividef(1.f, d * 0.25f) * 0.25f;
-    r = fmaf(r, fmaf(-df, r, 1.f), r);
-    const float q = z * r;
-    return fmaf(fmaf(-df, q, z), r, q);
+__device__ __forceinline__ float2 silu_rows(float2 z) {
+    constexpr float MOST = 3.402823466e38f;
+    const float2 d = make_float2(1.f + expf(-z.x), 1.f + expf(-z.y)), df = make_float2(-fminf(d.x, MOST), -fminf(d.y, MOST));
+    const float2 quarter = make_float2(0.25f, 0.25f), d4 = tc::mul2(d, quarter);        // (d = infinity: reciprocal and quotient 0)
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d4.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d4.y));
+    r = tc::mul2(r, quarter);
+    r = tc::fma2(r, tc::fma2(df, r, make_float2(1.f, 1.f)), r);
+    const float2 q = tc::mul2(z, r);
+    const float2 left = tc::fma2(df, q, z);                         // (z = infinity: not a number, and the quotient stands)
+    return tc::fma2(make_float2(fminf(left.x, MOST), fminf(left.y, MOST)), r, q);
 }
 __device__ __forceinline__ float softplus_fn(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+// max(z, 0) + log(1 + u), u = e^-|z|, for two entries at a time: log(1 + u) = u P(u), P of degree 9 from log(1 + u) / u at the Chebyshev
+// points of [0, 1] (interpolation error 2^-27; in fp32 at most 2.1 and in the mean square 0.55 of 2^-24, log1pf's 3.4 and 0.56).
+__device__ __forceinline__ float2 softplus_rows(float2 z) {
+    const float2 u = make_float2(expf(-fabsf(z.x)), expf(-fabsf(z.y)));
+    constexpr float c[10] = {1.000000000e+00f, -4.999989271e-01f, 3.332971036e-01f, -2.495161593e-01f, 1.966327429e-01f, -1.526966691e-01f, 1.054362357e-01f, -5.637361482e-02f, 1.954252832e-02f, -3.176057013e-03f};
+    float2 y = make_float2(c[9], c[9]);
+#pragma unroll
+    for (int i = 8; i >= 0; i--) y = tc::fma2(y, u, make_float2(c[i], c[i]));
+    return tc::fma2(y, u, make_float2(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f)));
+}
 // 2^x for x <= 0 on the special-function unit (relative error about 2^-22; results below the normal range become 0)
 __device__ __forceinline__ float exp2_neg(float x) {
     float y;
@@ -100,12 +116,13 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TI* __restrict__ 
     }
 }
 
-// The same for prompt rows where rows are whole pieces of four channels: a thread walks SV_TOKENS rows of four neighbouring channels, eight
-// rows' loads in flight together (wider pieces need 154 registers and leave ten warps on an SM: 96 us); where the rows of the tile break
-// (another sequence) is found once per warp.  The products, their order and the SiLU are those above (a quicker quotient turns some
-// roundings, which a state behind the convolution keeps).  Bound: bytes, of which enough are in flight only with many warps.  Measured on
-// B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 -> about 80 us (59 with a quicker quotient).
-constexpr int SV_TOKENS = 16;
+// The same for prompt rows where rows are whole pieces of four channels: a thread walks SV_TOKENS rows of four neighbouring channels, two at a
+// time in packed arithmetic, the next four rows' loads in flight beside the four it works on (wider pieces need 154 registers and leave
+// ten warps on an SM: 96 us; eight rows 60, two 58); where the rows of the tile break (another sequence) is found once per warp.  The products, their order and
+// the SiLU's value are those above (a quicker quotient turns some roundings, which a state behind the convolution keeps).  Bound: bytes,
+// of which enough are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 us by the kernel
+// above; a channel's SiLU with a branch, sixteen rows, loads after the work on the rows before them 75; now 54.
+constexpr int SV_TOKENS = 32;
 template <typename TI, typename TO, int K>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restrict__ xin, int64_t xin_stride, const float* __restrict__ w,
                                                              const float* __restrict__ bias, const TI* __restrict__ tail,
@@ -117,86 +134,92 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restric
     const int64_t tile0 = (int64_t)blockIdx.x * SV_TOKENS;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VW, lane = threadIdx.x & 31;
     const int nrows = (int)min((int64_t)SV_TOKENS, row_end - tile0);
-    // bit i: row tile0 - H + i continues the row above it (lanes H .. H + SV_TOKENS - 1 are the tile's own rows)
-    uint32_t goes_on;
-    int my_seq = -1, my_pos = -1;
-    {
-        const int64_t t = tile0 - H + lane;
-        const bool in = lane < H + SV_TOKENS && t >= 0 && t < row_end;
-        if (in) { my_seq = tok_seq[t]; my_pos = tok_pos[t]; }
-        const int above_seq = in && t > 0 ? tok_seq[t - 1] : -1, above_pos = in && t > 0 ? tok_pos[t - 1] : -2;
-        goes_on = __ballot_sync(0xffffffffu, in && t > 0 && above_seq == my_seq && above_pos + 1 == my_pos);
+    // bit i of the two: row tile0 - H + i continues the row above it (bits H .. H + SV_TOKENS - 1 are the tile's own rows)
+    uint32_t goes_on[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int64_t t = tile0 - H + lane + 32 * q;
+        const bool in = t > 0 && t < row_end && t < tile0 + SV_TOKENS;
+        goes_on[q] = __ballot_sync(0xffffffffu, in && tok_seq[in ? t : 0] == tok_seq[in ? t - 1 : 0] && tok_pos[in ? t : 0] == tok_pos[in ? t - 1 : 0] + 1);
     }
     const bool live = c < C;
     const int cc = live ? c : 0;
     const TI* col = xin + cc;
-    constexpr int AT_ONCE = 8;                          // rows whose loads are in flight together
-    In cur[AT_ONCE];
-    auto load = [&](int i0) {
+    constexpr int AT_ONCE = 4;                          // rows whose loads are in flight together
+    In cur[AT_ONCE], next[AT_ONCE];
+    auto load = [&](int i0, In (&to)[AT_ONCE]) {
         const TI* at = col + (tile0 + i0) * xin_stride;
 #pragma unroll
         for (int u = 0; u < AT_ONCE; u++, at += xin_stride)
-            if (i0 + u < nrows) cur[u] = *reinterpret_cast<const In*>(at);
+            if (i0 + u < nrows) to[u] = *reinterpret_cast<const In*>(at);
     };
-    load(0);
-    float wk[K][VW], b0[VW];
+    load(0, cur);
+    float2 wk[K][VW / 2], b0[VW / 2];                   // two channels at a time: packed arithmetic
 #pragma unroll
     for (int e = 0; e < VW; e++) {
-        b0[e] = bias != nullptr ? bias[cc + e] : 0.f;
+        float* b = &b0[e / 2].x + (e & 1);
+        *b = bias != nullptr ? bias[cc + e] : 0.f;
         if (K == 4) {
             const float4 f = *reinterpret_cast<const float4*>(w + (int64_t)(cc + e) * 4);
-            wk[3 % K][e] = f.x; wk[2][e] = f.y; wk[1][e] = f.z; wk[0][e] = f.w;
+            const float taps[4] = {f.w, f.z, f.y, f.x};
+#pragma unroll
+            for (int k = 0; k < K; k++) (&wk[k][e / 2].x)[e & 1] = taps[k];
         } else {
 #pragma unroll
-            for (int k = 0; k < K; k++) wk[k][e] = w[(int64_t)(cc + e) * K + (K - 1 - k)];
+            for (int k = 0; k < K; k++) (&wk[k][e / 2].x)[e & 1] = w[(int64_t)(cc + e) * K + (K - 1 - k)];
         }
     }
-    float hist[H][VW];                                  // hist[k - 1]: the input k positions back
+    float2 hist[H][VW / 2];                             // hist[k - 1]: the input k positions back
 #pragma unroll
     for (int k = 0; k < H; k++)
 #pragma unroll
-        for (int e = 0; e < VW; e++) hist[k][e] = 0.f;
-    auto refill = [&](int i) {                          // the window of row i, which does not go on from the row before it in registers
-        const int64_t t = tile0 + i;
-        const int seq = __shfl_sync(0xffffffffu, my_seq, H + i), pos = __shfl_sync(0xffffffffu, my_pos, H + i);
+        for (int e = 0; e < VW / 2; e++) hist[k][e] = make_float2(0.f, 0.f);
+    auto refill = [&](int i, uint32_t on) {             // the window of row i, which does not go on from the row before it in registers
+        const int64_t t = tile0 + i;                    // (on: goes_on from row i - H on)
+        const int seq = tok_seq[t], pos = tok_pos[t];
         int above = 0;                                  // rows above this one that are the sequence's previous positions
-        while (above < H && ((goes_on >> (H + i - above)) & 1)) above++;
+        while (above < H && ((on >> (H - above)) & 1)) above++;
 #pragma unroll
         for (int k = 1; k <= H; k++) {
             if (pos - k < 0) {
 #pragma unroll
-                for (int e = 0; e < VW; e++) hist[k - 1][e] = 0.f;
+                for (int e = 0; e < VW / 2; e++) hist[k - 1][e] = make_float2(0.f, 0.f);
             } else {
                 const In v = *reinterpret_cast<const In*>(k <= above ? col + (t - k) * xin_stride : tail + ((int64_t)seq * H + (H - (k - above))) * C + cc);
 #pragma unroll
-                for (int e = 0; e < VW; e++) hist[k - 1][e] = cvt_f(v.e[e]);
+                for (int e = 0; e < VW / 2; e++) hist[k - 1][e] = make_float2(cvt_f(v.e[2 * e]), cvt_f(v.e[2 * e + 1]));
             }
         }
     };
 #pragma unroll 1
     for (int i0 = 0; i0 < nrows; i0 += AT_ONCE) {
+        load(i0 + AT_ONCE, next);
 #pragma unroll
         for (int u = 0; u < AT_ONCE; u++) {
             const int i = i0 + u;
             if (i >= nrows) break;
-            if (i == 0 || !((goes_on >> (H + i)) & 1)) refill(i);
+            if (i == 0 || !((goes_on[0] >> (H + u)) & 1)) refill(i, goes_on[0] >> u);
             Out o;
 #pragma unroll
-            for (int e = 0; e < VW; e++) {
-                const float x = cvt_f(cur[u].e[e]);
-                float acc = b0[e] + wk[0][e] * x;
+            for (int e = 0; e < VW / 2; e++) {
+                const float2 x = make_float2(cvt_f(cur[u].e[2 * e]), cvt_f(cur[u].e[2 * e + 1]));
+                float2 acc = tc::fma2(wk[0][e], x, b0[e]);
 #pragma unroll
-                for (int k = 1; k < K; k++) acc += wk[k][e] * hist[k - 1][e];
-                if (act_silu) acc = silu_fn(acc);
-                if (add_input) acc += x;
-                stf(&o.e[e], acc);
+                for (int k = 1; k < K; k++) acc = tc::fma2(wk[k][e], hist[k - 1][e], acc);
+                if (act_silu) acc = silu_rows(acc);
+                if (add_input) acc = tc::add2(acc, x);
+                stf(&o.e[2 * e], acc.x);
+                stf(&o.e[2 * e + 1], acc.y);
 #pragma unroll
                 for (int k = H - 1; k >= 1; k--) hist[k][e] = hist[k - 1][e];
                 hist[0][e] = x;
             }
             if (live) *reinterpret_cast<Out*>(out + (tile0 + i) * C + c) = o;
         }
-        load(i0 + AT_ONCE);
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; u++) cur[u] = next[u];
+        goes_on[0] = __funnelshift_r(goes_on[0], goes_on[1], AT_ONCE);
+        goes_on[1] >>= AT_ONCE;
     }
 }
 
@@ -380,19 +403,15 @@ constexpr int SS_ITEMS = 8;
 constexpr int SS_BCR = 4;
 
 // VEC (16-bit rows in 16-byte pieces, states in whole eights): a thread brings eight neighbouring channels of ONE token and eight entries of
-// B or C per tile, with one address each, and stores eight outputs.  Measured on B200, bf16, 4 x 2048 tokens, 4096 channels, 16 states: 813 ->
-// 380 us (staging took 85 of 125 instructions per token; with the shape unknown to the compiler 541 us; a quick SiLU of the gate instead of
-// the exact one 370); one segment of 1024 tokens 426 -> 122 us.  What remains is shared memory (76 % of its rate), then issue and the
-// special-function unit (21 results per token and channel: 150 us).
-// NSL >= 0: 16 states on 2^NSL lanes, known to the compiler.
-template <typename T, typename TD, bool VEC, int NSL>
+// B or C per tile, with one address each, and stores eight outputs; staging with an address per entry took 85 of 125 instructions per
+// token.  16 states with fp32 step logits have a kernel of their own below.
+template <typename T, typename TD, bool VEC>
 __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
     const T* __restrict__ x, int64_t x_stride, const TD* __restrict__ dtl, int64_t dt_stride, const float* __restrict__ dt_bias,
     const float* __restrict__ A, const T* __restrict__ bc, int64_t bc_stride, int b_off, int c_off, const float* __restrict__ D,
     const T* __restrict__ z, int64_t z_stride, float* __restrict__ state, const int* __restrict__ seg_starts,
-    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C, int N_, int ns_log2_, int tt_) {
+    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C, int N, int ns_log2, int tt) {
     extern __shared__ __align__(16) float ssm[];
-    const int N = NSL >= 0 ? 16 : N_, ns_log2 = NSL >= 0 ? NSL : ns_log2_, tt = NSL >= 0 ? (NSL >= 2 ? 32 : SS_ITEMS << NSL) : tt_;
     const int NS = 1 << ns_log2, ch_log2 = 7 - ns_log2, CH = 1 << ch_log2, RE = (N + NS - 1) >> ns_log2;
     // whole groups of four states per lane, on 16-byte boundaries of the staged rows: B and C are read four at a time
     const bool vec = (N & 3) == 0 && (RE & 3) == 0;
@@ -488,10 +507,16 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                 for (int e = 0; e < 8; e++) f[e] = cvt_f(rx[e]);
                 put(xs + at, f);
 #pragma unroll
-                for (int e = 0; e < 8; e++) f[e] = softplus_fn(cvt_f(rd[e]) + vbias[e]);
+                for (int e = 0; e < 8; e += 2) {
+                    const float2 y = softplus_rows(make_float2(cvt_f(rd[e]) + vbias[e], cvt_f(rd[e + 1]) + vbias[e + 1]));
+                    f[e] = y.x; f[e + 1] = y.y;
+                }
                 put(ds + at, f);
 #pragma unroll
-                for (int e = 0; e < 8; e++) f[e] = silu_rows(cvt_f(rz[e]));
+                for (int e = 0; e < 8; e += 2) {
+                    const float2 y = silu_rows(make_float2(cvt_f(rz[e]), cvt_f(rz[e + 1])));
+                    f[e] = y.x; f[e + 1] = y.y;
+                }
                 put(zs + at, f);
             }
             auto stage_bc = [&](const T* from, int j, int k, bool of_c) {
@@ -537,7 +562,7 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
         const float* bp = bs + s * RE;
         const float* cp = cs + s * RE;
         const bool lane_live = s * RE < N;
-        if (NSL >= 0 || (vec && ns_log2 >= 2 && (tt & 3) == 0)) {
+        if (vec && ns_log2 >= 2 && (tt & 3) == 0) {
             // four tokens at a time, packed arithmetic; the four sums over the lanes of a channel are taken together, each lane quarter
             // keeping the token (2 (s & 1) + (s >> 1 & 1)) that it writes
             auto four = [&](int j, bool whole) {        // tokens j .. j + 3 (those below nt)
@@ -549,8 +574,8 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                         const float dt = ds[((j + u) << ch_log2) + cl], dx = dt * xs[((j + u) << ch_log2) + cl];
                         float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-                        for (int q = 0; q < (NSL >= 0 ? (16 >> NSL) / 4 : SS_R / 4); q++) {
-                            if (NSL >= 0 || (4 * q < RE && lane_live)) {
+                        for (int q = 0; q < SS_R / 4; q++) {
+                            if (4 * q < RE && lane_live) {
                                 const float4 b4 = reinterpret_cast<const float4*>(bp + (j + u) * N)[q], c4 = reinterpret_cast<const float4*>(cp + (j + u) * N)[q];
                                 float2 s0 = make_float2(S[4 * q], S[4 * q + 1]), s1 = make_float2(S[4 * q + 2], S[4 * q + 3]);
                                 const float2 e0 = make_float2(exp2_neg(dt * a[4 * q]), exp2_neg(dt * a[4 * q + 1]));
@@ -568,18 +593,12 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                 const bool odd = s & 1, high = s & 2;
                 const float k0 = odd ? y[2] : y[0], k1 = odd ? y[3] : y[1];                          // kept pair
                 const float p0 = k0 + __shfl_xor_sync(0xffffffffu, odd ? y[0] : y[2], 1), p1 = k1 + __shfl_xor_sync(0xffffffffu, odd ? y[1] : y[3], 1);
-                if (NSL == 1) {
-                    const int mine = j + 2 * (s & 1), at = (mine << ch_log2) + cl;
-                    if (whole || mine < nt) ys[at] = (p0 + dd * xs[at]) * zs[at];
-                    if (whole || mine + 1 < nt) ys[at + CH] = (p1 + dd * xs[at + CH]) * zs[at + CH];
-                } else {
-                    float v = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
-                    if (NSL < 0) for (int o = NS >> 1; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    const int mine = j + 2 * (s & 1) + ((s >> 1) & 1);
-                    if ((NSL >= 0 || s < 4) && (whole || mine < nt)) {
-                        const int at = (mine << ch_log2) + cl;
-                        ys[at] = (v + dd * xs[at]) * zs[at];
-                    }
+                float v = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
+                for (int o = NS >> 1; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                const int mine = j + 2 * (s & 1) + ((s >> 1) & 1);
+                if (s < 4 && (whole || mine < nt)) {
+                    const int at = (mine << ch_log2) + cl;
+                    ys[at] = (v + dd * xs[at]) * zs[at];
                 }
             };
             if (nt == tt) {
@@ -641,6 +660,186 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
             if (r < RE && k < N) sp[k] = S[r];
         }
     }
+}
+
+// Prompt portions of 16 states, 16-bit rows in 16-byte pieces, fp32 step logits: four lanes of four states per channel, CPL neighbouring
+// channels per lane.  grid (segments, ceil(C / (32 CPL))), four WALKERS that go through the tokens, and 4 CPL STAGERS, a tile of 32 tokens ahead
+// and one behind: a stager's thread brings eight neighbouring channels of a token, turns the step logits into
+// steps and leaves dt and dt x; once the walkers have left the sums over the states it adds D x, applies the gate and stores.  The rows
+// after next are asked for before that.
+// Bound: issue and the special-function unit (16 powers and 5 more results per token and channel: 150 us at the size below), once
+// nothing waits: with the same threads staging and walking in turn 325 us, at 0.39 instructions per cycle.  B and C are 128 bytes per
+// token and channel from shared memory, which gives 128 a cycle: two channels per lane share them where that still leaves every
+// scheduler a walker; beyond that (more powers by polynomial instead of the special-function unit: 275 us) nothing gave.  Measured on B200,
+// bf16, 4 x 2048 tokens, 4096 channels: 380 -> 247 us; one segment of 1024 tokens ONE.
+constexpr int SP_TILE = 32;
+template <int CPL> struct SpSmem {
+    static constexpr int CH = 32 * CPL, YP = CH + 8 * CPL;              // channels; floats between rows of y (no bank conflicts)
+    struct Tile {
+        float dt[SP_TILE * CH], dx[SP_TILE * CH], y[SP_TILE * YP], b[SP_TILE * 16], c[SP_TILE * 16];
+        uint4 x[128 * CPL], z[128 * CPL];                               // pieces as loaded, for the thread that brought them
+    } tile[2];
+};
+template <typename T, int CPL>
+__global__ void __launch_bounds__(128 + 128 * CPL, 2) selective_scan16_kernel(
+    const T* __restrict__ x, int64_t x_stride, const float* __restrict__ dtl, int64_t dt_stride, const float* __restrict__ dt_bias,
+    const float* __restrict__ A, const T* __restrict__ bc, int64_t bc_stride, int b_off, int c_off, const float* __restrict__ D,
+    const T* __restrict__ z, int64_t z_stride, float* __restrict__ state, const int* __restrict__ seg_starts,
+    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C) {
+    using Smem = SpSmem<CPL>;
+    constexpr int CH = Smem::CH, YP = Smem::YP, PIECES = CH / 8, ALL = 128 + 128 * CPL;    // pieces of a token: one thread each for a tile's
+    constexpr int FULL = 1, DONE = 3;                                   // named barriers, one per tile in shared memory
+    extern __shared__ __align__(16) unsigned char sp_raw[];
+    Smem& sm = *reinterpret_cast<Smem*>(sp_raw);
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, s = lane & 3;
+    const int t0 = seg_starts[b], n = seg_starts[b + 1] - t0;
+    if (n <= 0) return;
+    const int cbase = blockIdx.y * CH;
+    if (threadIdx.x >= 128) {
+        // ================ stagers: piece vp of token vj; the first four warps also eight entries of B or C of one token
+        const int st = tid - 128, vp = (st % PIECES) * 8, vj = st / PIECES, bj = st < 128 ? (st & 63) >> 1 : SP_TILE, bk = (st & 1) * 8;
+        const bool v_live = cbase + vp < C, second = st >= 64;
+        struct alignas(16) Piece { T e[8]; };
+        Piece rx, rz, rb;
+        float4 rd[2];
+        float bias[8], skip[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) { bias[e] = v_live ? dt_bias[cbase + vp + e] : 0.f; skip[e] = v_live ? D[cbase + vp + e] : 0.f; }
+        auto fetch = [&](int tile0) {
+            const int nt = min(SP_TILE, n - tile0);                     // <= 0 past the end: nothing is loaded
+            const int64_t t = t0 + tile0 + vj;
+            if (v_live && vj < nt) {
+                rx = *reinterpret_cast<const Piece*>(x + t * x_stride + cbase + vp);
+                rz = *reinterpret_cast<const Piece*>(z + t * z_stride + cbase + vp);
+                const float4* d = reinterpret_cast<const float4*>(dtl + t * dt_stride + cbase + vp);
+                rd[0] = d[0]; rd[1] = d[1];
+            }
+            if (bj < nt) rb = *reinterpret_cast<const Piece*>(bc + (t0 + tile0 + bj) * bc_stride + (second ? c_off : b_off) + bk);
+        };
+        auto stage = [&](int tile0) {                                   // what was fetched last
+            const int nt = min(SP_TILE, n - tile0), buf = tile0 / SP_TILE & 1;
+            typename Smem::Tile& to = sm.tile[buf];
+            if (v_live && vj < nt) {
+                to.x[st] = *reinterpret_cast<const uint4*>(&rx);
+                to.z[st] = *reinterpret_cast<const uint4*>(&rz);
+                const float* d = reinterpret_cast<const float*>(rd);
+                float f[8], g[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {
+                    const float2 dt = softplus_rows(tc::add2(make_float2(d[e], d[e + 1]), make_float2(bias[e], bias[e + 1])));
+                    const float2 v = tc::mul2(dt, make_float2(cvt_f(rx.e[e]), cvt_f(rx.e[e + 1])));
+                    f[e] = dt.x; f[e + 1] = dt.y; g[e] = v.x; g[e + 1] = v.y;
+                }
+#pragma unroll
+                for (int e = 0; e < 8; e += 4) {
+                    *reinterpret_cast<float4*>(&to.dt[vj * CH + vp + e]) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+                    *reinterpret_cast<float4*>(&to.dx[vj * CH + vp + e]) = make_float4(g[e], g[e + 1], g[e + 2], g[e + 3]);
+                }
+            }
+            if (bj < nt) {
+                float* at = (second ? to.c : to.b) + bj * 16 + bk;
+#pragma unroll
+                for (int e = 0; e < 8; e += 4)
+                    *reinterpret_cast<float4*>(at + e) = make_float4(cvt_f(rb.e[e]), cvt_f(rb.e[e + 1]), cvt_f(rb.e[e + 2]), cvt_f(rb.e[e + 3]));
+            }
+            tc::named_bar_arrive(FULL + buf, ALL);
+        };
+        fetch(0);
+        stage(0);
+        fetch(SP_TILE);
+        for (int tile0 = 0; tile0 < n; tile0 += SP_TILE) {
+            if (tile0 + SP_TILE < n) {
+                stage(tile0 + SP_TILE);                                 // the walkers are done with the tile before this one
+                fetch(tile0 + 2 * SP_TILE);
+            }
+            const int nt = min(SP_TILE, n - tile0), buf = tile0 / SP_TILE & 1;
+            const typename Smem::Tile& from = sm.tile[buf];
+            tc::named_bar_sync(DONE + buf, ALL);
+            if (v_live && vj < nt) {
+                Piece px, pz, o;
+                *reinterpret_cast<uint4*>(&px) = from.x[st];
+                *reinterpret_cast<uint4*>(&pz) = from.z[st];
+                const float* y = &from.y[vj * YP + vp];
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {
+                    const float2 g = silu_rows(make_float2(cvt_f(pz.e[e]), cvt_f(pz.e[e + 1])));
+                    const float2 w = tc::mul2(tc::fma2(make_float2(skip[e], skip[e + 1]), make_float2(cvt_f(px.e[e]), cvt_f(px.e[e + 1])), *reinterpret_cast<const float2*>(y + e)), g);
+                    stf(o.e + e, w.x);
+                    stf(o.e + e + 1, w.y);
+                }
+                *reinterpret_cast<Piece*>(out + (t0 + tile0 + vj) * C + cbase + vp) = o;
+            }
+        }
+        return;
+    }
+    // ================ walkers
+    const int cl = (tid >> 5) * 8 * CPL + (lane >> 2) * CPL;            // this lane's first channel, in the CTA
+    const bool fresh = tok_pos[t0] == 0;
+    const int64_t row0 = (int64_t)seq_ids[b] * C;
+    float2 S[CPL][2], a[CPL][2];
+#pragma unroll
+    for (int c = 0; c < CPL; c++) {
+        const int cc = min(cbase + cl + c, C - 1);                      // channels past the end take part in the shuffles
+        const float4 f = *reinterpret_cast<const float4*>(A + (int64_t)cc * 16 + 4 * s);
+        constexpr float L = 1.4426950408889634f;                        // exp(dt A) = 2^(dt A log2 e)
+        a[c][0] = make_float2(f.x * L, f.y * L); a[c][1] = make_float2(f.z * L, f.w * L);
+        const float4 h = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(state + (row0 + cc) * 16 + 4 * s);
+        S[c][0] = make_float2(h.x, h.y); S[c][1] = make_float2(h.z, h.w);
+    }
+    for (int tile0 = 0; tile0 < n; tile0 += SP_TILE) {
+        const int nt = min(SP_TILE, n - tile0), buf = tile0 / SP_TILE & 1;
+        typename Smem::Tile& tile = sm.tile[buf];
+        // four tokens at a time; their sums over a channel's lanes are taken together, lane s keeps token 2 (s & 1) + (s >> 1)
+        auto four = [&](int j, bool all) {                              // tokens j .. j + 3 (those below nt)
+            float y[4][CPL];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+#pragma unroll
+                for (int c = 0; c < CPL; c++) y[u][c] = 0.f;
+                if (!all && j + u >= nt) continue;
+                const float4 b4 = *reinterpret_cast<const float4*>(&tile.b[(j + u) * 16 + 4 * s]), c4 = *reinterpret_cast<const float4*>(&tile.c[(j + u) * 16 + 4 * s]);
+                float dt[CPL], dx[CPL];
+                if constexpr (CPL == 2) {
+                    const float2 d2 = *reinterpret_cast<const float2*>(&tile.dt[(j + u) * CH + cl]), x2 = *reinterpret_cast<const float2*>(&tile.dx[(j + u) * CH + cl]);
+                    dt[0] = d2.x; dt[CPL - 1] = d2.y; dx[0] = x2.x; dx[CPL - 1] = x2.y;
+                } else {
+                    dt[0] = tile.dt[(j + u) * CH + cl]; dx[0] = tile.dx[(j + u) * CH + cl];
+                }
+#pragma unroll
+                for (int c = 0; c < CPL; c++) {
+                    const float2 d2 = make_float2(dt[c], dt[c]), x2 = make_float2(dx[c], dx[c]);
+                    const float2 p0 = tc::mul2(d2, a[c][0]), p1 = tc::mul2(d2, a[c][1]);
+                    S[c][0] = tc::fma2(make_float2(exp2_neg(p0.x), exp2_neg(p0.y)), S[c][0], tc::mul2(x2, make_float2(b4.x, b4.y)));
+                    S[c][1] = tc::fma2(make_float2(exp2_neg(p1.x), exp2_neg(p1.y)), S[c][1], tc::mul2(x2, make_float2(b4.z, b4.w)));
+                    const float2 acc = tc::fma2(S[c][1], make_float2(c4.z, c4.w), tc::mul2(S[c][0], make_float2(c4.x, c4.y)));
+                    y[u][c] = acc.x + acc.y;
+                }
+            }
+            const bool odd = s & 1, high = s & 2;
+            float v[CPL];
+#pragma unroll
+            for (int c = 0; c < CPL; c++) {
+                const float p0 = (odd ? y[2][c] : y[0][c]) + __shfl_xor_sync(0xffffffffu, odd ? y[0][c] : y[2][c], 1);
+                const float p1 = (odd ? y[3][c] : y[1][c]) + __shfl_xor_sync(0xffffffffu, odd ? y[1][c] : y[3][c], 1);
+                v[c] = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
+            }
+            float* to = &tile.y[(j + 2 * (s & 1) + (s >> 1)) * YP + cl];                    // rows up to SP_TILE - 1 exist whatever nt
+            if constexpr (CPL == 2) *reinterpret_cast<float2*>(to) = make_float2(v[0], v[CPL - 1]);
+            else *to = v[0];
+        };
+        tc::named_bar_sync(FULL + buf, ALL);
+        if (nt == SP_TILE) {
+#pragma unroll 2
+            for (int j = 0; j < SP_TILE; j += 4) four(j, true);
+        } else {
+            for (int j = 0; j < nt; j += 4) four(j, false);
+        }
+        tc::named_bar_arrive(DONE + buf, ALL);
+    }
+#pragma unroll
+    for (int c = 0; c < CPL; c++)
+        if (cbase + cl + c < C)
+            *reinterpret_cast<float4*>(state + (row0 + cbase + cl + c) * 16 + 4 * s) = make_float4(S[c][0].x, S[c][0].y, S[c][1].x, S[c][1].y);
 }
 
 }  // namespace sllm
@@ -766,15 +965,27 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
         const bool vec = dtype != SLLM_F32 && states % 8 == 0 && channels % 8 == 0 && ns_tiled <= 4 && x_stride % 8 == 0 && z_stride % 8 == 0 &&
                          bc_stride % 8 == 0 && b_off % 8 == 0 && c_off % 8 == 0 && dt_stride % dv == 0 &&
                          (((uintptr_t)x | (uintptr_t)dt | (uintptr_t)z | (uintptr_t)bc | (uintptr_t)out) & 15) == 0;
-#define SS_TILED(TT, TD, VEC, NSL) selective_scan_tiled_kernel<TT, TD, VEC, NSL><<<SS_GRID(num_prefill_segs, ns_tiled), smem, st>>>(SS_ARGS(TD, 0, ns_tiled), tt)
-        const bool n16 = states == 16 && (ns_tiled == 1 || ns_tiled == 2);
-        if (vec) {
-            if (dt_f32 && n16 && ns_tiled == 1) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, 1))); }
-            else if (dt_f32 && n16) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, 2))); }
-            else if (dt_f32) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, -1))); }
-            else { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, T, true, -1))); }
-        } else if (dt_f32) { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, float, false, -1))); }
-        else { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, T, false, -1))); }
+#define SS_TILED(TT, TD, VEC) selective_scan_tiled_kernel<TT, TD, VEC><<<SS_GRID(num_prefill_segs, ns_tiled), smem, st>>>(SS_ARGS(TD, 0, ns_tiled), tt)
+        if (vec && dt_f32 && states == 16 && (((uintptr_t)A | (uintptr_t)state) & 15) == 0) {
+            int sms = 0;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
+            // two channels per lane from a warp per scheduler on
+            const bool two = (int64_t)num_prefill_segs * channels >= (int64_t)64 * sms;
+#define SP_LAUNCH(CPL) do {                                                                                                     \
+            static unsigned long long attr_mask = 0;                                                                            \
+            auto kern = selective_scan16_kernel<T, CPL>;                                                                        \
+            if (first_use_on_this_device(attr_mask)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpSmem<CPL>)); \
+            kern<<<dim3((unsigned)num_prefill_segs, (unsigned)cdiv(channels, 32 * (CPL))), 128 + 128 * (CPL), sizeof(SpSmem<CPL>), st>>>(     \
+                (const T*)x, x_stride, (const float*)dt, dt_stride, (const float*)dt_bias, (const float*)A, (const T*)bc, bc_stride, b_off, c_off, \
+                (const float*)D, (const T*)z, z_stride, (float*)state, (const int*)seg_starts, (const int*)seq_ids, (const int*)tok_pos, (T*)out, channels); \
+        } while (0)
+            SLLM_DISPATCH_DTYPE(dtype, { if (two) SP_LAUNCH(2); else SP_LAUNCH(1); });
+#undef SP_LAUNCH
+        } else if (vec) {
+            if (dt_f32) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true))); }
+            else { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, T, true))); }
+        } else if (dt_f32) { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, float, false))); }
+        else { SLLM_DISPATCH_DTYPE_F32(dtype, (SS_TILED(T, T, false))); }
 #undef SS_TILED
         if (check_launch("selective_scan (prompt portions)")) return 1;
     }

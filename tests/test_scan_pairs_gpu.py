@@ -1,0 +1,59 @@
+"""GPU: the selective scan of 16 states with staged steps (csrc/scan_ops.cu), one and two channels per lane, and the convolution's tiles,
+against the rules in 64 bits."""
+import pytest
+import torch
+
+from test_tile_edges_gpu import _normal, _segments
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("lens,firsts,C", [
+    ((1,), (0,), 8), ((31, 2), (5, 0), 72), ((32, 33, 64), (0, 9, 3), 40),                 # one channel per lane
+    ((33, 1, 32, 65), (0, 7, 3, 0), 2400), ((66, 4), (2, 0), 4808)])                       # two
+def test_scan_of_sixteen_states(dtype, lens, firsts, C):
+    """Outputs are rounded once; the state's relative error is that of its decays' exponents: products of about 10 at most, rounded to
+    24 bits, in sums of up to 66 tokens whose older part fades."""
+    from swiftllm_b200.worker.kernels.scan_ops import selective_scan
+    N, st, T = 16, _segments(lens, firsts), sum(lens)
+    base = _normal(T, 2 * C + 2 * N + 8, seed=C, dtype=dtype)
+    x, z, bc = base[:, :C], base[:, C:2 * C], base[:, 2 * C:]
+    dt, bias = _normal(T, C, seed=1), _normal(C, seed=2) - 3
+    A, D, S0 = -(_normal(C, N, seed=3).abs() + 0.1), _normal(C, seed=4), _normal(len(lens), C, N, seed=5)
+    state = S0.clone()
+    y = selective_scan(x, dt, bias, A, bc, 0, N, D, z, state, st)
+    steps = torch.nn.functional.softplus(dt.double() + bias.double())
+    want, at = torch.empty(T, C, dtype=torch.float64, device=x.device), 0
+    for i, (n, first) in enumerate(zip(lens, firsts)):
+        row = int(st.seq_ids[i])
+        S = S0[row].double() if first > 0 else torch.zeros(C, N, dtype=torch.float64, device=x.device)
+        for t in range(at, at + n):
+            S = torch.exp(steps[t, :, None] * A.double()) * S + (steps[t] * x[t].double())[:, None] * bc[t, None, :N].double()
+            want[t] = ((S * bc[t, None, N:2 * N].double()).sum(1) + D.double() * x[t].double()) * torch.nn.functional.silu(z[t].double())
+        at += n
+        assert float((state[row].double() - S).norm() / S.norm()) < 2e-6
+    assert float((y.double() - want).norm() / want.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+
+
+@pytest.mark.parametrize("taps", [3, 4])
+def test_convolution_tiles(taps):
+    """Segments that begin and end on every row near a tile's edge; as many channels as the vector kernel asks for at these rows."""
+    from swiftllm_b200.worker.kernels.scan_ops import short_conv
+    lens, firsts = (31, 1, 2, 30, 33, 5, 64, 1, 1, 88), (0, 3, 1, 0, 2, 0, 9, 1, 0, 4)
+    C, T, st = 4104, sum(lens), _segments(lens, firsts)
+    assert T * C >= 1 << 20
+    x, w, b = _normal(T, C, seed=1, dtype=torch.bfloat16), _normal(C, taps, seed=2), _normal(C, seed=3)
+    tail0 = _normal(len(lens), taps - 1, C, seed=4, dtype=torch.bfloat16)
+    tail = tail0.clone()
+    y = short_conv(x, w, b, tail, st, torch.bfloat16, silu=True, move_tail=True)
+    at = 0
+    for i, (n, first) in enumerate(zip(lens, firsts)):
+        row = int(st.seq_ids[i])
+        before = tail0[row].double() * (torch.arange(first - taps + 1, first, device=x.device) >= 0)[:, None]
+        full = torch.cat((before, x[at:at + n].double()))
+        acc = sum(full[k:k + n] * w[:, k].double() for k in range(taps)) + b.double()
+        want = torch.nn.functional.silu(acc)
+        assert float((y[at:at + n].double() - want).norm() / want.norm()) < 2.0 ** -8, i
+        assert torch.equal(tail[row].double(), full[n:])
+        at += n
