@@ -669,9 +669,9 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
 // after next are asked for before that.
 // Bound: issue and the special-function unit (16 powers and 5 more results per token and channel: 150 us at the size below), once
 // nothing waits: with the same threads staging and walking in turn 325 us, at 0.39 instructions per cycle.  B and C are 128 bytes per
-// token and channel from shared memory, which gives 128 a cycle: two channels per lane share them where that still leaves every
-// scheduler a walker; beyond that (more powers by polynomial instead of the special-function unit: 275 us) nothing gave.  Measured on B200,
-// bf16, 4 x 2048 tokens, 4096 channels: 380 -> 247 us; one segment of 1024 tokens ONE.
+// token and channel from shared memory, which gives 128 a cycle: two channels per lane share them where there are warps enough; beyond
+// that (more powers by polynomial instead of the special-function unit: 275 us) nothing gave.  Measured on B200,
+// bf16, 4 x 2048 tokens, 4096 channels: 380 -> 247 us; one segment of 1024 tokens 122 -> 59.
 constexpr int SP_TILE = 32;
 template <int CPL> struct SpSmem {
     static constexpr int CH = 32 * CPL, YP = CH + 8 * CPL;              // channels; floats between rows of y (no bank conflicts)
@@ -681,7 +681,7 @@ template <int CPL> struct SpSmem {
     } tile[2];
 };
 template <typename T, int CPL>
-__global__ void __launch_bounds__(128 + 128 * CPL, 2) selective_scan16_kernel(
+__global__ void __launch_bounds__(128 + 128 * CPL, CPL == 1 ? 3 : 2) selective_scan16_kernel(
     const T* __restrict__ x, int64_t x_stride, const float* __restrict__ dtl, int64_t dt_stride, const float* __restrict__ dt_bias,
     const float* __restrict__ A, const T* __restrict__ bc, int64_t bc_stride, int b_off, int c_off, const float* __restrict__ D,
     const T* __restrict__ z, int64_t z_stride, float* __restrict__ state, const int* __restrict__ seg_starts,
@@ -969,8 +969,9 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
         if (vec && dt_f32 && states == 16 && (((uintptr_t)A | (uintptr_t)state) & 15) == 0) {
             int sms = 0;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
-            // two channels per lane from a warp per scheduler on
-            const bool two = (int64_t)num_prefill_segs * channels >= (int64_t)64 * sms;
+            // one channel per lane while all CTAs are on the SMs at once, three each (us, one / two channels: 2 x 777 tokens, 4096 channels
+            // 65 / -, 2 x 777, 8192 channels 124 / 100, 3 x 2048, 4096 channels 217 / 248, 4 x 2048, 4096 channels 315 / 247)
+            const bool two = (int64_t)num_prefill_segs * cdiv(channels, 32) > 3 * (int64_t)sms;
 #define SP_LAUNCH(CPL) do {                                                                                                     \
             static unsigned long long attr_mask = 0;                                                                            \
             auto kern = selective_scan16_kernel<T, CPL>;                                                                        \

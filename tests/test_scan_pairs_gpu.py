@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("lens,firsts,C", [
     ((1,), (0,), 8), ((31, 2), (5, 0), 72), ((32, 33, 64), (0, 9, 3), 40),                 # one channel per lane
-    ((33, 1, 32, 65), (0, 7, 3, 0), 2400), ((66, 4), (2, 0), 4808)])                       # two
+    ((66, 4), (2, 0), 4808), ((33, 1, 32, 65), (0, 7, 3, 0), 4808)])                       # two (the last)
 def test_scan_of_sixteen_states(dtype, lens, firsts, C):
     """Outputs are rounded once; the state's relative error is that of its decays' exponents: products of about 10 at most, rounded to
     24 bits, in sums of up to 66 tokens whose older part fades."""
