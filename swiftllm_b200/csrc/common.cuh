@@ -90,6 +90,30 @@ static inline bool first_use_on_this_device(unsigned long long& mask) {
     return (old & bit) == 0;
 }
 
+// ---------------------------------------------------------------- launches that begin early
+// A kernel launched by launch_early may begin while the kernel before it in the stream still runs, once every CTA of that one has called
+// launch_next (or has ended): its launch and its CTAs' set-up hide behind the other's last CTAs.  It calls wait_previous before it touches
+// what earlier kernels read or write, which waits until all of them have ended and their writes are seen, and launch_next after that,
+// so that a kernel behind it that shares nothing with it need not wait for anything but the launch's own end.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A pointer as it is after wait_previous: what is read through a const __restrict__ argument the compiler takes for constant, and could read
+// sooner.
+template <typename T> __device__ __forceinline__ T* after_wait(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
+template <typename... P, typename... A>
+static inline void launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = stream;
+    config.attrs = &attr; config.numAttrs = 1;
+    cudaLaunchKernelEx(&config, kern, static_cast<P>(args)...);          // an error is what check_launch reports
+}
+
 // dispatch on the dtype tag
 #define SLLM_DISPATCH_DTYPE(dtype, ...)                                     \
     do {                                                                    \

@@ -25,6 +25,9 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(T* __restrict__ x, T* __re
     extern __shared__ uint4 row_smem[];
     __shared__ float red[16];
     using TT = Traits<T>;
+    wait_previous();
+    launch_next();
+    x = after_wait(x); residual = after_wait(residual); rows = after_wait(rows);
     const int64_t t = GATHER ? rows[blockIdx.x] : (int64_t)blockIdx.x;
     if (GATHER) assert(t >= 0 && t < num_rows);
     T* xr = x + t * hidden;
@@ -101,7 +104,7 @@ static int launch_rmsnorm(void* x, void* residual, const void* weight, float eps
     const int nvec = hidden / 8;
     const char* what = GATHER ? "add_rmsnorm_rows" : FUSED ? "fused_add_rmsnorm" : "rmsnorm";
     auto launch = [&](auto kern, int threads, size_t smem) {
-        kern<<<(unsigned)T_, threads, smem, stream>>>((T*)x, (T*)residual, (const T*)weight, eps, hidden, rows, (T*)out, num_rows);
+        launch_early(kern, (unsigned)T_, threads, smem, stream, (T*)x, (T*)residual, (const T*)weight, eps, hidden, rows, (T*)out, num_rows);
         return check_launch(what);
     };
     // rows of 4 x 128 .. 4 x 256 vectors (hidden 4096 .. 8192): 4 vectors per thread, 128 .. 256 threads, no shared-memory staging
@@ -149,6 +152,9 @@ __global__ void __launch_bounds__(256) rotary_kernel(T* __restrict__ q, T* __res
 template <typename T>
 __global__ void __launch_bounds__(256) silu_and_mul_kernel(T* __restrict__ x, int64_t total_vec, int64_t F) {
     using TT = Traits<T>;
+    wait_previous();
+    launch_next();
+    x = after_wait(x);
     const int64_t idx0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (idx0 >= total_vec) return;
     const int64_t vec_per_row = F >> 3;
@@ -233,7 +239,7 @@ int sllm_silu_and_mul_inplace(void* x, int64_t num_tokens, int64_t F, sllm_dtype
     const int64_t total = num_tokens * (F / 8);
     const int threads = 256;
     const unsigned blocks = (unsigned)(((total + 1) / 2 + threads - 1) / threads);
-    SLLM_DISPATCH_DTYPE(dtype, (silu_and_mul_kernel<T><<<blocks, threads, 0, (cudaStream_t)stream>>>((T*)x, total, F)));
+    SLLM_DISPATCH_DTYPE(dtype, (launch_early(silu_and_mul_kernel<T>, blocks, threads, 0, (cudaStream_t)stream, (T*)x, total, F)));
     return check_launch("silu_and_mul");
 }
 

@@ -353,6 +353,9 @@ template <typename T>
 __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* __restrict__ partial, const T* __restrict__ gate,
                                                                   int64_t gate_stride_t, T* __restrict__ out, int64_t out_stride_t,
                                                                   int64_t out_stride_h, int H, int r, int nsplit) {
+    wait_previous();
+    launch_next();
+    partial = after_wait(partial); gate = after_wait(gate);
     const int lane = threadIdx.x & 31;
     const int64_t idx = blockIdx.x, t = idx / H;
     const int h = (int)(idx - t * H);
@@ -522,8 +525,8 @@ static int latent_attention(bool portions, const void* q_lat, int64_t q_lat_stri
         a.out_vec = ((uintptr_t)out & 15) == 0 && out_stride_t % 8 == 0 && out_stride_h % 8 == 0;
         if (int rc = launch_latent_attn_tc(a, portions, dtype, (cudaStream_t)stream)) return rc;
         if (a.nsplit > 1)
-            SLLM_DISPATCH_DTYPE(dtype, (latent_attn_combine_kernel<T><<<(unsigned)(num_tokens * num_heads), 128, 0, (cudaStream_t)stream>>>(
-                a.partial, (const T*)gate, gate_stride_t, (T*)out, out_stride_t, out_stride_h, num_heads, r, a.nsplit)));
+            SLLM_DISPATCH_DTYPE(dtype, (launch_early(latent_attn_combine_kernel<T>, (unsigned)(num_tokens * num_heads), 128, 0, (cudaStream_t)stream, a.partial,
+                                                     (const T*)gate, gate_stride_t, (T*)out, out_stride_t, out_stride_h, num_heads, r, a.nsplit)));
         return check_launch("latent_attention (combine)");
     }
     const size_t mma_smem = ((size_t)(16 + LM_KT) * (r + dr + 8) + 16 * (LM_KT + 8)) * 2 + (16 * (LM_KT + 1) + 48) * sizeof(float);

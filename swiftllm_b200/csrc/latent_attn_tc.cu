@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;            // the last tokens of a prompt have the most keys: first
     int ntok = min(p.qt, p.num_tokens - t_first);
     if constexpr (ROWS == LT_SHARED) {               // one segment each, the last CTA what is left
+        wait_previous();
         auto length = [&](int left) {                // tokens of the segment at t_first
             const int a = t_first + min(lane, left - 1), b = t_first + min(lane + 32, left - 1);
             const int sa = p.tok_seq[a], sb = p.tok_seq[b], qa = p.tok_pos[a], qb = p.tok_pos[b];
@@ -126,6 +127,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_s;
+    wait_previous();
+    launch_next();
 
     int n_done = 0;                                  // tiles of the passes before: every barrier's phase follows from it
     int pass = 0, solo = -1;                         // solo >= 0: the pass is for this token of the segment alone
@@ -583,7 +586,7 @@ int launch_latent_attn_tc(LatentTc& p, bool portions, sllm_dtype_t dtype, cudaSt
                     SLLM_REQUIRE(e == cudaSuccess, "latent_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
                 }
         }
-        kernels[full][rows]<<<grid, LT_THREADS, LT_SMEM, stream>>>(p);
+        launch_early(kernels[full][rows], grid, LT_THREADS, LT_SMEM, stream, p);
     });
     return check_launch("latent_attention (tcgen05)");
 }

@@ -232,6 +232,9 @@ template <typename T>
 __global__ void paged_attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
                                         T* __restrict__ o, const int32_t* __restrict__ seq_lens, int nq, int D,
                                         int num_splits, int split_tokens) {
+    wait_previous();
+    launch_next();
+    part_o = after_wait(part_o); part_lse = after_wait(part_lse); seq_lens = after_wait(seq_lens);
     const int head = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
     const int n = (seq_lens[seq] + split_tokens - 1) / split_tokens;
     const int64_t base = ((int64_t)seq * nq + head) * num_splits;
@@ -362,8 +365,8 @@ int sllm_paged_attention(const void* q, const void* k_cache, const void* v_cache
         if (e) return e;
         if (p.num_splits > 1) {
             dim3 g2(nq, num_decoding_seqs);
-            SLLM_DISPATCH_DTYPE(dtype, (paged_attn_merge_kernel<T><<<g2, head_dim, 0, st>>>(p.part_o, p.part_lse, (T*)o, seq_lens, nq,
-                                                                                          head_dim, p.num_splits, p.split_tokens)));
+            SLLM_DISPATCH_DTYPE(dtype, (launch_early(paged_attn_merge_kernel<T>, g2, head_dim, 0, st, p.part_o, p.part_lse, (T*)o, seq_lens, nq,
+                                                     head_dim, p.num_splits, p.split_tokens)));
             return check_launch("paged_attention(phase 2)");
         }
         return 0;

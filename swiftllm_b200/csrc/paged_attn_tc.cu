@@ -192,6 +192,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_base_s;
+    wait_previous();                                                 // so far nothing in memory was touched
+    launch_next();
 
     if (warp == 0) {
         producer_loop<true>(p, &kmap, &qmap, k_sm, bars->k_full, bars->k_empty, TC_KSTAGES, bars, q_sm, g, lane);
@@ -495,7 +497,7 @@ int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, con
         static unsigned long long configured = 0;                                                                        \
         if (first_use_on_this_device(configured))                                                                        \
             cudaFuncSetAttribute(paged_attn_tc_kernel<TT, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES); \
-        paged_attn_tc_kernel<TT, GG><<<grid, TC_THREADS, TC_SMEM_BYTES, stream>>>(kmap, vmap, qmap, p);                  \
+        launch_early(paged_attn_tc_kernel<TT, GG>, grid, TC_THREADS, TC_SMEM_BYTES, stream, kmap, vmap, qmap, p);       \
     } while (0)
     if (dtype == SLLM_F16) {
         if (g <= 4) SLLM_TC_LAUNCH(__half, 4); else if (g <= 8) SLLM_TC_LAUNCH(__half, 8); else SLLM_TC_LAUNCH(__half, 16);

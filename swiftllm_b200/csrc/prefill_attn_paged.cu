@@ -36,6 +36,9 @@ template <typename T>
 __global__ void __launch_bounds__(256) prefill_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                             T* __restrict__ o, const int32_t* __restrict__ start_locs,
                                                             const int32_t* __restrict__ seq_lens, int nq, int64_t units, int nsplit) {
+    wait_previous();
+    launch_next();
+    part_o = after_wait(part_o); part_ml = after_wait(part_ml); start_locs = after_wait(start_locs); seq_lens = after_wait(seq_lens);
     const int lane = threadIdx.x & 31;
     const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int start = start_locs[blockIdx.y], len = seq_lens[blockIdx.y];
@@ -89,16 +92,16 @@ static int launch_prefill_paged_tc(const void* q, const void* k_cache, const voi
     if (dtype == SLLM_F16) {
         static unsigned long long c = 0;
         if (first_use_on_this_device(c)) cudaFuncSetAttribute(prefill_attn_tc_kernel<__half, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
-        prefill_attn_tc_kernel<__half, true><<<grid, PT_THREADS, PT_SMEM_BYTES, stream>>>(qmap, kmap, vmap, p, pg);
+        launch_early(prefill_attn_tc_kernel<__half, true>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, pg);
     } else {
         static unsigned long long c = 0;
         if (first_use_on_this_device(c)) cudaFuncSetAttribute(prefill_attn_tc_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
-        prefill_attn_tc_kernel<__nv_bfloat16, true><<<grid, PT_THREADS, PT_SMEM_BYTES, stream>>>(qmap, kmap, vmap, p, pg);
+        launch_early(prefill_attn_tc_kernel<__nv_bfloat16, true>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, pg);
     }
     if (check_launch("prefill_attention_paged(tcgen05)")) return 1;
     if (pg.nsplit > 1) {
         const dim3 rows((unsigned)cdiv((int64_t)max_chunk_len * nq, 8), (unsigned)num_seqs);
-        SLLM_DISPATCH_DTYPE(dtype, (prefill_merge_kernel<T><<<rows, 256, 0, stream>>>(pg.part_o, pg.part_ml, (T*)o, start_locs, chunk_lens, nq, num_tokens * nq, pg.nsplit)));
+        SLLM_DISPATCH_DTYPE(dtype, (launch_early(prefill_merge_kernel<T>, rows, 256, 0, stream, pg.part_o, pg.part_ml, (T*)o, start_locs, chunk_lens, nq, num_tokens * nq, pg.nsplit)));
         return check_launch("prefill_attention_paged(merge)");
     }
     return 0;

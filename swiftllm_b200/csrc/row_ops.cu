@@ -17,6 +17,9 @@ template <typename P>
 __global__ void __launch_bounds__(256) gather_rows_kernel(const int* __restrict__ idx, int offset, int64_t table_rows,
                                                           const P* __restrict__ table_a, P* __restrict__ out_a, int na,
                                                           const P* __restrict__ table_b, P* __restrict__ out_b, int nb) {
+    wait_previous();
+    launch_next();
+    idx = after_wait(idx);
     const int64_t t = blockIdx.x, r = (int64_t)idx[t] + offset;
     assert(r >= 0 && r < table_rows);
     for (int i = threadIdx.x; i < na; i += blockDim.x) out_a[t * na + i] = table_a[r * na + i];
@@ -27,8 +30,8 @@ template <typename P>
 static void launch_gather(const int* idx, int offset, int64_t table_rows, const void* ta, void* oa, int64_t bytes_a, const void* tb, void* ob,
                           int64_t bytes_b, int64_t n, cudaStream_t s) {
     const int na = (int)(bytes_a / (int64_t)sizeof(P)), nb = (int)(bytes_b / (int64_t)sizeof(P)), most = na > nb ? na : nb;
-    gather_rows_kernel<P><<<(unsigned)n, most >= 256 ? 256 : (most + 31) / 32 * 32, 0, s>>>(idx, offset, table_rows, (const P*)ta, (P*)oa, na,
-                                                                                           (const P*)tb, (P*)ob, nb);
+    launch_early(gather_rows_kernel<P>, (unsigned)n, most >= 256 ? 256 : (most + 31) / 32 * 32, 0, s, idx, offset, table_rows, (const P*)ta, (P*)oa, na,
+                 (const P*)tb, (P*)ob, nb);
 }
 
 // The greater of two (value, index) pairs: NaN above everything, the smaller index among equals.
@@ -48,6 +51,9 @@ __global__ void __cluster_dims__(AM_CTAS, 1, 1) __launch_bounds__(AM_THREADS) ar
     struct alignas(VEC * sizeof(T)) Piece { T e[VEC]; };
     __shared__ float wv[AM_THREADS / 32], cv[AM_CTAS];
     __shared__ int wi[AM_THREADS / 32], ci[AM_CTAS];
+    wait_previous();
+    launch_next();
+    x = after_wait(x);
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t row = blockIdx.x / AM_CTAS;
@@ -128,9 +134,9 @@ int sllm_argmax_rows(const void* x, int64_t row_stride, int64_t num_rows, int64_
     SLLM_DISPATCH_DTYPE_F32(dtype, {
         constexpr int W = 16 / (int)sizeof(T);
         if (n % W == 0 && row_stride % W == 0 && ((uintptr_t)x & 15) == 0)
-            argmax_rows_kernel<T, W><<<grid, AM_THREADS, 0, s>>>((const T*)x, row_stride, (int)n, (int64_t*)out);
+            launch_early(argmax_rows_kernel<T, W>, grid, AM_THREADS, 0, s, (const T*)x, row_stride, (int)n, (int64_t*)out);
         else
-            argmax_rows_kernel<T, 1><<<grid, AM_THREADS, 0, s>>>((const T*)x, row_stride, (int)n, (int64_t*)out);
+            launch_early(argmax_rows_kernel<T, 1>, grid, AM_THREADS, 0, s, (const T*)x, row_stride, (int)n, (int64_t*)out);
     });
     return check_launch("argmax_rows");
 }

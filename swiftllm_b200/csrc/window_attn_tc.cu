@@ -95,6 +95,8 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_s;
+    wait_previous();
+    launch_next();
 
     // ---- a segment: tokens ts .. ts + n - 1 of one sequence at positions pos0 ..
     struct Segment { int ts, n, seq, pos0, lo, hi, nk, steps_a, steps_b, end_a, end_b; };
@@ -722,7 +724,7 @@ int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) 
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM);                      \
             SLLM_REQUIRE(e == cudaSuccess, "window_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));                  \
         }                                                                                                                          \
-        kern<<<grid, WX_THREADS, WX_SMEM, stream>>>(p);                                                                            \
+        launch_early(kern, grid, WX_THREADS, WX_SMEM, stream, p);                                                                  \
     } while (0)
 #define SLLM_WX(EXT, CAP)                                                                                                          \
     do {                                                                                                                           \
