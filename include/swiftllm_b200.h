@@ -102,6 +102,9 @@ int sllm_rotary_store_kvcache_decode(void* q, void* k, const void* v, const void
  * (the reference allocates mid_o / mid_o_logexpsum per call, paged_attn.py:170-180). */
 int64_t sllm_paged_attention_workspace_bytes(int num_decoding_seqs, int num_q_heads, int head_dim, int max_seq_len,
                                              int seq_block_size, int num_kv_heads);
+/* the same for a 16-bit cache of these blocks: 0 also where a small launch merges its splits on chip (workspace may then be NULL) */
+int64_t sllm_paged_attention_workspace_needed(int num_decoding_seqs, int nq, int head_dim, int max_seq_len, int seq_block_size, int nkv,
+                                              int block_size, int64_t num_blocks, int num_layers);
 int sllm_paged_attention(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_table,
                          const int32_t* seq_ids, const int32_t* seq_lens, void* o, void* workspace,
                          int64_t workspace_bytes, float softmax_scale, int num_decoding_seqs, int max_seq_len,

@@ -33,6 +33,7 @@ SIGNATURES = {
     "sllm_store_kvcache": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _L, _I, _I, _I, _I, _I, _I, _I, _L, _L, _I, _P]),
     "sllm_rotary_store_kvcache_decode": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _L, _L, _L, _I, _P]),
     "sllm_paged_attention_workspace_bytes": (_L, [_I, _I, _I, _I, _I, _I]),
+    "sllm_paged_attention_workspace_needed": (_L, [_I, _I, _I, _I, _I, _I, _I, _L, _I]),
     "sllm_paged_attention": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _L, _F, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _L, _L, _I, _P]),
     "sllm_prefill_attention": (_I, [_P, _P, _P, _P, _P, _P, _F, _I, _I, _L, _I, _I, _I, _L, _L, _L, _I, _P]),
     "sllm_store_kvcache_chunked": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _L, _I, _I, _I, _I, _I, _I, _I, _L, _L, _I, _P]),
@@ -173,9 +174,14 @@ def dtype_tag_f32(dtype: torch.dtype) -> int:
     return F32 if dtype == torch.float32 else dtype_tag(dtype)
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream() -> int:
     """The current torch CUDA stream as a raw cudaStream_t (the reference's convention:
-    csrc/src/block_swapping.cpp:15-17, Triton launches)."""
+    csrc/src/block_swapping.cpp:15-17, Triton launches), without a stream object where torch gives the handle itself."""
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

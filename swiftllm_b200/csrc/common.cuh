@@ -103,15 +103,22 @@ template <typename T> __device__ __forceinline__ T* after_wait(T* p) {
     asm volatile("" : "+l"(p) : : "memory");
     return p;
 }
+// in clusters of `cluster` neighbouring CTAs
 template <typename... P, typename... A>
-static inline void launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+static inline void launch_early_clusters(int cluster, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = (unsigned)cluster; attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t config = {};
     config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = stream;
-    config.attrs = &attr; config.numAttrs = 1;
+    config.attrs = attrs; config.numAttrs = cluster > 1 ? 2 : 1;
     cudaLaunchKernelEx(&config, kern, static_cast<P>(args)...);          // an error is what check_launch reports
+}
+template <typename... P, typename... A>
+static inline void launch_early(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    launch_early_clusters(1, kern, grid, block, smem, stream, args...);
 }
 
 // dispatch on the dtype tag

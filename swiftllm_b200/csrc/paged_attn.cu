@@ -280,13 +280,19 @@ bool tc_paged_supported(int head_dim, int block_size, int nq, int nkv, int64_t n
 int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_table, const int32_t* seq_ids,
                     const int32_t* seq_lens, void* o, float* part_o, float* part_lse, float scale_log2e, int num_seqs,
                     int split_tokens, int num_splits, int cur_layer, int num_layers, int nq, int nkv, int max_blocks_per_seq,
-                    int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, int num_sms, cudaStream_t stream);
+                    int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, int num_sms, bool clustered, cudaStream_t stream);
 
 // SLLM_PAGED_ATTN_GEN=1 forces the cp.async/mma.sync kernel (A/B measurements, debugging); default: tcgen05/TMA
 // whenever the shape is covered (head_dim 128, block_size 16).
 static int forced_generation() {
     const char* e = getenv("SLLM_PAGED_ATTN_GEN");      // re-read every call so tests can toggle it
     return (e && e[0] == '1') ? 1 : (e && e[0] == '2') ? 2 : 0;
+}
+
+// Whether the splits of a (sequence, kv head) meet in a cluster: portable cluster sizes, and CTAs that find their clusters' SMs at once (a
+// GPC of 16 or more SMs holds two clusters of eight).
+static bool meets_in_cluster(int num_seqs, int nkv, int num_splits) {
+    return num_splits > 1 && num_splits <= 8 && (int64_t)num_seqs * nkv * num_splits <= num_sms() * 3 / 4;
 }
 
 template <typename T, int D>
@@ -324,6 +330,15 @@ int64_t sllm_paged_attention_workspace_bytes(int num_decoding_seqs, int nq, int 
     return (int64_t)num_decoding_seqs * nq * ns * (head_dim + 1) * (int64_t)sizeof(float);
 }
 
+int64_t sllm_paged_attention_workspace_needed(int num_decoding_seqs, int nq, int head_dim, int max_seq_len, int seq_block_size, int nkv,
+                                              int block_size, int64_t num_blocks, int num_layers) {
+    const int64_t bytes = sllm_paged_attention_workspace_bytes(num_decoding_seqs, nq, head_dim, max_seq_len, seq_block_size, nkv);
+    if (bytes == 0) return 0;
+    const int st = choose_split_tokens(num_decoding_seqs, nkv, max_seq_len, seq_block_size);
+    return forced_generation() != 1 && tc_paged_supported(head_dim, block_size, nq, nkv, num_blocks, num_layers) &&
+           meets_in_cluster(num_decoding_seqs, nkv, (max_seq_len + st - 1) / st) ? 0 : bytes;
+}
+
 int sllm_paged_attention(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_table,
                          const int32_t* seq_ids, const int32_t* seq_lens, void* o, void* workspace,
                          int64_t workspace_bytes, float softmax_scale, int num_decoding_seqs, int max_seq_len,
@@ -349,7 +364,9 @@ int sllm_paged_attention(const void* q, const void* k_cache, const void* v_cache
     p.cur_layer = cur_layer; p.num_layers = num_layers; p.nq = nq; p.nkv = nkv; p.block_size = block_size;
     p.max_blocks_per_seq = max_blocks_per_seq; p.q_stride = q_row_stride;
     p.part_o = nullptr; p.part_lse = nullptr;
-    if (p.num_splits > 1) {
+    const bool tc = forced_generation() != 1 && dtype <= SLLM_BF16 && tc_paged_supported(head_dim, block_size, nq, nkv, num_blocks, num_layers);
+    const bool clustered = tc && meets_in_cluster(num_decoding_seqs, nkv, p.num_splits);
+    if (p.num_splits > 1 && !clustered) {
         const int64_t need = (int64_t)num_decoding_seqs * nq * p.num_splits * (head_dim + 1) * (int64_t)sizeof(float);
         SLLM_REQUIRE(workspace && workspace_bytes >= need, "paged_attention: workspace too small (%lld < %lld bytes)",
                      (long long)workspace_bytes, (long long)need);
@@ -357,13 +374,12 @@ int sllm_paged_attention(const void* q, const void* k_cache, const void* v_cache
         p.part_lse = p.part_o + (int64_t)num_decoding_seqs * nq * p.num_splits * head_dim;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    if (forced_generation() != 1 && tc_paged_supported(head_dim, block_size, nq, nkv, num_blocks, num_layers) &&
-        dtype <= SLLM_BF16) {
+    if (tc) {
         int e = launch_paged_tc(q, k_cache, v_cache, block_table, seq_ids, seq_lens, o, p.part_o, p.part_lse, p.scale_log2e,
                                 num_decoding_seqs, p.split_tokens, p.num_splits, cur_layer, num_layers, nq, nkv,
-                                max_blocks_per_seq, num_blocks, q_row_stride, dtype, num_sms(), st);
+                                max_blocks_per_seq, num_blocks, q_row_stride, dtype, num_sms(), clustered, st);
         if (e) return e;
-        if (p.num_splits > 1) {
+        if (p.num_splits > 1 && !clustered) {
             dim3 g2(nq, num_decoding_seqs);
             SLLM_DISPATCH_DTYPE(dtype, (launch_early(paged_attn_merge_kernel<T>, g2, head_dim, 0, st, p.part_o, p.part_lse, (T*)o, seq_lens, nq,
                                                      head_dim, p.num_splits, p.split_tokens)));

