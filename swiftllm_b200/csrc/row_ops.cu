@@ -2,6 +2,7 @@
 // of logits.
 #include <assert.h>
 #include <cooperative_groups.h>
+#include <utility>
 
 #include "typed_io.cuh"
 
@@ -41,9 +42,10 @@ __device__ __forceinline__ bool above(float v, int i, float w, int j) {
 }
 
 // Eight CTAs (a cluster) per row, each over every eighth run of 256 pieces of VEC entries; the eight results meet in the first CTA's shared
-// memory.  One launch whatever the number of rows: a row has eight CTAs' loads in flight, 256 rows fill the GPU.  Bound: the bytes of the
-// logits (in L2 behind the head's product), below about 32 rows one load's latency per run.  Measured on B200, 128256 entries of 16 bits: 16
-// rows 6 us against 45 us of the tensor library's reduction, 256 rows 18 us.
+// memory, which may be written once that CTA is known to run: all arrive at the cluster's barrier as they start, and wait at it behind
+// their loads.  One launch whatever the number of rows: a row has eight CTAs' loads in flight, 256 rows fill the GPU.  Bound: the bytes
+// of the logits (in L2 behind the head's product), below about 32 rows one load's latency per run.  Measured on B200, 128256 entries of
+// 16 bits: 16 rows 6 us against 45 us of the tensor library's reduction, 256 rows 18 us.
 constexpr int AM_CTAS = 8, AM_THREADS = 256, AM_RUNS = 4;
 template <typename T, int VEC>
 __global__ void __cluster_dims__(AM_CTAS, 1, 1) __launch_bounds__(AM_THREADS) argmax_rows_kernel(const T* __restrict__ x, int64_t stride, int n,
@@ -51,10 +53,11 @@ __global__ void __cluster_dims__(AM_CTAS, 1, 1) __launch_bounds__(AM_THREADS) ar
     struct alignas(VEC * sizeof(T)) Piece { T e[VEC]; };
     __shared__ float wv[AM_THREADS / 32], cv[AM_CTAS];
     __shared__ int wi[AM_THREADS / 32], ci[AM_CTAS];
+    cg::cluster_group cluster = cg::this_cluster();
+    auto here = cluster.barrier_arrive();                            // this CTA has started
     wait_previous();
     launch_next();
     x = after_wait(x);
-    cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t row = blockIdx.x / AM_CTAS;
     const T* p = x + row * stride;
@@ -86,6 +89,7 @@ __global__ void __cluster_dims__(AM_CTAS, 1, 1) __launch_bounds__(AM_THREADS) ar
     };
     across(best, at, 32);
     if (lane == 0) { wv[warp] = best; wi[warp] = at; }
+    cluster.barrier_wait(std::move(here));                           // the first CTA has: its shared memory may be written
     __syncthreads();
     if (warp == 0) {
         best = wv[lane & 7]; at = wi[lane & 7];
