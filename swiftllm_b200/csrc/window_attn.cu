@@ -33,6 +33,7 @@
 //                      krot + dk - 1 of the key part) and the value its first dk columns
 //   sinks              a learned number per head: the softmax's denominator also contains exp(sinks[h])
 // diff_combine: per token and head, o = a1 - lambda * a2 of two maps' outputs, o / sqrt(mean(o^2) + eps) * factor * sigmoid(gate).
+#include <mutex>
 #include <type_traits>
 
 #include "mma_helpers.cuh"
@@ -742,7 +743,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_attn_decode_kernel(
     int G, int dk, int dv, int rot_dims, int window, float scale_log2, float sink, int halves, float qk_norm_eps,
     float softcap, const float* __restrict__ vcos, const float* __restrict__ vsin, float out_scale,
     const float* __restrict__ qnorm_w, float prenorm_eps, int chunk, int vshare, int out_f32, const float* __restrict__ slopes_,
-    int keep_first_, int gate_per_head_, int shared_kv_, int krot_, const float* __restrict__ sinks_, int beside) {
+    int keep_first_, int gate_per_head_, int shared_kv_, int krot_, const float* __restrict__ sinks_) {
     const float* slopes = EXT ? slopes_ : nullptr;
     const float* sinks = EXT ? sinks_ : nullptr;
     const int keep_first = EXT ? keep_first_ : 0, krot = EXT ? krot_ : 0;
@@ -1037,7 +1038,6 @@ __global__ void __launch_bounds__(WD_WARPS * 32) window_attn_decode_kernel(
         if (out_f32) reinterpret_cast<float*>(out)[t * out_stride_t + h * dv + d] = y;
         else stf(out + t * out_stride_t + h * dv + d, y);
     }
-    if (beside && blockIdx.x == 0 && blockIdx.y == 0) wait_previous();         // this launch ends no sooner than the prompt rows' one
 }
 
 // ------------------------------------------------------------------ two maps -> one head
@@ -1079,6 +1079,69 @@ __global__ void __launch_bounds__(256) diff_combine_kernel(const float* __restri
 
 static bool g_window_simt = false;
 
+// ------------------------------------------------------------------ a launch beside another one
+// A stream that begins where the caller's stands as this is made, and that the caller's waits for from join() on: what is launched on it
+// runs beside what the caller's stream is given in between, and touches nothing that that writes.  Where a graph is being captured, or no
+// stream is to be had, it is the caller's own.  Streams and their events go back to a list of at most KEPT, whose lock is held for
+// the list alone (the next user's work merely queues behind what is left on a stream).
+class StreamBeside {
+    struct Lane { cudaStream_t stream; cudaEvent_t begin, end; int device; };
+    static constexpr int KEPT = 16;
+    static inline std::mutex lock;
+    static inline Lane idle[KEPT];
+    static inline int num_idle = 0;
+    cudaStream_t caller;
+    Lane lane = {nullptr, nullptr, nullptr, -1};
+
+    void drop() {
+        if (lane.begin) cudaEventDestroy(lane.begin);
+        if (lane.end) cudaEventDestroy(lane.end);
+        if (lane.stream) cudaStreamDestroy(lane.stream);                      // once its work has ended
+        lane.stream = nullptr;
+    }
+    bool take() {
+        lane.device = current_device();
+        {
+            std::lock_guard<std::mutex> held(lock);
+            for (int i = num_idle - 1; i >= 0; i--)
+                if (idle[i].device == lane.device) { lane = idle[i]; idle[i] = idle[--num_idle]; return true; }
+        }
+        return cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking) == cudaSuccess &&
+               cudaEventCreateWithFlags(&lane.begin, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&lane.end, cudaEventDisableTiming) == cudaSuccess;
+    }
+    bool give_back() {
+        std::lock_guard<std::mutex> held(lock);
+        if (num_idle == KEPT) return false;
+        idle[num_idle++] = lane;
+        lane.stream = nullptr;
+        return true;
+    }
+
+  public:
+    StreamBeside(cudaStream_t of, bool wanted) : caller(of) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+        if (!wanted) return;
+        const bool known = cudaStreamIsCapturing(of, &capture) == cudaSuccess;
+        if (known && capture != cudaStreamCaptureStatusNone) return;
+        if (known && take() && cudaEventRecord(lane.begin, of) == cudaSuccess && cudaStreamWaitEvent(lane.stream, lane.begin, 0) == cudaSuccess) return;
+        drop();
+        cudaGetLastError();                                                   // not an error of the call: it goes on without
+    }
+    StreamBeside(const StreamBeside&) = delete;
+    StreamBeside& operator=(const StreamBeside&) = delete;
+    ~StreamBeside() { join(); }
+    cudaStream_t stream() const { return lane.stream ? lane.stream : caller; }
+    int join() {                                                              // an error: the caller's stream does not wait
+        if (!lane.stream) return 0;
+        cudaError_t e = cudaEventRecord(lane.end, lane.stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(caller, lane.end, 0);
+        if (e != cudaSuccess || !give_back()) drop();
+        SLLM_REQUIRE(e == cudaSuccess, "a launch beside another one: %s", cudaGetErrorString(e));
+        return 0;
+    }
+};
+
 // rows [0, num_prefill) are prompt portions (many consecutive tokens of a sequence share a CTA), the rest single decoded tokens
 template <typename T, int DMAX, bool EXT>
 static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void* cosb, const void* sinb, const void* gate,
@@ -1109,12 +1172,16 @@ static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void*
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, current_device());
     const float scale_log2 = scale * 1.4426950408889634f;
     const int64_t parts[2][2] = {{0, num_prefill}, {num_prefill, num_tokens - num_prefill}};
-    int prompts_tc = 0;                                                        // the launch before this one: prompt rows on tcgen05
+    // Decoded rows beside prompt rows of the tcgen05 kernel: neither launch touches what the other writes, so the decoded rows run on a
+    // stream beside the caller's, on the SMs that the prompt rows' last CTAs leave over (3 prompts of up to 2048 tokens and 40 decoded
+    // rows, 16 / 4 heads: 118 -> 92 us).  The prompt rows are launched first, which find their SMs first.
+    const bool prompts_tc = num_prefill > 0 && window_tc_supported(dk, dv, krot, hq, scale, cache, num_prefill);
+    StreamBeside beside(stream, prompts_tc && num_tokens > num_prefill && hq <= 16);
     for (int k = 0; k < 2; k++) {
         const int64_t first = parts[k][0], count = parts[k][1];
         if (count <= 0) continue;
         // prompt rows: tcgen05 (window_attn_tc.cu) where the products can be cut from the rows
-        if (k == 0 && window_tc_supported(dk, dv, krot, hq, scale, cache, count)) {
+        if (k == 0 && prompts_tc) {
             WindowTc w;
             w.q = q; w.q_st = q_stride_t; w.cosb = (const float*)cosb; w.sinb = (const float*)sinb; w.gate = gate; w.gate_st = gate_stride_t;
             w.cache = cache; w.n_slots = n_slots; w.slot = slot; w.block_size = block_size; w.block_table = (const int*)block_table;
@@ -1131,27 +1198,18 @@ static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void*
             w.gate_vec = ((uintptr_t)gate & 15) == 0 && gate_stride_t % 8 == 0;
             w.out_vec = ((uintptr_t)out & 15) == 0 && out_stride_t % 8 == 0;
             if (int rc = launch_window_attn_tc(w, std::is_same<T, __half>::value ? SLLM_F16 : SLLM_BF16, stream)) return rc;
-            prompts_tc = 1;
             continue;
         }
         if (k == 1 && hq <= 16) {
             size_t smem = 16 * (size_t)(dk * 2 + 16) + WD_WARPS * WD_STAGES * (size_t)KT * (tile_pitch(dk + krot) + (shared_kv ? sizeof(float) : dv * 2 + 16));
             const size_t merge = ((size_t)WD_WARPS * hq * dv + 2 * WD_WARPS * 16) * sizeof(float);
             if (smem < merge) smem = merge;
-            // Beside prompt rows of the tcgen05 kernel the two launches share nothing that either writes: this one begins once every CTA of that
-            // one has, on the SMs that its last CTAs leave over, and one of its CTAs waits for that launch's end (3 prompts of up to 2048 tokens
-            // and 40 decoded rows, 16 / 4 heads: 118 -> 88 us).
-            const int beside = prompts_tc;
-            const dim3 grid((unsigned)count, (unsigned)G);
-            auto launch = [&](auto... args) {
-                if (beside) launch_early(kern_split, grid, WD_WARPS * 32, smem, stream, args...);
-                else kern_split<<<grid, WD_WARPS * 32, smem, stream>>>(args...);
-            };
-            launch((const T*)q, q_stride_t, (const float*)cosb, (const float*)sinb, (const T*)gate, gate_stride_t, (const T*)cache,
+            kern_split<<<dim3((unsigned)count, (unsigned)G), WD_WARPS * 32, smem, beside.stream()>>>(
+                (const T*)q, q_stride_t, (const float*)cosb, (const float*)sinb, (const T*)gate, gate_stride_t, (const T*)cache,
                 n_slots, slot, block_size, (const int*)block_table, max_blocks_per_seq, (const int*)tok_seq, (const int*)tok_pos,
                 (T*)out, out_stride_t, (int)first, hq, G, dk, dv, rot_dims, window, scale_log2, sink, halves, qk_norm_eps, softcap,
                 (const float*)vcos, (const float*)vsin, out_scale, (const float*)qnorm_w, prenorm_eps, chunk, vshare, out_f32,
-                (const float*)slopes, keep_first, gate_per_head, shared_kv, krot, (const float*)sinks, beside);
+                (const float*)slopes, keep_first, gate_per_head, shared_kv, krot, (const float*)sinks);
             continue;
         }
         const int qt = k == 0 ? WT_ROWS >> hqp_log2 : 1;
@@ -1167,6 +1225,7 @@ static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void*
             halves, qk_norm_eps, softcap, (const float*)vcos, (const float*)vsin, out_scale, (const float*)qnorm_w, prenorm_eps,
             chunk, vshare, out_f32, (const float*)slopes, keep_first, gate_per_head, shared_kv, krot, (const float*)sinks);
     }
+    if (int rc = beside.join()) return rc;
     return check_launch("window_attention (tensor cores)");
 }
 

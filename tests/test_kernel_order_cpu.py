@@ -44,3 +44,38 @@ def test_other_ctas_have_started_before_their_shared_memory_is_touched(kernel):
     waits = [m.start() for m in re.finditer(r"\bcluster_sync_all\(|\bcluster\.(?:sync|barrier_wait)\(", body)]
     remote = [m.start() for m in REMOTE.finditer(body)]
     assert waits and waits[0] < remote[0] and waits[-1] > remote[0]           # started; and nobody leaves, or reads, too early
+
+
+def _launched_early():
+    """The kernels that files hand to launch_early, by name or through a variable."""
+    names = set()
+    for name, text in _files():
+        for m in re.finditer(r"(?<!void )\blaunch_early(_clusters)?\(", text):
+            args = text[m.end():_closing(text, m.end() - 1, "()")]
+            kern = args.split(",")[1 if m.group(1) else 0].strip()
+            if kern == "kern" and name == "common.cuh":
+                continue
+            direct = re.match(r"\w+_kernel\b", kern)
+            if direct:
+                names.add(direct.group(0))
+                continue
+            variable = re.match(r"\w+", kern).group(0)              # every kernel that it is given in this file
+            given = "".join(re.findall(r"\b%s\b[^;=]*=([^;]*);" % variable, text))
+            if not given:                                           # the parameter of a local launcher
+                given = "".join(re.findall(r"\blaunch\(([^;]*);", text))
+            found = re.findall(r"\w+_kernel\b", given)
+            assert found, (name, kern)
+            names.update(found)
+    return sorted(names)
+
+
+@pytest.mark.parametrize("kernel", _launched_early())
+def test_kernels_launched_early_wait_before_they_touch_memory(kernel):
+    params, body = KERNELS[kernel][1:]
+    assert "wait_previous();" in body, "never waits"
+    before, after = body.split("wait_previous();", 1)
+    structs = re.findall(r"const \w+ (p|pg)\b", params)
+    for p in re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)", params):
+        assert not re.search(r"\b%s\b" % p, before), f"{p} is used before the wait"
+    for p in structs:                                                # sizes may be read; what their pointers lead to may not
+        assert not re.search(r"\b%s\.\w+\[" % p, before), f"an array of {p} is read before the wait"
