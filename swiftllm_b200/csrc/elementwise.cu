@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(T* __restrict__ x, T* __re
     using TT = Traits<T>;
     wait_previous();
     launch_next();
-    x = after_wait(x); residual = after_wait(residual); rows = after_wait(rows);
+    x = after_wait(x); residual = after_wait(residual); weight = after_wait(weight); rows = after_wait(rows);
     const int64_t t = GATHER ? rows[blockIdx.x] : (int64_t)blockIdx.x;
     if (GATHER) assert(t >= 0 && t < num_rows);
     T* xr = x + t * hidden;

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const int* __restrict_
                                                           const P* __restrict__ table_b, P* __restrict__ out_b, int nb) {
     wait_previous();
     launch_next();
-    idx = after_wait(idx);
+    idx = after_wait(idx); table_a = after_wait(table_a); table_b = after_wait(table_b);
     const int64_t t = blockIdx.x, r = (int64_t)idx[t] + offset;
     assert(r >= 0 && r < table_rows);
     for (int i = threadIdx.x; i < na; i += blockDim.x) out_a[t * na + i] = table_a[r * na + i];

@@ -79,3 +79,11 @@ def test_kernels_launched_early_wait_before_they_touch_memory(kernel):
         assert not re.search(r"\b%s\b" % p, before), f"{p} is used before the wait"
     for p in structs:                                                # sizes may be read; what their pointers lead to may not
         assert not re.search(r"\b%s\.\w+\[" % p, before), f"an array of {p} is read before the wait"
+
+
+@pytest.mark.parametrize("kernel", [k for k, (_, _, body) in KERNELS.items() if "wait_previous();" in body])
+def test_arguments_taken_for_constant_are_taken_anew_behind_the_wait(kernel):
+    """Loads through a const __restrict__ argument may be moved ahead of the wait: the pointer goes through after_wait."""
+    params, body = KERNELS[kernel][1:]
+    for p in re.findall(r"const [^,]*?\*\s*__restrict__\s*(\w+)", params):
+        assert re.search(r"\b%s = after_wait\(%s\);" % (p, p), body.split("wait_previous();", 1)[1]), f"{p} is not"
