@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) silu_and_mul_kernel(T* __restrict__ x, in
         up_p[u] = x + (idx / vec_per_row) * 2 * F + 8 * (idx % vec_per_row);
     }
 #pragma unroll
-    for (int u = 0; u < 2; u++) { up[u] = ld_vec8(up_p[u]); gate[u] = ld_vec8_stream(up_p[u] + F); }
+    for (int u = 0; u < 2; u++) { up[u] = ld_vec8(up_p[u]); gate[u] = ld_vec8(up_p[u] + F); }
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         if (u == 1 && !two) break;

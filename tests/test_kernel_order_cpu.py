@@ -87,3 +87,9 @@ def test_arguments_taken_for_constant_are_taken_anew_behind_the_wait(kernel):
     params, body = KERNELS[kernel][1:]
     for p in re.findall(r"const [^,]*?\*\s*__restrict__\s*(\w+)", params):
         assert re.search(r"\b%s = after_wait\(%s\);" % (p, p), body.split("wait_previous();", 1)[1]), f"{p} is not"
+
+
+@pytest.mark.parametrize("kernel", [k for k, (_, _, body) in KERNELS.items() if "wait_previous();" in body])
+def test_no_non_coherent_loads_in_kernels_launched_early(kernel):
+    """They ask that nobody writes the memory for as long as the kernel lives, which begins while the kernel ahead still writes."""
+    assert not re.search(r"ld_vec8_stream|__ldg|ld\.global\.nc", KERNELS[kernel][2])
