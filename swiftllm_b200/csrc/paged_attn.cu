@@ -236,7 +236,7 @@ __global__ void paged_attn_merge_kernel(const float* __restrict__ part_o, const 
     launch_next();
     part_o = after_wait(part_o); part_lse = after_wait(part_lse); seq_lens = after_wait(seq_lens);
     const int head = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
-    const int n = (seq_lens[seq] + split_tokens - 1) / split_tokens;
+    const int n = min((seq_lens[seq] + split_tokens - 1) / split_tokens, num_splits);        // (tokens past them are not seen)
     const int64_t base = ((int64_t)seq * nq + head) * num_splits;
     float m = -INFINITY;
     for (int s = 0; s < n; s++) m = fmaxf(m, part_lse[base + s]);

@@ -22,6 +22,9 @@
 // merges a share of the heads.  No workspace, no second launch: one sequence of 700 tokens, 32 / 8 heads, 13.6 -> 9 us on the device.
 // Larger launches keep the merge kernel, which costs them nothing beside their tiles.
 // HBM roofline: algorithmic bytes = sum_i len_i * nkv * 128 * 2 * sizeof(T) + 2 * Bd * nq * 128 * sizeof(T).
+#include <limits.h>
+
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -48,7 +51,7 @@ struct TcParams {
     const int32_t* block_table; const int32_t* seq_ids; const int32_t* seq_lens;
     void* o; float* part_o; float* part_lse;
     float scale_log2e;
-    int split_tokens, num_splits, cur_layer, num_layers, nq, nkv, max_blocks_per_seq, num_seqs, num_items;
+    int split_tokens, num_splits, longest, cur_layer, num_layers, nq, nkv, max_blocks_per_seq, num_seqs, num_items;
     // shared-memory placement of the 1 KiB atoms of a KV tile and the matching descriptor strides
     int page_stride, tg_stride, half_stride, k_sbo, v_lbo, v_sbo, tma_4d;
     int counted;                      // items are the splits that exist (see Items)
@@ -64,6 +67,8 @@ struct Barriers {       // all mbarriers of the CTA (shared memory)
     uint64_t o_full[2], o_empty[2];
 };
 
+// Tokens past the launch's splits (a length above the longest that the caller stated, for which there is neither workspace nor a CTA of
+// the cluster) are not seen: every length is cut to p.longest.
 struct Item { int seq, kvh, split, split_start, split_len, ntiles; };
 
 // The launch's items.  Counted: idx runs over the whole splits of all sequences, kv heads fastest, and then over their last, shorter ones, so
@@ -99,7 +104,7 @@ __device__ __forceinline__ bool get_item(const TcParams& p, const Items& w, int 
     }
     // every caller is a converged warp: broadcasting the loaded length makes it (and everything derived from it)
     // provably warp-uniform for the compiler
-    const int len = __shfl_sync(0xffffffffu, p.seq_lens[it.seq], 0);
+    const int len = min(__shfl_sync(0xffffffffu, p.seq_lens[it.seq], 0), p.longest);
     it.split_start = it.split * p.split_tokens;
     if (it.split_start >= len) return false;
     it.split_len = min(p.split_tokens, len - it.split_start);
@@ -235,7 +240,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
         if (warp == 0) {
             int total = 0;
             for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
-                const int mine = s0 + lane < p.num_seqs ? p.seq_lens[s0 + lane] / p.split_tokens : 0;
+                const int mine = s0 + lane < p.num_seqs ? max(min(p.seq_lens[s0 + lane], p.longest), 0) / p.split_tokens : 0;
                 int sum = mine;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) { const int x = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += x; }
@@ -441,7 +446,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
         cluster_sync_all();
         if (warp >= 2 && warp < 6) {
             const int idx = blockIdx.x, split = idx % p.num_splits, kvh = idx / p.num_splits % p.nkv, seq = idx / (p.num_splits * p.nkv);
-            const int row = (warp & 3) * 32 + lane, n = (p.seq_lens[seq] + p.split_tokens - 1) / p.split_tokens;
+            const int row = (warp & 3) * 32 + lane, n = (min(p.seq_lens[seq], p.longest) + p.split_tokens - 1) / p.split_tokens;
             for (int h = split; h < g; h += p.num_splits) {
                 float m = -INFINITY, L = 0.f, O = 0.f;
                 for (int s = 0; s < n; s++) m = fmaxf(m, ld_cluster(smem_u32(lse_sm + h), s));
@@ -561,7 +566,8 @@ int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, con
 
     TcParams p;
     p.block_table = block_table; p.seq_ids = seq_ids; p.seq_lens = seq_lens; p.o = o; p.part_o = part_o; p.part_lse = part_lse;
-    p.scale_log2e = scale_log2e; p.split_tokens = split_tokens; p.num_splits = num_splits; p.cur_layer = cur_layer;
+    p.scale_log2e = scale_log2e; p.split_tokens = split_tokens; p.num_splits = num_splits;
+    p.longest = (int)std::min<int64_t>((int64_t)num_splits * split_tokens, INT_MAX - split_tokens); p.cur_layer = cur_layer;
     p.num_layers = num_layers; p.nq = nq; p.nkv = nkv; p.max_blocks_per_seq = max_blocks_per_seq; p.num_seqs = num_seqs;
     p.num_items = num_seqs * nkv * num_splits;
     p.clustered = clustered;

@@ -40,3 +40,27 @@ def test_splits_in_a_cluster(dtype, lens, H, G, sbs, clustered):
         want = torch.einsum("hn,nhd->hd", p, v).flatten()
         # the output and the softmax's weights are rounded once each
         assert float((out[i].double() - want).norm() / want.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), i
+
+
+@pytest.mark.parametrize("B,G", [(2, 2), (3, 8), (60, 2)])
+def test_lengths_above_the_longest_are_cut(B, G):
+    """Tokens past the launch's splits are not seen, and nothing is written past the workspace: splits in a cluster, counted splits and the
+    merge, with every third length above the stated longest."""
+    H, D, st_tokens, longest = 2 * G, 128, 256, 1024
+    lens = [3 * longest if i % 3 == 1 else 700 + 13 * i % 300 for i in range(B)]
+    blocks = 3 * longest // 16
+    kc, vc = (_normal(blocks, 1, G, 16, D, seed=i, dtype=torch.bfloat16) for i in (1, 2))
+    table = torch.stack([torch.randperm(blocks, generator=torch.Generator().manual_seed(i)) for i in range(B)]).to(torch.int32).to(DEV)
+    q = _normal(B, H, D, seed=4, dtype=torch.bfloat16)
+    ids, l = _ints(range(B)), _lib.lib()
+    floats = l.sllm_paged_attention_workspace_bytes(B, H, D, longest, st_tokens, G) // 4
+    outs = []
+    for stated in (lens, [min(n, longest) for n in lens]):
+        ws = torch.full((floats + (1 << 20),), 7.0, device=DEV)
+        out, n = torch.empty(B, H * D, dtype=torch.bfloat16, device=DEV), _ints(stated)
+        _lib.check(l.sllm_paged_attention(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), table.data_ptr(), ids.data_ptr(), n.data_ptr(), out.data_ptr(),
+                                          ws.data_ptr(), 4 * floats, D ** -0.5, B, longest, st_tokens, 0, 1, H, G, 16, D, blocks, blocks, H * D,
+                                          _lib.dtype_tag(q.dtype), _lib.stream()), "paged_attention")
+        assert bool((ws[floats:] == 7.0).all())
+        outs.append(out)
+    assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0], outs[1])
