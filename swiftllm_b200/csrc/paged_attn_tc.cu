@@ -17,8 +17,8 @@
 // Tokens are the MMA M dimension (the transposed problem), so no tensor work is spent on padded query rows and the
 // softmax uses all 128 threads; the GQA group is the N dimension (padded to 16 by reading neighbouring heads whose
 // columns are simply never read back).
-// CLUSTERS: in launches of at most one item per SM with two to eight splits the splits of a (sequence, kv head) are a cluster, and their
-// parts meet through distributed shared memory: every CTA leaves its part in its own (in the K ring, which nobody needs any more), and
+// CLUSTERS: in launches of two to eight splits whose items fill at most three quarters of the SMs (meets_in_cluster, paged_attn.cu) the splits
+// of a (sequence, kv head) are a cluster, and their parts meet through distributed shared memory: every CTA leaves its part in its own (in the K ring, which nobody needs any more), and
 // merges a share of the heads.  No workspace, no second launch: one sequence of 700 tokens, 32 / 8 heads, 13.6 -> 9 us on the device.
 // Larger launches keep the merge kernel, which costs them nothing beside their tiles.
 // HBM roofline: algorithmic bytes = sum_i len_i * nkv * 128 * 2 * sizeof(T) + 2 * Bd * nq * 128 * sizeof(T).
@@ -44,7 +44,7 @@ constexpr int TC_NPAD = 16;               // UMMA N (heads, padded)
 constexpr int TC_K_BYTES = TC_TILE * TC_D * 2;                 // 32 KiB per K (or V) tile
 constexpr int TC_Q_BYTES = 2 * TC_NPAD * 128;                  // [half][16 rows][128 B] = 4 KiB
 constexpr int TC_P_BYTES = 2 * TC_NPAD * 128;                  // [token half][16 rows][128 B] = 4 KiB
-constexpr int TC_SMEM_BYTES = (TC_KSTAGES + TC_VSTAGES) * TC_K_BYTES + 2 * TC_Q_BYTES + 2 * TC_P_BYTES + 2048;
+constexpr int TC_SMEM_BYTES = (TC_KSTAGES + TC_VSTAGES) * TC_K_BYTES + 2 * TC_Q_BYTES + 2 * TC_P_BYTES + 3072;
 constexpr int TC_TMEM_COLS = 64;          // S: 2 x 16, O: 2 x 16
 
 struct TcParams {
@@ -54,8 +54,6 @@ struct TcParams {
     int split_tokens, num_splits, longest, cur_layer, num_layers, nq, nkv, max_blocks_per_seq, num_seqs, num_items;
     // shared-memory placement of the 1 KiB atoms of a KV tile and the matching descriptor strides
     int page_stride, tg_stride, half_stride, k_sbo, v_lbo, v_sbo, tma_4d;
-    int counted;                      // items are the splits that exist (see Items)
-    int clustered;                    // the splits of a (sequence, kv head) are a cluster; every CTA has one item or none
 };
 
 struct Barriers {       // all mbarriers of the CTA (shared memory)
@@ -71,32 +69,35 @@ struct Barriers {       // all mbarriers of the CTA (shared memory)
 // the cluster) are not seen: every length is cut to p.longest.
 struct Item { int seq, kvh, split, split_start, split_len, ntiles; };
 
-// The launch's items.  Counted: idx runs over the whole splits of all sequences, kv heads fastest, and then over their last, shorter ones, so
-// that every CTA gets its share and the launch ends on short items (idx over all splits that the longest sequence has gave some CTAs twice
-// the work of others: a Llama step of 16 sequences of up to 1500 tokens 428 -> 419 us).  `before`: whole splits of the sequences before each,
-// for as many sequences as there is room for.
-constexpr int TC_COUNTED = 200;
-struct Items { const int* before; int count; };
+// A launch's items (compiled into the kernel: as a branch per item, the search below cost launches without it 2 to 13 %; 256 sequences of
+// 64 tokens, 32 / 8 heads, 32 us without and 34 with the branch):
+//   NUMBERED   idx runs over all splits that the longest sequence has
+//   COUNTED    idx runs over the whole splits of all sequences, kv heads fastest, and then over their last, shorter ones, so that every CTA
+//              gets its share and the launch ends on short items (numbered, some CTAs get twice the work of others: 32 sequences of up to
+//              1500 tokens, 16 / 4 heads, 28 us instead of 18.6; 100 of 700 each, 64 / 8 heads, 68 instead of 71)
+//   CLUSTERED  as NUMBERED, one item or none per CTA: the splits of a (sequence, kv head) are a cluster
+enum PagedItems { NUMBERED, COUNTED, CLUSTERED };
+constexpr int TC_COUNTED = 200;      // sequences whose sums find room behind the barriers and the reduction scratch: more are numbered
+static_assert(TC_COUNTED <= 256, "get_item looks through eights of 32 lanes");
+struct Items { const int* before; const int* lens; int count; };     // counted: whole splits of the sequences before each [num_seqs + 1], lengths
 
+template <PagedItems MODE>
 __device__ __forceinline__ bool get_item(const TcParams& p, const Items& w, int idx, Item& it) {
-    if (w.before != nullptr) {
-        const int s = idx / p.nkv;
+    if constexpr (MODE == COUNTED) {
+        const int s = idx / p.nkv, lane = threadIdx.x & 31;
         it.kvh = idx - s * p.nkv;
         const int whole = w.before[p.num_seqs];
-        int lo = s - whole, split = -1;                              // a last split
-        if (s < whole) {
-            int hi = p.num_seqs;                                     // before[lo] <= s < before[hi]
-            lo = 0;
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (w.before[mid] <= s) lo = mid; else hi = mid;
-            }
-            split = s - w.before[lo];
-        } else {
-            split = w.before[lo + 1] - w.before[lo];                 // (of no tokens where the whole ones are all)
+        if (s < whole) {                                             // the last sequence with before[seq] <= s: its eight, then itself
+            const uint32_t eights = __ballot_sync(0xffffffffu, 8 * lane < p.num_seqs && w.before[min(8 * lane, p.num_seqs)] <= s);
+            const int q = 8 * (__popc(eights) - 1) + (lane & 7);
+            const uint32_t mine = __ballot_sync(0xffffffffu, lane < 8 && q < p.num_seqs && w.before[min(q, p.num_seqs)] <= s);
+            it.seq = 8 * (__popc(eights) - 1) + __popc(mine) - 1;
+            it.split = s - w.before[it.seq];
+        } else {                                                     // a last split (of no tokens where the whole ones are all)
+            it.seq = s - whole;
+            it.split = w.before[it.seq + 1] - w.before[it.seq];
         }
-        it.seq = __shfl_sync(0xffffffffu, lo, 0);
-        it.split = __shfl_sync(0xffffffffu, split, 0);
+        it.split = __shfl_sync(0xffffffffu, it.split, 0);
     } else {
         it.split = idx % p.num_splits;
         it.kvh = (idx / p.num_splits) % p.nkv;
@@ -104,7 +105,7 @@ __device__ __forceinline__ bool get_item(const TcParams& p, const Items& w, int 
     }
     // every caller is a converged warp: broadcasting the loaded length makes it (and everything derived from it)
     // provably warp-uniform for the compiler
-    const int len = min(__shfl_sync(0xffffffffu, p.seq_lens[it.seq], 0), p.longest);
+    const int len = __shfl_sync(0xffffffffu, MODE == COUNTED ? w.lens[it.seq] : min(p.seq_lens[it.seq], p.longest), 0);
     it.split_start = it.split * p.split_tokens;
     if (it.split_start >= len) return false;
     it.split_len = min(p.split_tokens, len - it.split_start);
@@ -113,7 +114,7 @@ __device__ __forceinline__ bool get_item(const TcParams& p, const Items& w, int 
 }
 
 // Walks this CTA's work items tile by tile (every role runs the same deterministic schedule).
-struct TileCursor {
+template <PagedItems MODE> struct TileCursor {
     int idx;            // global item index (blockIdx.x + k * gridDim.x)
     Item it;
     int j;              // tile within the item
@@ -122,7 +123,7 @@ struct TileCursor {
     __device__ __forceinline__ void seek(const TcParams& p, const Items& w) {            // position on the next non-empty item
         valid = false;
         while (idx < w.count) {
-            if (get_item(p, w, idx, it)) { valid = true; j = 0; return; }
+            if (get_item<MODE>(p, w, idx, it)) { valid = true; j = 0; return; }
             idx += gridDim.x;
         }
     }
@@ -135,13 +136,13 @@ struct TileCursor {
 
 // One producer warp streams either the K or the V tiles (plus Q when IS_K): 32 block-table entries are fetched per
 // 4 tiles (prefetched one group ahead), lanes 0..7 each issue the TMA of one page.
-template <bool IS_K>
+template <bool IS_K, PagedItems MODE>
 __device__ __forceinline__ void producer_loop(const TcParams& p, const Items& w, const CUtensorMap* map, const CUtensorMap* qmap, uint8_t* ring,
                                               uint64_t* full, uint64_t* empty, int nstages, Barriers* bars, uint8_t* q_sm, int g, int lane) {
     uint32_t t = 0, n = 0;
     for (int idx = blockIdx.x; idx < w.count; idx += gridDim.x) {
         Item it;
-        if (!get_item(p, w, idx, it)) continue;
+        if (!get_item<MODE>(p, w, idx, it)) continue;
         if (IS_K) {       // Q of this item: heads [kvh*g, +16) of sequence seq, 128 d as two 64-wide boxes
             const int qb = n & 1;
             if (lane == 0) {
@@ -189,7 +190,7 @@ __device__ __forceinline__ void producer_loop(const TcParams& p, const Items& w,
     }
 }
 
-template <typename T, int G>      // G = number of S/O columns read back (GQA group padded to 4, 8 or 16)
+template <typename T, int G, PagedItems MODE>      // G = number of S/O columns read back (GQA group padded to 4, 8 or 16)
 __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __grid_constant__ CUtensorMap kmap,
                                                                       const __grid_constant__ CUtensorMap vmap,
                                                                       const __grid_constant__ CUtensorMap qmap,
@@ -234,30 +235,32 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
     const uint32_t tmem = *tmem_base_s;
     wait_previous();                                                 // so far nothing in memory was touched
     launch_next();
-    Items w{nullptr, p.num_items};
-    if (p.counted) {
+    Items w{nullptr, nullptr, p.num_items};
+    if constexpr (MODE == COUNTED) {
         int* before = reinterpret_cast<int*>(misc + 1216);           // [num_seqs + 1]
+        int* lens = reinterpret_cast<int*>(misc + 2048);             // [num_seqs]
+        static_assert(1216 + 4 * (TC_COUNTED + 1) <= 2048 && 2048 + 4 * TC_COUNTED <= 3072, "");
         if (warp == 0) {
             int total = 0;
             for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
-                const int mine = s0 + lane < p.num_seqs ? max(min(p.seq_lens[s0 + lane], p.longest), 0) / p.split_tokens : 0;
+                const int len = s0 + lane < p.num_seqs ? max(min(p.seq_lens[s0 + lane], p.longest), 0) : 0, mine = len / p.split_tokens;
                 int sum = mine;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) { const int x = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += x; }
-                if (s0 + lane < p.num_seqs) before[s0 + lane] = total + sum - mine;
+                if (s0 + lane < p.num_seqs) { before[s0 + lane] = total + sum - mine; lens[s0 + lane] = len; }
                 total += __shfl_sync(0xffffffffu, sum, 31);
             }
             if (lane == 0) before[p.num_seqs] = total;
         }
         __syncthreads();
-        w.before = before;
+        w.before = before; w.lens = lens;
         w.count = (before[p.num_seqs] + p.num_seqs) * p.nkv;
     }
 
     if (warp == 0) {
-        producer_loop<true>(p, w, &kmap, &qmap, k_sm, bars->k_full, bars->k_empty, TC_KSTAGES, bars, q_sm, g, lane);
+        producer_loop<true, MODE>(p, w, &kmap, &qmap, k_sm, bars->k_full, bars->k_empty, TC_KSTAGES, bars, q_sm, g, lane);
     } else if (warp == 6) {
-        producer_loop<false>(p, w, &vmap, &qmap, v_sm, bars->v_full, bars->v_empty, TC_VSTAGES, bars, q_sm, g, lane);
+        producer_loop<false, MODE>(p, w, &vmap, &qmap, v_sm, bars->v_full, bars->v_empty, TC_VSTAGES, bars, q_sm, g, lane);
     } else if (warp == 1) {
         // =========================================================== MMA issuer: two in-order queues, polled.  The whole warp
         // runs the loop converged (votes keep the control flow warp-uniform) and one elected lane issues (see elect_one).
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
             const uint64_t dq0 = make_smem_desc(smem_u32(q_sm), 16, 1024);
             const uint64_t dv0 = make_smem_desc(smem_u32(v_sm), p.v_lbo, p.v_sbo);
             const uint64_t dp0 = make_smem_desc(smem_u32(p_sm), 16, 1024);
-            TileCursor cs, cp;                  // next S tile / next PV tile
+            TileCursor<MODE> cs, cp;                  // next S tile / next PV tile
             cs.init(p, w); cp.init(p, w);
             uint32_t spins = 0;
             while (cp.valid) {
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
         T* const out = reinterpret_cast<T*>(p.o);
         for (int idx = blockIdx.x; idx < w.count; idx += gridDim.x) {
             Item it;
-            if (!get_item(p, w, idx, it)) continue;
+            if (!get_item<MODE>(p, w, idx, it)) continue;
             float m_run[G], l_part[G], acc[G], alpha_prev[G];
 #pragma unroll
             for (int h = 0; h < G; h++) { m_run[h] = -INFINITY; l_part[h] = 0.f; acc[h] = 0.f; alpha_prev[h] = 0.f; }
@@ -426,9 +429,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
                     const float L = (rp[h] + rp[16 + h]) + (rp[32 + h] + rp[48 + h]);
                     const float val = acc[h] / L;
                     const int head = it.kvh * g + h;
-                    if (p.num_splits == 1) {
+                    if (MODE == NUMBERED && p.num_splits == 1) {
                         out[((int64_t)it.seq * p.nq + head) * TC_D + row] = Traits<T>::from_f(val);
-                    } else if (p.clustered) {
+                    } else if constexpr (MODE == CLUSTERED) {
                         part_sm[h * TC_D + row] = val;
                         if (row == 0) lse_sm[h] = log2f(L) + m_run[h];
                     } else {
@@ -441,7 +444,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
         }
     }
 
-    if (p.clustered) {                                               // the splits' parts meet: like the merge kernel, a share of the heads each
+    if constexpr (MODE == CLUSTERED) {                               // the splits' parts meet: like the merge kernel, a share of the heads each
         __syncwarp();
         cluster_sync_all();
         if (warp >= 2 && warp < 6) {
@@ -570,26 +573,28 @@ int launch_paged_tc(const void* q, const void* k_cache, const void* v_cache, con
     p.longest = (int)std::min<int64_t>((int64_t)num_splits * split_tokens, INT_MAX - split_tokens); p.cur_layer = cur_layer;
     p.num_layers = num_layers; p.nq = nq; p.nkv = nkv; p.max_blocks_per_seq = max_blocks_per_seq; p.num_seqs = num_seqs;
     p.num_items = num_seqs * nkv * num_splits;
-    p.clustered = clustered;
-    p.counted = num_splits > 1 && !clustered && num_seqs <= TC_COUNTED;
     p.tma_4d = g_kv_4d_ok == 1;
     if (p.tma_4d) { p.page_stride = 4096; p.tg_stride = 2048; p.half_stride = 1024; p.k_sbo = 2048; p.v_lbo = 1024; p.v_sbo = 2048; }
     else          { p.page_stride = 2048; p.tg_stride = 1024; p.half_stride = 16384; p.k_sbo = 1024; p.v_lbo = 16384; p.v_sbo = 1024; }
     const int grid = p.num_items < num_sms ? p.num_items : num_sms;
     const int g = nq / nkv;
 
-#define SLLM_TC_LAUNCH(TT, GG)                                                                                          \
+#define SLLM_TC_LAUNCH(TT, GG, MODE)                                                                                    \
     do {                                                                                                                 \
         static unsigned long long configured = 0;                                                                        \
+        auto kern = paged_attn_tc_kernel<TT, GG, MODE>;                                                                  \
         if (first_use_on_this_device(configured))                                                                        \
-            cudaFuncSetAttribute(paged_attn_tc_kernel<TT, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES); \
-        launch_early_clusters(clustered ? num_splits : 1, paged_attn_tc_kernel<TT, GG>, grid, TC_THREADS, TC_SMEM_BYTES, stream, kmap, vmap, qmap, p); \
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES);                      \
+        launch_early_clusters(MODE == CLUSTERED ? num_splits : 1, kern, grid, TC_THREADS, TC_SMEM_BYTES, stream, kmap, vmap, qmap, p); \
     } while (0)
-    if (dtype == SLLM_F16) {
-        if (g <= 4) SLLM_TC_LAUNCH(__half, 4); else if (g <= 8) SLLM_TC_LAUNCH(__half, 8); else SLLM_TC_LAUNCH(__half, 16);
-    } else {
-        if (g <= 4) SLLM_TC_LAUNCH(__nv_bfloat16, 4); else if (g <= 8) SLLM_TC_LAUNCH(__nv_bfloat16, 8); else SLLM_TC_LAUNCH(__nv_bfloat16, 16);
-    }
+#define SLLM_TC_MODE(TT, GG)                                                                                            \
+    do {                                                                                                                 \
+        if (clustered) SLLM_TC_LAUNCH(TT, GG, CLUSTERED);                                                                \
+        else if (num_splits > 1 && num_seqs <= TC_COUNTED) SLLM_TC_LAUNCH(TT, GG, COUNTED);                              \
+        else SLLM_TC_LAUNCH(TT, GG, NUMBERED);                                                                           \
+    } while (0)
+    SLLM_DISPATCH_DTYPE(dtype, { if (g <= 4) SLLM_TC_MODE(T, 4); else if (g <= 8) SLLM_TC_MODE(T, 8); else SLLM_TC_MODE(T, 16); });
+#undef SLLM_TC_MODE
 #undef SLLM_TC_LAUNCH
     return check_launch("paged_attention(tcgen05)");
 }

@@ -1,5 +1,6 @@
-"""GPU: paged attention of small batches whose splits meet in a cluster (csrc/paged_attn_tc.cu) against 64 bits: two to eight splits, splits
-that a shorter sequence does not have, every width of a group, and the largest launch that takes the path beside the first that does not."""
+"""GPU: the items of a paged-attention launch (csrc/paged_attn_tc.cu) against 64 bits.  Splits that meet in a cluster: two to eight, splits
+that a shorter sequence does not have, every width of a group, the largest launch that takes the path beside the first that does not.
+Counted splits: batches around every edge of the scan and of the search, lengths that are whole multiples of a split."""
 import types
 
 import pytest
@@ -40,6 +41,34 @@ def test_splits_in_a_cluster(dtype, lens, H, G, sbs, clustered):
         want = torch.einsum("hn,nhd->hd", p, v).flatten()
         # the output and the softmax's weights are rounded once each
         assert float((out[i].double() - want).norm() / want.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), i
+
+
+@pytest.mark.parametrize("kind", ["mixed", "whole", "short", "one_long"])
+@pytest.mark.parametrize("B", [31, 32, 33, 64, 65, 128, 199, 200, 201])
+def test_counted_splits(B, kind):
+    """Up to 200 sequences are counted, 201 are numbered; `short`: sequences without a whole split among them and at the end."""
+    from swiftllm_b200.worker.kernels.paged_attn import paged_attention
+    H, G, sbs, dtype = 8, 2, 256, torch.bfloat16
+    some = {"mixed": (700, 256, 1, 255, 257, 512, 1024, 300), "whole": (256, 512, 1024, 768), "short": (17, 255, 900, 16, 1, 200, 3),
+            "one_long": (40,)}[kind]
+    lens = [some[i % len(some)] for i in range(B)]
+    lens[B // 2] = 1500
+    blocks = [-(-n // 16) for n in lens]
+    kc, vc = (_normal(sum(blocks), 1, G, 16, 128, seed=i, dtype=dtype) for i in (1, 2))
+    table = torch.zeros(B, max(blocks), dtype=torch.int32)
+    for i, n in enumerate(blocks):
+        table[i, :n] = torch.arange(sum(blocks[:i]), sum(blocks[:i + 1]))
+    q = _normal(B, H, 128, seed=4, dtype=dtype)
+    st = types.SimpleNamespace(num_decoding_seqs=B, num_prefill_seqs=0, seq_ids=_ints(range(B)), decoding_seq_lens=_ints(lens),
+                               softmax_scale=128 ** -0.5, max_decoding_len=max(lens), paged_attn_seq_block_size=sbs)
+    out = torch.full((B, H * 128), float("nan"), dtype=dtype, device=DEV)
+    paged_attention(q, kc, vc, table.to(DEV), None, types.SimpleNamespace(block_size=16), st, 0, out)
+    keys, values = (c[:, 0].transpose(1, 2).flatten(0, 1).double().repeat_interleave(H // G, 1) for c in (kc, vc))
+    for i, n in enumerate(lens):
+        at = 16 * sum(blocks[:i])
+        p = torch.softmax(torch.einsum("hd,nhd->hn", q[i].double(), keys[at:at + n]) * 128 ** -0.5, dim=1)
+        want = torch.einsum("hn,nhd->hd", p, values[at:at + n]).flatten()
+        assert float((out[i].double() - want).norm() / want.norm()) < 2.0 ** -8, i      # output and weights are rounded once each
 
 
 @pytest.mark.parametrize("B,G", [(2, 2), (3, 8), (60, 2)])
