@@ -128,7 +128,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
     tc_fence_after();
     const uint32_t tmem = *tmem_s;
     wait_previous();
-    launch_next();
+    // A merge of splits begins as the CTAs end: they leave no registers for its CTAs, which would all gather on the idle SMs (16 decoded tokens at
+    // up to 4000, 16 heads: 29 us, launched earlier 36; the merge behind the launch's end 29, alone 31 instead of 30)
+    if (p.nsplit == 1) launch_next();
 
     int n_done = 0;                                  // tiles of the passes before: every barrier's phase follows from it
     int pass = 0, solo = -1;                         // solo >= 0: the pass is for this token of the segment alone

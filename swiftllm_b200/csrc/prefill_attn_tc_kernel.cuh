@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if constexpr (PAGED) {                                      // (long launches over packed rows gain nothing: 594 -> 598 us)
         wait_previous();
-        launch_next();
+        if (pg.nsplit == 1) launch_next();                      // (a merge begins as the CTAs end: it would gather on the idle SMs; 64 tokens at 3000: 18.6 -> 17.2 us)
     }
     const int qblk = gridDim.x - 1 - blockIdx.x;                // latest (heaviest) query blocks first
     const int nsplit = PAGED ? pg.nsplit : 1;
