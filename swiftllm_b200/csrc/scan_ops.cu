@@ -118,12 +118,12 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TI* __restrict__ 
 
 // The same for prompt rows where rows are whole pieces of four channels: a thread walks SV_TOKENS rows of four neighbouring channels, two at a
 // time in packed arithmetic, the next four rows' loads in flight beside the four it works on (wider pieces need 154 registers and leave
-// ten warps on an SM: 96 us; eight rows 60, two 58); where the rows of the tile break (another sequence) is found once per warp.  The products, their order and
-// the SiLU's value are those above (a quicker quotient turns some roundings, which a state behind the convolution keeps).  Bound: bytes,
-// of which enough are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels, 4 taps: 179 us by the kernel
-// above; a channel's SiLU with a branch, sixteen rows, loads after the work on the rows before them 75; now 54.
-constexpr int SV_TOKENS = 32;
-template <typename TI, typename TO, int K>
+// ten warps on an SM: 96 us; eight rows 60, two 58); where the rows of the tile break (another sequence) is found once per warp.  The
+// products, their order and the SiLU's value are those above (a quicker quotient turns some roundings, which a state behind the
+// convolution keeps).  Bound: bytes, of which enough are in flight only with many warps.  Measured on B200, bf16, 8192 rows x 4096 channels,
+// 4 taps: 179 us by the kernel above; a channel's SiLU with a branch, sixteen rows, loads after the work on the rows before them 75;
+// now 54.
+template <typename TI, typename TO, int K, int SV_TOKENS>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const TI* __restrict__ xin, int64_t xin_stride, const float* __restrict__ w,
                                                              const float* __restrict__ bias, const TI* __restrict__ tail,
                                                              const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
@@ -869,10 +869,20 @@ int sllm_short_conv(const void* xin, int64_t xin_stride, sllm_dtype_t in_dtype, 
     // both, 2048 x 2048 31 against 18)
     const bool vec = num_prefill_tokens * channels >= (1 << 20) && (taps == 3 || taps == 4) && channels % 4 == 0 && xin_stride % 4 == 0 &&
                      (((uintptr_t)xin | (uintptr_t)tail | (uintptr_t)out | (uintptr_t)w) & 15) == 0;
-#define SC_VEC(TI, K)                                                                                                          \
-    short_conv_vec_kernel<TI, T, K><<<dim3((unsigned)cdiv(num_prefill_tokens, SV_TOKENS), (unsigned)cdiv(channels, 512)), 128, 0, st>>>( \
+    // rows of a tile: the fewer, the more CTAs and the shorter a thread's chain of loads; the more, the fewer rows are read twice (4 taps,
+    // bf16, us, 8 / 16 / 32 rows: 2^20 entries 8 / 10 / 14, 4 x 2^20 12.5 / 13.4 / 15.7, 6 x 15.9 / 16.5 / 17.7, 8 x 18.7 / 18.4 / 20.5, 24 x
+    // 46 / 44 / 46, 32 x 60 / 58 / 57)
+    const int64_t entries = num_prefill_tokens * channels;
+#define SC_VEC_TILES(TI, K, ROWS)                                                                                              \
+    short_conv_vec_kernel<TI, T, K, ROWS><<<dim3((unsigned)cdiv(num_prefill_tokens, ROWS), (unsigned)cdiv(channels, 512)), 128, 0, st>>>( \
         (const TI*)xin, xin_stride, (const float*)w, (const float*)bias, (const TI*)tail, (const int*)tok_seq, (const int*)tok_pos, \
         (T*)out, num_prefill_tokens, channels, add_input, act_silu)
+#define SC_VEC(TI, K)                                                                                                          \
+    do {                                                                                                                       \
+        if (entries < (7 << 20)) SC_VEC_TILES(TI, K, 8);                                                                       \
+        else if (entries < (28 << 20)) SC_VEC_TILES(TI, K, 16);                                                                \
+        else SC_VEC_TILES(TI, K, 32);                                                                                          \
+    } while (0)
     if (num_prefill_tokens > 0 && vec) {
         if (in_dtype == SLLM_F32) { SLLM_DISPATCH_DTYPE_F32(out_dtype, { if (taps == 3) SC_VEC(float, 3); else SC_VEC(float, 4); }); }
         else { SLLM_DISPATCH_DTYPE_F32(out_dtype, { if (taps == 3) SC_VEC(T, 3); else SC_VEC(T, 4); }); }
@@ -888,6 +898,7 @@ int sllm_short_conv(const void* xin, int64_t xin_stride, sllm_dtype_t in_dtype, 
     }
 #undef SC_LAUNCH
 #undef SC_VEC
+#undef SC_VEC_TILES
     return check_launch("short_conv");
 }
 

@@ -57,3 +57,22 @@ def test_convolution_tiles(taps):
         assert float((y[at:at + n].double() - want).norm() / want.norm()) < 2.0 ** -8, i
         assert torch.equal(tail[row].double(), full[n:])
         at += n
+
+
+@pytest.mark.parametrize("times,taps", [(7, 3), (8, 4), (27, 4), (28, 3), (29, 4)])
+def test_convolution_tile_heights(times, taps):
+    """Tiles of 8, 16 and 32 rows, by the number of entries: on both sides of the lines between them."""
+    from swiftllm_b200.worker.kernels.scan_ops import short_conv
+    lens = (31, 1, 2, 30, 33, 5, 64, 1, 1, 87) * times + (3,)
+    firsts = (0, 3, 1, 0, 2, 0, 9, 1, 0, 4) * times + (0,)
+    C, T, st = 4104, sum(lens), _segments(lens, firsts)
+    x, w, b = _normal(T, C, seed=1, dtype=torch.bfloat16), _normal(C, taps, seed=2), _normal(C, seed=3)
+    tail0 = _normal(len(lens), taps - 1, C, seed=4, dtype=torch.bfloat16)
+    y = short_conv(x, w, b, tail0.clone(), st, torch.bfloat16, silu=True, move_tail=True)
+    at = 0
+    for i, (n, first) in enumerate(zip(lens, firsts)):
+        before = tail0[i].double() * (torch.arange(first - taps + 1, first, device=x.device) >= 0)[:, None]
+        full = torch.cat((before, x[at:at + n].double()))
+        want = torch.nn.functional.silu(sum(full[k:k + n] * w[:, k].double() for k in range(taps)) + b.double())
+        assert float((y[at:at + n].double() - want).norm() / want.norm()) < 2.0 ** -8, i
+        at += n
