@@ -79,6 +79,7 @@ SIGNATURES = {
     "sllm_conv_tail_update": (_I, [_P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _P]),
     "sllm_mingru_scan": (_I, [_P, _L, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P]),
     "sllm_selective_scan": (_I, [_P, _L, _P, _L, _I, _P, _P, _P, _L, _I, _I, _P, _P, _L, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),
+    "sllm_selective_scan_rows": (_I, [_P, _L, _P, _L, _I, _P, _P, _P, _L, _I, _I, _P, _P, _L, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _P]),
     "sllm_embed_pair_hash": (_I, [_P, _P, _P, _P, _P, _P, _I, _L, _L, _F, _P, _P, _P, _L, _I, _I, _P]),
     "sllm_store_last_tokens": (_I, [_P, _P, _P, _P, _I, _P]),
     "sllm_silu_glu": (_I, [_P, _P, _L, _I, _I, _P]),

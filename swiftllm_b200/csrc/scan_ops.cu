@@ -405,13 +405,16 @@ constexpr int SS_BCR = 4;
 // VEC (16-bit rows in 16-byte pieces, states in whole eights): a thread brings eight neighbouring channels of ONE token and eight entries of
 // B or C per tile, with one address each, and stores eight outputs; staging with an address per entry took 85 of 125 instructions per
 // token.  16 states with fp32 step logits have a kernel of their own below.
-template <typename T, typename TD, bool VEC>
+// N16: 16 states on two lanes, known to the compiler (many short portions, and states that are not aligned; with the shape unknown 1.4
+// times as long).
+template <typename T, typename TD, bool VEC, bool N16 = false>
 __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
     const T* __restrict__ x, int64_t x_stride, const TD* __restrict__ dtl, int64_t dt_stride, const float* __restrict__ dt_bias,
     const float* __restrict__ A, const T* __restrict__ bc, int64_t bc_stride, int b_off, int c_off, const float* __restrict__ D,
     const T* __restrict__ z, int64_t z_stride, float* __restrict__ state, const int* __restrict__ seg_starts,
-    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C, int N, int ns_log2, int tt) {
+    const int* __restrict__ seq_ids, const int* __restrict__ tok_pos, T* __restrict__ out, int C, int N_, int ns_log2_, int tt_) {
     extern __shared__ __align__(16) float ssm[];
+    const int N = N16 ? 16 : N_, ns_log2 = N16 ? 1 : ns_log2_, tt = N16 ? 2 * SS_ITEMS : tt_;
     const int NS = 1 << ns_log2, ch_log2 = 7 - ns_log2, CH = 1 << ch_log2, RE = (N + NS - 1) >> ns_log2;
     // whole groups of four states per lane, on 16-byte boundaries of the staged rows: B and C are read four at a time
     const bool vec = (N & 3) == 0 && (RE & 3) == 0;
@@ -562,7 +565,7 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
         const float* bp = bs + s * RE;
         const float* cp = cs + s * RE;
         const bool lane_live = s * RE < N;
-        if (vec && ns_log2 >= 2 && (tt & 3) == 0) {
+        if (N16 || (vec && ns_log2 >= 2 && (tt & 3) == 0)) {
             // four tokens at a time, packed arithmetic; the four sums over the lanes of a channel are taken together, each lane quarter
             // keeping the token (2 (s & 1) + (s >> 1 & 1)) that it writes
             auto four = [&](int j, bool whole) {        // tokens j .. j + 3 (those below nt)
@@ -575,7 +578,7 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                         float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
                         for (int q = 0; q < SS_R / 4; q++) {
-                            if (4 * q < RE && lane_live) {
+                            if (N16 || (4 * q < RE && lane_live)) {
                                 const float4 b4 = reinterpret_cast<const float4*>(bp + (j + u) * N)[q], c4 = reinterpret_cast<const float4*>(cp + (j + u) * N)[q];
                                 float2 s0 = make_float2(S[4 * q], S[4 * q + 1]), s1 = make_float2(S[4 * q + 2], S[4 * q + 3]);
                                 const float2 e0 = make_float2(exp2_neg(dt * a[4 * q]), exp2_neg(dt * a[4 * q + 1]));
@@ -593,12 +596,18 @@ __global__ void __launch_bounds__(128) selective_scan_tiled_kernel(
                 const bool odd = s & 1, high = s & 2;
                 const float k0 = odd ? y[2] : y[0], k1 = odd ? y[3] : y[1];                          // kept pair
                 const float p0 = k0 + __shfl_xor_sync(0xffffffffu, odd ? y[0] : y[2], 1), p1 = k1 + __shfl_xor_sync(0xffffffffu, odd ? y[1] : y[3], 1);
-                float v = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
-                for (int o = NS >> 1; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                const int mine = j + 2 * (s & 1) + ((s >> 1) & 1);
-                if (s < 4 && (whole || mine < nt)) {
-                    const int at = (mine << ch_log2) + cl;
-                    ys[at] = (v + dd * xs[at]) * zs[at];
+                if constexpr (N16) {
+                    const int mine = j + 2 * (s & 1), at = (mine << ch_log2) + cl;
+                    if (whole || mine < nt) ys[at] = (p0 + dd * xs[at]) * zs[at];
+                    if (whole || mine + 1 < nt) ys[at + CH] = (p1 + dd * xs[at + CH]) * zs[at + CH];
+                } else {
+                    float v = (high ? p1 : p0) + __shfl_xor_sync(0xffffffffu, high ? p0 : p1, 2);
+                    for (int o = NS >> 1; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    const int mine = j + 2 * (s & 1) + ((s >> 1) & 1);
+                    if (s < 4 && (whole || mine < nt)) {
+                        const int at = (mine << ch_log2) + cl;
+                        ys[at] = (v + dd * xs[at]) * zs[at];
+                    }
                 }
             };
             if (nt == tt) {
@@ -940,22 +949,31 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
                         const void* A, const void* bc, int64_t bc_stride, int b_off, int c_off, const void* D, const void* z,
                         int64_t z_stride, void* state, const void* seg_starts, const void* seq_ids, const void* tok_pos, void* out,
                         int num_segs, int num_prefill_segs, int channels, int states, sllm_dtype_t dtype, sllm_stream_t stream) {
+    return sllm_selective_scan_rows(x, x_stride, dt, dt_stride, dt_f32, dt_bias, A, bc, bc_stride, b_off, c_off, D, z, z_stride, state, seg_starts,
+                                    seq_ids, tok_pos, out, -1, num_segs, num_prefill_segs, channels, states, dtype, stream);
+}
+
+int sllm_selective_scan_rows(const void* x, int64_t x_stride, const void* dt, int64_t dt_stride, int dt_f32, const void* dt_bias,
+                             const void* A, const void* bc, int64_t bc_stride, int b_off, int c_off, const void* D, const void* z,
+                             int64_t z_stride, void* state, const void* seg_starts, const void* seq_ids, const void* tok_pos, void* out,
+                             int64_t num_tokens, int num_segs, int num_prefill_segs, int channels, int states, sllm_dtype_t dtype,
+                             sllm_stream_t stream) {
     SLLM_REQUIRE(num_prefill_segs >= 0 && num_prefill_segs <= num_segs, "selective_scan: bad number of prompt segments");
     SLLM_REQUIRE(num_segs >= 0 && channels > 0 && states > 0 && states <= 32 * SS_R, "selective_scan: 1 <= states <= %d (got %d)",
                  32 * SS_R, states);
     if (num_segs == 0) return 0;
+    const int64_t num_prefill_tokens = num_tokens - (num_segs - num_prefill_segs);         // (used where num_tokens >= 0)
     SLLM_REQUIRE(x && dt && dt_bias && A && bc && D && z && state && seg_starts && seq_ids && tok_pos && out,
                  "selective_scan: null pointer");
     int ns_plain = 0;                                  // lanes per channel (log2): the fewest that hold all states
     while ((SS_R << ns_plain) < states) ns_plain++;
-    int ns_tiled = ns_plain;
+    int ns_tiled = ns_plain, sms = 0;
     if (num_prefill_segs > 0) {
         // prompt portions walk their tokens one after the other: with few (segment, channel) pairs more lanes per channel (fewer
         // states per thread) put more warps on the SMs, but not below four states a lane where these are read and multiplied together, four
         // tokens at a time, which takes 16 states or more (512 tokens, 16 states, us: 162 with one state a lane, 68 with four; 24: 174 and
         // 167; 32: 193 and 113; 64: 248 and 134), or where one state a lane would be more than eight warps an SM (8 states: 64 to
         // 4096 channels 156 - 170 and 168, f32 152 - 168 and 195; 8192 channels 215 and 168, f32 211 and 195; 4 states 162 and 287)
-        int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
         const int64_t pairs = (int64_t)num_prefill_segs * channels, few = 8 * (int64_t)sms;
         const bool fours = (states & 3) == 0 && (states >= 16 || (states >= 8 && pairs * states / 32 > few));
@@ -976,10 +994,16 @@ int sllm_selective_scan(const void* x, int64_t x_stride, const void* dt, int64_t
         const bool vec = dtype != SLLM_F32 && states % 8 == 0 && channels % 8 == 0 && ns_tiled <= 4 && x_stride % 8 == 0 && z_stride % 8 == 0 &&
                          bc_stride % 8 == 0 && b_off % 8 == 0 && c_off % 8 == 0 && dt_stride % dv == 0 &&
                          (((uintptr_t)x | (uintptr_t)dt | (uintptr_t)z | (uintptr_t)bc | (uintptr_t)out) & 15) == 0;
-#define SS_TILED(TT, TD, VEC) selective_scan_tiled_kernel<TT, TD, VEC><<<SS_GRID(num_prefill_segs, ns_tiled), smem, st>>>(SS_ARGS(TD, 0, ns_tiled), tt)
-        if (vec && dt_f32 && states == 16 && (((uintptr_t)A | (uintptr_t)state) & 15) == 0) {
-            int sms = 0;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
+#define SS_TILED(TT, TD, ...) selective_scan_tiled_kernel<TT, TD, __VA_ARGS__><<<SS_GRID(num_prefill_segs, ns_tiled), smem, st>>>(SS_ARGS(TD, 0, ns_tiled), tt)
+        // Portions that fill one tile of the kernel for 16 states in part leave its stagers idle, and it holds two or three CTAs on an SM where
+        // the tiled one holds eight: many short portions (on the average) stay with that one.  Tiled / own kernel, us: 64 x 8 tokens, 4096
+        // channels 28 / 36, 64 x 16, 8192 channels 76 / 104, 8 x 16, 4096 channels 8.1 / 8.2, 32 x 40 41.0 / 43.1; but 4 x 16 5.2 / 4.8, 8 x 1
+        // 5.8 / 4.7, 32 x 64 61.1 / 60.9.
+        const int64_t pairs = (int64_t)num_prefill_segs * channels, mean = num_prefill_tokens / num_prefill_segs;
+        const bool brief = num_tokens >= 0 && ((mean <= 48 && pairs > 600 * (int64_t)sms) || (mean >= 8 && mean <= 24 && pairs > 140 * (int64_t)sms));
+        const bool n16 = vec && dt_f32 && states == 16, own = n16 && (((uintptr_t)A | (uintptr_t)state) & 15) == 0;
+        if (n16 && ns_tiled == 1 && (brief || !own)) { SLLM_DISPATCH_DTYPE(dtype, (SS_TILED(T, float, true, true))); }
+        else if (own) {
             // one channel per lane while all CTAs are on the SMs at once, three each (us, one / two channels: 2 x 777 tokens, 4096 channels
             // 65 / -, 2 x 777, 8192 channels 124 / 100, 3 x 2048, 4096 channels 217 / 248, 4 x 2048, 4096 channels 315 / 247)
             const bool two = (int64_t)num_prefill_segs * cdiv(channels, 32) > 3 * (int64_t)sms;

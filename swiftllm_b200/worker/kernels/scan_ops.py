@@ -79,9 +79,9 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, A: 
     _lib.require_device(x)
     st = infer_state
     out = torch.empty((T, C), dtype=x.dtype, device=x.device)
-    _lib.check(_lib.lib().sllm_selective_scan(
+    _lib.check(_lib.lib().sllm_selective_scan_rows(
         x.data_ptr(), _stride0(x), dt.data_ptr(), _stride0(dt), 1 if dt.dtype == torch.float32 else 0, dt_bias.data_ptr(), A.data_ptr(),
         bc.data_ptr(), _stride0(bc), b_off, c_off, D.data_ptr(), z.data_ptr(), _stride0(z), state.data_ptr(), st.seg_starts.data_ptr(),
-        st.seq_ids.data_ptr(), st.token_positions.data_ptr(), out.data_ptr(), st.batch_size, _prefill_segs(st), C, N,
+        st.seq_ids.data_ptr(), st.token_positions.data_ptr(), out.data_ptr(), T, st.batch_size, _prefill_segs(st), C, N,
         _lib.dtype_tag_f32(x.dtype), _lib.stream()), "selective_scan")
     return out

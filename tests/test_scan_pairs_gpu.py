@@ -76,3 +76,28 @@ def test_convolution_tile_heights(times, taps):
         want = torch.nn.functional.silu(sum(full[k:k + n] * w[:, k].double() for k in range(taps)) + b.double())
         assert float((y[at:at + n].double() - want).norm() / want.norm()) < 2.0 ** -8, i
         at += n
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("lens,C", [((8, 24, 3, 17, 9), 4808), ((1, 16, 33, 2, 40, 7), 16008), ((28, 24, 24, 24, 25), 4808), ((8, 7, 8, 8, 8), 4808)])
+def test_scan_of_short_portions(dtype, lens, C):
+    """Many short portions (the first two; the others are on the other side of the lines), and a state off the 16-byte grid; outputs are
+    rounded once, states as in the test of longer ones."""
+    from swiftllm_b200.worker.kernels.scan_ops import selective_scan
+    N, firsts, T = 16, [3 * (i % 2) for i in range(len(lens))], sum(lens)
+    st = _segments(lens, firsts)
+    x, z, bc = _normal(T, 2 * C, seed=C, dtype=dtype)[:, :C], _normal(T, C, seed=9, dtype=dtype), _normal(T, 2 * N, seed=8, dtype=dtype)
+    dt, bias = _normal(T, C, seed=1), _normal(C, seed=2) - 3
+    A, D, S0 = -(_normal(C, N, seed=3).abs() + 0.1), _normal(C, seed=4), _normal(len(lens), C, N, seed=5)
+    states = [S0.clone(), torch.zeros(S0.numel() + 1, device=x.device)[1:].view_as(S0).copy_(S0)]
+    outs = [selective_scan(x, dt, bias, A, bc, 0, N, D, z, s, st) for s in states]
+    steps, want, at = torch.nn.functional.softplus(dt.double() + bias.double()), torch.empty(T, C, dtype=torch.float64, device=x.device), 0
+    for i, (n, first) in enumerate(zip(lens, firsts)):
+        S = S0[i].double() if first > 0 else torch.zeros(C, N, dtype=torch.float64, device=x.device)
+        for t in range(at, at + n):
+            S = torch.exp(steps[t, :, None] * A.double()) * S + (steps[t] * x[t].double())[:, None] * bc[t, None, :N].double()
+            want[t] = ((S * bc[t, None, N:].double()).sum(1) + D.double() * x[t].double()) * torch.nn.functional.silu(z[t].double())
+        at += n
+        assert all(float((s[i].double() - S).norm() / S.norm()) < 2e-6 for s in states)
+    for y in outs:
+        assert float((y.double() - want).norm() / want.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
