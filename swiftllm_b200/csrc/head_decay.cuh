@@ -607,7 +607,10 @@ __global__ void __launch_bounds__(256) hd_norm_kernel(const HeadDecayArgs p, int
 
 // The same for dv <= 128 in whole fours: a warp takes HD_UNITS neighbouring (row, head) pairs and asks for all their read-outs and gates at
 // once.  Bound: bytes (fp32 read-outs, gate, output), of which one pair's per warp are too few in flight: 8192 rows x 16 heads x 128
-// columns, bf16, 47 -> 36 us with cold caches.
+// columns, bf16, 47 -> 36 us with cold caches.  Only where there are enough pairs for that: with few of them a warp's four norms, one after
+// the other, are what the launch takes (the delta rule over prompts, this kernel / the one above, us, 16 heads: 128 columns, 64 tokens 12.6 /
+// 11.4, 512 tokens 23.9 / 24.0, 4096 tokens 131 / 136, 8192 tokens 252 / 264; 64 columns, of which half a warp is idle, 64 tokens 11.7 / 9.3,
+// 8192 tokens 189 / 188, 32 heads 235 / 240).
 constexpr int HD_UNITS = 4;
 template <typename T, bool DELTA>
 __global__ void __launch_bounds__(256) hd_norm_narrow_kernel(const HeadDecayArgs p, int64_t units) {
@@ -882,7 +885,7 @@ template <bool DELTA, typename F> static int hd_run(HeadDecayArgs a, sllm_dtype_
         if (slices > 1) {
             const int64_t n = num_prefill_tokens * a.H;
             SLLM_DISPATCH_DTYPE_F32(dtype, {
-                if (a.vec && a.dv <= 128) hd_norm_narrow_kernel<T, DELTA><<<(unsigned)cdiv(n, 8 * HD_UNITS), 256, 0, s>>>(a, n);
+                if (a.vec && a.dv <= 128 && n >= (a.dv > 64 ? 1 << 14 : 1 << 18)) hd_norm_narrow_kernel<T, DELTA><<<(unsigned)cdiv(n, 8 * HD_UNITS), 256, 0, s>>>(a, n);
                 else if (a.vec) hd_norm_kernel<T, DELTA, true><<<(unsigned)cdiv(n, 8), 256, 0, s>>>(a, n);
                 else hd_norm_kernel<T, DELTA, false><<<(unsigned)cdiv(n, 8), 256, 0, s>>>(a, n);
             });
