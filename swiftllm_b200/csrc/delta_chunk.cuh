@@ -671,18 +671,32 @@ template <typename T, int DKP> static int delta_chunk_width(const HeadDecayArgs&
     return delta_chunk_launch<T, DKP, 1>(a, s);
 }
 
-// Rows in 16-byte pieces, at most 128 state rows (more do not fit an owner's registers).
-static inline bool delta_chunk_takes(const HeadDecayArgs& a, sllm_dtype_t dtype) {
-    return dtype != SLLM_F32 && a.dk <= 128 && a.dk % 8 == 0 && a.dv % 8 == 0 && ((a.q_stride | a.k_stride | a.v_stride) & 7) == 0 &&
-           (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.o_raw) & 15) == 0;
+// The narrowest slices of a head that give no SM two CTAs: an SM holds one, and its owners go the faster the fewer they are.
+static inline int delta_chunk_slice(const HeadDecayArgs& a, int num_sms) {
+    int cw = 1;
+    while (cw < 8 && (int64_t)a.num_segs * a.H * cdiv(a.dv, 16 * cw) > num_sms) cw *= 2;
+    return cw;
+}
+
+// Rows in 16-byte pieces, at most 128 state rows (more do not fit an owner's registers), and portions that are not too short on the average:
+// three staged phases and the inverse take 9 us whatever a chunk holds, a batch of eight tokens 2 to 4, and where a batch kernel's CTA owns a
+// head (`owned`) there is no launch for the norm.  Batches / chunks, us, 16 heads: 128 x 128, 1 portion of 8 tokens 7.4 / 10.1, 4 x 8 9.8 / 11.1,
+// 9 x 8 14.0 / 12.7, 1 x 16 10.1 / 10.5, 4 x 12 12.5 / 11.2; 64 x 128, 9 x 8 9.3 / 9.7, 9 x 12 12.0 / 9.7; 64 x 64, 4 x 16 8.9 / 9.4, 4 x 20
+// 10.8 / 9.3, 9 x 24 9.8 / 10.0, 16 x 24 18.2 / 20.4, 16 x 32 22.2 / 20.5; 32 x 32, 1 x 24 8.5 / 8.9, 16 x 32 19.6 / 20.0; 96 x 160, 2 x 8 10.0 / 11.2, 6 x 8
+// 17.8 / 23.9, but 3 x 8, whose chunk kernel has 144 CTAs, 14.7 / 11.5.
+static inline bool delta_chunk_takes(const HeadDecayArgs& a, sllm_dtype_t dtype, int64_t num_tokens, int num_sms) {
+    const int64_t units = (int64_t)a.num_segs * a.H, ctas = units * cdiv(a.dv, 16 * delta_chunk_slice(a, num_sms));
+    const bool owned = a.dv <= 32 || 5 * units >= 3 * (int64_t)num_sms, full = 10 * ctas >= 9 * (int64_t)num_sms && ctas <= num_sms;
+    int shortest = 9;
+    if (a.dv <= 64) shortest = owned ? 25 : 17;
+    else if (a.dv > 128 ? full : owned && a.dk > 64) shortest = 1;
+    return num_tokens >= (int64_t)shortest * a.num_segs && dtype != SLLM_F32 && a.dk <= 128 && a.dk % 8 == 0 && a.dv % 8 == 0 &&
+           ((a.q_stride | a.k_stride | a.v_stride) & 7) == 0 && (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.o_raw) & 15) == 0;
 }
 
 // -> 1: the outputs are finished; 2: the read-outs are in o_raw
 template <typename T> static int delta_chunk(const HeadDecayArgs& a, int num_sms, cudaStream_t s) {
-    // the narrowest slices of a head that give no SM two CTAs: an SM holds one, and its owners go the faster the fewer they are
-    const int64_t units = (int64_t)a.num_segs * a.H;
-    int cw = 1;
-    while (cw < 8 && (units * cdiv(a.dv, 16 * cw) > num_sms)) cw *= 2;
+    const int cw = delta_chunk_slice(a, num_sms);
     return a.dk <= 64 ? delta_chunk_width<T, 64>(a, cw, s) : delta_chunk_width<T, 128>(a, cw, s);
 }
 

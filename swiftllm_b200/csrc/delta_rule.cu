@@ -20,8 +20,8 @@ extern "C" int sllm_delta_rule(const void* q, int64_t q_stride, const void* k, i
     a.o_raw = (float*)workspace; a.out = out; a.out_stride = out_stride;
     a.num_segs = num_segs; a.H = num_heads; a.G = num_kv_heads; a.dk = dk; a.dv = dv;
     return hd_run<true>(a, dtype, num_tokens, num_prefill_tokens, num_prefill_segs, workspace_floats, (cudaStream_t)stream,
-                        [&](const HeadDecayArgs& x, int num_sms, cudaStream_t s) {
-                            if (!delta_chunk_takes(x, dtype)) return 0;
+                        [&](const HeadDecayArgs& x, int64_t num_prompt_tokens, int num_sms, cudaStream_t s) {
+                            if (!delta_chunk_takes(x, dtype, num_prompt_tokens, num_sms)) return 0;
                             return dtype == SLLM_F16 ? delta_chunk<__half>(x, num_sms, s) : delta_chunk<__nv_bfloat16>(x, num_sms, s);
                         });
 }

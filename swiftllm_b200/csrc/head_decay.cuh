@@ -847,8 +847,8 @@ template <typename T, bool DELTA> static void hd_decode(const HeadDecayArgs& a, 
     }
 }
 
-// chunked(args, num_sms, stream): launches another kernel for the prompt portions and returns its CTAs per head, or 0 where it does not take
-// them
+// chunked(args, prompt tokens, num_sms, stream): launches another kernel for the prompt portions and returns its CTAs per head, or 0 where it
+// does not take them
 template <bool DELTA, typename F> static int hd_run(HeadDecayArgs a, sllm_dtype_t dtype, int64_t num_tokens, int64_t num_prefill_tokens,
                                                     int num_prefill_segs, int64_t workspace_floats, cudaStream_t s, F chunked) {
     const int total_segs = a.num_segs;
@@ -879,7 +879,7 @@ template <bool DELTA, typename F> static int hd_run(HeadDecayArgs a, sllm_dtype_
         int want = 1;
         if (a.dv > 64 && 5 * units * cdiv(a.dv, 128) >= 3 * num_sms) want = 4;
         else if (a.dv > 32 && 5 * units * cdiv(a.dv, 64) >= 3 * num_sms) want = 2;
-        int slices = chunked(a, num_sms, s);
+        int slices = chunked(a, num_prefill_tokens, num_sms, s);
         if (slices == 0) SLLM_DISPATCH_DTYPE_F32(dtype, (slices = hd_prompt<T, DELTA>(a, want, s)));
         if (check_launch("head decay (prompt portions)")) return 1;
         if (slices > 1) {

@@ -21,5 +21,5 @@ extern "C" int sllm_matrix_memory(const void* q, int64_t q_stride, const void* k
     a.seg_starts = (const int*)seg_starts; a.seq_ids = (const int*)seq_ids; a.tok_pos = (const int*)tok_pos;
     a.o_raw = (float*)workspace; a.out = out; a.out_stride = out_stride;
     a.num_segs = num_segs; a.H = num_heads; a.G = num_heads; a.dk = dk; a.dv = dv;
-    return hd_run<false>(a, dtype, num_tokens, num_prefill_tokens, num_prefill_segs, workspace_floats, (cudaStream_t)stream, [](const HeadDecayArgs&, int, cudaStream_t) { return 0; });
+    return hd_run<false>(a, dtype, num_tokens, num_prefill_tokens, num_prefill_segs, workspace_floats, (cudaStream_t)stream, [](const HeadDecayArgs&, int64_t, int, cudaStream_t) { return 0; });
 }

@@ -106,3 +106,15 @@ def test_values_that_are_not_finite_reach_what_follows(what, value):
             keep = [e for e in range(dv) if e != 5]
             assert _off(state[1][head][:, keep], clean_state[1][head][:, keep].double()) < 32 * 2.0 ** -24
             assert not state[1][head][:, 5].isfinite().any()
+
+
+@pytest.mark.parametrize("lens,H,G,dk,dv", [
+    ([8], 4, 4, 128, 128), ([9], 4, 4, 128, 128), ([1, 8, 15], 6, 3, 128, 128), ([9, 9], 48, 24, 128, 128), ([8, 8], 48, 24, 128, 128),
+    ([8] * 6, 20, 10, 64, 128), ([17, 16], 4, 2, 64, 64), ([16] * 3, 4, 2, 64, 64), ([24] * 5, 20, 10, 64, 64), ([25] * 5, 20, 10, 64, 64),
+    ([24], 4, 4, 32, 32), ([25], 4, 4, 32, 32), ([8] * 3, 16, 8, 96, 160), ([8] * 4, 16, 8, 96, 160)])
+def test_short_portions(lens, H, G, dk, dv):
+    """Both sides of the lines between batches of eight tokens and chunks."""
+    x, st = _case(torch.bfloat16, lens, H, G, dk, dv, seed=sum(lens) + dv)
+    out, state = _run(x, st, H, G, dk, dv)
+    ref, states = _exact(x, lens, H, G, dk, dv)
+    assert _off(out, ref) < 2.0 ** -9 and all(_off(state[r], S) < 32 * 2.0 ** -24 for r, S in states.items())
