@@ -6,7 +6,7 @@
 // mma.m16n8k16 (64 registers at dk = 128), and accumulators are the left operands of the next product as they lie: S^T against the
 // chunk's keys and queries, rhs^T against (I + A)^-1 - I, u^T against the score matrix and, weighted, against the keys.  Owners
 // exchange nothing.  Two more warpgroups work ahead of them, chunk by chunk: STAGERS bring keys and queries (as fp16, each row times a
-// power of two that brings its norm near 2^8, which keeps every bit of theirs down to 2^-25 of that norm) and make the chunk's two
+// power of two that brings its norm near 2^14, which keeps every bit of theirs down to 2^-28 of that norm) and make the chunk's two
 // 32 x 32 matrices (exact products of 16-bit numbers, decays in fp32); MAKERS turn logits into decays, invert I + A in fp32 and finish the
 // last chunk's outputs.
 //
@@ -14,12 +14,15 @@
 // cycles each, and at 64 chains (4 sequences x 16 heads) only 64 SMs busy.  Here a chain is spread over four to eight warps that never wait for
 // one another's numbers.  Bound: the owner's chain of dependent products (4900 of 5500 cycles per chunk; its 228 products take 1824 on the
 // tensor cores), with three warps per scheduler at 0.5 instructions per cycle; code beyond what fits the instruction caches costs more
-// than it saves, so loops are kept short (all unrolled: 385 us).  Measured on B200, bf16, 4 x 2048 tokens, 16 heads, 128 x 128: 717 -> 248 us
+// than it saves, so loops are kept short (all unrolled: 385 us).  Measured on B200, bf16, 4 x 2048 tokens, 16 heads, 128 x 128: 717 -> 255 us
 // with the head norm's 25.
 //
-// Precision: S, rhs, u and both matrices are fp32 numbers; as operands they are two fp16 numbers each (22 bits and a sign, against the
-// column's largest entry, which is brought to 2^13 by a power of two), products are summed in fp32, and the chunk's own sums are made
-// from zero and added to the decayed state once.  The state's distance to 64 bits after 2048 tokens: 1.20e-7 (token by token in fp32: 1.22e-7).
+// Precision: S, rhs, u and both matrices are fp32 numbers; as operands they are two fp16 numbers each (22 bits and a sign), the second
+// one times 2^11 and with sums of its own, so that it has fp16's whole range too: with a column's largest entry at 2^13 (by a power of
+// two) an entry keeps its 22 bits down to 2^-27 of that one, and nothing is lost above 2^-49 of it.  The product of two second parts (2^-24 of
+// theirs) is left out.  Products are summed in fp32, and the chunk's own sums are made from zero and added to the decayed state once.  The
+// state's distance to 64 bits after 2048 tokens: 1.20e-7 (token by token in fp32: 1.22e-7); that of state rows 2^20 below the others of their
+// columns, written and read by nearly one-hot keys, at most 3.7e-7 of the row (4.1e-7; 1.4e-5 with one sum for both parts, which is 3 % faster, and 7e-3 for rows 2^30 below).
 // Every factor is a product of decays <= 1, summed as logarithms over its own range: nothing overflows, whatever the decays.
 // A column in which something is not finite, although its state was, goes through the rule token by token in fp32, so that rows before
 // the one that brought it stay as they are.
@@ -38,6 +41,7 @@ constexpr int dc_owner_warps(int cw) { return cw == 8 ? 8 : 4; }               /
 constexpr int dc_threads(int cw) { return dc_owner_warps(cw) * 32 + 2 * DC_GROUP; }
 constexpr int DC_PITCH = 40;                 // entries between rows of the 32 x 32 matrices (no bank conflicts)
 constexpr float DC_UP = 16384.f;             // entries of both matrices (at most 1) are kept times 2^14
+constexpr float DC_LOW = 2048.f;             // low parts are kept times 2^11: as large as the high ones, they lose nothing below them
 
 // one chunk's staged data
 template <int DKP, int COLS> struct alignas(16) DcBuf {
@@ -81,11 +85,11 @@ __device__ __forceinline__ void dc_scale(float top, float& up, float& down) {
     down = dc_pow2(254 - b);
 }
 __device__ __forceinline__ uint32_t dc_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-// x, y (times up: below 2^14) as two fp16 numbers each
+// x, y (times up: below 2^14) as two fp16 numbers each, the second times DC_LOW
 __device__ __forceinline__ void dc_split(float2 x, float2 up, uint32_t& hi, uint32_t& lo) {
     const float2 s = tc::mul2(x, up);
     const __half2 h = __floats2half2_rn(s.x, s.y);
-    const float2 f = __half22float2(h), l = tc::add2(s, make_float2(-f.x, -f.y));
+    const float2 f = __half22float2(h), l = tc::mul2(tc::add2(s, make_float2(-f.x, -f.y)), make_float2(DC_LOW, DC_LOW));
     hi = dc_bits(h);
     lo = dc_bits(__floats2half2_rn(l.x, l.y));
 }
@@ -200,7 +204,7 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
                     const float y = j > lane ? x[e] * DC_UP : 0.f;
                     const __half hi = __float2half_rn(y);
                     B.n_hi[j * DC_PITCH + lane] = hi;
-                    B.n_lo[j * DC_PITCH + lane] = __float2half_rn(y - __half2float(hi));
+                    B.n_lo[j * DC_PITCH + lane] = __float2half_rn((y - __half2float(hi)) * DC_LOW);
                 }
             }
         };
@@ -344,8 +348,8 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
                 float ss = s2.x + s2.y;
                 ss += __shfl_xor_sync(0xffffffffu, ss, 1);
                 ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-                const int e = (int)((__float_as_uint(ss) >> 23) & 255u);         // a norm of 2^((e - 127) / 2) -> near 2^8
-                const int up = e == 255 ? 1 : min(max(127 + 8 - ((e - 127) >> 1), 1), 253);
+                const int e = (int)((__float_as_uint(ss) >> 23) & 255u);         // a norm of 2^((e - 127) / 2) -> near 2^14
+                const int up = e == 255 ? 1 : min(max(127 + 14 - ((e - 127) >> 1), 1), 253);
                 const float f = dc_pow2(up);
 #pragma unroll
                 for (int i = 0; i < KP; i++) {
@@ -453,7 +457,7 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
         float up[2], down[2];
         dc_scale(top[0], up[0], down[0]); dc_scale(top[1], up[1], down[1]);
         // ---- the state against keys (R) and queries (Z)
-        float R[4][4], Rl[4][4], Z[4][4];
+        float R[4][4], Rl[4][4], Z[4][4], Zl[4][4];
 #pragma unroll
         for (int ks = 0; ks < KS; ks++) {
             uint32_t hi[4], lo[4], kb[8], qb[8];
@@ -466,20 +470,26 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
 #pragma unroll
                 for (int i = 0; i < 4; i++) dc_mma0(Rl[i], lo, kb + 2 * i);
 #pragma unroll
-                for (int i = 0; i < 4; i++) dc_mma0(Z[i], lo, qb + 2 * i);
+                for (int i = 0; i < 4; i++) dc_mma0(Zl[i], lo, qb + 2 * i);
 #pragma unroll
                 for (int i = 0; i < 4; i++) dc_mma0(R[i], hi, kb + 2 * i);
+#pragma unroll
+                for (int i = 0; i < 4; i++) dc_mma0(Z[i], hi, qb + 2 * i);
             } else {
 #pragma unroll
                 for (int i = 0; i < 4; i++) dc_mma(Rl[i], lo, kb + 2 * i);
 #pragma unroll
-                for (int i = 0; i < 4; i++) dc_mma(Z[i], lo, qb + 2 * i);
+                for (int i = 0; i < 4; i++) dc_mma(Zl[i], lo, qb + 2 * i);
 #pragma unroll
                 for (int i = 0; i < 4; i++) dc_mma(R[i], hi, kb + 2 * i);
-            }
 #pragma unroll
-            for (int i = 0; i < 4; i++) dc_mma(Z[i], hi, qb + 2 * i);
+                for (int i = 0; i < 4; i++) dc_mma(Z[i], hi, qb + 2 * i);
+            }
         }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) Z[i][e] = fmaf(Zl[i][e], 1.f / DC_LOW, Z[i][e]);
         // ---- rhs = beta (v - D(j) S^T k), in R
         float xt[2] = {0.f, 0.f};
         {
@@ -493,7 +503,7 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
                     const uint32_t w = vb[2 * i + r];
-                    const float x = (R[i][2 * r] + Rl[i][2 * r]) * down[r], y = (R[i][2 * r + 1] + Rl[i][2 * r + 1]) * down[r];
+                    const float x = fmaf(Rl[i][2 * r], 1.f / DC_LOW, R[i][2 * r]) * down[r], y = fmaf(Rl[i][2 * r + 1], 1.f / DC_LOW, R[i][2 * r + 1]) * down[r];
                     R[i][2 * r] = fmaf(-bd.x, x, bt.x * dc_lo<T>(w));
                     R[i][2 * r + 1] = fmaf(-bd.y, y, bt.y * dc_hi<T>(w));
                     xt[r] = dc_top(xt[r], R[i][2 * r], R[i][2 * r + 1]);
@@ -506,7 +516,7 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
         for (int pass = 0; pass < 2; pass++) {
             xt[0] = dc_top4(xt[0]); xt[1] = dc_top4(xt[1]);
             odd = odd || (sound[0] && !dc_finite(xt[0])) || (sound[1] && !dc_finite(xt[1]));
-            float u2[2], dn[2], E[4][4];
+            float u2[2], dn[2], E[4][4], El[4][4];
             dc_scale(xt[0], u2[0], dn[0]); dc_scale(xt[1], u2[1], dn[1]);
             dn[0] *= 1.f / DC_UP; dn[1] *= 1.f / DC_UP;
             const uint32_t mh = smem_u32(pass ? B.p_hi : B.n_hi) + (r16 * DC_PITCH + 8 * ch2) * 2;
@@ -518,20 +528,24 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
             ldmatrix_x4(mh + LO + DOWN, l1[0], l1[1], l1[2], l1[3]);
             dc_operand(R[0], R[1], u2, hi, lo);
 #pragma unroll
-            for (int i = 0; i < 2; i++) { dc_mma0(E[i], hi, l0 + 2 * i); dc_mma0(E[2 + i], hi, l1 + 2 * i); }
+            for (int i = 0; i < 2; i++) { dc_mma0(El[i], hi, l0 + 2 * i); dc_mma0(El[2 + i], hi, l1 + 2 * i); }
 #pragma unroll
-            for (int i = 0; i < 2; i++) { dc_mma(E[i], lo, b0 + 2 * i); dc_mma(E[2 + i], lo, b1 + 2 * i); }
+            for (int i = 0; i < 2; i++) { dc_mma(El[i], lo, b0 + 2 * i); dc_mma(El[2 + i], lo, b1 + 2 * i); }
 #pragma unroll
-            for (int i = 0; i < 2; i++) { dc_mma(E[i], hi, b0 + 2 * i); dc_mma(E[2 + i], hi, b1 + 2 * i); }
+            for (int i = 0; i < 2; i++) { dc_mma0(E[i], hi, b0 + 2 * i); dc_mma0(E[2 + i], hi, b1 + 2 * i); }
             ldmatrix_x4(mh + DOWN + RIGHT, b1[0], b1[1], b1[2], b1[3]);
             ldmatrix_x4(mh + LO + DOWN + RIGHT, l1[0], l1[1], l1[2], l1[3]);
             dc_operand(R[2], R[3], u2, hi, lo);
 #pragma unroll
-            for (int i = 0; i < 2; i++) dc_mma(E[2 + i], hi, l1 + 2 * i);
+            for (int i = 0; i < 2; i++) dc_mma(El[2 + i], hi, l1 + 2 * i);
 #pragma unroll
-            for (int i = 0; i < 2; i++) dc_mma(E[2 + i], lo, b1 + 2 * i);
+            for (int i = 0; i < 2; i++) dc_mma(El[2 + i], lo, b1 + 2 * i);
 #pragma unroll
             for (int i = 0; i < 2; i++) dc_mma(E[2 + i], hi, b1 + 2 * i);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) E[i][e] = fmaf(El[i][e], 1.f / DC_LOW, E[i][e]);
             if (pass == 0) {
 #pragma unroll
                 for (int i = 0; i < 4; i++)
@@ -617,7 +631,7 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
         constexpr int TILES = 4;                                                  // tiles of eight keys at a time
 #pragma unroll
         for (int i1 = 0; i1 < DKP / 8; i1 += TILES) {
-            float acc[TILES][4];
+            float acc[TILES][4], low[TILES][4];
             uint32_t kb[2][2 * TILES];
 #pragma unroll
             for (int ks = 0; ks < 2; ks++)
@@ -625,11 +639,11 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
                 for (int i = 0; i < TILES; i += 2)                               // rows (tokens) 16 ks .. + 15, pieces i1 + i and i1 + i + 1
                     ldmatrix_x4_trans(kt + tile_off<DKP>(16 * ks + (lane & 15), i1 + i + (lane >> 4)), kb[ks][2 * i], kb[ks][2 * i + 1], kb[ks][2 * i + 2], kb[ks][2 * i + 3]);
 #pragma unroll
-            for (int i = 0; i < TILES; i++) dc_mma0(acc[i], wl[0], kb[0] + 2 * i);
+            for (int i = 0; i < TILES; i++) dc_mma0(low[i], wl[0], kb[0] + 2 * i);
 #pragma unroll
-            for (int i = 0; i < TILES; i++) dc_mma(acc[i], wl[1], kb[1] + 2 * i);
+            for (int i = 0; i < TILES; i++) dc_mma0(acc[i], wh[0], kb[0] + 2 * i);
 #pragma unroll
-            for (int i = 0; i < TILES; i++) dc_mma(acc[i], wh[0], kb[0] + 2 * i);
+            for (int i = 0; i < TILES; i++) dc_mma(low[i], wl[1], kb[1] + 2 * i);
 #pragma unroll
             for (int i = 0; i < TILES; i++) dc_mma(acc[i], wh[1], kb[1] + 2 * i);
 #pragma unroll
@@ -637,7 +651,8 @@ __global__ void __launch_bounds__(dc_threads(CW), 1) delta_chunk_kernel(const He
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
                     float* x = &S[i1 + i][2 * r];
-                    const float2 y = tc::fma2(make_float2(acc[i][2 * r], acc[i][2 * r + 1]), make_float2(wd[r], wd[r]), tc::mul2(make_float2(x[0], x[1]), keep));
+                    const float2 a = tc::fma2(make_float2(low[i][2 * r], low[i][2 * r + 1]), make_float2(1.f / DC_LOW, 1.f / DC_LOW), make_float2(acc[i][2 * r], acc[i][2 * r + 1]));
+                    const float2 y = tc::fma2(a, make_float2(wd[r], wd[r]), tc::mul2(make_float2(x[0], x[1]), keep));
                     x[0] = y.x; x[1] = y.y;
                     top[r] = dc_top(top[r], y.x, y.y);
                 }

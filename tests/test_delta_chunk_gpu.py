@@ -118,3 +118,31 @@ def test_short_portions(lens, H, G, dk, dv):
     out, state = _run(x, st, H, G, dk, dv)
     ref, states = _exact(x, lens, H, G, dk, dv)
     assert _off(out, ref) < 2.0 ** -9 and all(_off(state[r], S) < 32 * 2.0 ** -24 for r, S in states.items())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("noise,lens,H,dv", [(0.0, [40, 33], 2, 128), (0.0, [257], 12, 128), (1e-3, [64, 97], 2, 128), (0.0, [70], 6, 160), (0.0, [50, 64], 3, 64)])
+def test_rows_of_very_different_sizes(dtype, noise, lens, H, dv):
+    """Every other row of the state is 2^20 below the rest of its columns, and so are the values that (nearly) one-hot keys write into it,
+    among the others in the same chunks.  A row's entries are sums of as many fp32 numbers as tokens touch it (a dozen at most, and the
+    decays' product): 2^-20 of the row is sixteen units in the last place of such a number, where operands cut at 2^-38 of their column
+    would leave 2^-18 and more.  With noise the small rows also
+    hold the products of all keys with the large ones: twice that."""
+    dk, T = 128, sum(lens)
+    x, st = _case(dtype, lens, H, H, dk, dv, seed=T + dv)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    at = torch.randint(0, dk, (T,), generator=g, device=DEV)
+    small = torch.where(torch.arange(dk, device=DEV) % 2 == 0, 1.0, 2.0 ** -20)
+    least = small if dtype == torch.bfloat16 else small.clamp_min(2.0 ** -10)               # what fp16 values can be
+    hot = torch.nn.functional.one_hot(at, dk).float() + noise * torch.randn(T, dk, generator=g, device=DEV)
+    x["k"] = hot.repeat(1, H).to(dtype)
+    x["q"] = torch.nn.functional.one_hot(torch.randint(0, dk // 2, (T,), generator=g, device=DEV) * 2 + 1, dk).float().repeat(1, H).to(dtype)
+    x["v"] = (x["v"].float() * least[at][:, None]).to(dtype)
+    x["state"] = x["state"] * small[:, None]
+    x["rate"] = torch.full((H,), 0.01, device=DEV)                               # rows stay within 2^-27 of their columns
+    out, state = _run(x, st, H, H, dk, dv)
+    ref, states = _exact(x, lens, H, H, dk, dv)
+    assert _off(out, ref) < (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
+    for r, S in states.items():
+        row = (state[r].double() - S).norm(dim=-1) / S.norm(dim=-1).clamp_min(1e-30)
+        assert float(row.max()) < 2.0 ** (-19 if noise else -20)
