@@ -101,3 +101,27 @@ def test_scan_of_short_portions(dtype, lens, C):
         assert all(float((s[i].double() - S).norm() / S.norm()) < 2e-6 for s in states)
     for y in outs:
         assert float((y.double() - want).norm() / want.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+
+
+@pytest.mark.parametrize("n", [1, 16, 33])
+def test_steps_are_as_exact_as_the_plain_functions(n):
+    """One input of 1 through B = 1 and no decay leaves the step in the state: no further off 64 bits, in the mean square, than log1p(exp(z))
+    of the tensor library's fp32 functions, in both kernels of 16 states; logits of any size."""
+    from swiftllm_b200.worker.kernels.scan_ops import selective_scan
+    C, N, st = 1 << 16, 16, _segments((n,), (0,))
+    z = torch.rand(C, generator=torch.Generator(device="cuda").manual_seed(n), device="cuda") * 24 - 12
+    ends = torch.tensor([-104.0, float("-inf"), -87.0, -30.0, 20.5, 88.0, 1e30, 0.0, -0.0], device="cuda")
+    logits = torch.full((n, C), float("-inf"), device="cuda")            # steps of 0 but for the first token
+    logits[0] = z
+    logits[0, :9] = ends
+    one = torch.ones(n, C, dtype=torch.bfloat16, device="cuda")
+    state = torch.zeros(1, C, N, device="cuda")
+    selective_scan(one, logits, torch.zeros(C, device="cuda"), torch.zeros(C, N, device="cuda"), one[:, :2 * N], 0, N,
+                   torch.zeros(C, device="cuda"), one, state, st)
+    want = torch.nn.functional.softplus(logits[0].double(), threshold=1e9)
+    assert torch.equal(state[0], state[0, :, :1].expand(C, N))
+    off = lambda y: float(((y.double() - want) / want)[9:].square().mean().sqrt())
+    assert off(state[0, :, 0]) <= off(torch.log1p(torch.exp(logits[0])))
+    got = state[0, :9, 0].double()
+    assert float(got[0]) < 1e-44 and float(got[1]) == 0.0
+    assert bool(((got - want[:9]).abs() <= 2.0 ** -20 * want[:9])[2:].all())
