@@ -92,9 +92,10 @@ static inline bool first_use_on_this_device(unsigned long long& mask) {
 
 // ---------------------------------------------------------------- launches that begin early
 // A kernel launched by launch_early may begin while the kernel before it in the stream still runs, once every CTA of that one has called
-// launch_next (or has ended): its launch and its CTAs' set-up hide behind the other's last CTAs.  It calls wait_previous before it touches
-// what earlier kernels read or write, which waits until all of them have ended and their writes are seen, and launch_next after that,
-// so that a kernel behind it that shares nothing with it need not wait for anything but the launch's own end.
+// launch_next (or has ended): its launch and its CTAs' set-up hide behind the other's last CTAs.  Every CTA of it calls wait_previous before
+// it touches anything in memory, which waits until all earlier kernels have ended and their writes are seen, and launch_next after that, or
+// not at all (the end of its CTAs stands for it): what begins behind it waits in its turn.  It uses no non-coherent loads, which ask that
+// nobody writes the memory for as long as the kernel lives.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A pointer as it is after wait_previous: what is read through a const __restrict__ argument the compiler takes for constant, and could read

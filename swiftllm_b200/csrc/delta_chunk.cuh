@@ -22,7 +22,8 @@
 // two) an entry keeps its 22 bits down to 2^-27 of that one, and nothing is lost above 2^-49 of it.  The product of two second parts (2^-24 of
 // theirs) is left out.  Products are summed in fp32, and the chunk's own sums are made from zero and added to the decayed state once.  The
 // state's distance to 64 bits after 2048 tokens: 1.20e-7 (token by token in fp32: 1.22e-7); that of state rows 2^20 below the others of their
-// columns, written and read by nearly one-hot keys, at most 3.7e-7 of the row (4.1e-7; 1.4e-5 with one sum for both parts, which is 3 % faster, and 7e-3 for rows 2^30 below).
+// columns, written and read by nearly one-hot keys, at most 3.7e-7 of the row (4.1e-7; with one sum for both parts, which is 3 % faster, 1.4e-5,
+// and 7e-3 for rows 2^30 below).
 // Every factor is a product of decays <= 1, summed as logarithms over its own range: nothing overflows, whatever the decays.
 // A column in which something is not finite, although its state was, goes through the rule token by token in fp32, so that rows before
 // the one that brought it stay as they are.

@@ -18,9 +18,9 @@
 // softmax uses all 128 threads; the GQA group is the N dimension (padded to 16 by reading neighbouring heads whose
 // columns are simply never read back).
 // CLUSTERS: in launches of two to eight splits whose items fill at most three quarters of the SMs (meets_in_cluster, paged_attn.cu) the splits
-// of a (sequence, kv head) are a cluster, and their parts meet through distributed shared memory: every CTA leaves its part in its own (in the K ring, which nobody needs any more), and
-// merges a share of the heads.  No workspace, no second launch: one sequence of 700 tokens, 32 / 8 heads, 13.6 -> 9 us on the device.
-// Larger launches keep the merge kernel, which costs them nothing beside their tiles.
+// of a (sequence, kv head) are a cluster, and their parts meet through distributed shared memory: every CTA leaves its part in its own (in
+// the K ring, which nobody needs any more), and merges a share of the heads.  No workspace, no second launch: one sequence of 700 tokens,
+// 32 / 8 heads, 13.6 -> 9 us on the device.  Larger launches keep the merge kernel, which costs them nothing beside their tiles.
 // HBM roofline: algorithmic bytes = sum_i len_i * nkv * 128 * 2 * sizeof(T) + 2 * Bd * nq * 128 * sizeof(T).
 #include <limits.h>
 

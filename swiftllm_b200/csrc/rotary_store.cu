@@ -17,7 +17,8 @@ __global__ void __launch_bounds__(256) rotary_store_decode_kernel(
     int64_t q_stride, int64_t k_stride, int64_t v_stride, int cur_layer, int num_layers, int bs, int max_blocks_per_seq) {
     wait_previous();
     launch_next();
-    q = after_wait(q); k = after_wait(k); v = after_wait(v); cosb = after_wait(cosb); sinb = after_wait(sinb); block_table = after_wait(block_table); seq_ids = after_wait(seq_ids); seq_lens = after_wait(seq_lens);
+    q = after_wait(q); k = after_wait(k); v = after_wait(v); cosb = after_wait(cosb); sinb = after_wait(sinb);
+    block_table = after_wait(block_table); seq_ids = after_wait(seq_ids); seq_lens = after_wait(seq_lens);
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int chunks = head_dim >> 4;             // 8-wide chunks in half a head
@@ -92,7 +93,6 @@ extern "C" int sllm_rotary_store_kvcache_decode(void* q, void* k, const void* v,
     const int threads = 256;
     const unsigned blocks = (unsigned)((total + threads - 1) / threads);
     SLLM_DISPATCH_DTYPE(dtype, (launch_early(rotary_store_decode_kernel<T>, blocks, threads, 0, (cudaStream_t)stream,
-        
                                    (T*)q, (T*)k, (const T*)v, (const T*)cosb, (const T*)sinb, (T*)k_cache, (T*)v_cache, block_table,
                                    seq_ids, decoding_seq_lens, total, num_q_heads, num_kv_heads, head_dim, q_row_stride,
                                    k_row_stride, v_row_stride, cur_layer, num_layers, block_size, max_blocks_per_seq)));

@@ -18,8 +18,9 @@
 // see, the segment is done over, token by token, with the keys that the token does not see left zero: a result depends on its own keys only.
 //
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
-// ones 312 us with the mma.sync kernel of window_attn.cu for the prompts -> 118 us (the decoded rows alone 32; two rounds of CTAs here; a CTA's
-// step of 80 keys is about 2200 cycles, its queries and first keys 12 k, its output 5 k).
+// ones 312 us with the mma.sync kernel of window_attn.cu for the prompts -> 118 us, 92 with the decoded rows beside the prompts' last CTAs
+// (the prompts alone 87, the decoded rows 31; two rounds of CTAs here; a CTA's step of 80 keys is about 2200 cycles, its queries and first
+// keys 12 k, its output 5 k).
 //
 // EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores;
 // FULL: heads of 128 + 128 entries without turned ones beside shared keys (the producers are bound by their instructions).
