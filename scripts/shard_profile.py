@@ -28,6 +28,7 @@ def main():
     ap.add_argument("--model", default="llama3-8b", choices=["llama3-8b", "llama3-70b"])
     ap.add_argument("--fuse-rotary-store", action="store_true")
     ap.add_argument("--tag", default="")
+    ap.add_argument("--out", default=".", help="folder of the launch list")
     args = ap.parse_args()
     import torch.distributed as dist
     import swiftllm_b200
@@ -82,8 +83,8 @@ def main():
     rows = {ev.key: [ev.count, float(ev.device_time_total)] for ev in prof.key_averages()
             if ev.device_type == DeviceType.CUDA and ev.device_time_total > 0}
     tot = sum(r[1] for r in rows.values())
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    path = os.path.join(ROOT, "gpurun_out", f"shard_launches_tp{args.tp}_b{B}_s{S}{args.tag}.csv")
+    os.makedirs(args.out, exist_ok=True)
+    path = os.path.join(args.out, f"shard_launches_tp{args.tp}_b{B}_s{S}{args.tag}.csv")
     with open(path, "w") as f:
         f.write("kernel,launches_per_step,us_per_step,us_per_launch,share\n")
         for k, (c, us) in sorted(rows.items(), key=lambda kv: -kv[1][1]):

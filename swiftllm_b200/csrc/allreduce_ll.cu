@@ -1,5 +1,5 @@
 // Tensor-parallel exchange, low-latency variant: reduce-scatter + residual add + RMSNorm + all-gather in
-// ONE kernel with NO barrier.  Measured on B200/NVSwitch (profiles/r2_p2p_latency_n2.log): a flag round trip costs 5.5 us,
+// ONE kernel with NO barrier.  Measured on B200/NVSwitch: a flag round trip costs 5.5 us,
 // i.e. every "publish a flag, wait for everybody's flag" barrier costs ~3 us one way, and the flag-based two-shot kernel
 // (allreduce_norm.cu) pays two of them plus a peer-load round trip plus a system fence: ~28 us per exchange for 2 MiB.
 // Here data is PUSHED and carries its own validity (the NCCL "LL" idea): every 8-byte unit that crosses NVLink is

@@ -1,7 +1,7 @@
 // Blackwell (sm_100a) primitives used by the tcgen05/TMA kernels: mbarrier, TMA tensor loads, UMMA shared-memory
 // and instruction descriptors, tcgen05.mma / commit / ld, TMEM allocation.  Inline PTX only.
 // Descriptor bit layouts follow the PTX ISA "tcgen05 matrix descriptors" (cross-checked against the field
-// definitions in CUTLASS cute/arch/mma_sm100_desc.hpp) and were validated on hardware with probes/umma_probe.cu.
+// definitions in CUTLASS cute/arch/mma_sm100_desc.hpp) and were validated on hardware.
 #pragma once
 #include <cuda.h>
 

@@ -174,7 +174,7 @@ def test_tp_world8_matches_single_gpu():
 
     History: the first version of this test ran all eleven modes (22 tensor-parallel models, ~80 symmetric-memory buffers with
     multicast bindings) in one process group and did not finish within 400 s on an 8-GPU box, while every mode takes
-    2-4 s at world 4 (profiles/r2_pytest_tp_n4*.log) and the 8-GPU sweeps of the same kernels ran cleanly
+    2-4 s at world 4 and the 8-GPU sweeps of the same kernels ran cleanly
     (profiles/r2_tp_sweep_n8_b256.jsonl) - which mode stalled is unknown (no per-mode progress lines then; they exist now)."""
     if torch.cuda.device_count() < 8:
         pytest.skip("needs 8 GPUs")
