@@ -1080,7 +1080,7 @@ def run_ours(args):
                 "h2d_bytes_per_step": 3 * B * 4, "d2h_bytes_per_step": B * 8},
         "gpu_launches": launches_per_step * args.steps,
         "gpu_launches_note": f"{launches_per_step} native (libswiftllm_b200.so) launch calls per decode step "
-                             f"({'replayed from a CUDA graph' if graph is not None else 'eager'}); GEMMs/embedding/argmax are library calls on top",
+                             f"({'replayed from a CUDA graph' if graph is not None else 'eager'}); GEMMs are library calls on top",
         "roofline": {"kernel": kname, "bound": "hbm", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_src, "peak_source": peak_src,
                      "algorithmic_bytes_per_launch": alg_bytes, "mean_launch_ms": pa_ms, "launches_timed": len(durs),

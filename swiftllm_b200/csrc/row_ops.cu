@@ -45,7 +45,7 @@ __device__ __forceinline__ bool above(float v, int i, float w, int j) {
 // memory, which may be written once that CTA is known to run: all arrive at the cluster's barrier as they start, and wait at it behind
 // their loads.  One launch whatever the number of rows: a row has eight CTAs' loads in flight, 256 rows fill the GPU.  Bound: the bytes
 // of the logits (in L2 behind the head's product), below about 32 rows one load's latency per run.  Measured on B200, 128256 entries of
-// 16 bits: 16 rows 6 us against 45 us of the tensor library's reduction, 256 rows 18 us.
+// 16 bits, us, this / the tensor library's reduction: 16 rows 6.4 / 26, 64 rows 12 / 26, 128 rows 18, 256 rows 31 / 37.
 constexpr int AM_CTAS = 8, AM_THREADS = 256, AM_RUNS = 4;
 template <typename T, int VEC>
 __global__ void __cluster_dims__(AM_CTAS, 1, 1) __launch_bounds__(AM_THREADS) argmax_rows_kernel(const T* __restrict__ x, int64_t stride, int n,

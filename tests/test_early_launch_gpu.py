@@ -100,7 +100,7 @@ def _stepwise_and_back_to_back(load, stages, result):
 
 
 def _mixed_window(seed, H, G, prompts, decodes, dtype=torch.bfloat16):
-    """A windowed layer's step: norm of the projection, store of its keys and values, attention of prompt and decoded rows."""
+    """A windowed layer's step: norm of the projection, store of its keys and values, attention of prompt and decoded rows, norm of both."""
     from swiftllm_b200.worker.kernels.rmsnorm import rmsnorm_inplace
     from swiftllm_b200.worker.kernels.window_attn import window_attention, window_kv_store
     rows = [(n, 700) for n in prompts] + [(1, n - 1) for n in decodes]
@@ -113,7 +113,7 @@ def _mixed_window(seed, H, G, prompts, decodes, dtype=torch.bfloat16):
     old = _normal(sum(blocks), 1, 16, 2 * G * D, seed=seed + 7, dtype=dtype)
     proj, cache = torch.empty_like(projs[0]), torch.empty_like(old)
     out = torch.empty(T, H * D, dtype=dtype, device=DEV)
-    w = _normal(proj.shape[1], seed=seed + 8, dtype=dtype)
+    w, w2 = _normal(proj.shape[1], seed=seed + 8, dtype=dtype), _normal(H * D, seed=seed + 9, dtype=dtype)
     st = types.SimpleNamespace(num_tokens=T, num_prefill_tokens=sum(prompts), num_prefill_seqs=len(prompts), num_decoding_seqs=len(decodes),
                                token_seq_ids=_ints(i for i, (n, _) in enumerate(rows) for _ in range(n)),
                                token_positions=_ints(p + j for n, p in rows for j in range(n)), max_prefill_len=max(prompts))
@@ -124,7 +124,8 @@ def _mixed_window(seed, H, G, prompts, decodes, dtype=torch.bfloat16):
         proj.copy_(projs[i])
     stages = [lambda: rmsnorm_inplace(proj, w, 1e-5),
               lambda: window_kv_store(k, v, cache, 0, table, st, G, D, D, 0, None, None),
-              lambda: window_attention(q, gate, cache, 0, table, st, out, H, G, D, D, 0, 512, D ** -0.5, True, None, None)]
+              lambda: window_attention(q, gate, cache, 0, table, st, out, H, G, D, D, 0, 512, D ** -0.5, True, None, None),
+              lambda: rmsnorm_inplace(out, w2, 1e-5)]
     return load, stages, lambda: [out, cache]
 
 
