@@ -81,23 +81,24 @@ static int launch_prefill_paged_tc(const void* q, const void* k_cache, const voi
                                    const int32_t* chunk_lens, float scale_log2e, int num_seqs, int max_chunk_len,
                                    int64_t num_tokens, int nq, int nkv, int64_t qs, int64_t cache_rows, const PtPaged& pg,
                                    sllm_dtype_t dtype, cudaStream_t stream) {
+    PtParams p;
+    p.o = o; p.start_locs = start_locs; p.seq_lens = chunk_lens; p.scale_log2e = scale_log2e; p.nq = nq; p.nkv = nkv;
+    bool many;
+    const dim3 grid = pt_grid(p, num_seqs, max_chunk_len, num_tokens, pg.nsplit, true, many);
     CUtensorMap qmap, kmap, vmap;
-    SLLM_REQUIRE(pt_map(&qmap, q, (uint64_t)num_tokens, nq * PT_D, qs, PT_BQ, dtype) &&
+    SLLM_REQUIRE(pt_query_map(&qmap, q, (uint64_t)num_tokens, nq, qs, p.pack_log2, dtype) &&
                  pt_map(&kmap, k_cache, (uint64_t)cache_rows, PT_D, PT_D, PT_PAGE, dtype) &&
                  pt_map(&vmap, v_cache, (uint64_t)cache_rows, PT_D, PT_D, PT_PAGE, dtype),
                  "prefill_attention_paged: cuTensorMapEncodeTiled failed");
-    PtParams p;
-    p.o = o; p.start_locs = start_locs; p.seq_lens = chunk_lens; p.scale_log2e = scale_log2e; p.nq = nq; p.nkv = nkv;
-    dim3 grid((max_chunk_len + 2 * PT_BQ - 1) / (2 * PT_BQ), nq, num_seqs * pg.nsplit);
-    if (dtype == SLLM_F16) {
-        static unsigned long long c = 0;
-        if (first_use_on_this_device(c)) cudaFuncSetAttribute(prefill_attn_tc_kernel<__half, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
-        launch_early(prefill_attn_tc_kernel<__half, true>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, pg);
-    } else {
-        static unsigned long long c = 0;
-        if (first_use_on_this_device(c)) cudaFuncSetAttribute(prefill_attn_tc_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
-        launch_early(prefill_attn_tc_kernel<__nv_bfloat16, true>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, pg);
-    }
+    SLLM_DISPATCH_DTYPE(dtype, {
+        static unsigned long long configured = 0;
+        if (first_use_on_this_device(configured)) {
+            cudaFuncSetAttribute(prefill_attn_tc_kernel<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
+            cudaFuncSetAttribute(prefill_attn_tc_kernel<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
+        }
+        if (many) launch_early(prefill_attn_tc_kernel<T, true, true>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, pg);
+        else launch_early(prefill_attn_tc_kernel<T, true, false>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, pg);
+    });
     if (check_launch("prefill_attention_paged(tcgen05)")) return 1;
     if (pg.nsplit > 1) {
         const dim3 rows((unsigned)cdiv((int64_t)max_chunk_len * nq, 8), (unsigned)num_seqs);
