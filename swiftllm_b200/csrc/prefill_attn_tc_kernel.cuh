@@ -88,21 +88,6 @@ struct PtPaged {
 };
 constexpr int PT_PAGE = 16;               // tokens per KV page (PAGED only)
 
-// The next CTA of the grid that has not been launched, in place of this one: asked for by one thread, the answer (16 bytes) completes on `bar`.
-__device__ __forceinline__ void pt_ask_next(uint32_t dst, uint32_t bar) {
-    fence_proxy_async();                                        // the last answer has been read
-    mbar_arrive_expect_tx(bar, 16);
-    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst), "r"(bar) : "memory");
-}
-__device__ __forceinline__ bool pt_next(uint32_t src, int& x, int& y) {
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n .reg .b128 a;\n ld.shared.b128 a, [%3];\n clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n"
-                 " selp.u32 %0, 1, 0, p;\n mov.u32 %1, 0;\n mov.u32 %2, 0;\n"
-                 " @p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, a;\n"
-                 " @p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, a;\n}\n"
-                 : "=&r"(ok), "=&r"(x), "=&r"(y) : "r"(src) : "memory");
-    return ok != 0;
-}
 // All sequences' query blocks, those of the highest rows first (they have the most keys).  Each by a whole warp
 __device__ __forceinline__ int pt_blocks(const PtParams& p, int s, int len) {            // of sequence s, which has that many rows
     const int log2 = (p.tiles == 2 ? 8 : 7) - p.pack_log2;
@@ -313,7 +298,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 __syncwarp();
                 if (!it.valid) break;
                 if (lane == 0) {
-                    if (MANY && !asked) pt_ask_next(next_at, next_bar);
+                    if (MANY && !asked) ask_next_cta(next_at, next_bar);
                     if (n > 0) {
                         mbar_wait(smem_u32(&bars->q_empty), (n & 1) ^ 1);
                         load_queries(it);
@@ -330,7 +315,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 if constexpr (MANY) {
                     mbar_wait(next_bar, answers++ & 1);
                     int x, y;
-                    if (pt_next(next_at, x, y)) { head_block = PAGED ? y : x; slot = PAGED ? x : y; }
+                    if (next_cta(next_at, x, y)) { head_block = PAGED ? y : x; slot = PAGED ? x : y; }
                 }
             }
         } else if (warp == 2) {

@@ -74,6 +74,23 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
 
+// ------------------------------------------------------------------ cluster launch control
+// The next CTA of the grid that has not been launched, in place of this one: asked for by one thread, the answer (16 bytes) completes on `bar`.
+__device__ __forceinline__ void ask_next_cta(uint32_t dst, uint32_t bar) {
+    fence_proxy_async();                                        // the last answer has been read
+    mbar_arrive_expect_tx(bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool next_cta(uint32_t src, int& x, int& y) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n .reg .b128 a;\n ld.shared.b128 a, [%3];\n clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n"
+                 " selp.u32 %0, 1, 0, p;\n mov.u32 %1, 0;\n mov.u32 %2, 0;\n"
+                 " @p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, a;\n"
+                 " @p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, a;\n}\n"
+                 : "=&r"(ok), "=&r"(x), "=&r"(y) : "r"(src) : "memory");
+    return ok != 0;
+}
+
 // ------------------------------------------------------------------ UMMA descriptors
 // Shared-memory matrix descriptor, SWIZZLE_128B.  K-major operand: rows of 128 B (64 x 16-bit along K), 8-row
 // atoms 1 KiB apart by `sbo` bytes (LBO unused).  MN-major operand: atoms of 8 K-rows x 64 MN-elements; `lbo` =

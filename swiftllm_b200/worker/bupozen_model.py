@@ -7,7 +7,7 @@ from swiftllm_b200.worker.weight import load_bupozen_weights
 
 
 class BupozenModel(ParallelBlockModel):
-    NATIVE_SOURCES = ParallelBlockModel.NATIVE_SOURCES + ("latent_attn.cu", "latent_attn_tc.cu",)
+    NATIVE_SOURCES = ParallelBlockModel.NATIVE_SOURCES + ("latent_attn.cu", "latent_attn_tc.cu", "latent_attn_prompt.cu",)
     CONFIG_CLASS = BupozenModelConfig
 
     @staticmethod

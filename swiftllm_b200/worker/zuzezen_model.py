@@ -23,7 +23,7 @@ from .token_model import TokenBatchModel
 
 
 class ZuzezenModel(TokenBatchModel):
-    NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("parallel_block.cu", "stream_ops.cu", "latent_attn.cu", "latent_attn_tc.cu", "window_attn.cu", "window_attn_tc.cu", "gla.cu")
+    NATIVE_SOURCES = TokenBatchModel.NATIVE_SOURCES + ("parallel_block.cu", "stream_ops.cu", "latent_attn.cu", "latent_attn_tc.cu", "latent_attn_prompt.cu", "window_attn.cu", "window_attn_tc.cu", "gla.cu")
     CONFIG_CLASS = ZuzezenModelConfig
 
     @staticmethod
