@@ -4,8 +4,8 @@
 // A CTA owns two tiles of 128 query ROWS of one key/value group, row = (token, head of the group) with the heads padded to a power of
 // two: 64 tokens for four heads per group.  Tokens are walked in segments (runs of one sequence at consecutive positions), so any order
 // of rows is correct; a segment's rows share ONE list of keys (kept first positions, then the window), taken in steps of 80.
-//   warps 0, 2   producers: gather cache rows through the block table by cp.async into a four-stage ring (keys past the segment's last
-//                position are zero)
+//   warps 0, 2   producers: cache rows through the block table into a four-stage ring, in TMA boxes of 16 rows (BOXES) or by cp.async (keys past
+//                the segment's last position are zero)
 //   warps 1, 3   product issuers of tile A / B:  S_X(j + 1) = Q_X . K(j + 1) as soon as S_X(j) is in registers,
 //                O_X += P_X(j) . V(j) when P_X(j) is there; with shared_kv the key tile is also the value tile
 //   warps 4-7    queries, softmax and output of tile A, warps 8-11 of tile B: thread = query row = TMEM lane, P as 16-bit A operand in TMEM,
@@ -18,9 +18,9 @@
 // see, the segment is done over, token by token, with the keys that the token does not see left zero: a result depends on its own keys only.
 //
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
-// ones 312 us with the mma.sync kernel of window_attn.cu for the prompts -> 118 us, 92 with the decoded rows beside the prompts' last CTAs
-// (the prompts alone 87, the decoded rows 31; two rounds of CTAs here; a CTA's step of 80 keys is about 2200 cycles, its queries and first
-// keys 12 k, its output 5 k).
+// ones 312 us with the mma.sync kernel of window_attn.cu for the prompts -> 118 us, 91 with the decoded rows beside the prompts' last CTAs, 83 with
+// boxes (the prompts alone 85 -> 74, one of 2048 51 -> 42, 600 rows at 1500 41 -> 31, 32 heads at 1000, window 2048 170 -> 144).  Two rounds of
+// CTAs here; a CTA's step of 80 keys is 2000 cycles of softmax, its queries 10 k, its output 10 k (gates one by one 15 k).
 //
 // EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores;
 // FULL: heads of 128 + 128 entries without turned ones beside shared keys (the producers are bound by their instructions).
@@ -45,27 +45,38 @@ constexpr int WX_SMEM = WX_MISC_OFF + 256;
 constexpr int WX_S_COL = 0, WX_P_COL = 160, WX_O_COL = 256;      // tile B: + 80, + 40, + 128
 constexpr float WX_LOG2E = 1.4426950408889634f;
 // registers: 384 threads are launched with 168 each; the softmax warpgroups hold a row of scores and of P
-constexpr int WX_REGS_FEW = 72, WX_REGS_MANY = 216;
+constexpr int WX_REGS_FEW = 88, WX_REGS_MANY = 208;
 static_assert(WX_REGS_FEW + 2 * WX_REGS_MANY <= 3 * 168, "the warpgroups' shares must fit what the block was launched with");
 constexpr int WX_LAG = 1;                             // steps whose rows are in flight behind the one being asked for
 
 struct WindowTcBars {
     uint64_t full[WX_STAGES], empty[WX_STAGES];
     uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2];
+    uint64_t landed[2];                              // [keys, values]: boxes of a step whose unseen rows have yet to become zero
 };
 
 __device__ __forceinline__ uint32_t wx_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
 
-// 1 / (1 + e^-z): the quick reciprocal and one step of Newton's iteration, r + r (1 - d r), which leaves about half a unit in the last place
-// and has no branch, so that the gates of a row are worked on together (with a quotient rounded exactly the case below
-// took 127 us instead of 115).
-__device__ __forceinline__ float sigmoid_nr(float z) {
-    const float d = 1.f + __expf(-z), r = __fdividef(1.f, d);       // r is 0 from d = 2^126 on
-    return fmaf(r, fmaf(-fminf(d, 0x1p127f), r, 1.f), r);
+// y / (1 + e^-z), two at a time: the quick reciprocal and one step of Newton's iteration, r + r (1 - d r), which leaves about half a unit in the last place
+// and has no branch, so that the gates of a row are worked on together (with a quotient rounded exactly the case below took 127 us
+// instead of 115).  Five to six instructions a gate: a row's 128 take 1.9 k cycles of its warp when it has the scheduler to itself (one by one 3.8 k).
+__device__ __forceinline__ float rcp_quick(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float2 gate_pair(float2 y, float2 z) {
+    const float2 one = make_float2(1.f, 1.f), t = mul2(z, make_float2(-WX_LOG2E, -WX_LOG2E));
+    const float2 d = add2(make_float2(fast_exp2_tc(t.x), fast_exp2_tc(t.y)), one), r = make_float2(rcp_quick(d.x), rcp_quick(d.y));
+    const float2 low = make_float2(-fminf(d.x, 0x1p127f), -fminf(d.y, 0x1p127f));      // r is 0 from d = 2^126 on
+    return mul2(y, fma2(r, fma2(low, r, one), r));
 }
 
-template <typename T, bool EXT, bool CAP, bool FULL>
-__global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const WindowTc p) {
+// BOXES: keys and values come in TMA boxes of 16 cache rows, each producer warp its half of a step's columns (a step's 5120 16-byte pieces by cp.async take
+// two warps 2500 to 3000 cycles to ask for, softmax and products 2100)
+template <typename T, bool EXT, bool CAP, bool FULL, bool BOXES>
+__global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const WindowTc p) {
+    static_assert(!BOXES || (FULL && !EXT), "boxes of 128 + 128 columns, of one run of positions");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_sm = smem;                             // [tile][chunk][128 rows][128 B]
     uint8_t* kv_sm = smem + 2 * WX_Q_BYTES;           // [stage][chunk][80 keys][128 B]
@@ -88,8 +99,10 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
         for (int x = 0; x < 2; x++) {
             mbar_init(smem_u32(&bars->s_full[x]), 1); mbar_init(smem_u32(&bars->s_empty[x]), 128);
             mbar_init(smem_u32(&bars->p_full[x]), 128); mbar_init(smem_u32(&bars->p_empty[x]), 1);
+            mbar_init(smem_u32(&bars->landed[x]), 1);
         }
         mbar_fence_init();
+        if constexpr (BOXES) tma_prefetch_desc(&map);
     }
     if (warp == 1) tmem_alloc<512>(smem_u32(tmem_s));
     tc_fence_before();
@@ -114,12 +127,15 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
         const int left = ntok - i0;
         s.seq = p.tok_seq[s.ts]; s.pos0 = p.tok_pos[s.ts];
         s.n = left;
-        for (int b = 0; b < left; b += 32) {
-            const int i = b + min(lane, left - 1 - b);
-            const uint32_t cut = __ballot_sync(0xffffffffu, p.tok_seq[s.ts + i] != s.seq || p.tok_pos[s.ts + i] != s.pos0 + i);
+        for (int b = 0; b < left; b += 64) {              // (all loads of 64 tokens in flight together)
+            const int i = min(b + lane, left - 1), k = min(i + 32, left - 1);
+            const int qi = p.tok_seq[s.ts + i], qk = p.tok_seq[s.ts + k], pi = p.tok_pos[s.ts + i], pk = p.tok_pos[s.ts + k];
+            const uint32_t cut = __ballot_sync(0xffffffffu, qi != s.seq || pi != s.pos0 + i), later = __ballot_sync(0xffffffffu, qk != s.seq || pk != s.pos0 + k);
             if (cut) { s.n = b + __ffs(cut) - 1; break; }
+            if (later) { s.n = b + 31 + __ffs(later); break; }
         }
         s.lo = first_seen(s.pos0); s.hi = s.pos0 + s.n - 1;
+        if constexpr (BOXES) s.lo &= ~15;                 // (a box's first row)
         s.nk = EXT && p.window > 0 ? min(keep_first, s.lo) : 0;
         const int na = min(s.n, tpt), nb = s.n - na;
         // entry v of the list of keys is position v (v < nk) or v - nk + lo; entries a tile's last token sees
@@ -161,6 +177,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
     };
     if (warp < 4) {
         reg_dec<WX_REGS_FEW>();
+        int landed_done = 0;                          // phases of `landed`
         for (int i0 = 0; i0 < ntok;) {
             pass++;
             const Segment sg = segment(i0);
@@ -169,7 +186,43 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
             const int* bt = p.block_table + (int64_t)sg.seq * p.max_blocks_per_seq;
             const int own = sg.pos0 + max(solo, 0), total = solo < 0 ? max(sg.end_a, sg.end_b) : nk + own - lo + 1;
             const int hidden = solo < 0 ? 0 : nk + first_seen(own) - lo;             // entries vkeep .. hidden - 1 are not
-            if (warp == 0 || warp == 2) {
+            if (BOXES && (warp == 0 || warp == 2)) {
+                // ======================================================= producers: warp 0 the keys, warp 2 the values; lanes 0 .. 4 a box each
+                const int seen = (solo < 0 ? first_seen(sg.pos0) : first_seen(own)) - lo;      // entries seen .. total - 1 are visible
+                const int col = warp == 0 ? kofs : vofs;
+                auto box_row = [&](int j) {
+                    const int kp = lo + j * WX_BK + 16 * lane;
+                    if (lane >= WX_BK / 16 || j >= nsteps || kp >= lo + total) return -1;
+                    const int b = kp / p.block_size;
+                    return (int)(((long long)bt[b] * p.n_slots + p.slot) * p.block_size + (kp - b * p.block_size));
+                };
+                int next = box_row(0);
+                for (int j = 0; j < nsteps; j++) {
+                    const int it = n_done + j, st = it % WX_STAGES, row = next;
+                    next = box_row(j + 1);
+                    const bool ragged = j * WX_BK < seen || (j + 1) * WX_BK > total;
+                    const uint32_t full = smem_u32(&bars->full[st]), bar = ragged ? smem_u32(&bars->landed[warp >> 1]) : full;
+                    uint8_t* half = kv_sm + st * WX_STAGE + warp * WX_CHUNK;                  // this warp's two chunks
+                    const int boxes = __popc(__ballot_sync(0xffffffffu, row >= 0));
+                    if (lane == 0) {
+                        mbar_wait(smem_u32(&bars->empty[st]), ((it / WX_STAGES) & 1) ^ 1);
+                        mbar_arrive_expect_tx(bar, (uint32_t)boxes * 16 * 256);
+                    }
+                    __syncwarp();
+                    if (row >= 0) {
+                        tma_load_2d(smem_u32(half) + lane * 2048, &map, bar, col, row);
+                        tma_load_2d(smem_u32(half) + WX_CHUNK + lane * 2048, &map, bar, col + 64, row);
+                    }
+                    if (!ragged) continue;
+                    mbar_wait(bar, landed_done++ & 1);        // rows that are not seen become zero
+                    for (int r = lane >> 4; r < WX_BK; r += 2)
+                        if (j * WX_BK + r < seen || j * WX_BK + r >= total)
+                            *reinterpret_cast<uint4*>(half + ((lane >> 3) & 1) * WX_CHUNK + r * 128 + (lane & 7) * 16) = make_uint4(0, 0, 0, 0);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full);
+                }
+            } else if (warp == 0 || warp == 2) {
                 // ======================================================= producers: keys 40 (warp / 2) .. of every step, eight lanes a 128-byte piece
                 const int r0 = 20 * warp, piece = lane & 7;
                 const T* cache = reinterpret_cast<const T*>(p.cache);
@@ -235,10 +288,11 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                 const int kd_steps = dk >> 4;
                 auto scores = [&](int j) {
                     const int it = n_done + j, st = it % WX_STAGES;
+                    const uint64_t kd = dk0 + (uint64_t)((st * WX_STAGE) >> 4);
                     mbar_wait(smem_u32(&bars->full[st]), (it / WX_STAGES) & 1);
+                    if (j > 0) mbar_wait(smem_u32(&bars->s_empty[x]), (x_done + j - 1) & 1);
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint64_t kd = dk0 + (uint64_t)((st * WX_STAGE) >> 4);
 #pragma unroll
                         for (int k = 0; k < 8; k++)
                             if (k < kd_steps) {
@@ -255,16 +309,13 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                     scores(0);
                     for (int j = 0; j < mine; j++) {
                         const int xi = x_done + j;
-                        if (j + 1 < mine) {
-                            mbar_wait(smem_u32(&bars->s_empty[x]), xi & 1);
-                            scores(j + 1);
-                        }
+                        if (j + 1 < mine) scores(j + 1);
                         const int st = (n_done + j) % WX_STAGES;
+                        const int k16 = min(WX_BK / 16, (end - j * WX_BK + 15) / 16);         // none past the last key the tile can see
+                        const uint64_t vd = dv0 + (uint64_t)((st * WX_STAGE) >> 4) + vfirst;
                         mbar_wait(smem_u32(&bars->p_full[x]), xi & 1);
                         tc_fence_after();
                         if (elect_one()) {
-                            const int k16 = min(WX_BK / 16, (end - j * WX_BK + 15) / 16);     // none past the last key the tile can see
-                            const uint64_t vd = dv0 + (uint64_t)((st * WX_STAGE) >> 4) + vfirst;
 #pragma unroll
                             for (int k = 0; k < WX_BK / 16; k++)
                                 if (k < k16) umma_ts(o_addr, p_addr + 8 * k, vd + (uint64_t)((k * 2048) >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
@@ -318,20 +369,42 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
 #pragma unroll
                     for (int e = 0; e < 8; e++) nw[e] = p.qnorm_w != nullptr ? p.qnorm_w[dc + e] : 1.f;
                     const bool turns = d < p.rot_dims;
+                    // 64 rows on, a lane's row is that of the same head (at most 64 of a group) some tokens on: its pointers move by constants
+                    const int start = 2 * me + (lane >> 4), hop = 64 >> p.hqp_log2;
+                    const T* qp[4];
+                    const float* cp[4];
+                    const float* sp[4];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        const int row = start + 16 * b;
+                        const int64_t t = ts + (row >> p.hqp_log2);
+                        qp[b] = reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + min(row & (hqp - 1), hq - 1)) * dk + dc;
+                        cp[b] = p.cosb + t * half + dr; sp[b] = p.sinb + t * half + dr;
+                    }
+                    const int64_t q_hop = hop * p.q_st;
+                    const int a_hop = hop * half;
+                    Vec8<T> nu[4];                    // the next rows are on their way while these are turned
+                    float4 nc[4], ns[4];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) nc[b] = ns[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    auto ask = [&](int r0) {
+#pragma unroll
+                        for (int b = 0; b < 4; b++) {
+                            if (((r0 + 16 * b) >> p.hqp_log2) < n) {          // (other rows are made zero below)
+                                nu[b] = ld_vec8(qp[b]);
+                                if (p.rot_dims > 0) { nc[b] = *reinterpret_cast<const float4*>(cp[b]); ns[b] = *reinterpret_cast<const float4*>(sp[b]); }
+                            }
+                            qp[b] += q_hop; cp[b] += a_hop; sp[b] += a_hop;
+                        }
+                    };
+                    ask(start);
 #pragma unroll 1
-                    for (int r0 = 2 * me + (lane >> 4); r0 < nrows; r0 += 64) {
+                    for (int r0 = start; r0 < nrows; r0 += 64) {
                         Vec8<T> u[4];
                         float4 c4[4], s4[4];
 #pragma unroll
-                        for (int b = 0; b < 4; b++) {
-                            const int row = r0 + 16 * b;
-                            const int64_t t = ts + min(row >> p.hqp_log2, n - 1);
-                            u[b] = ld_vec8(reinterpret_cast<const T*>(p.q) + t * p.q_st + (int64_t)(g * hq + min(row & (hqp - 1), hq - 1)) * dk + dc);
-                            if (p.rot_dims > 0) {
-                                c4[b] = *reinterpret_cast<const float4*>(p.cosb + t * half + dr);
-                                s4[b] = *reinterpret_cast<const float4*>(p.sinb + t * half + dr);
-                            }
-                        }
+                        for (int b = 0; b < 4; b++) { u[b] = nu[b]; c4[b] = nc[b]; s4[b] = ns[b]; }
+                        if (r0 + 64 < nrows) ask(r0 + 64);
 #pragma unroll
                         for (int b = 0; b < 4; b++) {
                             const int row = r0 + 16 * b;
@@ -521,14 +594,31 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                 if (j > 0 && __any_sync(0xffffffffu, need)) {
                     mbar_wait(smem_u32(&bars->p_empty[x]), (xi - 1) & 1);          // the products of step j - 1 are done: O is stable
                     tc_fence_after();
+                    if constexpr (FULL && !EXT) {     // a round trip to TMEM takes as long for 64 columns as for 16
 #pragma unroll 1
-                    for (int d = 0; d < dv; d += 16) {
-                        uint32_t t[16];
-                        tmem_ld<16>(o_addr + d, t);
-                        tmem_ld_wait();
+                        for (int d = 0; d < 128; d += 64) {
+                            uint32_t t[2][32];
+                            tmem_ld32(o_addr + d, t[0]);
+                            tmem_ld32(o_addr + d + 32, t[1]);
+                            tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-                        tmem_st16(o_addr + d, t);
+                            for (int i = 0; i < 64; i += 2) {
+                                const float2 y = mul2(make_float2(__uint_as_float(t[i >> 5][i & 31]), __uint_as_float(t[i >> 5][(i & 31) + 1])), make_float2(alpha, alpha));
+                                t[i >> 5][i & 31] = __float_as_uint(y.x); t[i >> 5][(i & 31) + 1] = __float_as_uint(y.y);
+                            }
+                            tmem_st32(o_addr + d, t[0]);
+                            tmem_st32(o_addr + d + 32, t[1]);
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int d = 0; d < dv; d += 16) {
+                            uint32_t t[16];
+                            tmem_ld<16>(o_addr + d, t);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
+                            tmem_st16(o_addr + d, t);
+                        }
                     }
                 }
                 if (need) m_ref = m_new;
@@ -572,8 +662,8 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                 auto gate8 = [&](const Vec8<T>& u, float (&y)[8]) {
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
-                        const float2 z = Traits<T>::to_f2(u.v[e]);
-                        y[2 * e] *= sigmoid_nr(z.x); y[2 * e + 1] *= sigmoid_nr(z.y);
+                        const float2 q = gate_pair(make_float2(y[2 * e], y[2 * e + 1]), Traits<T>::to_f2(u.v[e]));
+                        y[2 * e] = q.x; y[2 * e + 1] = q.y;
                     }
                 };
                 auto store8 = [&](int64_t to, float (&y)[8]) {
@@ -613,42 +703,72 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const Win
                     float* xs = reinterpret_cast<float*>(q_sm + x * WX_Q_BYTES);
                     auto cell = [&](int rr, int quarter) { return reinterpret_cast<float4*>(xs + rr * 64 + ((quarter ^ (rr & 15)) << 2)); };
                     const int l8 = lane & 7;
-                    // this lane's part of row 32 quad + 4 i + lane / 8: its index in gate and out, -1 where there is nothing to store
-                    auto part = [&](int i, int d0, int64_t stride) {
+                    // this lane's part of row 32 quad + 4 i + lane / 8, where there is something to store: its token and head
+                    uint32_t there = 0;
+                    int64_t gate_at[8], out_at[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
                         const int rr = quad * 32 + 4 * i + (lane >> 3), rt = x * tpt + (rr >> p.hqp_log2), rh = rr & (hqp - 1);
-                        return rt < n && rh < hq && (solo < 0 || rt == solo) && d0 + 8 * l8 < dv ? (ts + rt) * stride + (int64_t)(g * hq + rh) * dv + d0 + 8 * l8 : -1ll;
-                    };
-                    for (int d0 = 0; d0 < dv; d0 += 64) {
-                        Vec8<T> z[8];                 // all gates of the pass are asked for before the first is used
-                        if (gated) {
-#pragma unroll
-                            for (int i = 0; i < 8; i++) z[i] = ld_vec8(gate + max(part(i, d0, p.gate_st), 0ll));
-                        }
-                        const int cols = min(64, dv - d0);
-#pragma unroll 1
-                        for (int d = 0; d < cols; d += 16) {
-                            uint32_t v[16];
-                            tmem_ld<16>(o_addr + d0 + d, v);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < 16; e += 2) look(v[e], v[e + 1]);
-#pragma unroll
-                            for (int e = 0; e < 4; e++)
-                                *cell(row, (d >> 2) + e) = make_float4(__uint_as_float(v[4 * e]) * f, __uint_as_float(v[4 * e + 1]) * f,
-                                                                       __uint_as_float(v[4 * e + 2]) * f, __uint_as_float(v[4 * e + 3]) * f);
-                        }
-                        __syncwarp();                 // a warp reads the rows that it wrote
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const int rr = quad * 32 + 4 * i + (lane >> 3);
-                            const float4 lo4 = *cell(rr, 2 * l8), hi4 = *cell(rr, 2 * l8 + 1);
-                            float y[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
-                            if (gated) gate8(z[i], y);
-                            const int64_t to = part(i, d0, p.out_st);
-                            if (to >= 0) store8(to, y);
-                        }
-                        __syncwarp();
+                        const bool is = rt < n && rh < hq && (solo < 0 || rt == solo);
+                        const int64_t col = (int64_t)(g * hq + rh) * dv + 8 * l8;
+                        there |= is ? 1u << i : 0u;
+                        gate_at[i] = is ? (ts + rt) * p.gate_st + col : 0; out_at[i] = is ? (ts + rt) * p.out_st + col : 0;
                     }
+                    // (no branches between one row's numbers and the next one's: the rows' exponentials and quotients run side by side)
+                    auto rows = [&](auto to_f32, auto with_gate) {
+#pragma unroll 1
+                        for (int d0 = 0; d0 < dv; d0 += 64) {
+                            const bool here = d0 + 8 * l8 < dv;
+                            Vec8<T> z[8];             // all gates of the pass are asked for before the first is used
+                            if constexpr (with_gate.value) {
+#pragma unroll
+                                for (int i = 0; i < 8; i++) z[i] = ld_vec8(gate + (here ? gate_at[i] + d0 : 0));
+                            }
+                            const int cols = min(64, dv - d0);
+#pragma unroll 1
+                            for (int d = 0; d < cols; d += 16) {
+                                uint32_t v[16];
+                                tmem_ld<16>(o_addr + d0 + d, v);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int e = 0; e < 16; e += 2) look(v[e], v[e + 1]);
+#pragma unroll
+                                for (int e = 0; e < 4; e++)
+                                    *cell(row, (d >> 2) + e) = make_float4(__uint_as_float(v[4 * e]) * f, __uint_as_float(v[4 * e + 1]) * f,
+                                                                           __uint_as_float(v[4 * e + 2]) * f, __uint_as_float(v[4 * e + 3]) * f);
+                            }
+                            __syncwarp();             // a warp reads the rows that it wrote
+#pragma unroll
+                            for (int i0 = 0; i0 < 8; i0 += 4) {
+                                float y[4][8];
+#pragma unroll
+                                for (int k = 0; k < 4; k++) {
+                                    const int rr = quad * 32 + 4 * (i0 + k) + (lane >> 3);
+                                    const float4 lo4 = *cell(rr, 2 * l8), hi4 = *cell(rr, 2 * l8 + 1);
+                                    y[k][0] = lo4.x; y[k][1] = lo4.y; y[k][2] = lo4.z; y[k][3] = lo4.w;
+                                    y[k][4] = hi4.x; y[k][5] = hi4.y; y[k][6] = hi4.z; y[k][7] = hi4.w;
+                                    if constexpr (with_gate.value) gate8(z[i0 + k], y[k]);
+                                }
+#pragma unroll
+                                for (int k = 0; k < 4; k++) {
+                                    if (!here || !(there >> (i0 + k) & 1)) continue;
+                                    if constexpr (to_f32.value) {
+                                        float* o = reinterpret_cast<float*>(p.out) + out_at[i0 + k] + d0;
+                                        *reinterpret_cast<float4*>(o) = make_float4(y[k][0], y[k][1], y[k][2], y[k][3]);
+                                        *reinterpret_cast<float4*>(o + 4) = make_float4(y[k][4], y[k][5], y[k][6], y[k][7]);
+                                    } else {
+                                        *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.out) + out_at[i0 + k] + d0) =
+                                            make_uint4(pack2<T>(y[k][0], y[k][1]), pack2<T>(y[k][2], y[k][3]), pack2<T>(y[k][4], y[k][5]), pack2<T>(y[k][6], y[k][7]));
+                                    }
+                                }
+                            }
+                            __syncwarp();
+                        }
+                    };
+                    using Yes = std::true_type; using No = std::false_type;
+                    if (p.out_f32) { if (gated) rows(Yes(), Yes()); else rows(Yes(), No()); }
+                    else if (gated) rows(No(), Yes());
+                    else rows(No(), No());
                 } else {
                 const int hv = dv >> 1;
 #pragma unroll 1
@@ -717,20 +837,33 @@ int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) 
     while (p.qt > least && p.qt > 1 && (int64_t)cdiv(p.num_rows, p.qt >> 1) * p.G <= num_sms) p.qt >>= 1;
     const dim3 grid((unsigned)cdiv(p.num_rows, p.qt), (unsigned)p.G);
     const bool ext = p.slopes != nullptr || p.keep_first > 0 || p.gate_per_head || p.shared_kv || p.sinks != nullptr, cap = p.softcap > 0.f;
-#define SLLM_WX3(EXT, CAP, FULL)                                                                                                          \
+    // boxes: whole cache blocks of 16 rows, 16-byte rows and columns of theirs (a block table names only blocks that there are: the map need not know how
+    // many)
+    CUtensorMap map = {};
+    bool boxes = !ext && p.dk == 128 && p.dv == 128 && p.krot == 0 && p.block_size % 16 == 0 && p.row_elems % 8 == 0 && p.koff % 8 == 0;
+    if (boxes) {
+        const cuuint64_t dims[2] = {(cuuint64_t)p.row_elems, (cuuint64_t)1 << 31}, strides[1] = {(cuuint64_t)p.row_elems * 2};
+        const cuuint32_t box[2] = {64, 16}, es[2] = {1, 1};
+        TensorMapEncodeFn enc = get_tensor_map_encoder();
+        boxes = enc != nullptr && enc(&map, dtype == SLLM_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p.cache), dims,
+                                      strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+#define SLLM_WX3(EXT, CAP, FULL, BOXES)                                                                                                          \
     do {                                                                                                                           \
         static unsigned long long configured = 0;                                                                                  \
-        auto kern = window_attn_tc_kernel<T, EXT, CAP, FULL>;                                                                            \
+        auto kern = window_attn_tc_kernel<T, EXT, CAP, FULL, BOXES>;                                                                            \
         if (first_use_on_this_device(configured)) {                                                                                \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_SMEM);                      \
             SLLM_REQUIRE(e == cudaSuccess, "window_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));                  \
         }                                                                                                                          \
-        launch_early(kern, grid, WX_THREADS, WX_SMEM, stream, p);                                                                  \
+        launch_early(kern, grid, WX_THREADS, WX_SMEM, stream, map, p);                                                                \
     } while (0)
 #define SLLM_WX(EXT, CAP)                                                                                                          \
     do {                                                                                                                           \
-        if (p.dk == 128 && p.dv == 128 && p.krot == 0) SLLM_WX3(EXT, CAP, true);                                                   \
-        else SLLM_WX3(EXT, CAP, false);                                                                                            \
+        if (!EXT && boxes) SLLM_WX3(EXT, CAP, true, !EXT);                                                                         \
+        else if (p.dk == 128 && p.dv == 128 && p.krot == 0) SLLM_WX3(EXT, CAP, true, false);                                       \
+        else SLLM_WX3(EXT, CAP, false, false);                                                                                           \
     } while (0)
     SLLM_DISPATCH_DTYPE(dtype, {
         if (ext && cap) SLLM_WX(true, true);
