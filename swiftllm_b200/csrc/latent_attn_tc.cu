@@ -27,8 +27,8 @@
 //
 // Bound: at M = 64 the tensor core runs at half rate, (D + r) * 64 * 64 multiply-adds per tile = 2176 cycles at D = 576, r = 512, and
 // S's operands are 4 KiB of shared memory per 32 cycles; a decoded token is bound by its rows' bytes.  Measured on B200, bf16, 16 heads,
-// r = 512: four prompts of 2048 tokens 3214 us with the mma.sync kernel of latent_attn.cu -> 573 us (509 TFLOP/s); 64 decoded tokens at
-// 2048 keys 88 -> 49 us with the merge.
+// r = 512: four prompts of 2048 tokens 3214 us with the mma.sync kernel of latent_attn.cu -> 573 us (509 TFLOP/s; large launches of
+// such rows now run latent_attn_prompt.cu, 450 us); 64 decoded tokens at 2048 keys 88 -> 49 us with the merge.
 #include "latent_attn_tc.cuh"
 #include "mma_helpers.cuh"
 #include "tc_helpers.cuh"
