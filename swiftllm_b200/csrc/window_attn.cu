@@ -1191,6 +1191,7 @@ static int launch_window_attn_mma(const void* q, int64_t q_stride_t, const void*
             w.vsin = (const float*)vsin; w.out_scale = out_scale; w.qnorm_w = (const float*)qnorm_w; w.prenorm_eps = prenorm_eps; w.chunk = chunk;
             w.vshare = vshare; w.out_f32 = out_f32; w.slopes = (const float*)slopes; w.keep_first = keep_first; w.gate_per_head = gate_per_head;
             w.shared_kv = shared_kv; w.krot = krot; w.sinks = (const float*)sinks;
+            w.beside = beside.stream() != stream ? (int)std::min<int64_t>(parts[1][1] * G, 1 << 30) : 0;
             w.row_elems = shared_kv ? shared_kv_row(G, dk + krot) : G * dk + (G / vshare) * dv;
             w.koff = shared_kv ? shared_kv_key_offset(G) : 0;
             w.q_vec = ((uintptr_t)q & 15) == 0 && q_stride_t % 8 == 0 && (!halves || rot_dims % 16 == 0);

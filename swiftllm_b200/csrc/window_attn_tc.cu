@@ -19,8 +19,8 @@
 //
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
 // ones 312 us with the mma.sync kernel of window_attn.cu for the prompts -> 118 us, 91 with the decoded rows beside the prompts' last CTAs, 83 with
-// boxes (the prompts alone 85 -> 74, one of 2048 51 -> 42, 600 rows at 1500 41 -> 31, 32 heads at 1000, window 2048 170 -> 144).  Two rounds of
-// CTAs here; a CTA's step of 80 keys is 2000 cycles of softmax, its queries 10 k, its output 10 k (gates one by one 15 k).
+// boxes (the prompts alone 85 -> 74, one of 2048 51 -> 42, 600 rows at 1500 41 -> 31, 32 heads at 1000, window 2048 170 -> 144; with the long
+// CTAs of all groups first 74 -> 64, 144 -> 117).  Two rounds of CTAs here; a CTA's step of 80 keys is 2000 cycles of softmax, its queries 10 k, its output 10 k (gates one by one 15 k).
 //
 // EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores;
 // FULL: heads of 128 + 128 entries without turned ones beside shared keys (the producers are bound by their instructions).
@@ -88,9 +88,12 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const __g
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool shared_kv = EXT && p.shared_kv;
     const int krot = EXT && !FULL ? p.krot : 0, keep_first = EXT ? p.keep_first : 0;
-    const int dk = FULL ? 128 : p.dk, dv = FULL ? 128 : p.dv, KW = dk + krot, hq = p.H / p.G, hqp = 1 << p.hqp_log2, g = blockIdx.y;
+    const int dk = FULL ? 128 : p.dk, dv = FULL ? 128 : p.dv, KW = dk + krot, hq = p.H / p.G, hqp = 1 << p.hqp_log2;
     const int kch = (KW + 63) >> 6, vch = shared_kv ? 0 : (dv + 63) >> 6;         // chunks of a key / value row
-    const int t_first = (gridDim.x - 1 - blockIdx.x) * p.qt;                       // the last tokens of a prompt have the most keys: first
+    // The last tokens of a prompt have the most keys: first, in all groups (p.group_blocks: in one group behind the other)
+    const int behind = gridDim.x - 1 - blockIdx.x, of = p.group_blocks ? p.group_blocks : p.G, k = behind / of;
+    const int block = p.group_blocks ? behind - k * of : k, g = p.group_blocks ? k : behind - k * of;
+    const int t_first = block * p.qt;
     const int ntok = min(p.qt, p.num_rows - t_first);
 
     if (tid == 0) {
@@ -835,8 +838,14 @@ int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) 
     p.qt = (2 * WX_ROWS) >> p.hqp_log2;
     const int least = (WX_ROWS / 2) >> p.hqp_log2;
     while (p.qt > least && p.qt > 1 && (int64_t)cdiv(p.num_rows, p.qt >> 1) * p.G <= num_sms) p.qt >>= 1;
-    const dim3 grid((unsigned)cdiv(p.num_rows, p.qt), (unsigned)p.G);
+    const dim3 grid((unsigned)cdiv(p.num_rows, p.qt) * (unsigned)p.G);
     const bool ext = p.slopes != nullptr || p.keep_first > 0 || p.gate_per_head || p.shared_kv || p.sinks != nullptr, cap = p.softcap > 0.f;
+    // The long CTAs of all groups first: with one group behind the other the last one's long CTAs begin when most SMs have run out of work (us, one group
+    // behind the other / now, three prompts of up to 2048, 16 / 4 heads 74 / 64, 32 / 8 heads at 1000, window 2048 144 / 117, shared keys 181 instead of 229).
+    // More than a round of them beside a round of decoded rows keeps the groups apart: those fill the ragged end, and find no SM before the last prompt row's
+    // CTA has one (us, apart / together, three prompts of up to 2048 and 38 decoded 83 / 90, 64 decoded 90 / 92, at 300 keys 75 / 76, 32 / 8 heads
+    // 178 / 180; two at 1000 and 64 147 / 136; ten decoded 83 / 70, one prompt of 1000 58 / 52; shared keys, 40 decoded 106 / 100, 216 / 204)
+    p.group_blocks = !ext && p.beside >= num_sms && (int64_t)grid.x > num_sms ? cdiv(p.num_rows, p.qt) : 0;
     // boxes: whole cache blocks of 16 rows, 16-byte rows and columns of theirs (a block table names only blocks that there are: the map need not know how
     // many)
     CUtensorMap map = {};

@@ -13,6 +13,8 @@ struct WindowTc {
     const int* block_table; int max_blocks_per_seq;
     const int* tok_seq; const int* tok_pos;
     void* out; int64_t out_st;
+    int beside;                                          // CTAs of decoded rows on a stream beside this launch's
+    int group_blocks;                                    // set at the launch: blocks of rows a group, where its CTAs keep together
     int num_rows, H, G, dk, dv, rot_dims, window;
     float scale, sink;
     int halves;
