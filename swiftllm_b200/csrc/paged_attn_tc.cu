@@ -44,7 +44,7 @@ constexpr int TC_NPAD = 16;               // UMMA N (heads, padded)
 constexpr int TC_K_BYTES = TC_TILE * TC_D * 2;                 // 32 KiB per K (or V) tile
 constexpr int TC_Q_BYTES = 2 * TC_NPAD * 128;                  // [half][16 rows][128 B] = 4 KiB
 constexpr int TC_P_BYTES = 2 * TC_NPAD * 128;                  // [token half][16 rows][128 B] = 4 KiB
-constexpr int TC_SMEM_BYTES = (TC_KSTAGES + TC_VSTAGES) * TC_K_BYTES + 2 * TC_Q_BYTES + 2 * TC_P_BYTES + 3072;
+constexpr int TC_SMEM_BYTES = (TC_KSTAGES + TC_VSTAGES) * TC_K_BYTES + 2 * TC_Q_BYTES + 2 * TC_P_BYTES + 3328;
 constexpr int TC_TMEM_COLS = 64;          // S: 2 x 16, O: 2 x 16
 
 struct TcParams {
@@ -68,6 +68,7 @@ struct Barriers {       // all mbarriers of the CTA (shared memory)
 // Tokens past the launch's splits (a length above the longest that the caller stated, for which there is neither workspace nor a CTA of
 // the cluster) are not seen: every length is cut to p.longest.
 struct Item { int seq, kvh, split, split_start, split_len, ntiles; };
+struct Place { int seq, kvh, split; };      // where an item's output goes
 
 // A launch's items (compiled into the kernel: as a branch per item, the search below cost launches without it 2 to 13 %; 256 sequences of
 // 64 tokens, 32 / 8 heads, 32 us without and 34 with the branch):
@@ -205,9 +206,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
     uint8_t* misc = p_sm + 2 * TC_P_BYTES;                           // barriers, tmem base, reduction scratch
     Barriers* bars = reinterpret_cast<Barriers*>(misc);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(misc + 256);
-    float* red = reinterpret_cast<float*>(misc + 320);               // [2 parity][4 warps][16] + [4][16] sums
+    float* red = reinterpret_cast<float*>(misc + 320);               // [2 parity][4 warps][16] of a tile
+    float* sums = reinterpret_cast<float*>(misc + 832);              // [2 parity][4 warps][16] of an item
+    float* tops = reinterpret_cast<float*>(misc + 1344);             // [2 parity][16]: the maximum that they refer to
     float* part_sm = reinterpret_cast<float*>(k_sm);                 // clusters: [heads][128 d] of this split, once its last tile is done with
-    float* lse_sm = reinterpret_cast<float*>(misc + 1152);           // clusters: [heads]
+    float* lse_sm = reinterpret_cast<float*>(misc + 1472);           // clusters: [heads]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = p.nq / p.nkv;
@@ -239,9 +242,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
     launch_next();
     Items w{nullptr, nullptr, p.num_items};
     if constexpr (MODE == COUNTED) {
-        int* before = reinterpret_cast<int*>(misc + 1216);           // [num_seqs + 1]
-        int* lens = reinterpret_cast<int*>(misc + 2048);             // [num_seqs]
-        static_assert(1216 + 4 * (TC_COUNTED + 1) <= 2048 && 2048 + 4 * TC_COUNTED <= 3072, "");
+        int* before = reinterpret_cast<int*>(misc + 1536);           // [num_seqs + 1]
+        int* lens = reinterpret_cast<int*>(misc + 2432);             // [num_seqs]
+        static_assert(1536 + 4 * (TC_COUNTED + 1) <= 2432 && 2432 + 4 * TC_COUNTED <= 3328, "");
         if (warp == 0) {
             int total = 0;
             for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
@@ -343,10 +346,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
         const int sw = warp - 2;                       // 0..3 index for the reduction scratch
         uint32_t t = 0;
         T* const out = reinterpret_cast<T*>(p.o);
-        // An item's last products and its output come behind the next item's first weights: the tensor core's latency, and the sums' way through shared
-        // memory, pass beside them (one item after the other / now, us, ragged, 32 / 8 heads: 200 sequences of up to 40 tokens 24.0 / 20.3, 256 of
-        // up to 130 32.9 / 27.3, 128 of up to 300 25.2 / 22.7, 256 of up to 600 58.8 / 57.5, 256 x 4096 618 both)
-        float m_run[G], l_part[G], acc[G], alpha_prev[G], m_done[G], l_done[G];
+        // BEHIND: an item's last products and its output come behind the next item's first weights: the tensor core's latency, and the sums' way
+        // through shared memory, pass beside them (one item after the other / now, us, ragged, 32 / 8 heads: 200 sequences of up to 40 tokens
+        // 24.0 / 20.1, 128 of up to 300 24.9 / 22.2, 64 of up to 1000 37.2 / 35.2, 256 x 4096 618 both).  Not above eight heads a group, whose state
+        // does not fit the registers twice (255 and spills in every tile's loop; behind the next item / before it, us, 256 ragged sequences of up to
+        // 2000 tokens, 32 / 2 heads 104.8 / 91.7, 16 / 1 heads 73.7 / 66.0, 210 of up to 4000 79.8 / 71.3, 256 of up to 130 13.0 / 12.3).
+        float m_run[G], l_part[G], acc[G], alpha_prev[G];
 #pragma unroll
         for (int h = 0; h < G; h++) acc[h] = alpha_prev[h] = 0.f;
         auto fold_o = [&](uint32_t tt) {                // acc = acc * alpha(tt) + O_tile(tt)
@@ -361,18 +366,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
 #pragma unroll
             for (int h = 0; h < G; h++) acc[h] = acc[h] * alpha_prev[h] + __uint_as_float(r[h]);
         };
-        // l = sum over the 128 token-threads, out[h][d=row] = acc / l
-        auto finish = [&](const Item& it) {
-            float* rp = red + 128;                                             // [4 warps][16] scratch for the sums
-            float lsum[G];
+        // An item's sums, and the maximum that they refer to, wait for finish() in one of two places of shared memory.  A barrier of the four warps lies
+        // between the two (that of the next item's first tile, or its own), and one behind finish() before the place's next use.
+        auto leave = [&](int n) {
 #pragma unroll
-            for (int h = 0; h < G; h++) lsum[h] = warp_sum(l_done[h]);
-            // (a barrier lies between the previous item's reads of rp and this: that of the next item's first tile)
-            if (lane == 0) {
-#pragma unroll
-                for (int h = 0; h < G; h++) rp[sw * 16 + h] = lsum[h];
+            for (int h = 0; h < G; h++) {
+                const float l = warp_sum(l_part[h]);
+                if (lane == 0) sums[(n & 1) * 64 + sw * 16 + h] = l;
+                if (row == 0) tops[(n & 1) * 16 + h] = m_run[h];
             }
-            named_bar_sync(1, 128);
+        };
+        // l = sum over the 128 token-threads, out[h][d=row] = acc / l
+        auto finish = [&](const Place& it, int n) {
+            const float* rp = sums + (n & 1) * 64;
 #pragma unroll
             for (int h = 0; h < G; h++) {
                 if (h < g) {
@@ -383,11 +389,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
                         out[((int64_t)it.seq * p.nq + head) * TC_D + row] = Traits<T>::from_f(val);
                     } else if constexpr (MODE == CLUSTERED) {
                         part_sm[h * TC_D + row] = val;
-                        if (row == 0) lse_sm[h] = log2f(L) + m_done[h];
+                        if (row == 0) lse_sm[h] = log2f(L) + tops[(n & 1) * 16 + h];
                     } else {
                         const int64_t pi = ((int64_t)it.seq * p.nq + head) * p.num_splits + it.split;
                         p.part_o[pi * TC_D + row] = val;
-                        if (row == 0) p.part_lse[pi] = log2f(L) + m_done[h];
+                        if (row == 0) p.part_lse[pi] = log2f(L) + tops[(n & 1) * 16 + h];
                     }
                 }
             }
@@ -397,11 +403,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
                 if (get_item<MODE>(p, w, idx, it)) return true;
             return false;
         };
-        constexpr bool LONE = MODE == CLUSTERED;        // one item or none: nothing to come behind
-        Item it, next, done;
-        int idx = blockIdx.x;
-        bool more = seek(idx, it), any = false;
-        while (more) {
+        constexpr bool LONE = MODE == CLUSTERED, BEHIND = !LONE && G <= 8;      // LONE: one item or none
+        Item it, next;
+        Place done;
+        int idx = blockIdx.x, n = 0;                    // n: items of this CTA
+        for (bool more = seek(idx, it); more; n++) {
 #pragma unroll
             for (int h = 0; h < G; h++) { m_run[h] = -INFINITY; l_part[h] = 0.f; }
             for (int j = 0; j < it.ntiles; j++, t++) {
@@ -449,26 +455,30 @@ __global__ void __launch_bounds__(TC_THREADS, 1) paged_attn_tc_kernel(const __gr
                 }
                 fence_proxy_async();
                 mbar_arrive(smem_u32(&bars->p_full[b]));
-                if (!LONE && j == 0) { idx += gridDim.x; more = seek(idx, next); }
-                if (t > 0) fold_o(t - 1);
-                if (!LONE && j == 0) {
-                    if (any) finish(done);
+                if (BEHIND && j == 0) { idx += gridDim.x; more = seek(idx, next); }
+                if (BEHIND ? t > 0 : j > 0) fold_o(t - 1);
+                if (j == 0) {
+                    if (BEHIND && n > 0) finish(done, n - 1);
 #pragma unroll
                     for (int h = 0; h < G; h++) acc[h] = 0.f;
                 }
 #pragma unroll
                 for (int h = 0; h < G; h++) alpha_prev[h] = x[h];
             }
-            any = true;
-            done = it;
-            if (LONE) more = false; else it = next;
-#pragma unroll
-            for (int h = 0; h < G; h++) { m_done[h] = m_run[h]; l_done[h] = l_part[h]; }
+            leave(n);
+            done = Place{it.seq, it.kvh, it.split};
+            if (BEHIND) it = next;
+            else {
+                fold_o(t - 1);
+                named_bar_sync(1, 128);
+                finish(done, n);
+                idx += gridDim.x; more = !LONE && seek(idx, it);
+            }
         }
-        if (any) {
+        if (BEHIND && n > 0) {
             fold_o(t - 1);
-            if (!LONE) named_bar_sync(1, 128);          // (no next item: the sums of the one before may still be read)
-            finish(done);
+            named_bar_sync(1, 128);
+            finish(done, n - 1);
         }
     }
 

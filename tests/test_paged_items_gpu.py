@@ -34,3 +34,9 @@ def test_items_behind_one_another(dtype, H, G, B, sbs):
         k, v = (c[table[i, :blocks[i]].long(), 0].transpose(1, 2).flatten(0, 1)[:n].double().repeat_interleave(H // G, 1) for c in (kc, vc))
         w = torch.softmax(torch.einsum("hd,nhd->hn", q[i].double(), k) * 128 ** -0.5, dim=1)
         assert rel(out[i], torch.einsum("hn,nhd->hd", w, v).flatten()) < UNIT[dtype], (i, n)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("H,G,B,sbs", [(9, 1, 260, 0), (24, 2, 60, 128), (32, 2, 230, 256), (11, 1, 3, 128)])
+def test_wide_groups_one_item_after_the_other(dtype, H, G, B, sbs):
+    test_items_behind_one_another(dtype, H, G, B, sbs)
