@@ -1,0 +1,75 @@
+"""CPU: the numbering of query blocks that persistent prefill CTAs search (pt_block, csrc/prefill_attn_tc_kernel.cuh), in Python as the kernel does it, against a
+plain enumeration: blocks of the highest number first, the sequences of a number in order."""
+import pytest
+import torch
+
+WARP, WIDE = 32, 128
+
+
+class Search:
+    """pt_block with its cursor; `reads`: lengths of sequences past the warp's own 32 that were read."""
+
+    def __init__(self, blocks, max_blocks):
+        self.blocks, self.max_blocks, self.reads = [min(b, max_blocks) for b in blocks], max_blocks, 0
+        self.total = sum(self.blocks)
+        self.block = self.first = self.count = self.s0 = self.before = 0
+
+    def _from(self, b):
+        self.reads += max(0, len(self.blocks) - WARP)
+        return sum(max(n - b, 0) for n in self.blocks)
+
+    def __call__(self, rank):
+        if rank < self.first or rank >= self.first + self.count:
+            lo, hi, from_lo, from_hi = 0, self.max_blocks, self.total, 0
+            while hi - lo > 1:
+                mid = (lo + hi) // 2
+                n = self._from(mid)
+                if n > rank:
+                    lo, from_lo = mid, n
+                else:
+                    hi, from_hi = mid, n
+            self.block, self.first, self.count, self.s0, self.before = lo, from_hi, from_lo - from_hi, 0, 0
+        elif rank < self.first + self.before:
+            self.s0 = self.before = 0
+        r = rank - self.first
+        while self.s0 < len(self.blocks):
+            n = self.before
+            for s in range(self.s0, self.s0 + WIDE):
+                self.reads += WARP <= s < len(self.blocks)
+                if s < len(self.blocks) and self.blocks[s] > self.block:
+                    if n == r:
+                        return s, self.block
+                    n += 1
+            self.before = n
+            self.s0 += WIDE
+        raise AssertionError("a rank without a sequence")
+
+
+def enumeration(blocks, max_blocks):
+    return [(s, b) for b in reversed(range(max_blocks)) for s, n in enumerate(blocks) if n > b]
+
+
+def _blocks(kind, n):
+    g = torch.Generator().manual_seed(n)
+    if kind == "one long":
+        return [37 if s == n // 2 else 1 for s in range(n)]
+    if kind == "empty ones":
+        return [s % 3 for s in range(n)]
+    return (torch.rand(n, generator=g) * (1 if kind == "single" else 12)).ceil().int().tolist()
+
+
+@pytest.mark.parametrize("kind", ["single", "spread", "one long", "empty ones"])
+@pytest.mark.parametrize("n", [1, 31, 33, 128, 129, 300, 1000])
+@pytest.mark.parametrize("heads,by_head", [(1, True), (8, True), (8, False)])
+def test_every_cta_finds_its_blocks(kind, n, heads, by_head):
+    blocks = _blocks(kind, n)
+    most = max(1, max(blocks)) + 1                           # (the caller's longest may be longer than any)
+    order = enumeration(blocks, most)
+    grid = [(h, r) for r in range(len(order)) for h in range(heads)] if by_head else [(h, r) for h in range(heads) for r in range(len(order))]
+    for cta in (0, 1, 147):                                  # ranks of a CTA among 148 that take the grid's next in turn
+        search = Search(blocks, most)
+        mine = grid[cta::148]
+        for _, rank in mine:
+            assert search(rank) == order[rank]
+        if kind == "single" and heads == 8 and by_head and n > WARP:      # the lengths are read about once a CTA, not several times an item
+            assert search.reads <= 2 * (n + WIDE) + WIDE * len(mine)

@@ -79,3 +79,30 @@ def test_sequences_that_share_rows_and_a_longest_below():
     prefill_attention(q, k, v, out, None, None, _state([600] * 12, [0] * 12, 300))
     ref = _causal(q, k.repeat_interleave(4, 1), v.repeat_interleave(4, 1), 0)
     assert rel(out[:512], ref[:512]) < UNIT[torch.float16] and bool((out[512:] == 7.0).all())
+
+
+# more sequences than a warp has lanes: several numbers of blocks, sequences without rows among them, one long one among short ones
+MANY = [tuple((37 * i) % 150 for i in range(300)), tuple(900 if i == 170 else 1 + i % 9 for i in range(333)), (70,) * 129]
+
+
+@pytest.mark.parametrize("H,G", [(8, 8), (8, 2), (8, 1)])
+@pytest.mark.parametrize("lens", MANY)
+def test_many_prompts(H, G, lens):
+    from swiftllm_b200.worker.kernels.prefill_attn import prefill_attention
+    T = sum(lens)
+    q, k, v = _packed(torch.float16, H, G, T)
+    out = torch.full((T + 1, H, 128), 7.0, dtype=torch.float16, device=DEV)
+    prefill_attention(q, k, v, out[:-1], None, None, _state(lens))
+    at = 0
+    for n in lens:
+        s = slice(at, at + n)
+        at += n
+        if n:
+            assert rel(out[s], _causal(q[s], k[s].repeat_interleave(H // G, 1), v[s].repeat_interleave(H // G, 1), 0)) < UNIT[torch.float16], n
+    assert bool((out[-1] == 7.0).all())
+
+
+@pytest.mark.parametrize("lens", MANY)
+@pytest.mark.parametrize("splits", [1, 2])
+def test_many_portions(lens, splits):
+    test_portions(torch.bfloat16, 8, 2, tuple(max(n, 1) for n in lens), splits)
