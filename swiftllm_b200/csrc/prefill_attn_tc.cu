@@ -82,6 +82,7 @@ dim3 pt_grid(PtParams& p, int num_seqs, int max_len, int64_t num_tokens, int nsp
     many = items > (!paged && max_len <= 4 * PT_BK ? 2 * sms : sms);
     if (!many) return dim3((unsigned)each, (unsigned)heads, (unsigned)(num_seqs * nsplit));
     const unsigned slots = (unsigned)std::min<int64_t>(blocks(p.tiles) * nsplit, 65535);
+    p.takes = heads * slots > sms;
     return paged ? dim3(slots, (unsigned)heads) : dim3((unsigned)heads, slots);
 }
 

@@ -20,7 +20,11 @@
 // TMEM: S_A 0..79, S_B 80..159, P_A 160..199, P_B 200..239, O_A 256..383, O_B 384..511.
 //
 // Items come from the launch's grid, the longest first: a CTA that is about to finish one takes a CTA that has not been launched yet in its own
-// stead (cluster launch control), so that the SMs share the items as they get to them whatever the lengths are, and beside other kernels.
+// stead (cluster launch control), so that the SMs share the items as they get to them whatever the lengths are, and beside other kernels.  It asks
+// when the last PT_STAGES steps' keys are yet to load: asked at an item's beginning, the CTAs of the longest items, which begin first, had taken a
+// second one before the others ended (us, at the beginning / now: one prompt of 4096 tokens, 16 / 4 heads, 85 / 64; two of up to 2000, 32 / 8
+// heads, 51 / 41; three of up to 1000, 64 / 8 heads, 44 / 45.6; twelve of up to 1777, 16 / 4 heads, 72 both).  Portions in no more CTAs
+// than SMs do not ask: a request that finds none costs their steps 7 % (one of 1024 tokens at 5000, 24 / 4 heads, 93 us with and 87 without).
 // With a CTA per (sequence, head, 256 tokens) 4000 cycles passed before its first product, over a quarter of a prompt of 450 tokens, and a tile's rows
 // multiplied 104 keys on the average that they do not see, now 56 at four heads a tile.  Measured on B200, us: 4 x 4096 bf16, 32 / 8 heads 590 -> 550
 // (1020 TFLOP/s), twelve ragged fp16 prompts of up to 1777 tokens 202 -> 160, 64 of up to 100 tokens 72 -> 31, 512 tokens at 3584 47.2 -> 45.5.
@@ -68,6 +72,7 @@ struct PtParams {
     int nq, nkv;
     int pack_log2;                        // query heads of one key/value head that lie side by side in a tile
     int num_seqs, tiles, max_blocks;      // query blocks of one or two tiles; those of a sequence that count
+    int takes;                            // portions: more CTAs than SMs, whose items CTAs take over
 };
 // what the warps of a CTA have to know of an item; tile A takes part in nkt_a steps of 80 keys, B in nkt_b, from step j0 on
 struct PtItem {
@@ -172,6 +177,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
 
     // what warp 0 knows: the slot, how many there are, the lane's sequence (without MANY: the CTA's)
     constexpr bool BY_HEAD = MANY && !PAGED;
+    const bool takes = MANY && (!PAGED || p.takes);
     int head_block = BY_HEAD ? blockIdx.x : blockIdx.y, slot = BY_HEAD ? blockIdx.y : MANY ? blockIdx.x : gridDim.x - 1 - blockIdx.x, slots = 0;
     const int slot_step = BY_HEAD ? gridDim.y : gridDim.x;
     PtCursor cursor = {0, 0, 0, 0, 0};
@@ -261,10 +267,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
 
     if (warp < 4) {
         reg_dec<PT_REGS_FEW>();
-        // An item's steps of a ring; k0: the ring's steps before it.  PAGED (one whole warp per ring): step j = pages 5j .. 5j+4 of the
-        // sequence.  The block-table entries of the NEXT step are fetched before this step's stage is waited for; lane 0 arms the mbarrier with
-        // the bytes of the pages that exist, then lanes 0..4 issue the two (64 d x 16 token) boxes of one page each.
-        auto paged_producer = [&](const PtItem& it, int k0, const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty) {
+        const uint32_t next_bar = smem_u32(&bars->next), next_at = smem_u32(answer);
+        // An item's steps of a ring; k0: the ring's steps before it; ask_at: the step at which the grid's next CTA is asked for.  PAGED (one whole
+        // warp per ring): step j = pages 5j .. 5j+4 of the sequence.  The block-table entries of the NEXT step are fetched before this step's stage
+        // is waited for; lane 0 arms the mbarrier with the bytes of the pages that exist, then lanes 0..4 issue the two (64 d x 16 token) boxes of
+        // one page each.
+        auto paged_producer = [&](const PtItem& it, int k0, const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty, int ask_at) {
             const int32_t* bt = pg.block_table + (int64_t)it.seq_id * pg.max_blocks_per_seq;
             const int kvlen = it.pre + it.len, npages = (kvlen + PT_PAGE - 1) / PT_PAGE, nkt = it.steps();
             const int kvh = it.head0 / (p.nq / p.nkv);
@@ -278,6 +286,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 const int valid = min(PPS, npages - (it.j0 + j) * PPS);      // >= 1: step j exists because page 5j does
                 const uint32_t bar = smem_u32(&full[st]);
                 if (lane == 0) {
+                    if (MANY && j == ask_at) ask_next_cta(next_at, next_bar);
                     mbar_wait(smem_u32(&empty[st]), (((k0 + j) / PT_STAGES) & 1) ^ 1);
                     mbar_arrive_expect_tx(bar, (uint32_t)valid * PT_PAGE * PT_D * 2);
                 }
@@ -291,10 +300,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 }
             }
         };
-        auto packed_producer = [&](const PtItem& it, int k0, const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty) {
+        auto packed_producer = [&](const PtItem& it, int k0, const CUtensorMap& map, uint8_t* ring, uint64_t* full, uint64_t* empty, int ask_at) {
             const int nkt = it.steps(), kvh = it.head0 / (p.nq / p.nkv);
             for (int j = 0; lane == 0 && j < nkt; j++) {
                 const int st = (k0 + j) % PT_STAGES;
+                if (MANY && j == ask_at) ask_next_cta(next_at, next_bar);
                 mbar_wait(smem_u32(&empty[st]), (((k0 + j) / PT_STAGES) & 1) ^ 1);
                 const uint32_t bar = smem_u32(&full[st]), dst = smem_u32(ring + st * PT_KV_BYTES);
                 mbar_arrive_expect_tx(bar, PT_KV_BYTES);
@@ -305,8 +315,6 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
         };
         if (warp == 0) {
             // ======================================================= items; TMA producer: Q of an item, then its K tiles
-            const uint32_t next_bar = smem_u32(&bars->next), next_at = smem_u32(answer);
-            bool asked = false;
             for (int n = 0, k0 = 0, answers = 0;; n++) {
                 const PtItem it = n == 0 ? first : find();
                 if (lane == 0) {
@@ -316,22 +324,20 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                 }
                 __syncwarp();
                 if (!it.valid) break;
-                if (lane == 0) {
-                    if (MANY && !asked) ask_next_cta(next_at, next_bar);
-                    if (n > 0) {
-                        mbar_wait(smem_u32(&bars->q_empty), (n & 1) ^ 1);
-                        load_queries(it);
-                    }
+                if (lane == 0 && n > 0) {
+                    mbar_wait(smem_u32(&bars->q_empty), (n & 1) ^ 1);
+                    load_queries(it);
                 }
                 __syncwarp();
-                if constexpr (PAGED) paged_producer(it, k0, kmap, k_sm, bars->k_full, bars->k_empty);
-                else packed_producer(it, k0, kmap, k_sm, bars->k_full, bars->k_empty);
+                const int ask_at = takes && slot + slot_step >= slots ? max(it.steps() - PT_STAGES, 0) : -1;      // (behind the CTA's last slot alone)
+                if constexpr (PAGED) paged_producer(it, k0, kmap, k_sm, bars->k_full, bars->k_empty, ask_at);
+                else packed_producer(it, k0, kmap, k_sm, bars->k_full, bars->k_empty, ask_at);
                 k0 += it.steps();
                 slot += slot_step;
-                asked = slot < slots;                            // (more query blocks than the grid has: only where sequences share rows)
-                if (asked) continue;
+                if (slot < slots) continue;                      // (more query blocks than the grid has: only where sequences share rows)
                 slot = slots;
-                if constexpr (MANY) {
+                if (takes) {
+                    if (lane == 0 && it.steps() == 0) ask_next_cta(next_at, next_bar);
                     mbar_wait(next_bar, answers++ & 1);
                     int x, y;
                     if (next_cta(next_at, x, y)) { head_block = PAGED ? y : x; slot = PAGED ? x : y; }
@@ -342,8 +348,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
             for (int n = 0, k0 = 0;; n++) {
                 const PtItem it = take(n);
                 if (!it.valid) break;
-                if constexpr (PAGED) paged_producer(it, k0, vmap, v_sm, bars->v_full, bars->v_empty);
-                else packed_producer(it, k0, vmap, v_sm, bars->v_full, bars->v_empty);
+                if constexpr (PAGED) paged_producer(it, k0, vmap, v_sm, bars->v_full, bars->v_empty, -1);
+                else packed_producer(it, k0, vmap, v_sm, bars->v_full, bars->v_empty, -1);
                 k0 += it.steps();
             }
         } else {

@@ -8,6 +8,7 @@ import types
 import pytest
 import torch
 
+from prefill_grid import prefill_grid
 from tile_cases import DEV, TYPES, UNIT, ints, normal, rel, table
 
 pytestmark = pytest.mark.gpu
@@ -106,3 +107,37 @@ def test_many_prompts(H, G, lens):
 @pytest.mark.parametrize("splits", [1, 2])
 def test_many_portions(lens, splits):
     test_portions(torch.bfloat16, 8, 2, tuple(max(n, 1) for n in lens), splits)
+
+
+# more query blocks than the grid has, because sequences share rows: a CTA goes on by so many, and takes the grid's next only behind its last
+def _shared(n):
+    g = prefill_grid(64, 8, n, 700, 600, 1, False, torch.cuda.get_device_properties(0).multi_processor_count)
+    assert g.many and g.asks and n * -(-600 // g.tokens) > 2 * g.slots
+    return g
+
+
+def test_packed_prompts_that_share_rows_and_take_ctas():
+    from swiftllm_b200.worker.kernels.prefill_attn import prefill_attention
+    H, G, T, n = 64, 8, 600, 40
+    _shared(n)
+    q, k, v = _packed(torch.bfloat16, H, G, T)
+    out = torch.full((T, H, 128), 7.0, dtype=torch.bfloat16, device=DEV)
+    prefill_attention(q, k, v, out, None, None, _state([T] * n, [0] * n, 700))
+    assert rel(out, _causal(q, k.repeat_interleave(8, 1), v.repeat_interleave(8, 1), 0)) < UNIT[torch.bfloat16]
+
+
+@pytest.mark.parametrize("splits", [1, 3])
+def test_portions_that_share_rows_and_take_ctas(splits):
+    from swiftllm_b200 import _lib
+    H, G, T, n, pre, dtype = 64, 8, 600, 40, 333, torch.float16
+    _shared(n)
+    bt, nb = table([T + pre], 16, 3)
+    kc, vc = (normal(nb, 2, G, 16, 128, seed=i, dtype=dtype) for i in (1, 2))
+    q, out = normal(T, H, 128, seed=3, dtype=dtype), torch.full((T, H, 128), 7.0, dtype=dtype, device=DEV)
+    ws = torch.full((splits * T * H * 130,), float("nan"), device=DEV)
+    zeros, lens, prefix = ints([0] * n), ints([T] * n), ints([pre] * n)
+    _lib.check(_lib.lib().sllm_prefill_attention_paged_split(
+        q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), bt.data_ptr(), zeros.data_ptr(), zeros.data_ptr(), lens.data_ptr(), prefix.data_ptr(),
+        128 ** -0.5, n, 700, T, 1, 2, H, G, 16, 128, bt.shape[1], nb, H * 128, _lib.dtype_tag(dtype), _lib.stream(), splits, ws.data_ptr()), "portions")
+    k, v = (c[bt[0].long(), 1].transpose(1, 2).flatten(0, 1)[:T + pre].repeat_interleave(8, 1) for c in (kc, vc))
+    assert rel(out, _causal(q, k, v, pre)) < UNIT[dtype]
