@@ -65,6 +65,8 @@ struct PtBarriers {
     uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2], o_empty[2];      // [tile]
 };
 
+enum PtOrder { PT_AT_ONCE, PT_BY_SLOT, PT_BY_HEAD };      // portions whose CTAs all have an SM; others: grid (slots, heads) or (heads, slots)
+
 struct PtParams {
     void* o;
     const int32_t* start_locs; const int32_t* seq_lens;
@@ -72,7 +74,7 @@ struct PtParams {
     int nq, nkv;
     int pack_log2;                        // query heads of one key/value head that lie side by side in a tile
     int num_seqs, tiles, max_blocks;      // query blocks of one or two tiles; those of a sequence that count
-    int takes;                            // portions: more CTAs than SMs, whose items CTAs take over
+    int order;                            // of a MANY launch: a PtOrder
 };
 // what the warps of a CTA have to know of an item; tile A takes part in nkt_a steps of 80 keys, B in nkt_b, from step j0 on
 struct PtItem {
@@ -148,8 +150,8 @@ __device__ __forceinline__ int pt_block(const PtParams& p, int mine, int total, 
 // [half][80 rows][128 B] layout, so the product issuer and its descriptors are shared by both variants.  Page slots that a tail step does not
 // load keep what lay there: their scores are masked, and P . V stops before them.
 // MANY: more items than SMs.  grid: heads / pack and slots (all sequences' query blocks; a CTA takes every so many, if they are more than the grid
-// has).  The order of the grid is the order of the work: packed prompts (heads, slots), the longest items of all heads first; portions
-// (slots, heads), whose items differ little and whose keys may be more than L2 holds.  Else grid (query blocks from the last
+// has).  The order of the grid is the order of the work: (heads, slots), the longest items of all heads first, for packed prompts and for portions
+// of up to four items an SM; (slots, heads) for other portions, whose keys may be more than L2 holds.  Else grid (query blocks from the last
 // one, heads / pack, sequence * nsplit + split), a CTA for an item.
 template <typename T, bool PAGED, bool MANY>
 __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap qmap,
@@ -176,10 +178,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     const int tile_tokens = PT_BQ >> p.pack_log2;
 
     // what warp 0 knows: the slot, how many there are, the lane's sequence (without MANY: the CTA's)
-    constexpr bool BY_HEAD = MANY && !PAGED;
-    const bool takes = MANY && (!PAGED || p.takes);
-    int head_block = BY_HEAD ? blockIdx.x : blockIdx.y, slot = BY_HEAD ? blockIdx.y : MANY ? blockIdx.x : gridDim.x - 1 - blockIdx.x, slots = 0;
-    const int slot_step = BY_HEAD ? gridDim.y : gridDim.x;
+    const bool takes = MANY && (!PAGED || p.order != PT_AT_ONCE), by_head = MANY && (!PAGED || p.order == PT_BY_HEAD);
+    int head_block = by_head ? blockIdx.x : blockIdx.y, slot = by_head ? blockIdx.y : MANY ? blockIdx.x : gridDim.x - 1 - blockIdx.x, slots = 0;
+    const int slot_step = by_head ? gridDim.y : gridDim.x;
     PtCursor cursor = {0, 0, 0, 0, 0};
     int mine = lane, my_split = 0, my_blocks = 0, my_len = 0, my_start = 0, my_pre = 0, my_id = 0;
     if constexpr (!MANY) {
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
                     if (lane == 0 && it.steps() == 0) ask_next_cta(next_at, next_bar);
                     mbar_wait(next_bar, answers++ & 1);
                     int x, y;
-                    if (next_cta(next_at, x, y)) { head_block = PAGED ? y : x; slot = PAGED ? x : y; }
+                    if (next_cta(next_at, x, y)) { head_block = by_head ? x : y; slot = by_head ? y : x; }
                 }
             }
         } else if (warp == 2) {

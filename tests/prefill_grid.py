@@ -14,4 +14,4 @@ def prefill_grid(H, G, seqs, longest, rows, splits, paged, sms=148):
     many = heads * seqs * splits * up(longest, tokens) > (2 * sms if short else sms)
     slots = min(blocks(tiles) * splits, 65535)
     return types.SimpleNamespace(pack=pack, heads=heads, tiles=tiles, tokens=tokens, most=up(longest, 256) * 256 // tokens, many=many, slots=slots,
-                                 asks=many and (not paged or heads * slots > sms))
+                                 asks=many and (not paged or heads * slots > sms), by_head=many and (not paged or sms < heads * slots <= 4 * sms))

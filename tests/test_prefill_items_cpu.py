@@ -73,3 +73,14 @@ def test_every_cta_finds_its_blocks(kind, n, heads, by_head):
             assert search(rank) == order[rank]
         if kind == "single" and heads == 8 and by_head and n > WARP:      # the lengths are read about once a CTA, not several times an item
             assert search.reads <= 2 * (n + WIDE) + WIDE * len(mine)
+
+
+@pytest.mark.parametrize("H,G,lens", [(16, 16, (1024, 121, 754, 363)), (32, 32, (300, 35, 221, 106)), (24, 4, (1024, 121, 754, 363))])
+def test_the_last_items_are_the_shortest(H, G, lens):
+    """Portions of one to four items an SM, in the grid's order: what is left for the second round are no long items."""
+    from prefill_grid import prefill_grid
+    g = prefill_grid(H, G, len(lens), max(lens), sum(lens), 1, True)
+    order = enumeration([-(-n // g.tokens) for n in lens], g.most)
+    assert g.many and g.by_head and 148 < g.heads * g.slots <= 4 * 148
+    items = [b for _, b in order for _ in range(g.heads)]
+    assert max(items[148:]) <= min(items[:148])
