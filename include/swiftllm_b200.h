@@ -157,6 +157,9 @@ int sllm_prefill_attention_paged_split(const void* q, const void* k_cache, const
                                  int num_q_heads, int num_kv_heads, int block_size, int head_dim,
                                  int max_blocks_per_seq, int64_t num_blocks, int64_t q_row_stride, sllm_dtype_t dtype,
                                  sllm_stream_t stream, int num_splits, void* workspace);
+/* The most query blocks (x heads that do not lie side by side in one) of one or two 128-row tiles that the tcgen05 kernel makes of such a step
+ * for each key split: what a caller divides the SMs by.  0 for sizes that are none. */
+int64_t sllm_prefill_attention_blocks(int num_q_heads, int num_kv_heads, int num_prefill_seqs, int max_prefill_len, int64_t num_prefill_tokens, int tiles);
 
 /* ---- Block-table maintenance: swiftllm/worker/kernels/block_mgmt.py:26-46, :66-80, :106-127
  * block_table int32 [max_seqs, max_blocks_per_seq]; num_seq_allocated_blocks int32 [max_seqs];

@@ -54,6 +54,17 @@ bool pt_query_map(CUtensorMap* out, const void* ptr, uint64_t rows, int heads, i
 
 // Up to eight query heads of a key/value head lie side by side in a tile: rows of fewer tokens, so that a tile of 128 rows multiplies fewer keys that most
 // of its rows do not see, and short prompts fill their tiles.
+static int pt_pack_log2(int nq, int nkv) {
+    int n = 0;
+    while (n < 3 && (nq / nkv) % (2 << n) == 0) n++;
+    return n;
+}
+// Query blocks of one or two tiles of all sequences, for one of the heads / pack: every sequence ends in a block of its own
+static int64_t pt_blocks_of_all(int pack_log2, int num_seqs, int max_len, int64_t num_tokens, int tiles) {
+    const int tokens = tiles * PT_BQ >> pack_log2;
+    return std::min<int64_t>((int64_t)num_seqs * cdiv(max_len, tokens), num_tokens / tokens + num_seqs);
+}
+
 // Blocks of one tile where that leaves no SM two of them (a step of one tile ends sooner: a prompt of 300 tokens, 32 / 8 heads, 9.0 us, with two tiles 11.3),
 // or few of them that are short (20 prompts of up to 200 tokens, 16 / 4 heads: 14.4, with two 16.6; at 64 / 8 heads, seven an SM, 32.9 and 31.9).
 dim3 pt_grid(PtParams& p, int num_seqs, int max_len, int64_t num_tokens, int nsplit, bool paged, bool& many) {
@@ -64,15 +75,11 @@ dim3 pt_grid(PtParams& p, int num_seqs, int max_len, int64_t num_tokens, int nsp
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device());
         __atomic_store_n(&sm_count[dev], sms, __ATOMIC_RELAXED);
     }
-    p.pack_log2 = 0;
-    while (p.pack_log2 < 3 && (p.nq / p.nkv) % (2 << p.pack_log2) == 0) p.pack_log2++;
+    p.pack_log2 = pt_pack_log2(p.nq, p.nkv);
     p.num_seqs = num_seqs;
     const int64_t heads = p.nq >> p.pack_log2;
     const int whole = cdiv(max_len, 2 * PT_BQ) * 2 * PT_BQ;    // rows up to the whole 256 behind the longest that the caller states
-    auto blocks = [&](int tiles) {                             // of all sequences: every sequence ends in a block of its own
-        const int tokens = tiles * PT_BQ >> p.pack_log2;
-        return std::min<int64_t>((int64_t)num_seqs * cdiv(max_len, tokens), num_tokens / tokens + num_seqs);
-    };
+    auto blocks = [&](int tiles) { return pt_blocks_of_all(p.pack_log2, num_seqs, max_len, num_tokens, tiles); };
     const int64_t ones = heads * nsplit * blocks(1);
     p.tiles = ones <= sms || (!paged && max_len <= 4 * PT_BK && 2 * ones <= 5 * sms) ? 1 : 2;
     const int tokens = p.tiles * PT_BQ >> p.pack_log2, each = cdiv(max_len, tokens);
@@ -118,3 +125,10 @@ int launch_prefill_tc(const void* q, const void* k, const void* v, void* o, cons
 }
 
 }  // namespace sllm
+
+extern "C" int64_t sllm_prefill_attention_blocks(int nq, int nkv, int num_prefill_seqs, int max_prefill_len, int64_t num_prefill_tokens, int tiles) {
+    using namespace sllm;
+    if (nkv <= 0 || nq <= 0 || nq % nkv != 0 || num_prefill_seqs <= 0 || max_prefill_len <= 0 || num_prefill_tokens < 0 || tiles < 1 || tiles > 2) return 0;
+    const int pack_log2 = pt_pack_log2(nq, nkv);
+    return (nq >> pack_log2) * pt_blocks_of_all(pack_log2, num_prefill_seqs, max_prefill_len, num_prefill_tokens, tiles);
+}

@@ -1,5 +1,7 @@
 """Reference: swiftllm/worker/kernels/prefill_attn.py (prefill_attention :102-139); also replaces the
 vllm_flash_attn.flash_attn_varlen_func call at swiftllm/worker/layers/transformer_layer.py:86-96."""
+import functools
+
 import torch
 
 from swiftllm_b200 import _lib
@@ -32,14 +34,36 @@ def prefill_attention(
 _SM_COUNT = {}
 
 
-def _key_splits(heads: int, longest: int, kv_len: int) -> int:
-    """CTAs that share a query block's keys: as many as keep one CTA (256 query rows of a head) per SM when the portions alone leave SMs
-    idle, each with at least eight steps of 80 keys (shorter ones do not pay for the merge)."""
+def _key_splits(heads: int, longest: int, kv_len: int, blocks=None) -> int:
+    """CTAs that share a query block's keys when the portions alone leave SMs idle: as many as find an SM at once, each with at least eight steps of 80
+    keys, or six where eight leave half of the SMs idle (shorter ones do not pay for the merge).  `blocks`: the launch's query blocks if they have
+    one tile, and two (None: a block for 256 rows of a head).  Measured on B200, us, splits counted by 256 rows of a head / by the blocks, in which
+    heads lie side by side: 16 tokens at 5000, 64 / 8 heads, 35.2 / 17.8; four portions of up to 16 at 5000, 32 / 8 heads, 62.8 / 24.8; 300 at 3000,
+    32 / 8 heads, 36.3 / 30.6; 64 at 5000, 16 / 4 heads, 19.2 / 17.8; 512 at 3584, 32 / 8 heads, 43.8 both."""
     dev = torch.cuda.current_device()
     if dev not in _SM_COUNT:
         _SM_COUNT[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
-    blocks = heads * -(-longest // 256)
-    return max(1, min(_SM_COUNT[dev] // max(1, blocks), kv_len // 640, 16))
+    return _splits(_SM_COUNT[dev], kv_len, *(blocks or (heads * -(-longest // 256),) * 2), blocks is not None)
+
+
+@functools.lru_cache(maxsize=1024)
+def _splits(sms: int, kv_len: int, ones: int, twos: int, fewer_steps: bool) -> int:
+    most = kv_len // 640
+    if fewer_steps and most > 1 and ones * most <= sms // 2:
+        most = kv_len // 480
+    one, two = (min(sms // max(1, b), most, 16) for b in (ones, twos))
+    if two <= max(1, one):
+        return max(1, one)
+    # Blocks of two tiles leave room for more splits.  In tenths of a microsecond: a step takes them 12 and blocks of one tile 9; splits and their merge
+    # come to 95 and 50 (64 / 8 heads, 128 tokens at 5000: two splits of one tile 38.3 us, four of two 33.6; 16 / 4 heads, 512 at 2000: 23.8 and 26.2)
+    steps, of_one = -(-kv_len // 80), 9 if one else 12                 # (more blocks of one tile than SMs: a launch without splits has two)
+    alone = of_one * -(-steps // max(1, one)) + (50 if one > 1 else 0)
+    return two if 12 * -(-steps // two) + 95 < alone else max(1, one)
+
+
+@functools.lru_cache(maxsize=1024)
+def _blocks(nq: int, nkv: int, seqs: int, longest: int, rows: int):
+    return tuple(_lib.lib().sllm_prefill_attention_blocks(nq, nkv, seqs, longest, rows, tiles) for tiles in (1, 2))
 
 
 def prefill_attention_paged(
@@ -66,7 +90,8 @@ def prefill_attention_paged(
     if infer_state.num_prefill_seqs == 0:
         return
     num_blocks, num_layers, nkv, bs, _ = k_cache.shape
-    nsplit = _key_splits(nq * infer_state.num_prefill_seqs, infer_state.max_prefill_len, getattr(infer_state, "max_prefill_kv_len", 0)) \
+    n, longest = infer_state.num_prefill_seqs, infer_state.max_prefill_len
+    nsplit = _key_splits(nq * n, longest, getattr(infer_state, "max_prefill_kv_len", 0), _blocks(nq, nkv, n, longest, Tp)) \
         if D == 128 and bs == 16 else 1
     ws = torch.empty((nsplit * Tp * nq * (D + 2),), dtype=torch.float32, device=q.device) if nsplit > 1 else None
     _lib.check(_lib.lib().sllm_prefill_attention_paged_split(

@@ -84,3 +84,31 @@ def test_the_last_items_are_the_shortest(H, G, lens):
     assert g.many and g.by_head and 148 < g.heads * g.slots <= 4 * 148
     items = [b for _, b in order for _ in range(g.heads)]
     assert max(items[148:]) <= min(items[:148])
+
+
+SHAPES = [(64, 8, 1, 16, 16), (64, 8, 1, 64, 64), (32, 8, 4, 16, 45), (32, 8, 1, 300, 300), (32, 8, 1, 512, 512), (16, 4, 1, 64, 64), (24, 4, 4, 64, 150),
+          (16, 16, 1, 300, 300), (16, 1, 3, 40, 41), (64, 8, 1, 700, 700), (32, 8, 32, 500, 8000), (6, 2, 2, 1, 2), (48, 8, 7, 333, 334)]
+
+
+@pytest.mark.parametrize("H,G,n,longest,rows", SHAPES)
+def test_blocks_are_counted_as_the_launch_makes_them(H, G, n, longest, rows):
+    from prefill_grid import prefill_grid
+    from swiftllm_b200.worker.kernels.prefill_attn import _blocks
+    for tiles, got in zip((1, 2), _blocks(H, G, n, longest, rows)):
+        g = prefill_grid(H, G, n, longest, rows, 1, True, sms=1 << 30 if tiles == 1 else 0)
+        assert g.tiles == tiles and got == g.heads * min(n * -(-longest // g.tokens), rows // g.tokens + n)
+
+
+@pytest.mark.parametrize("H,G,n,longest,rows", SHAPES)
+@pytest.mark.parametrize("kv_len", [0, 479, 700, 1016, 3300, 5064, 30000])
+def test_key_splits_fill_the_sms_and_no_more(H, G, n, longest, rows, kv_len):
+    from prefill_grid import prefill_grid
+    from swiftllm_b200.worker.kernels.prefill_attn import _blocks, _splits
+    sms = 148
+    splits = _splits(sms, kv_len, *_blocks(H, G, n, longest, rows), True)
+    g = prefill_grid(H, G, n, longest, rows, splits, True, sms)
+    assert 1 <= splits <= 16 and (splits == 1 or kv_len // splits >= 480)
+    if splits > 1:
+        assert g.heads * g.slots <= sms or g.heads * n * splits * -(-longest // g.tokens) <= sms
+    if splits < min(16, kv_len // 640):                      # keys for more CTAs, but no SMs: at least half of them have one
+        assert 2 * splits * _blocks(H, G, n, longest, rows)[0] > sms
