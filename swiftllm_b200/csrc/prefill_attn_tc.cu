@@ -76,7 +76,7 @@ dim3 pt_grid(PtParams& p, int num_seqs, int max_len, int64_t num_tokens, int nsp
         __atomic_store_n(&sm_count[dev], sms, __ATOMIC_RELAXED);
     }
     p.pack_log2 = pt_pack_log2(p.nq, p.nkv);
-    p.num_seqs = num_seqs;
+    p.num_seqs = num_seqs; p.order = PT_AT_ONCE;
     const int64_t heads = p.nq >> p.pack_log2;
     const int whole = cdiv(max_len, 2 * PT_BQ) * 2 * PT_BQ;    // rows up to the whole 256 behind the longest that the caller states
     auto blocks = [&](int tiles) { return pt_blocks_of_all(p.pack_log2, num_seqs, max_len, num_tokens, tiles); };
@@ -84,9 +84,11 @@ dim3 pt_grid(PtParams& p, int num_seqs, int max_len, int64_t num_tokens, int nsp
     p.tiles = ones <= sms || (!paged && max_len <= 4 * PT_BK && 2 * ones <= 5 * sms) ? 1 : 2;
     const int tokens = p.tiles * PT_BQ >> p.pack_log2, each = cdiv(max_len, tokens);
     p.max_blocks = whole / tokens;
-    // a few short items over: their CTAs end sooner than the grid's next one is asked for (152 of up to four steps: 13.4 us, launched 11)
-    const int64_t items = heads * num_seqs * nsplit * each;
-    many = items > (!paged && max_len <= 4 * PT_BK ? 2 * sms : sms);
+    // a few short items over: their CTAs end sooner than the grid's next one is asked for (152 of up to four steps: 13.4 us, launched 11).  Portions
+    // whose blocks all find an SM: a CTA for each, which need not search, beside a few without a block (us, searched / launched: six of up to
+    // 400 tokens at 200, 16 / 4 heads, 17.3 / 16.3; four of up to 300 at 500, 16 / 16 heads, 15.9 / 14.9; two of up to 100 at 4000, 24 / 4 heads, 23.1 / 24.0)
+    const bool launched = paged ? heads * nsplit * blocks(p.tiles) <= sms : max_len <= 4 * PT_BK;
+    many = heads * num_seqs * nsplit * each > (!launched ? sms : paged ? 3 * sms / 2 : 2 * sms);
     if (!many) return dim3((unsigned)each, (unsigned)heads, (unsigned)(num_seqs * nsplit));
     const unsigned slots = (unsigned)std::min<int64_t>(blocks(p.tiles) * nsplit, 65535);
     // Portions of a few items an SM end on the shortest items of all heads, not on the last head's long ones.  With more, the items of a head together:
