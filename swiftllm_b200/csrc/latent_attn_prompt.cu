@@ -193,10 +193,13 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
                     if (group >= 0) tma_load_4d(smem_u32(smem + st * LP_STAGE) + lane * 2 * LP_GROUP, &map, bar, 0, 0, 0, group);
                     if (!ragged) continue;
                     mbar_wait(bar, ragged_done++ & 1);    // rows that are not seen become zero
-                    for (int row = 0; row < LP_KEYS; row++) {
+                    // four rows at a time, eight lanes to a row's 128 bytes of each chunk (a row at a time 200 cycles each: up to 7 us an item, which
+                    // for short prompts is most of it; us, 64 of up to 60 tokens, 16 heads, 73.7 / 52.0, 200 of up to 100, 4 heads, 91.7 / 65.0)
+                    for (int row = lane >> 3; row < LP_KEYS; row += 4) {
                         if (base + row >= it.see_lo && base + row <= it.see_hi) continue;
-                        uint8_t* at = smem + st * LP_STAGE + (row >> 3) * LP_GROUP + (row & 7) * 128;
-                        for (int i = lane; i < LP_CHUNKS * 8; i += 32) *reinterpret_cast<uint4*>(at + (i >> 3) * 1024 + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+                        uint8_t* at = smem + st * LP_STAGE + (row >> 3) * LP_GROUP + (row & 7) * 128 + (lane & 7) * 16;
+#pragma unroll
+                        for (int c = 0; c < LP_CHUNKS; c++) *reinterpret_cast<uint4*>(at + c * 1024) = make_uint4(0, 0, 0, 0);
                     }
                     fence_proxy_async();
                     __syncwarp();
