@@ -542,10 +542,12 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
     if (warp == 1) tmem_dealloc<512>(tmem);
 }
 
-// Where every SM has at least three CTAs' rows to do.  A first item takes 5 us longer to start than in latent_attn_tc.cu, which few short ones do not make up
-// for (16 heads, two prompts of 1658 tokens in all: 67.6 us and 63.3; one of 2048: 136 and 161).
+// Where every SM has at least two and a half CTAs' rows to do (us, latent_attn_tc.cu / here, no window: 16 heads, one prompt of 1539 tokens 97 / 70, 40 of 38
+// 38 / 29; 4 heads, two of 3078 163 / 142; 64 heads, two of 192 at 1500 175 / 125).  With fewer, few long segments end late here, where a CTA has taken its
+// second before its first is done (4 heads, two of 1894, 240 CTAs, 71 / 80, two of 2486, 312 CTAs, 108 / 117; 16 heads, two of 473 30 / 32), though
+// others gain (16 heads, 8 of 118 27 / 21).
 bool latent_prompt_takes(const LatentTc& p, dim3 grid, int num_sms) {
-    return (int64_t)grid.x * grid.y >= 3ll * num_sms && p.r == LP_R && p.dr == LP_DR && p.block_size % 16 == 0 && p.nsplit == 1 && p.q_vec && get_tensor_map_encoder() != nullptr;
+    return 2ll * grid.x * grid.y >= 5ll * num_sms && p.r == LP_R && p.dr == LP_DR && p.block_size % 16 == 0 && p.nsplit == 1 && p.q_vec && get_tensor_map_encoder() != nullptr;
 }
 
 int launch_latent_attn_prompt(const LatentTc& p, dim3 grid, sllm_dtype_t dtype, cudaStream_t stream) {
