@@ -545,9 +545,10 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
 // Where every SM has at least two and a half CTAs' rows to do (us, latent_attn_tc.cu / here, no window: 16 heads, one prompt of 1539 tokens 97 / 70, 40 of 38
 // 38 / 29; 4 heads, two of 3078 163 / 142; 64 heads, two of 192 at 1500 175 / 125).  With fewer, few long segments end late here, where a CTA has taken its
 // second before its first is done (4 heads, two of 1894, 240 CTAs, 71 / 80, two of 2486, 312 CTAs, 108 / 117; 16 heads, two of 473 30 / 32), though
-// others gain (16 heads, 8 of 118 27 / 21).
+// others gain (16 heads, 8 of 118 27 / 21).  Query views in which heads or tokens share their entries are left to latent_attn_tc.cu's plain loads.
 bool latent_prompt_takes(const LatentTc& p, dim3 grid, int num_sms) {
-    return 2ll * grid.x * grid.y >= 5ll * num_sms && p.r == LP_R && p.dr == LP_DR && p.block_size % 16 == 0 && p.nsplit == 1 && p.q_vec && get_tensor_map_encoder() != nullptr;
+    return 2ll * grid.x * grid.y >= 5ll * num_sms && p.r == LP_R && p.dr == LP_DR && p.block_size % 16 == 0 && p.nsplit == 1 && p.q_vec &&
+           p.ql_st > 0 && p.ql_sh > 0 && get_tensor_map_encoder() != nullptr;
 }
 
 int launch_latent_attn_prompt(const LatentTc& p, dim3 grid, sllm_dtype_t dtype, cudaStream_t stream) {
@@ -565,8 +566,7 @@ int launch_latent_attn_prompt(const LatentTc& p, dim3 grid, sllm_dtype_t dtype, 
     const cuuint64_t qdims[4] = {64, (cuuint64_t)p.H, (cuuint64_t)p.num_tokens, LP_R / 64};
     const cuuint64_t qstrides[3] = {(cuuint64_t)p.ql_sh * 2, (cuuint64_t)p.ql_st * 2, 128};
     const cuuint32_t qbox[4] = {64, 1u << p.hp_log2, (cuuint32_t)p.qt, LP_R / 64};
-    SLLM_REQUIRE(encode(&map, p.cache, dims, strides, box) == CUDA_SUCCESS && encode(&qmap, p.q_lat, qdims, qstrides, qbox) == CUDA_SUCCESS,
-                 "latent_attention: cuTensorMapEncodeTiled failed");
+    if (encode(&map, p.cache, dims, strides, box) != CUDA_SUCCESS || encode(&qmap, p.q_lat, qdims, qstrides, qbox) != CUDA_SUCCESS) return -1;
     SLLM_DISPATCH_DTYPE(dtype, {
         static unsigned long long configured = 0;
         if (first_use_on_this_device(configured)) {

@@ -576,7 +576,8 @@ int launch_latent_attn_tc(LatentTc& p, bool portions, sllm_dtype_t dtype, cudaSt
     const int64_t share = portions ? num_sms / ((int64_t)grid.x * grid.y * grid.z) : 1;
     if (share > 1) grid.z *= (unsigned)(share > p.qt ? p.qt : share);
     const int full = p.r == 512 && p.dr == 64, rows = grid.z > (unsigned)p.nsplit ? LT_SHARED : !portions && p.hp_log2 <= 4 ? LT_SINGLES : LT_PROMPTS;
-    if (portions && rows == LT_PROMPTS && latent_prompt_takes(p, grid, num_sms)) return launch_latent_attn_prompt(p, grid, dtype, stream);
+    if (portions && rows == LT_PROMPTS && latent_prompt_takes(p, grid, num_sms))
+        if (const int rc = launch_latent_attn_prompt(p, grid, dtype, stream); rc >= 0) return rc;
     SLLM_DISPATCH_DTYPE(dtype, {
         static unsigned long long configured = 0;
         void (*kernels[2][3])(LatentTc) = {

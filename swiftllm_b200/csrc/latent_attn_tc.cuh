@@ -29,7 +29,7 @@ bool latent_tc_supported(int r, int dr);
 // nsplit > 1 leaves [T, H, nsplit, r + 2] in `partial` for latent_attn_combine_kernel.
 int launch_latent_attn_tc(LatentTc& p, bool portions, sllm_dtype_t dtype, cudaStream_t stream);
 
-// latent_attn_prompt.cu: prompt rows of 512 + 64 entries in one key split, on launch_latent_attn_tc's grid
+// latent_attn_prompt.cu: prompt rows of 512 + 64 entries in one key split, on launch_latent_attn_tc's grid; -1: a view that has no tensor map
 bool latent_prompt_takes(const LatentTc& p, dim3 grid, int num_sms);
 int launch_latent_attn_prompt(const LatentTc& p, dim3 grid, sllm_dtype_t dtype, cudaStream_t stream);
 

@@ -49,7 +49,7 @@ def test_views_that_are_not_aligned():
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("H,window,portions", [(16, 0, [(1800, 5), (7, 90)]), (64, 33, [(200, 5), (300, 90)])])
 def test_keys_reach_only_rows_that_see_them(value, H, window, portions):
-    # every CTA from the odd key on meets it; more of them than a CTA keeps marks of
+    # every CTA from the odd key on meets it (64 heads: a token a CTA, whose keys are all its own)
     c = latent_case(torch.bfloat16, portions, [], H, 512, 64, 64, window, sink=True)
     spots, clean, cache, at = [41, 42, 66, 120, 130], latent_run(c), c.cache.clone(), 0
     for pos in spots:
@@ -60,3 +60,61 @@ def test_keys_reach_only_rows_that_see_them(value, H, window, portions):
     for pos in spots:
         sees[:q.shape[0]] |= (q >= pos) & ((q - pos < window) if window else True)
     assert torch.equal(got[~sees], clean[~sees]) and bool((~torch.isfinite(got[sees])).flatten(1).any(1).all())
+
+
+# 64 tokens a CTA whose runs end anywhere in it; two blocks of heads, the last one in part
+@pytest.mark.parametrize("H,window,portions", [(1, 0, [(33 + i % 31, (7 * i) % 90) for i in range(500)] + [(2500, 0), (2101, 33)]),
+                                               (1, 100, [(1, 4), (62, 0), (65, 128)] + [(4000, 900)] * 7 + [(500, 3)]), (72, 0, [(150, 20), (90, 0)]), (96, 70, [(233, 10)])])
+def test_one_head_and_more_than_64(H, window, portions):
+    c = latent_case(torch.bfloat16, portions, [], H, 512, 64, 64, window, sink=False, gated=True)
+    got, ref, at = latent_run(c), latent_exact(c), 0
+    for n, p in c.rows:
+        assert rel(got[at:at + n], ref[at:at + n]) < UNIT[torch.bfloat16], (n, p)
+        at += n
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("-inf")])
+def test_more_segments_than_a_cta_keeps_marks_of(value):
+    # 32 tokens a CTA, 16 segments of two, three CTAs or more in turn: the 32 marks are looked through in the middle of a CTA's work, and again
+    portions = [(2, (5 * i) % 130) for i in range(7200)]
+    c = latent_case(torch.bfloat16, portions, [], 2, 512, 64, 64, 0, sink=True)
+    clean, cache = latent_run(c), c.cache.clone()
+    first = torch.arange(len(portions), device=c.q.device)
+    bad = first % 3 != 1
+    pos = torch.tensor([p + 1 for _, p in portions], device=c.q.device)      # the second token's own key, which the first does not see
+    block = c.bt[first, pos // 16].long()
+    cache[block[bad], 1, pos[bad] % 16, 300] = value
+    got = latent_run(c, cache).unflatten(0, (-1, 2))
+    clean = clean.unflatten(0, (-1, 2))
+    assert torch.equal(got[:, 0], clean[:, 0]) and torch.equal(got[~bad], clean[~bad])
+    assert bool((~torch.isfinite(got[bad][:, 1])).flatten(1).any(1).all())
+
+
+@pytest.mark.parametrize("window", [33, 64, 1000])
+def test_keys_that_only_some_tokens_of_a_segment_see_through_a_window(window):
+    # four tokens a CTA: keys behind the first of them, and keys in front of the last one's window
+    n, p = 1800, 5
+    c = latent_case(torch.float16, [(n, p), (7, 90)], [], 16, 512, 64, 64, window, sink=True)
+    clean, cache, spots = latent_run(c), c.cache.clone(), [41, 42, 203, 1206, 1500]
+    for pos in spots:
+        cache[int(c.bt[0, pos // 16]), 1, pos % 16, [3, 511]] = float("nan")
+    got = latent_run(c, cache)
+    q = torch.arange(n, device=c.q.device) + p
+    sees = torch.zeros(c.q.shape[0], dtype=torch.bool, device=c.q.device)
+    for pos in spots:
+        sees[:n] |= (q >= pos) & (q - pos < window)
+    assert torch.equal(got[~sees], clean[~sees]) and bool((~torch.isfinite(got[sees])).flatten(1).any(1).all())
+
+
+@pytest.mark.parametrize("broadcast", ["heads", "tokens", "turned"])
+def test_query_views_of_other_strides(broadcast):
+    # heads or tokens that share their entries go to the kernel of other sizes; heads outside of tokens stay
+    from swiftllm_b200.worker.kernels.latent_attn import latent_attention
+    c = latent_case(torch.bfloat16, [(1400, 9), (533, 0)], [], 16, 512, 64, 64, 0, sink=True)
+    T = c.q.shape[0]
+    view = c.q[:, :1].expand(T, 16, 512) if broadcast == "heads" else c.q[:1].expand(T, 16, 512) if broadcast == "tokens" else \
+        c.q.transpose(0, 1).contiguous().transpose(0, 1)
+    c.q, out = view.contiguous(), torch.empty_like(c.q)
+    clean = latent_run(c)
+    latent_attention(view, c.qr, c.gate, c.cache, 1, c.bt, c.st, out, c.dims, 0, c.scale, c.cos, c.sin, c.sink)
+    assert torch.equal(out, clean) if broadcast == "turned" else rel(out, clean) < 2 * UNIT[torch.bfloat16]
