@@ -20,7 +20,8 @@
 // Measured on B200, bf16, 16 heads on 4 key/value heads of 128 entries, window 1024: prompts of 2048, 242 and 1507 tokens beside forty decoded
 // ones 312 us with the mma.sync kernel of window_attn.cu for the prompts -> 118 us, 91 with the decoded rows beside the prompts' last CTAs, 83 with
 // boxes (the prompts alone 85 -> 74, one of 2048 51 -> 42, 600 rows at 1500 41 -> 31, 32 heads at 1000, window 2048 170 -> 144; with the long
-// CTAs of all groups first 74 -> 64, 144 -> 117).  Two rounds of CTAs here; a CTA's step of 80 keys is 2000 cycles of softmax, its queries 10 k, its output 10 k (gates one by one 15 k).
+// CTAs of all groups first 74 -> 64, 144 -> 117).  Two rounds of CTAs here; a CTA's step of 80 keys is 2000 cycles of softmax, its queries 10 k, its
+// output 10 k (gates one by one 15 k).
 //
 // EXT: the kernel knows slopes, kept first positions, gates per head, shared_kv rows and learned sinks; CAP: a tanh cap on the scores;
 // FULL: heads of 128 + 128 entries without turned ones beside shared keys (the producers are bound by their instructions).
@@ -386,7 +387,10 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const __g
                     }
                     const int64_t q_hop = hop * p.q_st;
                     const int a_hop = hop * half;
-                    Vec8<T> nu[4];                    // the next rows are on their way while these are turned
+                    // The next rows are on their way while these are turned; not in EXT kernels, whose registers they cost more than their latency (us, ahead /
+                    // not, shared keys, 32 / 8 heads: two of up to 100 tokens 33.6 / 32.5, 16 of up to 128 47.1 / 45.2, three of up to 2048 105 / 104)
+                    constexpr bool AHEAD = !EXT;
+                    Vec8<T> nu[4];
                     float4 nc[4], ns[4];
 #pragma unroll
                     for (int b = 0; b < 4; b++) nc[b] = ns[b] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -400,14 +404,15 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const __g
                             qp[b] += q_hop; cp[b] += a_hop; sp[b] += a_hop;
                         }
                     };
-                    ask(start);
+                    if (AHEAD) ask(start);
 #pragma unroll 1
                     for (int r0 = start; r0 < nrows; r0 += 64) {
+                        if (!AHEAD) ask(r0);
                         Vec8<T> u[4];
                         float4 c4[4], s4[4];
 #pragma unroll
                         for (int b = 0; b < 4; b++) { u[b] = nu[b]; c4[b] = nc[b]; s4[b] = ns[b]; }
-                        if (r0 + 64 < nrows) ask(r0 + 64);
+                        if (AHEAD && r0 + 64 < nrows) ask(r0 + 64);
 #pragma unroll
                         for (int b = 0; b < 4; b++) {
                             const int row = r0 + 16 * b;
