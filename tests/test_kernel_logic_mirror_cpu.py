@@ -2,8 +2,9 @@
 csrc/prefill_attn_kernel.cuh with PAGED = true), step for step as the CUDA code does it - which kv steps a CTA visits, which
 pages a step loads (whole pages for the TMA kernel, row-wise zero fill for the cp.async kernel), when the causal / tail mask is
 applied (`need_mask`) and with which limit (`lim`), which warps skip a tile, which rows are written - with the tensor-core
-products replaced by fp64 matmuls.  It is checked against the fp64 definition (oracle/kernels.py) on random ragged
-(prefix, chunk) layouts, with NaN in every K slot and a large finite value in every V slot that must not contribute.
+products replaced by fp64 matmuls, and of the TMA kernel's items: its blocks, heads side by side, search and key splits.  It is checked against
+the fp64 definition (oracle/kernels.py) on random ragged (prefix, chunk) layouts, with NaN in every K slot and a large finite value in every
+V slot that must not contribute.
 
 This cannot validate the CUDA code (that needs a GPU: tests/test_chunked_prefill_gpu.py); it validates the ARITHMETIC OF THE
 INDICES that was changed without a GPU at hand (prefix offsets in nkt / need_mask / lim / skip), so an off-by-one there shows
@@ -14,6 +15,7 @@ import pytest
 import torch
 
 from oracle import kernels as K
+from prefill_grid import Search, prefill_grid
 
 BS = 16
 
@@ -22,74 +24,93 @@ def _gather_page(cache, blk, layer, kvh):
     return cache[blk, layer, kvh].double().numpy()          # [16, D]
 
 
-def mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, scale, layer, nsplit=1):
-    """prefill_attn_tc_kernel<T, PAGED=true>: CTA = (seq and key split, head, 256 query rows = tiles A and B), 80-token kv steps of which a
-    split takes `per`; then prefill_merge_kernel over the splits' (maximum, sum, O), which start as NaN: what nobody wrote is not read."""
+def _items(chunk, starts, prefix, nq, nkv, rows, nsplit, sms):
+    """What the launch's CTAs take: (sequence, block, split, first head) of every item, in the grid's order."""
+    g = prefill_grid(nq, nkv, len(chunk), max(chunk), rows, nsplit, True, sms)
+    each = -(-max(chunk) // g.tokens)
+    if g.many:
+        blocks = [-(-n // g.tokens) for n in chunk]
+        total = sum(min(n, g.most) for n in blocks) * nsplit
+        grid = [(h, s) for s in range(g.slots) for h in range(g.heads)] if g.by_head else [(h, s) for h in range(g.heads) for s in range(g.slots)]
+        search = {}
+        for h, first in grid:                                          # (a CTA, or another one in its stead)
+            for slot in range(first, total, g.slots):
+                seq, block = search.setdefault(h, Search(blocks, g.most))(slot // nsplit)
+                yield seq, block, slot % nsplit, h * g.pack
+    else:
+        for z, h, x in ((z, h, x) for z in range(len(chunk) * nsplit) for h in range(g.heads) for x in range(each)):
+            seq, split = divmod(z, nsplit)
+            for block in range(each - 1 - x, min(-(-chunk[seq] // g.tokens), g.most), each):
+                yield seq, block, split, h * g.pack
+
+
+def mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, scale, layer, nsplit=1, sms=148):
+    """prefill_attn_tc_kernel<T, PAGED=true>: item = (sequence, block of one or two 128-row tiles, key split, heads side by side in a tile: row =
+    (token, head)), 80-token kv steps of which a split takes `per`; then prefill_merge_kernel over the splits' (maximum, sum, O), which start as NaN:
+    what nobody wrote is not read, and neither is a page slot that a step does not load."""
     Tn, nq, D = q.shape
     nkv = kc.shape[2]
     out = np.zeros((Tn, nq, D))
-    BQ, BK = 128, 80
+    g = prefill_grid(nq, nkv, len(chunk), max(chunk), Tn, nsplit, True, sms)
+    BQ, BK, TT = 128, 80, 128 // g.pack                                # TT: tokens of a tile
     PPS = BK // BS                                                     # pages per step
     part_m, part_l, part_o = np.full((nsplit, Tn, nq), np.nan), np.full((nsplit, Tn, nq), np.nan), np.full((nsplit, Tn, nq, D), np.nan)
     cdiv = lambda a, b: (a + b - 1) // b
-    for seq in range(len(chunk)):
+    seen = set()
+    for seq, block, split, head0 in _items(chunk, starts, prefix, nq, nkv, Tn, nsplit, sms):
+        assert (seq, block, split, head0) not in seen
+        seen.add((seq, block, split, head0))
         ln, pre, tok0 = chunk[seq], prefix[seq], starts[seq]
         kvlen = pre + ln
         npages = cdiv(kvlen, BS)
-        for head in range(nq):
-            kvh = head // (nq // nkv)
-            for qblk, split in ((b, z) for b in range(cdiv(max(chunk), 2 * BQ)) for z in range(nsplit)):
-                q0 = qblk * 2 * BQ
-                if q0 >= ln:
-                    continue
-                active_b = q0 + BQ < ln
-                end = [min(kvlen, pre + q0 + BQ), min(kvlen, pre + q0 + 2 * BQ) if active_b else 0]
-                steps = [cdiv(e, BK) for e in end]
-                per = cdiv(max(steps), nsplit)
-                j0 = split * per
-                nkt = [min(max(n - j0, 0), per) for n in steps]
-                if max(nkt) == 0:                                      # a split past the last key: thread tid < 256 answers for row tid
-                    n = min(2 * BQ, ln - q0)
-                    part_m[split, tok0 + q0:tok0 + q0 + n, head], part_l[split, tok0 + q0:tok0 + q0 + n, head] = -np.inf, 0.0
-                    continue
-                for x in range(2):
-                    rows = q0 + x * BQ + np.arange(BQ)                 # chunk-relative query rows of this tile
-                    ok = tok0 + rows < Tn
-                    qrow = np.zeros((BQ, D))
-                    qrow[ok] = q[tok0 + rows[ok], head].double().numpy()          # TMA: rows past the tensor are zero-filled
-                    m, l, O = np.full((BQ, 1), -np.inf), np.zeros((BQ, 1)), np.zeros((BQ, D))
-                    for j in range(j0, j0 + nkt[x]):
-                        # producer: pages 5j .. 5j+4 that exist are loaded WHOLE; the rest of the stage is zero (or stale, finite)
-                        Kt, Vt = np.zeros((BK, D)), np.zeros((BK, D))
-                        valid = min(PPS, npages - j * PPS)
-                        assert valid >= 1
-                        for pg in range(valid):
-                            blk = int(bt[sids[seq], PPS * j + pg])
-                            Kt[pg * BS:(pg + 1) * BS] = _gather_page(kc, blk, layer, kvh)
-                            Vt[pg * BS:(pg + 1) * BS] = _gather_page(vc, blk, layer, kvh)
-                        with np.errstate(invalid="ignore"):
-                            S = qrow @ Kt.T
-                        c0 = j * BK
-                        if c0 + BK - 1 > pre + q0 + x * BQ or c0 + BK > kvlen:
-                            lim = np.minimum(pre + rows, kvlen - 1) - c0
-                            S = np.where(np.arange(BK)[None, :] <= lim[:, None], S, -np.inf)
-                        m_new = np.maximum(m, S.max(1, keepdims=True) * scale)
-                        with np.errstate(invalid="ignore"):
-                            alpha = np.where(m_new > m, np.exp(m - m_new), 1.0)
-                        m, l, O = m_new, l * alpha, O * alpha
-                        P = np.exp(S * scale - np.where(np.isneginf(m), 0.0, m))         # nothing seen yet: weights of 0
-                        l = l + P.sum(1, keepdims=True)
-                        k16 = min(PPS, cdiv(end[x] - c0, 16))          # P . V: none past the last key the tile can see
-                        assert k16 >= 1
-                        O = O + P[:, :16 * k16] @ Vt[:16 * k16]
-                    wr = rows < ln                                      # epilogue: only rows inside the chunk are written
-                    at = tok0 + rows[wr]
-                    if nsplit > 1:
-                        part_m[split, at, head], part_l[split, at, head] = m[wr, 0], l[wr, 0]
-                        if nkt[x] > 0:
-                            part_o[split, at, head] = O[wr]
-                    elif nkt[x] > 0:
-                        out[at, head] = O[wr] / l[wr]
+        kvh = head0 // (nq // nkv)
+        q0 = block * g.tiles * TT
+        assert q0 < ln
+        upto = lambda n: cdiv(pre + min(ln, n), BK)
+        steps = [upto(q0 + TT), upto(q0 + 2 * TT) if g.tiles == 2 and q0 + TT < ln else 0]
+        per = cdiv(max(steps), nsplit)
+        j0 = split * per
+        nkt = [min(max(n - j0, 0), per) for n in steps]
+        for x in range(g.tiles):
+            first = q0 + x * TT                                        # chunk-relative tokens and heads of this tile's rows
+            tok, head = first + np.arange(BQ) // g.pack, head0 + np.arange(BQ) % g.pack
+            ok = tok0 + tok < Tn
+            qrow = np.zeros((BQ, D))
+            qrow[ok] = q.double().numpy()[tok0 + tok[ok], head[ok]]    # TMA: rows past the tensor are zero-filled
+            end = min(kvlen, pre + first + TT)
+            m, l, O = np.full((BQ, 1), -np.inf), np.zeros((BQ, 1)), np.zeros((BQ, D))
+            for j in range(j0, j0 + nkt[x]):
+                # producer: pages 5j .. 5j+4 that exist are loaded WHOLE; the rest of the stage keeps what lay there
+                Kt, Vt = np.full((BK, D), np.nan), np.full((BK, D), np.nan)
+                valid = min(PPS, npages - j * PPS)
+                assert valid >= 1
+                for pg in range(valid):
+                    blk = int(bt[sids[seq], PPS * j + pg])
+                    Kt[pg * BS:(pg + 1) * BS] = _gather_page(kc, blk, layer, kvh)
+                    Vt[pg * BS:(pg + 1) * BS] = _gather_page(vc, blk, layer, kvh)
+                with np.errstate(invalid="ignore"):
+                    S = qrow @ Kt.T
+                c0 = j * BK
+                if c0 + BK - 1 > pre + first or c0 + BK > kvlen:
+                    lim = np.minimum(pre + tok, kvlen - 1) - c0
+                    S = np.where(np.arange(BK)[None, :] <= lim[:, None], S, -np.inf)
+                m_new = np.maximum(m, S.max(1, keepdims=True) * scale)
+                with np.errstate(invalid="ignore"):
+                    alpha = np.where(m_new > m, np.exp(m - m_new), 1.0)
+                m, l, O = m_new, l * alpha, O * alpha
+                P = np.exp(S * scale - np.where(np.isneginf(m), 0.0, m))         # nothing seen yet: weights of 0
+                l = l + P.sum(1, keepdims=True)
+                k16 = min(PPS, cdiv(end - c0, 16))                     # P . V: none past the last key the tile can see
+                assert k16 >= 1
+                O = O + P[:, :16 * k16] @ Vt[:16 * k16]
+            wr = tok < ln                                              # output: only rows inside the chunk are written
+            at = tok0 + tok[wr], head[wr]
+            if nsplit > 1:
+                part_m[split][at], part_l[split][at] = m[wr, 0], l[wr, 0]
+                if nkt[x] > 0:
+                    part_o[split][at] = O[wr]
+            elif nkt[x] > 0:
+                out[at] = O[wr] / l[wr]
     if nsplit > 1:
         for seq in range(len(chunk)):                                   # merge: the rows of the sequences, no others
             for u in range(starts[seq], starts[seq] + chunk[seq]):
@@ -192,9 +213,19 @@ def test_mirror_of_the_tcgen05_paged_prefill_kernel_matches_the_definition(seed)
     q, kc, vc, bt, sids, starts, chunk, prefix = _case(rng, BS, 32, 4, 2, 3)
     ref = K.prefix_prefill_attention_exact(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, BS, 1).numpy()
     for nsplit in (1, 2, 5, 16):
-        got = mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, 1, nsplit)
-        assert np.isfinite(got).all()
-        assert np.abs(got - ref).max() < 1e-9
+        for sms in (148, 13, 3):                             # blocks of one tile, each launched; of two, that CTAs take from the grid in either order
+            got = mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, 1, nsplit, sms)
+            assert np.isfinite(got).all()
+            assert np.abs(got - ref).max() < 1e-9
+
+
+@pytest.mark.parametrize("nq,nkv", [(8, 1), (6, 2), (2, 2)])
+def test_mirror_with_other_groups_of_heads(nq, nkv):
+    rng = np.random.default_rng(nq)
+    q, kc, vc, bt, sids, starts, chunk, prefix = _case(rng, BS, 32, nq, nkv, 2)
+    ref = K.prefix_prefill_attention_exact(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, BS, 1).numpy()
+    for nsplit, sms in ((1, 148), (3, 148), (1, 2), (3, 20)):
+        assert np.abs(mirror_tc(q, kc, vc, bt, sids, starts, chunk, prefix, 32 ** -0.5, 1, nsplit, sms) - ref).max() < 1e-9
 
 
 @pytest.mark.parametrize("seed,bs", [(0, 16), (1, 16), (2, 32), (3, 4)])

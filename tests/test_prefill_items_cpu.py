@@ -3,46 +3,7 @@ plain enumeration: blocks of the highest number first, the sequences of a number
 import pytest
 import torch
 
-WARP, WIDE = 32, 128
-
-
-class Search:
-    """pt_block with its cursor; `reads`: lengths of sequences past the warp's own 32 that were read."""
-
-    def __init__(self, blocks, max_blocks):
-        self.blocks, self.max_blocks, self.reads = [min(b, max_blocks) for b in blocks], max_blocks, 0
-        self.total = sum(self.blocks)
-        self.block = self.first = self.count = self.s0 = self.before = 0
-
-    def _from(self, b):
-        self.reads += max(0, len(self.blocks) - WARP)
-        return sum(max(n - b, 0) for n in self.blocks)
-
-    def __call__(self, rank):
-        if rank < self.first or rank >= self.first + self.count:
-            lo, hi, from_lo, from_hi = 0, self.max_blocks, self.total, 0
-            while hi - lo > 1:
-                mid = (lo + hi) // 2
-                n = self._from(mid)
-                if n > rank:
-                    lo, from_lo = mid, n
-                else:
-                    hi, from_hi = mid, n
-            self.block, self.first, self.count, self.s0, self.before = lo, from_hi, from_lo - from_hi, 0, 0
-        elif rank < self.first + self.before:
-            self.s0 = self.before = 0
-        r = rank - self.first
-        while self.s0 < len(self.blocks):
-            n = self.before
-            for s in range(self.s0, self.s0 + WIDE):
-                self.reads += WARP <= s < len(self.blocks)
-                if s < len(self.blocks) and self.blocks[s] > self.block:
-                    if n == r:
-                        return s, self.block
-                    n += 1
-            self.before = n
-            self.s0 += WIDE
-        raise AssertionError("a rank without a sequence")
+from prefill_grid import WARP, WIDE, Search, prefill_grid
 
 
 def enumeration(blocks, max_blocks):
@@ -78,7 +39,6 @@ def test_every_cta_finds_its_blocks(kind, n, heads, by_head):
 @pytest.mark.parametrize("H,G,lens", [(16, 16, (1024, 121, 754, 363)), (32, 32, (300, 35, 221, 106)), (24, 4, (1024, 121, 754, 363))])
 def test_the_last_items_are_the_shortest(H, G, lens):
     """Portions of one to four items an SM, in the grid's order: what is left for the second round are no long items."""
-    from prefill_grid import prefill_grid
     g = prefill_grid(H, G, len(lens), max(lens), sum(lens), 1, True)
     order = enumeration([-(-n // g.tokens) for n in lens], g.most)
     assert g.many and g.by_head and 148 < g.heads * g.slots <= 4 * 148
@@ -92,7 +52,6 @@ SHAPES = [(64, 8, 1, 16, 16), (64, 8, 1, 64, 64), (32, 8, 4, 16, 45), (32, 8, 1,
 
 @pytest.mark.parametrize("H,G,n,longest,rows", SHAPES)
 def test_blocks_are_counted_as_the_launch_makes_them(H, G, n, longest, rows):
-    from prefill_grid import prefill_grid
     from swiftllm_b200.worker.kernels.prefill_attn import _blocks
     for tiles, got in zip((1, 2), _blocks(H, G, n, longest, rows)):
         g = prefill_grid(H, G, n, longest, rows, 1, True, sms=1 << 30 if tiles == 1 else 0)
@@ -102,7 +61,6 @@ def test_blocks_are_counted_as_the_launch_makes_them(H, G, n, longest, rows):
 @pytest.mark.parametrize("H,G,n,longest,rows", SHAPES)
 @pytest.mark.parametrize("kv_len", [0, 479, 700, 1016, 3300, 5064, 30000])
 def test_key_splits_fill_the_sms_and_no_more(H, G, n, longest, rows, kv_len):
-    from prefill_grid import prefill_grid
     from swiftllm_b200.worker.kernels.prefill_attn import _blocks, _splits
     sms = 148
     splits = _splits(sms, kv_len, *_blocks(H, G, n, longest, rows), True)
