@@ -8,7 +8,8 @@
 // Every O_q is a tile's own, made from zero; accumulator warps add it to fp32 registers, O = O 2^(m_old - m_new) + O_q.  Rescales therefore cost
 // the tensor core nothing: with O in TMEM they stood between one tile's products and the next's, for the reference is the running maximum itself.
 //   warp 0        TMA producer: a tile is four boxes of 16 cache rows, (64 d | 8 rows | 9 chunks | row groups of 8), into a ring of three stages
-//   warps 1, 2    product issuers, of S and of O_0 .. O_3: one thread's instructions per product take as long as the product (both by one warp: 551 us, now 512)
+//   warps 1, 2    product issuers, of S and of O_0 .. O_3: one thread's instructions per product take as long as the product (both by one
+//                 warp 551 us, by two 512, with a CTA per 64 rows)
 //   warps 4-7     softmax: rows 16 w + lane / 4 (a) and + 8 (b), four lanes a row
 //   warps 8-15    accumulators, 16 rows of a quadrant each: warps 8-11 O_0 and O_2, 12-15 O_1 and O_3; 128 registers a thread
 // TMEM: an M = 64 operand fills 16 of every 32 lanes.  Lanes 0 .. 15: Q in columns 0 .. 287, two buffers of S behind it.  Lanes 16 .. 31: three buffers
@@ -51,23 +52,6 @@ struct LatentPromptBars {
     uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2], a_empty[2], f_full[2], f_empty[2];
     uint64_t o_full[LP_BUFS], o_empty[LP_BUFS];
 };
-
-// 16 lanes x 64 columns of fp32: register 4 i + j is row lane / 4 (+ 8 for j >= 2), column 8 i + 2 (lane % 4) + (j & 1)
-__device__ __forceinline__ void lp_ld_16x64(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-                   "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                   "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-}
-// 16 lanes x 32 words (P: 64 keys of 16 bits): register 2 i + j is row lane / 4 (+ 8 for j = 1), word 4 i + lane % 4
-__device__ __forceinline__ void lp_st_16x32(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                    "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ uint32_t lp_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
 
 __device__ __forceinline__ uint64_t lp_desc(uint64_t base, uint32_t low) { return (base & 0xffffffff00000000ull) | low; }
 
@@ -364,15 +348,15 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
                     uint32_t v[16];
 #pragma unroll
                     for (int i = 0; i < 8; i++) {
-                        v[2 * i] = *reinterpret_cast<const uint32_t*>(q_sm + ch * LP_QCHUNK + lp_off(ra, i) + 4 * (lane & 3));
-                        v[2 * i + 1] = *reinterpret_cast<const uint32_t*>(q_sm + ch * LP_QCHUNK + lp_off(rb, i) + 4 * (lane & 3));
+                        v[2 * i] = *reinterpret_cast<const uint32_t*>(q_sm + ch * LP_QCHUNK + swizzled(ra, i) + 4 * (lane & 3));
+                        v[2 * i + 1] = *reinterpret_cast<const uint32_t*>(q_sm + ch * LP_QCHUNK + swizzled(rb, i) + 4 * (lane & 3));
                     }
-                    lp_st_16x32(tlane + LP_Q_COL + 32 * ch, v);
+                    tmem_st_16x32(tlane + LP_Q_COL + 32 * ch, v);
                 }
                 turn(0);
                 angles(tok_b);
                 turn(1);
-                lp_st_16x32(tlane + LP_Q_COL + LP_R / 2, w);
+                tmem_st_16x32(tlane + LP_Q_COL + LP_R / 2, w);
                 tmem_st_wait();
                 tc_fence_before();
                 fence_proxy_async();                      // boxes overwrite the stage
@@ -395,7 +379,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
                 mbar_wait(smem_u32(&bars->s_full[b]), (t >> 1) & 1);
                 tc_fence_after();
                 uint32_t s[32];
-                lp_ld_16x64(tlane + LP_S_COL + 64 * b, s);
+                tmem_ld_16x64(tlane + LP_S_COL + 64 * b, s);
                 tmem_ld_wait();
                 tc_fence_before();
                 mbar_arrive(smem_u32(&bars->s_empty[b]));
@@ -438,7 +422,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
                 if ((lane & 3) == 0) { sh.alpha[b][ra] = al_a; sh.alpha[b][rb] = al_b; }
                 mbar_wait(smem_u32(&bars->p_empty[b]), ((t >> 1) & 1) ^ 1);
                 tc_fence_after();
-                lp_st_16x32(tlane + UPPER + LP_P_COL + 32 * b, w);
+                tmem_st_16x32(tlane + UPPER + LP_P_COL + 32 * b, w);
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(smem_u32(&bars->p_full[b]));
@@ -483,12 +467,14 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_attn_prompt_kernel(const
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
                     const int i = 4 * t + 2 * q + half, buf = i % LP_BUFS;
+                    // (This half waits for every other phase of a buffer.  The one between, of product i - 3, is over: the products' warp issues one behind the
+                    // other, and i - 2, which this half has waited for, came after it)
                     mbar_wait(smem_u32(&bars->o_full[buf]), (i / LP_BUFS) & 1);
                     tc_fence_after();
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         uint32_t v[32];
-                        lp_ld_16x64(tlane + LP_O_COL + 128 * buf + 64 * h, v);
+                        tmem_ld_16x64(tlane + LP_O_COL + 128 * buf + 64 * h, v);
                         tmem_ld_wait();
                         if (h == 1) {
                             tc_fence_before();

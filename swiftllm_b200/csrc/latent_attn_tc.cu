@@ -55,25 +55,6 @@ struct LatentTcBars {
     uint64_t s_full[2], s_empty[2], p_full[2], o_done[2];
 };
 
-// 16 lanes x 64 columns of fp32: register 4 i + j is row lane / 4 (+ 8 for j >= 2), column 8 i + 2 (lane % 4) + (j & 1)
-__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-                   "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                   "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-}
-// 16 lanes x 32 words (P: 64 keys of 16 bits): register 2 i + j is row lane / 4 (+ 8 for j = 1), word 4 i + lane % 4
-__device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                    "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-
-// byte offset of 16-byte piece `piece` (of 8) of row `row` in a chunk of 64 rows x 128 bytes, SWIZZLE_128B
-__device__ __forceinline__ uint32_t lt_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
-
 // FULL: r = 512 and dr = 64, known to the compiler (the producers' and the issuer's loops are bound by their instructions).  ROWS: prompt
 // rows (and single tokens of more heads); LT_SINGLES: single tokens of at most 16 heads, whose rows 16 .. 31 repeat rows 0 .. 15; LT_SHARED: prompt
 // rows of a launch that leaves SMs over, whose CTAs of the same tokens take one segment each (in the first kernel this costs 3 %)
@@ -172,7 +153,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 const long long ri = __shfl_sync(0xffffffffu, rowi, 4 * i + (lane >> 3));
                 const int bytes = ri >= 0 ? 16 : 0;
                 const T* src = reinterpret_cast<const T*>(p.cache) + (ri >= 0 ? ri * D + piece * 8 : 0);
-                const uint32_t dst = smem_u32(k_sm + st * LT_STAGE) + lt_off(row, piece);
+                const uint32_t dst = smem_u32(k_sm + st * LT_STAGE) + swizzled(row, piece);
                 if constexpr (FULL) {
                     if (g == 0) {
 #pragma unroll
@@ -221,7 +202,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                 const bool live = j < n && h < p.H;
                 const T* ql = reinterpret_cast<const T*>(p.q_lat) + (live ? (int64_t)(ts + j) * p.ql_st + (int64_t)h * p.ql_sh : 0);
                 for (int c = lane; c < (r >> 3); c += 32) {
-                    uint8_t* dst = q_sm + (c >> 3) * LT_CHUNK + lt_off(row, c & 7);
+                    uint8_t* dst = q_sm + (c >> 3) * LT_CHUNK + swizzled(row, c & 7);
                     if (p.q_vec) {
                         cp_async16(smem_u32(dst), live ? ql + 8 * c : ql, live ? 16 : 0);
                     } else {
@@ -267,7 +248,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attn_tc_kernel(const Lat
                     v = make_uint4(w[0], w[1], w[2], w[3]);
                 }
                 const int col = r + d;
-                *reinterpret_cast<uint4*>(q_sm + (col >> 6) * LT_CHUNK + lt_off(row, (col & 63) >> 3)) = v;
+                *reinterpret_cast<uint4*>(q_sm + (col >> 6) * LT_CHUNK + swizzled(row, (col & 63) >> 3)) = v;
             }
             cp_async_wait<0>();
             fence_proxy_async();

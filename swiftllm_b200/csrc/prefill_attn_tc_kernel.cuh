@@ -88,8 +88,8 @@ struct PtItem {
 struct PtPaged {
     const int32_t* block_table; const int32_t* seq_ids; const int32_t* prefix_lens;
     int cur_layer, num_layers, max_blocks_per_seq;
-    // key splits (steps with few query blocks): slot blockIdx.y = query block * nsplit + split; nsplit > 1 leaves fp32 rows of unnormalised O
-    // [nsplit, tokens, nq, 128] and their (reference maximum in base 2, sum) [nsplit, tokens, nq, 2] for prefill_merge_kernel
+    // key splits (steps with few query blocks): slot = query block * nsplit + split, without MANY blockIdx.z = sequence * nsplit + split; nsplit > 1
+    // leaves fp32 rows of unnormalised O [nsplit, tokens, nq, 128] and their (reference maximum in base 2, sum) [nsplit, tokens, nq, 2] for prefill_merge_kernel
     int nsplit; int64_t num_tokens;
     float* part_o; float* part_ml;
 };

@@ -56,8 +56,6 @@ struct WindowTcBars {
     uint64_t landed[2];                              // [keys, values]: boxes of a step whose unseen rows have yet to become zero
 };
 
-__device__ __forceinline__ uint32_t wx_off(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
-
 // y / (1 + e^-z), two at a time: the quick reciprocal and one step of Newton's iteration, r + r (1 - d r), which leaves about half a unit in the last place
 // and has no branch, so that the gates of a row are worked on together (with a quotient rounded exactly the case below took 127 us
 // instead of 115).  Five to six instructions a gate: a row's 128 take 1.9 k cycles of its warp when it has the scheduler to itself (one by one 3.8 k).
@@ -252,7 +250,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const __g
                         const long long ri = __shfl_sync(0xffffffffu, i < 8 ? a : b, l & 31);
                         const int bytes = ri >= 0 ? 16 : 0;
                         const T* src = ri >= 0 ? cache + ri * p.row_elems : cache;
-                        const uint32_t dst = stage + wx_off(row, piece);
+                        const uint32_t dst = stage + swizzled(row, piece);
                         if constexpr (FULL) {             // (a row that is not there reads nothing, wherever src points)
                             const T* ks = src + kofs + piece * 8;
                             cp_async16(dst, ks, bytes); cp_async16(dst + WX_CHUNK, ks + 64, bytes);
@@ -363,7 +361,7 @@ __global__ void __launch_bounds__(WX_THREADS, 1) window_attn_tc_kernel(const __g
                 auto stage_row = [&](int row, const float (&x)[8]) {
                     if (d < dk) {
                         const uint4 v = make_uint4(pack2<T>(x[0], x[1]), pack2<T>(x[2], x[3]), pack2<T>(x[4], x[5]), pack2<T>(x[6], x[7]));
-                        *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + wx_off(row & 127, (d & 63) >> 3)) = v;
+                        *reinterpret_cast<uint4*>(q_sm + (row >> 7) * WX_Q_BYTES + (d >> 6) * WX_QCHUNK + swizzled(row & 127, (d & 63) >> 3)) = v;
                     }
                 };
                 if (p.q_fast) {
