@@ -120,7 +120,9 @@ int launch_prefill_tc(const void* q, const void* k, const void* v, void* o, cons
             cudaFuncSetAttribute(prefill_attn_tc_kernel<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
             cudaFuncSetAttribute(prefill_attn_tc_kernel<T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM_BYTES);
         }
-        if (many) prefill_attn_tc_kernel<T, false, true><<<grid, PT_THREADS, PT_SMEM_BYTES, stream>>>(qmap, kmap, vmap, p, PtPaged{});
+        // (begun early or not, us called eagerly: eight prompts of up to 600 tokens, 32 / 8 heads, 28.7 / 31.4, twelve of up to 1777, 16 / 4 heads, 70.0 / 72.1,
+        // 4 x 4096, 32 / 8 heads, 477 / 476)
+        if (many) launch_early(prefill_attn_tc_kernel<T, false, true>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, PtPaged{});
         else launch_early(prefill_attn_tc_kernel<T, false, false>, grid, PT_THREADS, PT_SMEM_BYTES, stream, qmap, kmap, vmap, p, PtPaged{});
     });
     return check_launch("prefill_attention(tcgen05)");

@@ -170,10 +170,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prefill_attn_tc_kernel(const __
     static_assert(sizeof(PtBarriers) <= 512 && 528 + 2 * sizeof(PtItem) <= 640, "barriers, items and the answer share a kilobyte");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if constexpr (PAGED || !MANY) {                             // (long launches over packed rows gain nothing: 594 -> 598 us)
-        wait_previous();
-        if (!PAGED || pg.nsplit == 1) launch_next();                      // (a merge begins as the CTAs end: it would gather on the idle SMs; 64 tokens at 3000: 18.6 -> 17.2 us)
-    }
+    wait_previous();
+    if (!PAGED || pg.nsplit == 1) launch_next();                // (a merge begins as the CTAs end: it would gather on the idle SMs; 64 tokens at 3000: 18.6 -> 17.2 us)
     const int nsplit = PAGED ? pg.nsplit : 1;
     const int tile_tokens = PT_BQ >> p.pack_log2;
 
