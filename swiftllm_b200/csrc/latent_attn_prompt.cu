@@ -22,9 +22,9 @@
 // run (with a CTA per 64 rows 12 us of 36 passed around its products).
 //
 // Bound: at M = 64 the tensor core runs at half rate, 2176 cycles a tile (measured: 32, 64, 128 cycles for N = 64, 128, 256; a thread's loop that works out
-// descriptors and phases between products takes longer than that).  Its shared-memory reads and the boxes' writes take 1664.  Here a tile takes 2470, at the
-// clock that the power cap leaves; between two items 6000 cycles.  Measured on B200, bf16, 16 heads: four prompts of 2048 tokens 571 us with
-// latent_attn_tc.cu -> 449 (651 TFLOP/s); 32 heads, three ragged prompts of up to 1000 tokens at 1900, window 2048: 540 -> 419.
+// descriptors and phases between products takes longer than that).  Its shared-memory reads and the boxes' writes take 1664.  Measured on B200, bf16, 16
+// heads: four prompts of 2048 tokens 571 us with latent_attn_tc.cu -> 425 (688 TFLOP/s); at the clock that the power cap leaves (1.76 GHz in a loop of seconds)
+// the products are two thirds of that.  32 heads, three ragged prompts of up to 1000 tokens at 1900, window 2048: 544 -> 382.
 #include "latent_attn_tc.cuh"
 #include "mma_helpers.cuh"
 #include "tc_helpers.cuh"

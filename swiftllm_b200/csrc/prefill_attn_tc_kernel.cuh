@@ -23,11 +23,11 @@
 // stead (cluster launch control), so that the SMs share the items as they get to them whatever the lengths are, and beside other kernels.  It asks
 // when the last PT_STAGES steps' keys are yet to load: asked at an item's beginning, the CTAs of the longest items, which begin first, had taken a
 // second one before the others ended (us, at the beginning / now: one prompt of 4096 tokens, 16 / 4 heads, 85 / 64; two of up to 2000, 32 / 8
-// heads, 51 / 41; three of up to 1000, 64 / 8 heads, 44 / 45.6; twelve of up to 1777, 16 / 4 heads, 72 both).  Portions in no more CTAs
+// heads, 51 / 41; three of up to 1000, 64 / 8 heads, 44 / 45.6; twelve of up to 1777, 16 / 4 heads, 72 both; launched late, as both were then).  Portions in no more CTAs
 // than SMs do not ask: a request that finds none costs their steps 7 % (one of 1024 tokens at 5000, 24 / 4 heads, 93 us with and 87 without).
 // With a CTA per (sequence, head, 256 tokens) 4000 cycles passed before its first product, over a quarter of a prompt of 450 tokens, and a tile's rows
-// multiplied 104 keys on the average that they do not see, now 56 at four heads a tile.  Measured on B200, us: 4 x 4096 bf16, 32 / 8 heads 590 -> 550
-// (1020 TFLOP/s), twelve ragged fp16 prompts of up to 1777 tokens 202 -> 160, 64 of up to 100 tokens 72 -> 31, 512 tokens at 3584 47.2 -> 45.5.
+// multiplied 104 keys on the average that they do not see, now 56 at four heads a tile.  Measured on B200, us: 4 x 4096 bf16, 32 / 8 heads 590 -> 544
+// (1010 TFLOP/s), twelve ragged fp16 prompts of up to 1777 tokens 202 -> 157, 64 of up to 100 tokens 72 -> 29, 512 tokens at 3584 47.2 -> 45.3.
 // An issuer works out its operands before it waits: it sits between every softmax and the products behind it (3 to 6 %).
 //
 // Why steps of 80 keys: scores and P need places of their own, so that the next scores are multiplied while the softmax of the last ones

@@ -847,7 +847,9 @@ int launch_window_attn_tc(WindowTc& p, sllm_dtype_t dtype, cudaStream_t stream) 
     // behind the other / now, three prompts of up to 2048, 16 / 4 heads 74 / 64, 32 / 8 heads at 1000, window 2048 144 / 117, shared keys 181 instead of 229).
     // More than a round of them beside a round of decoded rows keeps the groups apart: those fill the ragged end, and find no SM before the last prompt row's
     // CTA has one (us, apart / together, three prompts of up to 2048 and 38 decoded 83 / 90, 64 decoded 90 / 92, at 300 keys 75 / 76, 32 / 8 heads
-    // 178 / 180; two at 1000 and 64 147 / 136; ten decoded 83 / 70, one prompt of 1000 58 / 52; shared keys, 40 decoded 106 / 100, 216 / 204)
+    // 178 / 180; less than a round of either, together: ten decoded 83 / 70, one prompt of 1000 58 / 52; shared keys 106 / 100, 216 / 204).  What
+    // decides is whether the decoded rows' work fits the ragged end, which their number alone does not say: 64 beside two prompts at 1000, 32 / 8 heads, keep
+    // the groups apart and take 147 where together they would take 136
     p.group_blocks = !ext && p.beside >= num_sms && (int64_t)grid.x > num_sms ? cdiv(p.num_rows, p.qt) : 0;
     // boxes: whole cache blocks of 16 rows, 16-byte rows and columns of theirs (a block table names only blocks that there are: the map need not know how
     // many)

@@ -4,6 +4,7 @@
  * vs the CPU oracle in bf16; CUDA-graph decode path == eager path."""
 import json
 import os
+import tempfile
 
 import numpy as np
 import pytest
@@ -13,7 +14,7 @@ from oracle.model import OracleLlama, OracleWeights
 
 pytestmark = pytest.mark.gpu
 T = torch.from_numpy
-OUT = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out")
+OUT = os.path.join(tempfile.gettempdir(), "swiftllm_b200_parity")
 
 
 def _hf_tensors(w: OracleWeights, F: int):
