@@ -298,3 +298,26 @@ def test_a_latent_layer(prompts, decodes):
               lambda: latent_attention(q[:, :, :r], q[:, :, r:], gate, cache, 0, table, st, out, 0, 0, (r + dr) ** -0.5, None, None),
               lambda: rmsnorm_inplace(out.view(T, H * r), w2, 1e-5)]
     _stepwise_and_back_to_back(load, stages, lambda: [out, cache])
+
+
+def _prompts(seed, H=32, G=8, lens=(900, 333, 700)):
+    from swiftllm_b200.worker.kernels.prefill_attn import prefill_attention
+    T = sum(lens)
+    qkv = _normal(T, (H + 2 * G) * 128, seed=seed, dtype=torch.bfloat16)
+    q, k, v = (x.unflatten(1, (-1, 128)) for x in qkv.split([H * 128, G * 128, G * 128], dim=1))
+    st = types.SimpleNamespace(prefill_seq_start_locs=_ints(sum(lens[:i]) for i in range(len(lens))), prefill_seq_lens=_ints(lens), softmax_scale=128 ** -0.5,
+                               num_prefill_seqs=len(lens), max_prefill_len=max(lens))
+    return lambda out: prefill_attention(q, k, v, out, None, None, st), (T, H, 128)
+
+
+def _latent_prompts(seed, H=16, n=1700):
+    from tile_cases import latent_case
+    from swiftllm_b200.worker.kernels.latent_attn import latent_attention
+    c = latent_case(torch.bfloat16, [(n, seed)], [], H, 512, 64, 64, 0, sink=True)
+    return lambda out: latent_attention(c.q, c.qr, c.gate, c.cache, 1, c.bt, c.st, out, c.dims, 0, c.scale, c.cos, c.sin, c.sink), (n, H, 512)
+
+
+@pytest.mark.parametrize("make", [_prompts, _latent_prompts])
+def test_ctas_that_take_others_back_to_back(make):
+    """Grids of more CTAs than SMs, whose CTAs take the next one's place: the launch behind them begins when none is left."""
+    test_back_to_back(make)
